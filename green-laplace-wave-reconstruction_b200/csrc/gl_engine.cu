@@ -4212,9 +4212,20 @@ static gl_status wit_upload_tables() {
 
 static size_t wit_binom_stride(int n_modes) { return (size_t)n_modes + 4; }
 
+// Table sizes of the sector-44 sum.  Pair states cost 24 M^2 bytes (0.4 GB at
+// the limit of 4096 modes, far beyond any sum that ends); triple states 8 M^3
+// (1 GB at 500 modes) and are formed per quartet above that.
+constexpr int WIT44_PAIR_MODES = 4096, WIT44_TRIPLE_MODES = 500;
+static size_t wit_pairs(int n) { return n <= WIT44_PAIR_MODES ? (size_t)n * (n + 1) / 2 : 0; }
+static size_t wit_triples(int n) { return n <= WIT44_TRIPLE_MODES ? (size_t)n * (n + 1) * (n + 2) / 6 : 0; }
+static size_t wit_head_bytes(int n_modes) {
+  return align_up(sizeof(WitStats)) + 5 * wit_binom_stride(n_modes) * sizeof(unsigned long long);
+}
+
 extern "C" size_t gl_wit_workspace_size(int n_modes) {
   if (n_modes < 1) return 0;
-  return align_up(sizeof(WitStats)) + 5 * wit_binom_stride(n_modes) * sizeof(unsigned long long);
+  const size_t subs = (n_modes <= WIT44_PAIR_MODES ? (size_t)n_modes : 0) + wit_pairs(n_modes) + wit_triples(n_modes);
+  return wit_head_bytes(n_modes) + (subs ? 256 + 3 * subs * sizeof(double2) : 0);  // 256: table alignment
 }
 
 extern "C" gl_status gl_wit_read_sector_stats(int sector, const void* d_work, int n_modes,
@@ -4314,7 +4325,53 @@ extern "C" gl_status gl_wit_sector_range(int sector, int n_modes, const int* d_m
   a.binom_stride = (int)stride;
   a.sector = sector;
   if (q_end == q_begin) return GL_OK;  // an empty share: zero fields, zero counts
-  const int blocks = (int)std::min<unsigned long long>((q_end - q_begin + 127) / 128, 148ull * 32);
+  const unsigned long long count = q_end - q_begin;
+  if (sector == 44 && n_modes <= WIT44_PAIR_MODES) {
+    // Real arithmetic over tabulated pair and triple states; 100 modes (4.4 M
+    // quartets): 13.4 ms by the general kernel below, 0.34 ms.  The
+    // triple table is built when the call's candidates outnumber its entries
+    // (a rank's small share forms its triples per quartet, by the same
+    // function).  Sectors 40 and 42 mix signs, and their intermediate sums
+    // resonate, so they keep the general recursion.
+    Wit44Tables t;
+    t.n_modes = n_modes;
+    t.n_pairs = wit_pairs(n_modes);
+    t.n_triples = count >= wit_triples(n_modes) ? wit_triples(n_modes) : 0;
+    double2* base = reinterpret_cast<double2*>(
+        (reinterpret_cast<uintptr_t>(work) + wit_head_bytes(n_modes) + 255) & ~(uintptr_t)255);
+    t.single = base;
+    t.pair = base + 3 * (size_t)n_modes;
+    t.triple = t.n_triples ? t.pair + 3 * t.n_pairs : nullptr;
+    {
+      LaunchScope ls("wit44_single_kernel", st, 0.0);
+      wit44_single_kernel<<<(n_modes + 127) / 128, 128, 0, st>>>(a.M, d_modes, dkx, dky, base, n_modes);
+    }
+    LAUNCH_CHECK("wit44_single_kernel");
+    {
+      LaunchScope ls("wit44_pair_kernel", st, 0.0);
+      wit44_pair_kernel<<<dim3((n_modes + 127) / 128, n_modes), 128, 0, st>>>(a.M, t);
+    }
+    LAUNCH_CHECK("wit44_pair_kernel");
+    if (t.n_triples) {
+      LaunchScope ls("wit44_triple_kernel", st, 0.0);
+      wit44_triple_kernel<<<dim3((n_modes + 127) / 128, n_modes, n_modes), 128, 0, st>>>(a.M, t);
+    }
+    LAUNCH_CHECK("wit44_triple_kernel");
+    // candidates per warp: enough warps for the GPU, 32 steps a lane or what
+    // keeps the grid below 2^30 blocks
+    const unsigned long long per = std::max<unsigned long long>(
+        std::min<unsigned long long>(32, 1 + count / (32ull * 148 * 32)), 1 + count / (128ull << 30));
+    const unsigned long long chunk = 32 * per, warps = (count + chunk - 1) / chunk;
+    const unsigned int grid = (unsigned int)((warps + 3) / 4);
+    {
+      LaunchScope ls("wit44_table_kernel", st, 0.0);
+      if (t.n_triples) wit44_table_kernel<true><<<grid, 128, 0, st>>>(a, t, chunk);
+      else wit44_table_kernel<false><<<grid, 128, 0, st>>>(a, t, chunk);
+    }
+    LAUNCH_CHECK("wit44_table_kernel");
+    return GL_OK;
+  }
+  const int blocks = (int)std::min<unsigned long long>((count + 127) / 128, 148ull * 32);
   {
     LaunchScope ls("wit44_kernel", st, 0.0);
     wit44_kernel<<<blocks, 128, 0, st>>>(a);

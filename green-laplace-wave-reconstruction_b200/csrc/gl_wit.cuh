@@ -355,6 +355,29 @@ GL_D int wit_unrank_step(const unsigned long long* row, int hi, unsigned long lo
   return lo;
 }
 
+// Folds a warp's counters into the statistics.
+GL_D void wit_fold_stats(WitStats* st, unsigned long long kept, unsigned long long near, unsigned long long szo,
+                         unsigned long long szi, double max_res, double min_det, double max_src) {
+  for (int o = 16; o > 0; o >>= 1) {
+    kept += __shfl_xor_sync(0xffffffffu, kept, o);
+    near += __shfl_xor_sync(0xffffffffu, near, o);
+    szo += __shfl_xor_sync(0xffffffffu, szo, o);
+    szi += __shfl_xor_sync(0xffffffffu, szi, o);
+    max_res = fmax(max_res, __shfl_xor_sync(0xffffffffu, max_res, o));
+    min_det = fmin(min_det, __shfl_xor_sync(0xffffffffu, min_det, o));
+    max_src = fmax(max_src, __shfl_xor_sync(0xffffffffu, max_src, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&st->kept, kept);
+    atomicAdd(&st->near, near);
+    atomicAdd(&st->strict_zero_output, szo);
+    atomicAdd(&st->strict_zero_intermediate, szi);
+    atomic_max_nonneg(&st->max_residual, max_res);
+    atomicMin(&st->min_detuning, (unsigned long long)__double_as_longlong(min_det));
+    atomic_max_nonneg(&st->max_strict_src, max_src);
+  }
+}
+
 // Sectors of the fourth-order sum (directional_eta4_openmp.cpp:604-734):
 //   44: unordered quartets of + parents, all targets inside the grid;
 //   40: unordered + pair x unordered - pair, analytic half-plane targets;
@@ -472,24 +495,335 @@ __global__ void __launch_bounds__(128) wit44_kernel(WitArgs a) {
     min_det = fmin(min_det, r.rho);
     max_src = fmax(max_src, r.strict_src);
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    kept += __shfl_xor_sync(0xffffffffu, kept, o);
-    near += __shfl_xor_sync(0xffffffffu, near, o);
-    szo += __shfl_xor_sync(0xffffffffu, szo, o);
-    szi += __shfl_xor_sync(0xffffffffu, szi, o);
-    max_res = fmax(max_res, __shfl_xor_sync(0xffffffffu, max_res, o));
-    min_det = fmin(min_det, __shfl_xor_sync(0xffffffffu, min_det, o));
-    max_src = fmax(max_src, __shfl_xor_sync(0xffffffffu, max_src, o));
+  wit_fold_stats(a.stats, kept, near, szo, szi, max_res, min_det, max_src);
+}
+
+// ---------------------------------------------------------------------------
+// Sector 44 over tabulated subset states
+// ---------------------------------------------------------------------------
+//
+// With all four signs equal the recursion is real: eta of every subset is
+// real and phi, psi, the vertical velocity and the kinematic source are
+// imaginary (eta = e, phi = i f, horizontal velocity (x, y), vertical i v).
+// A subset's state depends only on its modes, so the M (M+1)/2 pair states
+// (and, up to WIT44_TRIPLE_MODES modes, the M (M+1)(M+2)/6 triple states) are
+// tabulated once, and a quartet is left with its own degree: 14 proper
+// subsets, each entering the Taylor sums once -- the set partitions that
+// share a potential block collapse into one elevation factor per order
+// (unordered partitions; the block orders cancel the factorials).
+//
+// What bounds it: FP64 issue (about 250 operations a quartet) and the loads
+// of four triple and six pair states, which the lanes of a warp read
+// contiguously because consecutive candidates differ in their lowest mode,
+// and four FP64 atomics per quartet.
+// 100 modes (4.4 M quartets): 0.31 ms and 0.03 ms for the tables, against
+// 13.4 ms for the general kernel; 382 modes (901 M): 0.06 s against 3.2 s.
+
+struct WitSub {
+  double e, f, x, y, v, q;  // q with its sign bit set: a strict zero, e = its source
+};
+
+struct Wit44Tables {
+  const double2* single;  // [3][M]: (kx, ky), (om, q), (f, |k|^2)
+  double2* pair;          // [3][n_pairs]: (e, f), (x, y), (v, q)
+  double2* triple;        // [3][n_triples], null: formed per quartet
+  size_t n_pairs, n_triples;
+  int n_modes;
+};
+
+struct WitOne {
+  double kx, ky, om, q, f, m2;
+};
+
+GL_D WitOne wit_single(const Wit44Tables& T, int i) {
+  const double2 k = __ldg(T.single + i), w = __ldg(T.single + T.n_modes + i), p = __ldg(T.single + 2 * T.n_modes + i);
+  return WitOne{k.x, k.y, w.x, w.y, p.x, p.y};
+}
+
+// Multiset indices a <= b <= c, lowest mode fastest (the order of the
+// quartet candidates).
+GL_HD size_t wit_pair_at(int a, int b) { return (size_t)b * (b + 1) / 2 + a; }
+GL_HD size_t wit_triple_at(int a, int b, int c) {
+  return (size_t)c * (c + 1) * (c + 2) / 6 + (size_t)b * (b + 1) / 2 + a;
+}
+
+GL_D WitSub wit_sub_load(const double2* t, size_t n, size_t i) {
+  const double2 a = __ldg(t + i), b = __ldg(t + n + i), c = __ldg(t + 2 * n + i);
+  return WitSub{a.x, a.y, b.x, b.y, c.x, c.y};
+}
+GL_D void wit_sub_store(double2* t, size_t n, size_t i, const WitSub& s) {
+  t[i] = make_double2(s.e, s.f);
+  t[n + i] = make_double2(s.x, s.y);
+  t[2 * n + i] = make_double2(s.v, s.q);
+}
+
+// A stored strict zero: counts it, takes its source and clears the marker.
+GL_D void wit_sub_strict(WitSub& s, int& count, double& src) {
+  if (signbit(s.q)) {
+    ++count;
+    src = fmax(src, s.e);
+    s.e = 0.0;
+    s.q = -s.q;
   }
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd(&a.stats->kept, kept);
-    atomicAdd(&a.stats->near, near);
-    atomicAdd(&a.stats->strict_zero_output, szo);
-    atomicAdd(&a.stats->strict_zero_intermediate, szi);
-    atomic_max_nonneg(&a.stats->max_residual, max_res);
-    atomicMin(&a.stats->min_detuning, (unsigned long long)__double_as_longlong(min_det));
-    atomic_max_nonneg(&a.stats->max_strict_src, max_src);
+}
+
+// Taylor and source sums of one subset.
+struct WitSums {
+  double T, LV, LT, H, K, X, Y;
+};
+
+// Potential block (kx, ky, om, f) with its weighted vertical derivatives:
+// A = sum_o z_o prod(eta)/o!, B = sum_o z_{o+1} prod(eta)/o!.
+GL_D void wit_block(WitSums& s, double kx, double ky, double om, double f, double A, double B) {
+  const double fa = f * A;
+  s.T += fa;
+  s.LV += f * B;
+  s.LT += om * fa;
+  s.X += kx * fa;
+  s.Y += ky * fa;
+}
+// Advection and kinetic terms of a two-block partition (l, r), both orders.
+GL_D void wit_cross(WitSums& s, double lx, double ly, double lv, double le, double lkx, double lky, double rx,
+                    double ry, double rv, double re, double rkx, double rky) {
+  s.H += (lx * rkx + ly * rky) * re + (rx * lkx + ry * lky) * le;
+  s.K += lx * rx + ly * ry - lv * rv;
+}
+
+GL_D bool wit_is_strict(double mag) { return mag <= 100.0 * 2.220446049250313e-16 * fmax(mag, 1.0); }
+
+// Response of a pair or triple to its sources.
+GL_D WitSub wit_close(const WitModel& M, const WitSums& s, double kx, double ky, double om) {
+  const double mag = hypot(kx, ky);
+  WitSub o;
+  o.q = mag * tanh(M.h * mag);
+  const double s0 = s.LV - s.H - o.q * s.T;
+  const double s1 = om * s.T - (s.LT + s.K);
+  const bool strict = wit_is_strict(mag);
+  double psi = 0.0;
+  o.e = 0.0;
+  if (!strict) {
+    const double den = om * om - M.g * o.q;
+    o.e = -(om * s0 + o.q * s1) / den;
+    psi = (M.g * s0 + om * s1) / den;
   }
+  o.f = psi - s.T;
+  o.x = -(kx * o.f + s.X);
+  o.y = -(ky * o.f + s.Y);
+  o.v = o.q * o.f + s.LV;
+  if (strict) {
+    o.e = hypot(s0, s1);
+    o.q = -o.q;
+  }
+  return o;
+}
+
+__device__ __noinline__ WitSub wit_triple_state(const WitModel& M, const Wit44Tables& T, int a, int b, int c) {
+  const WitOne s[3] = {wit_single(T, a), wit_single(T, b), wit_single(T, c)};
+  WitSums w = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const WitOne &p = s[(k + 1) % 3], &r = s[(k + 2) % 3], &o = s[k];
+    const int lo = k == 0 ? b : a, hi = k == 2 ? b : c;  // the pair without slot k
+    WitSub q = wit_sub_load(T.pair, T.n_pairs, wit_pair_at(lo, hi));
+    int n = 0;
+    double src = 0.0;
+    wit_sub_strict(q, n, src);
+    const double pkx = p.kx + r.kx, pky = p.ky + r.ky, pom = p.om + r.om;
+    wit_block(w, o.kx, o.ky, o.om, o.f, o.q * q.e + 0.25 * o.m2, o.m2 * q.e + 0.25 * (o.m2 * o.q));
+    wit_block(w, pkx, pky, pom, q.f, 0.5 * q.q, 0.5 * (pkx * pkx + pky * pky));
+    wit_cross(w, -o.kx * o.f, -o.ky * o.f, o.q * o.f, 0.5, o.kx, o.ky, q.x, q.y, q.v, q.e, pkx, pky);
+  }
+  return wit_close(M, w, s[0].kx + s[1].kx + s[2].kx, s[0].ky + s[1].ky + s[2].ky, s[0].om + s[1].om + s[2].om);
+}
+
+__global__ void wit44_single_kernel(WitModel M, const int* modes, double dkx, double dky, double2* single, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double kx = modes[2 * i] * dkx, ky = modes[2 * i + 1] * dky;
+  const double m = hypot(kx, ky), q = m * tanh(M.h * m), om = sqrt(M.g * q);
+  single[i] = make_double2(kx, ky);
+  single[n + i] = make_double2(om, q);
+  single[2 * n + i] = make_double2(-om / (2.0 * q), m * m);
+}
+
+// One thread per pair (a <= b): blockIdx.y = b, threads over a.
+__global__ void __launch_bounds__(128) wit44_pair_kernel(WitModel M, Wit44Tables T) {
+  const int b = blockIdx.y, a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a > b) return;
+  const WitOne p = wit_single(T, a), r = wit_single(T, b);
+  WitSums w = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  wit_block(w, p.kx, p.ky, p.om, p.f, 0.5 * p.q, 0.5 * p.m2);
+  wit_block(w, r.kx, r.ky, r.om, r.f, 0.5 * r.q, 0.5 * r.m2);
+  wit_cross(w, -p.kx * p.f, -p.ky * p.f, p.q * p.f, 0.5, p.kx, p.ky, -r.kx * r.f, -r.ky * r.f, r.q * r.f, 0.5,
+            r.kx, r.ky);
+  wit_sub_store(T.pair, T.n_pairs, wit_pair_at(a, b), wit_close(M, w, p.kx + r.kx, p.ky + r.ky, p.om + r.om));
+}
+
+// One thread per triple (a <= b <= c): blockIdx.z = c, blockIdx.y = b.
+__global__ void __launch_bounds__(128) wit44_triple_kernel(WitModel M, Wit44Tables T) {
+  const int c = blockIdx.z, b = blockIdx.y, a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b > c || a > b) return;
+  wit_sub_store(T.triple, T.n_triples, wit_triple_at(a, b, c), wit_triple_state(M, T, a, b, c));
+}
+
+// One lane per quartet; a warp takes `chunk` consecutive candidates (a
+// multiple of 32), unranks its first ones and steps through the rest, so the
+// lanes share their three upper modes but for a carry and read the tables
+// contiguously along the lowest one.
+template <bool TRIPLES>
+__global__ void __launch_bounds__(128) wit44_table_kernel(WitArgs a, Wit44Tables T, unsigned long long chunk) {
+  unsigned long long kept = 0, near_count = 0, szo = 0, szi = 0;
+  double max_res = 0.0, min_det = INFINITY, max_src = 0.0;
+  const int M = a.n_modes;
+  const unsigned long long* b2 = a.binom + 2 * a.binom_stride;
+  const unsigned long long* b3 = a.binom + 3 * a.binom_stride;
+  const unsigned long long* b4 = a.binom + 4 * a.binom_stride;
+  const unsigned long long warp = (unsigned long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  unsigned long long qi = a.q_begin + warp * chunk + (threadIdx.x & 31);
+  const unsigned long long q_end = min(a.n_quartets, a.q_begin + (warp + 1) * chunk);
+  int i = 0, j = 0, k = 0, l = 0;
+  if (qi < q_end) {
+    unsigned long long q = qi;
+    l = wit_unrank_step(b4, M + 2, q);
+    q -= b4[l];
+    k = wit_unrank_step(b3, l - 1, q);
+    q -= b3[k];
+    j = wit_unrank_step(b2, k - 1, q);
+    q -= b2[j];
+    i = (int)q;
+    j -= 1;
+    k -= 2;
+    l -= 3;
+  }
+  for (; qi < q_end; qi += 32) {
+    const int idx[4] = {i, j, k, l};
+    i += 32;  // the next candidate of this lane
+    while (i > j) {
+      i -= j + 1;
+      if (++j > k) {
+        j = 0;
+        if (++k > l) {
+          k = 0;
+          ++l;
+        }
+      }
+    }
+    int tx = 0, ty = 0;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      tx += __ldg(a.modes + 2 * idx[s]);
+      ty += __ldg(a.modes + 2 * idx[s] + 1);
+    }
+    if (tx == 0 && ty == 0) {
+      ++szo;
+      continue;
+    }
+    if (abs(tx) >= a.nx / 2 || abs(ty) >= a.ny / 2) continue;
+    int strict = 0;
+    double src = 0.0;
+    WitOne s[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) s[p] = wit_single(T, idx[p]);
+    WitSums w = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    // the three splits into two pairs; r2[p]: elevations of the pairs without slot p
+    double r2[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int c = 1; c < 4; ++c) {
+      const int u = c == 1 ? 2 : 1, v = c == 3 ? 2 : 3;  // slots (0, c | u, v)
+      WitSub P = wit_sub_load(T.pair, T.n_pairs, wit_pair_at(idx[0], idx[c]));
+      WitSub Q = wit_sub_load(T.pair, T.n_pairs, wit_pair_at(idx[u], idx[v]));
+      wit_sub_strict(P, strict, src);
+      wit_sub_strict(Q, strict, src);
+      const double pkx = s[0].kx + s[c].kx, pky = s[0].ky + s[c].ky;
+      const double qkx = s[u].kx + s[v].kx, qky = s[u].ky + s[v].ky;
+      const double pm = pkx * pkx + pky * pky, qm = qkx * qkx + qky * qky;
+      wit_block(w, pkx, pky, s[0].om + s[c].om, P.f, P.q * Q.e + 0.25 * pm, pm * Q.e + 0.25 * (pm * P.q));
+      wit_block(w, qkx, qky, s[u].om + s[v].om, Q.f, Q.q * P.e + 0.25 * qm, qm * P.e + 0.25 * (qm * Q.q));
+      wit_cross(w, P.x, P.y, P.v, P.e, pkx, pky, Q.x, Q.y, Q.v, Q.e, qkx, qky);
+      r2[u] += P.e;
+      r2[v] += P.e;
+      r2[0] += Q.e;
+      r2[c] += Q.e;
+    }
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      const int t0 = p == 0 ? 1 : 0, t1 = p <= 1 ? 2 : 1, t2 = p == 3 ? 2 : 3;  // the triple without slot p
+      WitSub t = TRIPLES ? wit_sub_load(T.triple, T.n_triples, wit_triple_at(idx[t0], idx[t1], idx[t2]))
+                         : wit_triple_state(a.M, T, idx[t0], idx[t1], idx[t2]);
+      wit_sub_strict(t, strict, src);
+      const WitOne& o = s[p];
+      const double tkx = s[t0].kx + s[t1].kx + s[t2].kx, tky = s[t0].ky + s[t1].ky + s[t2].ky;
+      const double m2q = o.m2 * o.q, h2 = 0.5 * r2[p];
+      wit_block(w, o.kx, o.ky, o.om, o.f, o.q * t.e + o.m2 * h2 + 0.125 * m2q,
+                o.m2 * t.e + m2q * h2 + 0.125 * (o.m2 * o.m2));
+      wit_block(w, tkx, tky, s[t0].om + s[t1].om + s[t2].om, t.f, 0.5 * t.q, 0.5 * (tkx * tkx + tky * tky));
+      wit_cross(w, -o.kx * o.f, -o.ky * o.f, o.q * o.f, 0.5, o.kx, o.ky, t.x, t.y, t.v, t.e, tkx, tky);
+    }
+    // the quartet's own response
+    const double kx = s[0].kx + s[1].kx + s[2].kx + s[3].kx, ky = s[0].ky + s[1].ky + s[2].ky + s[3].ky;
+    const double om = s[0].om + s[1].om + s[2].om + s[3].om;
+    const double mag = hypot(kx, ky), q = mag * tanh(a.M.h * mag);
+    double s0 = w.LV - w.H - q * w.T, s1 = om * w.T - (w.LT + w.K);
+    const double lin = a.M.g * q, tem = om * om;
+    const double rho = fabs(lin - tem) / fmax(lin + tem, 2.2250738585072014e-308);
+    const bool near = rho < a.thr;
+    double eta = 0.0, psi = 0.0, ret = 0.0, ms = 0.0, ns = 0.0;
+    if (near) {
+      const double wo = sqrt(lin);
+      ms = sqrt(wo / (2.0 * a.M.g));
+      ns = sqrt(a.M.g / (2.0 * wo));
+    }
+    const double ts = om >= 0.0 ? 1.0 : -1.0;
+    if (wit_is_strict(mag)) {
+      ++strict;
+      src = fmax(src, hypot(s0, s1));
+      s0 = s1 = 0.0;
+    } else if (near) {
+      const double ra = s0 / (2.0 * ms), rb = ts * s1 / (2.0 * ns);
+      ret = ra + rb;
+      const double den = om + ts * sqrt(lin);
+      eta = -ms * (ra - rb) / den;
+      psi = -ts * ns * (ra - rb) / den;
+    } else {
+      const double den = tem - lin;
+      eta = -(om * s0 + q * s1) / den;
+      psi = (a.M.g * s0 + om * s1) / den;
+    }
+    // residual of the surface operator (kinematic imaginary, dynamic real)
+    const double er = -om * eta - q * psi - s0 + ms * ret;
+    const double pr = om * psi + a.M.g * eta - s1 + ts * ns * ret;
+    int rep = 1, run = 1;  // multiset repeat factor: product of factorials of run lengths
+#pragma unroll
+    for (int p = 1; p < 4; ++p) {
+      run = idx[p] == idx[p - 1] ? run + 1 : 1;
+      rep *= run;
+    }
+    const int ix = ((tx % a.nx) + a.nx) % a.nx, iy = ((ty % a.ny) + a.ny) % a.ny;
+    const size_t plane = (size_t)a.nx * a.ny, field = plane * a.n_cases;
+    for (int cs = 0; cs < a.n_cases; ++cs) {
+      const cplx* amp = a.amp + (size_t)cs * a.n_modes;
+      cplx wt = cscale(2.0, amp[idx[0]]);
+#pragma unroll
+      for (int p = 1; p < 4; ++p) wt = cmul(wt, amp[idx[p]]);
+      wt = cdiv_real(wt, (double)rep);
+      double* dst = reinterpret_cast<double*>(a.out + (size_t)cs * plane + (size_t)iy * a.nx + ix);
+      atomicAdd(dst, wt.x * eta);
+      atomicAdd(dst + 1, wt.y * eta);
+      atomicAdd(dst + 2 * field, -wt.y * psi);
+      atomicAdd(dst + 2 * field + 1, wt.x * psi);
+      if (near) {
+        atomicAdd(dst + 8 * field, -wt.y * ret);
+        atomicAdd(dst + 8 * field + 1, wt.x * ret);
+      }
+    }
+    ++kept;
+    near_count += near ? 1 : 0;
+    szi += strict;
+    max_res = fmax(max_res, hypot(er, pr));
+    min_det = fmin(min_det, rho);
+    max_src = fmax(max_src, src);
+  }
+  wit_fold_stats(a.stats, kept, near_count, szo, szi, max_res, min_det, max_src);
 }
 
 }  // namespace gl

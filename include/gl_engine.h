@@ -347,7 +347,7 @@ gl_status gl_box_synthesize_noalloc(int n_units, int nx, int ny, int box_x0, int
  * :747-773).  d_modes: (mx, my) int32 pairs; d_amp: [case][mode] complex128;
  * d_out: 5 planes [field][case][ny][nx] complex128 (eta, psi, etaCoordinate,
  * psiCoordinate, retained), zeroed and accumulated by the call; d_work:
- * gl_wit_workspace_size(n_modes) device bytes (statistics + binomial table). */
+ * gl_wit_workspace_size(n_modes) device bytes (statistics, binomial table, sector-44 pair and triple states). */
 typedef struct gl_wit_stats {
   unsigned long long candidates, kept, near, strict_zero_output, strict_zero_intermediate;
   double max_residual, min_detuning, max_strict_zero_source;
