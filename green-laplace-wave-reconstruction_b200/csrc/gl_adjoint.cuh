@@ -38,25 +38,33 @@ struct SeedArgs {
 // + sign transform along x of each residual row; only the box columns are
 // kept.  The column pass is col_fft_kernel with conj_io = 1.
 #ifdef GL_TRANSFORM_TU  // launched by gl_launch_cols.cu
+template <int N>
 __global__ void __launch_bounds__(256, 2) seed_row_kernel(SeedArgs a, const cplx* __restrict__ tw) {
   extern __shared__ cplx smem[];
-  const int n = a.nx;
-  const int L = padded_len(n);
-  int g, G;
-  const FftGroup f = fft_group(n, a.log2nx, g, G);
+  constexpr int T = FftLen<N>::T;
+  const int G = blockDim.x / T, g = threadIdx.x / T, t = threadIdx.x % T;
   const int y = blockIdx.x * G + g;
   const int unit = blockIdx.y;
   const bool active = y < a.ny;
   const int yy = active ? y : 0;
-  cplx* buf = smem + (size_t)g * L;
-  const double* row = a.r + ((size_t)unit * a.ny + yy) * n;
+  cplx* buf = smem + (size_t)g * FftLen<N>::ROW;
+  const double* row = a.r + ((size_t)unit * a.ny + yy) * N;
   cplx* orow = a.out + ((size_t)unit * a.ny + yy) * a.w;
-  auto load = [&](int xb) -> cplx { return cmk(row[xb], 0.0); };
-  auto store = [&](int xb, cplx v) {
-    const int xo = wrap(xb - a.x0, n);
-    if (xo < a.w) orow[xo] = v;
+  // the imaginary parts are a run-time zero: around a literal one the compiler
+  // contracts the first butterflies' products differently from every other
+  // transform's, and the roundoff floors downstream amplify that
+  double zero;
+  asm volatile("mov.f64 %0, 0d0000000000000000;" : "=d"(zero));
+  auto load = [&](int xb, int) -> cplx { return cmk(row[xb], zero); };
+  auto sink = [&](int e, int step, const cplx* v, int cnt) {
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      if (r >= cnt) continue;
+      const int xo = wrap_n<N>(e + r * step - a.x0);
+      if (xo < a.w) orow[xo] = v[r];
+    }
   };
-  fft_row<+1>(buf, f, active, tw, load, store);
+  fft_n<+1, N>(buf, t, 1 + g, active, tw, load, sink);
 }
 #endif  // GL_TRANSFORM_TU
 
@@ -112,39 +120,37 @@ GL_D double cmb_damping(const CmbArgs& a, int job, double nu) {
 // sign by groups of n/16 threads in parallel, and each box bin then sums its
 // banks' multiplied values in bank order (deterministic) into the bank's
 // output spectrum, with the job's damping, the scale and the mask applied.
-// MIX = m > 0: columns of the mixed length 16 m.
-template <int MIX>
+template <int N>
 __global__ void __launch_bounds__(256, 2) col_combine_kernel(CmbArgs a, const cplx* __restrict__ tw,
                                                             int cw) {
   extern __shared__ cplx smem[];
+  constexpr int T = FftLen<N>::T, L = FftLen<N>::COL;
   const int job = blockIdx.y;
   const int unit = job / a.jobs_per_unit;
   const int x_first = blockIdx.x * cw;
   const int ncol = min(cw, a.box.w - x_first);
   const int nb = a.nbanks;
-  const int n = a.n;
-  const int L = padded_len(n);
   const int h = a.box.h;
   const int plane = a.box.w * h;
   // stage: shared row (k * cw + c) holds bank k, column c
-  const cplx* src = a.in + (size_t)job * nb * n * a.box.w + x_first;
-  for (int t = threadIdx.x; t < nb * n * ncol; t += blockDim.x) {
-    const int k = t / (n * ncol), r = t % (n * ncol);
+  const cplx* src = a.in + (size_t)job * nb * N * a.box.w + x_first;
+  for (int q = threadIdx.x; q < nb * N * ncol; q += blockDim.x) {
+    const int k = q / (N * ncol), r = q % (N * ncol);
     const int y = r / ncol, c = r % ncol;
-    smem[(size_t)(k * cw + c) * L + phys(y)] = src[((size_t)k * n + y) * a.box.w + c];
+    smem[(size_t)(k * cw + c) * L + pos<N>(y)] = src[((size_t)k * N + y) * a.box.w + c];
   }
   __syncthreads();
-  int g, G;
-  const FftGroup f = fft_group(n, a.log2n, g, G);
+  const int G = blockDim.x / T, g = threadIdx.x / T, t = threadIdx.x % T;
+  const int y0 = mod_n<N>(a.box.y0);
   const int nrow = nb * ncol;
-  for (int it = 0; it < (nrow + G - 1) / G; ++it) {
-    const int r = it * G + g;
+  for (int it = 0; it < nrow; it += G) {
+    const int r = it + g;
     const bool active = r < nrow;
     const int rr = active ? r : 0;
     cplx* buf = smem + (size_t)((rr / ncol) * cw + rr % ncol) * L;
-    auto load = [&](int yb) -> cplx { return buf[phys(yb)]; };
-    auto store = [&](int yb, cplx v) { buf[phys(yb)] = v; };
-    fft_row<+1, MIX>(buf, f, active, tw, load, store);
+    auto load = [&](int, int e) -> cplx { return buf[pos_in<N>(t, e)]; };
+    auto sink = [&](int o, int step, const cplx* v, int cnt) { row_put<N>(buf, o, step, v, cnt); };
+    fft_n<+1, N>(buf, t, 1 + g, active, tw, load, sink);
   }
   __syncthreads();
   const unsigned char* mask = a.mask ? a.mask + (size_t)unit * plane : nullptr;
@@ -152,7 +158,7 @@ __global__ void __launch_bounds__(256, 2) col_combine_kernel(CmbArgs a, const cp
   for (int t = threadIdx.x; t < ncol * h; t += blockDim.x) {
     const int c = t % ncol, by = t / ncol;
     const int i = by * a.box.w + x_first + c;
-    const int yb = phys(wrap_any(a.box.y0 + by, n));
+    const int yb = pos<N>(wrap_n<N>(y0 + by));
     const GeoRef geo{a.geo, plane, i};
     cplx acc0 = czero(), acc1 = czero(), acc2 = czero(), acc3 = czero();
     for (int k = 0; k < nb; ++k) {

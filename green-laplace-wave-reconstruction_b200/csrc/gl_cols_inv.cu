@@ -1,0 +1,126 @@
+// Inverse column launches: multiplier banks of a spectral box, transformed
+// along y.
+#define GL_TRANSFORM_TU
+#include "gl_host.h"
+
+namespace gl {
+
+namespace {
+
+template <int N>
+void col_ifft_n(dim3 grid, size_t smem, cudaStream_t st, const ColArgs& a, const cplx* tw, int cw, int bpb) {
+  ensure_smem_attr((const void*)col_ifft_kernel<N>, (int)SMEM_LIMIT);
+  col_ifft_kernel<N><<<grid, 256, smem, st>>>(a, tw, cw, bpb);
+}
+
+// Per-stage names of the column launches in the launch accounting.
+const char* col_ifft_name(int kind) {
+  switch (kind) {
+    case COL_ETA22: case COL_PSI22: return "col_ifft_kernel[order2]";
+    case COL_INNER: return "col_ifft_kernel[inner]";
+    case COL_OUTER1: return "col_ifft_kernel[outer1]";
+    case COL_OUTER2: return "col_ifft_kernel[outer2]";
+    case COL_E44_PAIR: case COL_E44_FIRST3: case COL_E44_FIRST4: return "col_ifft_kernel[order4]";
+  }
+  return "col_ifft_kernel";
+}
+
+// A multiplier as rot(f s): its factor plane and rotation.
+void factor_of(int mult, signed char& fac, unsigned char& rot) {
+  constexpr int I = ROT_SWAP | ROT_NEG_RE, MI = ROT_SWAP | ROT_NEG_IM, NEG = ROT_NEG_RE | ROT_NEG_IM;
+  int f = F_DIRECT, r = 0;
+  switch (mult) {
+    case M_ONE: f = F_ONE; break;
+    case M_NU: f = F_NU; break;
+    case M_NU2: f = F_NU2; break;
+    case M_NU3: f = F_NU3; break;
+    case M_NU4: f = F_NU4; break;
+    case M_QX_SNU: f = F_QX_SNU; break;
+    case M_QY_SNU: f = F_QY_SNU; break;
+    case M_Q2_SNU: f = F_Q2_SNU; break;
+    case M_QX: f = F_QX; break;
+    case M_QY: f = F_QY; break;
+    case M_Q2: f = F_Q2; break;
+    case M_NUQX: f = F_NUQX; break;
+    case M_NUQY: f = F_NUQY; break;
+    case M_IQX: f = F_QX, r = I; break;
+    case M_IQY: f = F_QY, r = I; break;
+    case M_MI_NU: f = F_NU, r = MI; break;
+    case M_MI_Q2_SNU: f = F_Q2_SNU, r = MI; break;
+    case M_MI_Q2NU: f = F_Q2NU, r = MI; break;
+    case M_MINUS_A: f = F_A, r = NEG; break;
+    case M_MINUS_Q2: f = F_Q2, r = NEG; break;
+    case M_A: f = F_A; break;
+    case M_MI_NU2QX: f = F_NU2QX, r = MI; break;
+    case M_MI_NU2QY: f = F_NU2QY, r = MI; break;
+    case M_MINUS_Q2A: f = F_Q2A, r = NEG; break;
+    case M_I_ANU: f = F_ANU, r = I; break;
+    case M_Q2NU: f = F_Q2NU; break;
+    case M_NU2QX: f = F_NU2QX; break;
+    case M_NU2QY: f = F_NU2QY; break;
+    case M_IQXA: f = F_QXA, r = I; break;
+    case M_IQYA: f = F_QYA, r = I; break;
+    case M_Q2A: f = F_Q2A; break;
+  }
+  fac = (signed char)f;
+  rot = (unsigned char)r;
+}
+
+}  // namespace
+
+gl_status launch_col_ifft(const ColArgs& a0, int njobs, cudaStream_t st, const cplx* tw) {
+  ColArgs a = a0;
+  if (!is_pow2(a.n) && !mixed_len(a.n)) return fail(GL_ERR_UNSUPPORTED, "column length %d has no transform", a.n);
+  for (int k = 0; k < a.nbanks; ++k) factor_of(a.mult[k], a.fac[k], a.rot[k]);
+  const int T = is_pow2(a.n) ? a.n / 16 : 16, G = 256 / T;
+  const bool direct = T <= 16;
+  // the damped base spectrum of the block's columns is formed only for the
+  // kinds that share one base across their banks (col_ifft_kernel)
+  const bool shared_base = a.kind != COL_PLAIN && a.kind != COL_OUTER2 && a.kind != COL_FLOORED;
+  const int hp = a.box.h | 1, w = a.box.w;
+  auto smem_of = [&](int cw) {
+    return ((size_t)G * columns_row_len(a.n) + (shared_base ? (size_t)cw * hp : 0)) * sizeof(cplx);
+  };
+  // Columns per block and banks per block by a small cost model, in units of
+  // one transform round of a block's G groups: a block costs its rounds, the
+  // damped base (about a third of a round per element and thread) and half a
+  // round of prologue; blocks run in waves of the resident ones.  Splitting the
+  // banks repeats the base but fills the GPU when a launch has few columns and
+  // jobs (one 128^2 unit: 24 blocks of four serial rounds became 192 of one),
+  // and trims the last wave of large ones (16 units of the 1024^2 order-3
+  // workload: 640 blocks in 3 waves).
+  const int cw_top = fft_cols_per_block(a.n, w);
+  int best_cw = cw_top, best_bpb = a.nbanks;
+  double best = 1e30;
+  for (int cw = a.cw_max > 0 ? std::min(a.cw_max, cw_top) : cw_top; cw >= 1; cw /= 2) {
+    const size_t sm = smem_of(cw);
+    if (sm > SMEM_LIMIT) continue;
+    const double slots = (double)SM_COUNT * (2 * (sm + 1024) <= SMEM_LIMIT + 1024 ? 2 : 1);
+    for (int nz = 1; nz <= a.nbanks; ++nz) {
+      const int bpb = (a.nbanks + nz - 1) / nz;
+      const double blocks = (double)((w + cw - 1) / cw) * njobs * ((a.nbanks + bpb - 1) / bpb);
+      const int cols = std::min(cw, w);
+      const int rounds = direct ? (bpb * cols + G - 1) / G : bpb;
+      const int base_iters = shared_base ? (cw * a.box.h + 255) / 256 : 0;
+      const double q = blocks / slots;
+      const double waves = q <= 4.0 ? std::ceil(q) : q + 0.5;
+      const double cost = waves * (0.5 + 0.35 * base_iters + rounds) * (blocks <= SM_COUNT ? 0.7 : 1.0);
+      if (cost < best - 1e-9) {
+        best = cost;
+        best_cw = cw;
+        best_bpb = bpb;
+      }
+    }
+    if (a.cw_max > 0 || cw <= 2) break;
+  }
+  const size_t smem = smem_of(best_cw);
+  dim3 grid((w + best_cw - 1) / best_cw, njobs, (a.nbanks + best_bpb - 1) / best_bpb);
+  const double bytes = (double)njobs * (a.twins ? a.nout : a.nbanks) * w * a.n * sizeof(cplx) +
+                       (double)njobs * w * a.box.h * sizeof(cplx);
+  LaunchScope ls(col_ifft_name(a.kind), st, bytes);
+  GL_LEN_DISPATCH(a.n, col_ifft_n, grid, smem, st, a, tw, best_cw, best_bpb);
+  LAUNCH_CHECK("col_ifft_kernel");
+  return GL_OK;
+}
+
+}  // namespace gl

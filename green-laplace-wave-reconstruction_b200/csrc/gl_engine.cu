@@ -143,6 +143,43 @@ __global__ void geo_kernel(double* geo, Box box, int nx, int ny, double lx, doub
   }
 }
 
+// Factor planes of a box behind its geometry planes (Fac, the first `nfac`),
+// column-major [x][y]: the products in apply_mult's order of operations.
+__global__ void factor_kernel(double* geo, Box box, int nfac) {
+  const int plane = box.w * box.h;
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < plane; j += gridDim.x * blockDim.x) {
+    const int x = j / box.h, y = j % box.h;
+    const BinGeo g = load_geo(geo, plane, y * box.w + x);
+    const double sn = safe_nu(g.nu);
+    for (int f = 0; f < nfac; ++f) {
+      double v = 0.0;
+      switch (f) {
+        case F_A: v = g.a; break;
+        case F_Q2: v = g.q * g.q; break;
+        case F_QX: v = g.qx; break;
+        case F_QY: v = g.qy; break;
+        case F_QXA: v = g.qx * g.a; break;
+        case F_QYA: v = g.qy * g.a; break;
+        case F_Q2A: v = g.q * g.q * g.a; break;
+        case F_NU: v = g.nu; break;
+        case F_NU2: v = g.nu * g.nu; break;
+        case F_NU3: v = g.nu * g.nu * g.nu; break;
+        case F_QX_SNU: v = g.qx / sn; break;
+        case F_QY_SNU: v = g.qy / sn; break;
+        case F_Q2_SNU: v = (g.q * g.q) / sn; break;
+        case F_NUQX: v = g.nu * g.qx; break;
+        case F_NUQY: v = g.nu * g.qy; break;
+        case F_Q2NU: v = (g.q * g.q) * g.nu; break;
+        case F_NU4: v = g.nu * g.nu * g.nu * g.nu; break;
+        case F_NU2QX: v = g.nu * g.nu * g.qx; break;
+        case F_NU2QY: v = g.nu * g.nu * g.qy; break;
+        case F_ANU: v = g.a * g.nu; break;
+      }
+      geo[(size_t)(GEO_PLANES + f) * plane + j] = v;
+    }
+  }
+}
+
 // tw[m] = exp(-2 pi i m/TW_N) for m < TW_N; with count = TW_ALLOC also the
 // tables of the mixed lengths n = 16 m after it (W_n^e, e < n).
 __global__ void twiddle_kernel(cplx* tw, int count) {
@@ -1016,17 +1053,21 @@ extern "C" gl_status gl_plan_create(gl_plan** out, const gl_plan_desc* desc) {
   }
   // device tables
   cudaError_t e = cudaSuccess;
-  auto geo_alloc = [&](double** g, const Box& b) {
-    if (e == cudaSuccess) e = cudaMalloc(g, sizeof(double) * 6 * b.w * b.h);
+  // geometry planes, and behind them the factor planes of the box's column
+  // banks: eta22 and psi22 read the parent box's up to nu^2, order 3 its up to
+  // q^2 nu and the pair box's first four
+  auto geo_alloc = [&](double** g, const Box& b, int nfac) {
+    if (e == cudaSuccess) e = cudaMalloc(g, sizeof(double) * (GEO_PLANES + nfac) * b.w * b.h);
     if (e == cudaSuccess) {
-      const int plane = b.w * b.h;
-      geo_kernel<<<std::min(1024, (plane + 255) / 256), 256>>>(*g, b, d.nx, d.ny, d.lx, d.ly, d.depth, 0.0);
+      const int plane = b.w * b.h, blocks = std::min(1024, (plane + 255) / 256);
+      geo_kernel<<<blocks, 256>>>(*g, b, d.nx, d.ny, d.lx, d.ly, d.depth, 0.0);
+      if (nfac) factor_kernel<<<blocks, 256>>>(*g, b, nfac);
       e = cudaGetLastError();
     }
   };
-  geo_alloc(&p->geo1, p->b1);
-  geo_alloc(&p->geo2, p->b2);
-  geo_alloc(&p->geo3, p->b3);
+  geo_alloc(&p->geo1, p->b1, o3 ? F_Q2NU + 1 : (o2 ? F_NU2 + 1 : 0));
+  geo_alloc(&p->geo2, p->b2, o3 ? F_QY + 1 : 0);
+  geo_alloc(&p->geo3, p->b3, 0);
   if (e == cudaSuccess) e = cudaMalloc(&p->tw, sizeof(cplx) * TW_ALLOC);
   if (e == cudaSuccess) {
     twiddle_kernel<<<TW_ALLOC / 256 + 1, 256>>>(p->tw, TW_ALLOC);
@@ -2163,18 +2204,20 @@ extern "C" gl_status gl_eta44_plan_create(gl_plan** out, const gl_eta44_desc* de
   p->h_comp_scale[1] = want_psi ? e.depth * std::sqrt(e.gravity * e.depth) : 0.0;
   if (want_psi) p->d.gravity = e.gravity;
   cudaError_t err = cudaSuccess;
-  auto geo_alloc = [&](double** g, const Box& b) {
-    if (err == cudaSuccess) err = cudaMalloc(g, sizeof(double) * 6 * b.w * b.h);
+  // geometry planes and the factor planes of each box's column banks
+  auto geo_alloc = [&](double** g, const Box& b, int nfac) {
+    if (err == cudaSuccess) err = cudaMalloc(g, sizeof(double) * (GEO_PLANES + nfac) * b.w * b.h);
     if (err == cudaSuccess) {
-      const int plane = b.w * b.h;
-      geo_kernel<<<std::min(1024, (plane + 255) / 256), 256>>>(*g, b, e.n, e.n, p->d.lx, p->d.ly, e.depth, e.dk);
+      const int plane = b.w * b.h, blocks = std::min(1024, (plane + 255) / 256);
+      geo_kernel<<<blocks, 256>>>(*g, b, e.n, e.n, p->d.lx, p->d.ly, e.depth, e.dk);
+      if (nfac) factor_kernel<<<blocks, 256>>>(*g, b, nfac);
       err = cudaGetLastError();
     }
   };
-  geo_alloc(&p->geo1, p->b1);
-  geo_alloc(&p->geo2, p->b2);
-  geo_alloc(&p->geo3, p->b3);
-  geo_alloc(&p->geo4, p->b4);
+  geo_alloc(&p->geo1, p->b1, N_FAC);
+  geo_alloc(&p->geo2, p->b2, F_Q2A + 1);
+  geo_alloc(&p->geo3, p->b3, F_QY + 1);
+  geo_alloc(&p->geo4, p->b4, 0);
   if (err == cudaSuccess) err = cudaMalloc(&p->tw, sizeof(cplx) * TW_ALLOC);
   if (err == cudaSuccess) {
     twiddle_kernel<<<TW_ALLOC / 256 + 1, 256>>>(p->tw, TW_ALLOC);

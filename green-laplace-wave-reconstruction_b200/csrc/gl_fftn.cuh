@@ -1,0 +1,230 @@
+// Register-resident FFTs of a length known at compile time: the powers of two
+// 16..4096 and the mixed lengths 16 m, m in {3, 5, 6, 9, 10, 12, 15}.
+//
+// A power-of-two length-N transform is run by a group of T = N/16 threads
+// that each hold 16 complex values per pass.  Passes are Stockham autosort
+// steps of radix 16 (the last one radix 2, 4 or 8 when log2 N is not a
+// multiple of 4), so a 256-point transform is two passes and a 1024-point one
+// three, with one shared-memory round trip between passes.  A mixed length
+// 16 m is run by T = 16 threads in two passes: radix m (one butterfly per
+// thread, no twiddles), then radix 16 over the m butterflies (threads t < m)
+// with twiddles from a length-N table.  The first pass reads its inputs
+// through a caller functor (global memory, multipliers, zero outside a box) and
+// the last pass hands its outputs to one (kept columns only, physical scaling),
+// so intermediate rows never exist in global memory.
+//
+// Pass structure, strides and shared-memory offsets are constants: a thread's
+// sixteen values sit at one base address plus immediates, and a kernel carries
+// the code of one length.  Small launches are bound by exactly that -- the
+// fetches of cold instructions (5 of 9 stall cycles per issue in the 128^2
+// column launches with run-time lengths) and the per-element index
+// arithmetic -- and the transform rounds of large ones by the latter.
+//
+// Rows in shared memory keep the first pass's stores free of bank conflicts:
+// powers of two pad one element every 16, mixed lengths with even m one every
+// m, odd m none.  Groups of at most 32 threads synchronise with __syncwarp;
+// larger ones use one named barrier per group.
+#pragma once
+#include "gl_fftreg.cuh"
+
+namespace gl {
+
+// Elements of a padded row of length n; columns_row_len is odd, for kernels
+// that also access rows of consecutive columns.
+GL_HD constexpr int padded_row_len(int n) {
+  return n == 96 || n == 160 || n == 192 ? n + 16 : (n == 48 || n == 80 || n == 144 || n == 240 ? n : n + n / 16);
+}
+GL_HD constexpr int columns_row_len(int n) { return padded_row_len(n) | 1; }
+
+template <int N>
+struct FftLen {
+  static constexpr bool mixed =
+      N == 48 || N == 80 || N == 96 || N == 144 || N == 160 || N == 192 || N == 240;
+  static constexpr int M = mixed ? N / 16 : 0;
+  static constexpr int T = mixed ? 16 : N / 16;  // threads per transform
+  static constexpr int MP = M + (M % 2 == 0 ? 1 : 0);      // padded run of m elements
+  static constexpr int ROW = padded_row_len(N), COL = columns_row_len(N);
+  static_assert(!mixed || ROW == 16 * MP, "one pad element per run of an even m");
+};
+
+// Position of element i in a padded row.
+template <int N>
+GL_D int pos(int i) {
+  if constexpr (!FftLen<N>::mixed) return i + (i >> 4);
+  else if constexpr (FftLen<N>::M % 2) return i;
+  else return i + (int)((unsigned)i / (unsigned)FftLen<N>::M);
+}
+
+// Position of a thread's r-th first-pass input t + r T.
+template <int N>
+GL_D int pos_in(int t, int r) {
+  constexpr int T = FftLen<N>::T;
+  if constexpr (FftLen<N>::mixed) return pos<N>(t + T * r);
+  else return t + (t >> 4) + T * r + (T * r >> 4);
+}
+
+// m mod N for -N <= m < 2N (any m for a power of two).
+template <int N>
+GL_D int wrap_n(int m) {
+  if constexpr (!FftLen<N>::mixed) return m & (N - 1);
+  else return m < 0 ? m + N : (m >= N ? m - N : m);
+}
+
+// m mod N in [0, N), any m.
+template <int N>
+GL_D int mod_n(int m) {
+  if constexpr (!FftLen<N>::mixed) return m & (N - 1);
+  const int r = m % N;
+  return r < 0 ? r + N : r;
+}
+
+template <int N>
+GL_D void group_sync(int id) {
+  constexpr int T = FftLen<N>::T;
+  if constexpr (T <= 32) __syncwarp();
+  else asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(T) : "memory");
+}
+
+// One Stockham pass of radix R over sub-transforms of NS points: LAST hands its
+// butterflies to sink(o, step, v, R) -- element r of v is output o + r * step.
+template <int SIGN, int N, int R, int NS, bool LAST, class Load, class Sink>
+GL_D void pass_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__ tw, Load& load, Sink& sink) {
+  constexpr int T = FftLen<N>::T, B = 16 / R, stride = N / R;
+  constexpr int twstep = TW_N / (NS * R);
+  if constexpr (NS == 1) {
+    cplx v[16];
+    if (active) {
+#pragma unroll
+      for (int r = 0; r < 16; ++r) v[r] = load(t + r * stride, r);
+    }
+    group_sync<N>(id);
+    if (active) {
+      dft16<SIGN>(v);
+      if constexpr (LAST) {
+        sink(16 * t, 1, v, 16);
+      } else {
+        cplx* p = buf + 17 * t;
+#pragma unroll
+        for (int r = 0; r < 16; ++r) p[r] = v[r];
+      }
+    }
+  } else if constexpr (LAST) {
+    // the last pass's butterflies read and write the same elements (their
+    // stride is NS), so they run one after another with no barrier between
+    // reads and writes; short ones are not unrolled, which keeps the
+    // radix-2, 4 and 8 passes at the register count of the radix-16 one
+    if (active) {
+#pragma unroll 1
+      for (int b = 0; b < B; ++b) {
+        cplx v[R];
+        const cplx* p = buf + (T >= 16 ? t + (t >> 4) + b * (T + T / 16) : t + T * b);
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = p[r * (NS + NS / 16)];
+        const int j = t + T * b;
+        apply_twiddles<SIGN, R>(v, j * twstep, tw);
+        dftR<SIGN, R>(v);
+        sink(j, NS, v, R);
+      }
+    }
+  } else {
+    cplx v[16];
+    const int k = t & (NS - 1), o = (t - k) * 16 + k;
+    if (active) {
+      const cplx* p = buf + t + (t >> 4);
+#pragma unroll
+      for (int r = 0; r < 16; ++r) v[r] = p[r * (stride + stride / 16)];
+    }
+    group_sync<N>(id);
+    if (active) {
+      apply_twiddles<SIGN, 16>(v, k * twstep, tw);
+      dft16<SIGN>(v);
+      cplx* p = buf + o + (o >> 4);
+#pragma unroll
+      for (int r = 0; r < 16; ++r) p[r * (NS + NS / 16)] = v[r];
+    }
+  }
+  if constexpr (!LAST) group_sync<N>(id);
+}
+
+// Full transform of one row by its group's T threads (thread t): inputs from
+// load(i, r) (element i, the thread's r-th), outputs to sink(o, step, v, count) (elements o + r * step); the
+// passes between them go through the padded row `buf`.  Every thread of the
+// group makes the same call; `id` names the group's barrier when T > 32.
+// The first pass has read all its inputs before it writes `buf`, and the last
+// one has read element i when it hands it to the sink, so load may read `buf`
+// and sink may write each element back to its own place.  Other lanes may
+// still be reading `buf` when a thread returns.
+template <int SIGN, int N, class Load, class Sink>
+GL_D void fft_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__ tw, Load& load, Sink& sink) {
+  if constexpr (FftLen<N>::mixed) {
+    constexpr int M = FftLen<N>::M, MP = FftLen<N>::MP;
+    {
+      cplx v[M];
+      if (active) {
+#pragma unroll
+        for (int r = 0; r < M; ++r) v[r] = load(t + 16 * r, r);
+      }
+      group_sync<N>(id);
+      if (active) {
+        dft_mixed<SIGN, M>(v);
+        cplx* p = buf + t * MP;
+#pragma unroll
+        for (int r = 0; r < M; ++r) p[r] = v[r];
+      }
+    }
+    group_sync<N>(id);
+    const bool act = active && t < M;
+    cplx v[16];
+    if (act) {
+#pragma unroll
+      for (int r = 0; r < 16; ++r) v[r] = buf[t + MP * r];
+      if (t > 0) apply_twiddles<SIGN, 16>(v, t, tw + TW_N + mixed_tw_offset(N));
+      dft16<SIGN>(v);
+      sink(t, M, v, 16);
+    }
+  } else {
+    pass_n<SIGN, N, 16, 1, N == 16>(buf, t, id, active, tw, load, sink);
+    if constexpr (N >= 256) {
+      pass_n<SIGN, N, 16, 16, N == 256>(buf, t, id, active, tw, load, sink);
+      if constexpr (N == 4096) pass_n<SIGN, N, 16, 256, true>(buf, t, id, active, tw, load, sink);
+      else if constexpr (N > 256) pass_n<SIGN, N, N / 256, 256, true>(buf, t, id, active, tw, load, sink);
+    } else if constexpr (N > 16) {
+      pass_n<SIGN, N, N / 16, 16, true>(buf, t, id, active, tw, load, sink);
+    }
+  }
+}
+
+// Sink that writes a pass's outputs back to a padded row.
+template <int N>
+GL_D void row_put(cplx* buf, int o, int step, const cplx* v, int cnt) {
+  cplx* p = FftLen<N>::mixed ? buf + o : buf + o + (o >> 4);
+  const int d = FftLen<N>::mixed ? FftLen<N>::MP : step + step / 16;
+#pragma unroll
+  for (int r = 0; r < 16; ++r)
+    if (r < cnt) p[r * d] = v[r];
+}
+
+// Runs CALL<N>(args...) for the transform length n.
+#define GL_POW2_CASES(CALL, ...)                \
+  case 16: CALL<16>(__VA_ARGS__); break;        \
+  case 32: CALL<32>(__VA_ARGS__); break;        \
+  case 64: CALL<64>(__VA_ARGS__); break;        \
+  case 128: CALL<128>(__VA_ARGS__); break;      \
+  case 256: CALL<256>(__VA_ARGS__); break;      \
+  case 512: CALL<512>(__VA_ARGS__); break;      \
+  case 1024: CALL<1024>(__VA_ARGS__); break;    \
+  case 2048: CALL<2048>(__VA_ARGS__); break;    \
+  case 4096: CALL<4096>(__VA_ARGS__); break;
+#define GL_LEN_DISPATCH(n, CALL, ...)           \
+  switch (n) {                                  \
+    GL_POW2_CASES(CALL, __VA_ARGS__)            \
+    case 48: CALL<48>(__VA_ARGS__); break;      \
+    case 80: CALL<80>(__VA_ARGS__); break;      \
+    case 96: CALL<96>(__VA_ARGS__); break;      \
+    case 144: CALL<144>(__VA_ARGS__); break;    \
+    case 160: CALL<160>(__VA_ARGS__); break;    \
+    case 192: CALL<192>(__VA_ARGS__); break;    \
+    case 240: CALL<240>(__VA_ARGS__); break;    \
+  }
+
+}  // namespace gl

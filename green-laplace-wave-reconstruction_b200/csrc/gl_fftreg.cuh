@@ -1,30 +1,11 @@
-// Register-resident FFTs for power-of-two lengths 16..4096 and for the
-// mixed lengths 16 m, m in {3, 5, 6, 9, 10, 12, 15} (48 .. 240).
-//
-// A power-of-two length-n transform is run by a group of T = n/16 threads
-// that each hold 16 complex values per pass.  Passes are Stockham autosort
-// steps of radix 16 (the last one radix 2, 4 or 8 when log2 n is not a
-// multiple of 4), so a 256-point transform is two passes and a 1024-point one
-// three, with one shared-memory round trip between passes instead of one per
-// radix-4 stage.  A mixed length 16 m is run by T = 16 threads in two passes:
-// radix m (one butterfly per thread, no twiddles), then radix 16 over the m
-// butterflies (threads t < m) with twiddles from a length-n table.  The first
-// pass reads its inputs through a caller functor (global memory, on-the-fly
-// multipliers, zero outside a spectral box) and the last pass hands its
-// outputs to a caller functor (kept columns only, physical scaling), so
-// intermediate rows never exist in global memory.
-//
-// Shared rows use a padded layout, element i at i + i/16, which keeps the
-// stride-16 stores of the first pass free of bank conflicts.  Groups of at
-// most 32 threads synchronise with __syncwarp; larger groups use one named
-// barrier per group.
+// Register DFTs of radix 2..16, of the small odd radices and of the composite
+// radices of the mixed transform lengths 16 m, m in {3, 5, 6, 9, 10, 12, 15}
+// (48 .. 240), with their twiddles.  gl_fftn.cuh builds the transforms from
+// them.
 #pragma once
 #include "gl_fft.cuh"
 
 namespace gl {
-
-GL_HD int phys(int i) { return i + (i >> 4); }
-GL_HD int padded_len(int n) { return n + (n >> 4) + 1; }  // +1: odd stride between rows
 
 // cos(pi/8), sin(pi/8), sqrt(2)/2
 constexpr double FC8 = 0.92387953251128675613;
@@ -315,173 +296,6 @@ GL_D void apply_twiddles(cplx* v, int m, const cplx* __restrict__ tw) {
   v[13] = cmul(v[13], cmul(w1, w12));
   v[14] = cmul(v[14], cmul(w2, w12));
   v[15] = cmul(v[15], cmul(w3, w12));
-}
-
-// Synchronisation of one group of T threads.
-struct GroupSync {
-  int T, id;
-  GL_D void operator()() const {
-    if (T <= 32) {
-      __syncwarp();
-    } else {
-      asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(T) : "memory");
-    }
-  }
-};
-
-struct FftGroup {
-  int n, log2n;  // transform length (log2n unused for mixed lengths)
-  int m;         // mixed length n = 16 m, else 0
-  int T;         // threads in the group (n / 16, 16 for mixed lengths)
-  int t;         // thread index inside the group
-  GroupSync sync;
-};
-
-// Group geometry of thread tl of a team of `team` threads (a block, or one
-// row's share of a block that carries several rows) doing length-n
-// transforms; named barriers of the team's groups start at id_base.
-GL_D FftGroup fft_group_team(int n, int log2n, int tl, int team, int id_base, int& g, int& G) {
-  FftGroup f;
-  f.n = n;
-  f.log2n = log2n;
-  f.m = mixed_len(n) ? n >> 4 : 0;
-  f.T = f.m ? 16 : n >> 4;
-  G = team / f.T;
-  g = tl / f.T;
-  f.t = tl % f.T;
-  f.sync = GroupSync{f.T, id_base + g};
-  return f;
-}
-
-// Group geometry for a block of `threads` threads doing length-n transforms.
-GL_D FftGroup fft_group(int n, int log2n, int& g, int& G) {
-  FftGroup f;
-  f.n = n;
-  f.log2n = log2n;
-  f.m = mixed_len(n) ? n >> 4 : 0;
-  f.T = f.m ? 16 : n >> 4;
-  G = blockDim.x / f.T;
-  g = threadIdx.x / f.T;
-  f.t = threadIdx.x % f.T;
-  f.sync = GroupSync{f.T, 1 + g};  // named barrier id per group (used when T > 32)
-  return f;
-}
-
-// One Stockham pass of radix R over the padded row `buf`.
-//   FIRST: pass inputs come from load(i) (else from buf), LAST: outputs go to
-//   store(i, v) (else back to buf).  `active` = false runs the barriers only.
-template <int SIGN, int R, bool FIRST, bool LAST, class Load, class Store>
-GL_D void fft_pass(cplx* buf, const FftGroup& f, int ns, bool active, const cplx* __restrict__ tw,
-                   Load& load, Store& store) {
-  constexpr int B = 16 / R;
-  const int stride = f.n / R;
-  cplx v[16];
-#pragma unroll
-  for (int b = 0; b < B; ++b) {
-    const int j = f.t + f.T * b;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int i = j + r * stride;
-      v[b * R + r] = active ? (FIRST ? load(i) : buf[phys(i)]) : czero();
-    }
-  }
-  f.sync();
-  if (active) {
-    const int twstep = TW_N / (ns * R);
-#pragma unroll
-    for (int b = 0; b < B; ++b) {
-      const int j = f.t + f.T * b;
-      const int k = j & (ns - 1);
-      if (ns > 1) apply_twiddles<SIGN, R>(v + b * R, k * twstep, tw);
-      dftR<SIGN, R>(v + b * R);
-      const int o = (j - k) * R + k;
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int i = o + r * ns;
-        if (LAST)
-          store(i, v[b * R + r]);
-        else
-          buf[phys(i)] = v[b * R + r];
-      }
-    }
-  }
-  if (!LAST) f.sync();
-}
-
-// Second pass of a mixed length n = 16 m: radix 16 over the m butterflies
-// j = t < m, inputs buf[t + m r], twiddles W_n^(r t) from the length-n table.
-template <int SIGN, class Store>
-GL_D void fft_mixed_last(cplx* buf, const FftGroup& f, bool active, const cplx* __restrict__ twn,
-                         Store& store) {
-  const int M = f.m, t = f.t;
-  const bool act = active && t < M;
-  cplx v[16];
-  if (act) {
-#pragma unroll
-    for (int r = 0; r < 16; ++r) v[r] = buf[phys(t + M * r)];
-  }
-  f.sync();
-  if (act) {
-    if (t > 0) apply_twiddles<SIGN, 16>(v, t, twn);
-    dft16<SIGN>(v);
-#pragma unroll
-    for (int r = 0; r < 16; ++r) store(t + M * r, v[r]);
-  }
-}
-
-// Whole transform of a mixed length n = 16 m: pass 1 radix m over inputs
-// load(t + 16 r) (butterfly j = t), outputs at t m + r; then the radix-16 pass.
-template <int SIGN, int M, class Load, class Store>
-GL_D void fft_row_mixed(cplx* buf, const FftGroup& f, bool active, const cplx* __restrict__ tw, Load& load,
-                        Store& store) {
-  const int t = f.t;
-  cplx v[M];
-#pragma unroll
-  for (int r = 0; r < M; ++r) v[r] = active ? load(t + 16 * r) : czero();
-  f.sync();
-  if (active) {
-    dft_mixed<SIGN, M>(v);
-#pragma unroll
-    for (int r = 0; r < M; ++r) buf[phys(t * M + r)] = v[r];
-  }
-  f.sync();
-  fft_mixed_last<SIGN>(buf, f, active, tw + TW_N + mixed_tw_offset(f.n), store);
-}
-
-// Full transform of one row.  Requires n >= 16 and all T threads of the
-// group to call it with the same arguments (inactive groups pass
-// active = false and only meet the barriers).  MIX = 0: power-of-two
-// lengths; MIX = m: the mixed length n = 16 m (the twiddle buffer then holds
-// TW_ALLOC entries).  Kernels are instantiated per MIX: one kernel carrying
-// every radix behind a runtime switch spills heavily.
-template <int SIGN, int MIX = 0, class Load, class Store>
-GL_D void fft_row(cplx* buf, const FftGroup& f, bool active, const cplx* __restrict__ tw, Load& load,
-                  Store& store) {
-  if constexpr (MIX > 0) {
-    fft_row_mixed<SIGN, MIX>(buf, f, active, tw, load, store);
-    return;
-  }
-  const int full = f.log2n >> 2;  // radix-16 passes
-  const int rem = f.log2n & 3;    // last radix 2^rem (0: none)
-  const int passes = full + (rem ? 1 : 0);
-  int ns = 1;
-  for (int p = 0; p < passes; ++p) {
-    const bool first = p == 0, last = p == passes - 1;
-    const int R = (p < full) ? 16 : (1 << rem);
-    if (R == 16) {
-      if (first && last) fft_pass<SIGN, 16, true, true>(buf, f, ns, active, tw, load, store);
-      else if (first) fft_pass<SIGN, 16, true, false>(buf, f, ns, active, tw, load, store);
-      else if (last) fft_pass<SIGN, 16, false, true>(buf, f, ns, active, tw, load, store);
-      else fft_pass<SIGN, 16, false, false>(buf, f, ns, active, tw, load, store);
-    } else if (R == 8) {
-      fft_pass<SIGN, 8, false, true>(buf, f, ns, active, tw, load, store);
-    } else if (R == 4) {
-      fft_pass<SIGN, 4, false, true>(buf, f, ns, active, tw, load, store);
-    } else {
-      fft_pass<SIGN, 2, false, true>(buf, f, ns, active, tw, load, store);
-    }
-    ns *= R;
-  }
 }
 
 }  // namespace gl

@@ -112,7 +112,9 @@ constexpr size_t SMEM_LIMIT = 227 * 1024;
 // row kernels also hold a static mbarrier: their dynamic budget leaves 1 KB
 constexpr size_t ROW_SMEM_LIMIT = SMEM_LIMIT - 1024;
 
-inline size_t row_smem(int nbanks, int ncx) { return (size_t)nbanks * padded_len(ncx) * sizeof(cplx); }
+// Shared-memory budget of a row of `nbanks` banks, as plans are accepted by it
+// (padded_row_len plus one element of slack).
+inline size_t row_smem(int nbanks, int ncx) { return (size_t)nbanks * (ncx + ncx / 16 + 1) * sizeof(cplx); }
 
 inline int grid_for(size_t n, int threads, int cap = 4096) {
   size_t b = (n + threads - 1) / threads;
@@ -127,19 +129,8 @@ inline int fft_cols_per_block(int n, int w) {
   return std::max(1, std::min(256 / T, next_pow2(w)));
 }
 
-// Kernels instantiated per mixed radix (MIX = n/16 for the mixed lengths, 0
-// for powers of two).
-#define GL_MIX_DISPATCH(n, launcher, ...)                                   \
-  switch (mixed_len(n) ? (n) / 16 : 0) {                                   \
-    case 3: launcher<3>(__VA_ARGS__); break;                               \
-    case 5: launcher<5>(__VA_ARGS__); break;                               \
-    case 6: launcher<6>(__VA_ARGS__); break;                               \
-    case 9: launcher<9>(__VA_ARGS__); break;                               \
-    case 10: launcher<10>(__VA_ARGS__); break;                             \
-    case 12: launcher<12>(__VA_ARGS__); break;                             \
-    case 15: launcher<15>(__VA_ARGS__); break;                             \
-    default: launcher<0>(__VA_ARGS__); break;                              \
-  }
+// SMs of a B200 (launch shapes weigh their waves against it).
+constexpr int SM_COUNT = 148;
 
 // ---------------------------------------------------------------------------
 // transform launchers
@@ -161,9 +152,11 @@ gl_status launch_gen_rows(const GenRowArgs& a, int nuc, cudaStream_t st);
 
 // Row launches by kind family, one translation unit each.  Each returns
 // false when `a.kind` is not in its family or its row length has no
-// instantiation; `smem` is the per-row dynamic shared memory.
-bool row_dispatch_pair(const RowArgs& a, dim3 grid, int T, size_t smem, cudaStream_t st, const cplx* tw);
-bool row_dispatch_wide(const RowArgs& a, dim3 grid, int T, size_t smem, cudaStream_t st, const cplx* tw);
-bool row_dispatch_adj(const RowArgs& a, dim3 grid, int T, size_t smem, cudaStream_t st, const cplx* tw);
+// instantiation.
+bool row_dispatch_pair(const RowArgs& a, int njobs, cudaStream_t st, const cplx* tw);
+bool row_dispatch_inner(const RowArgs& a, int njobs, cudaStream_t st, const cplx* tw);
+bool row_dispatch_wide(const RowArgs& a, int njobs, cudaStream_t st, const cplx* tw);
+bool row_dispatch_e44(const RowArgs& a, int njobs, cudaStream_t st, const cplx* tw);
+bool row_dispatch_adj(const RowArgs& a, int njobs, cudaStream_t st, const cplx* tw);
 
 }  // namespace gl

@@ -21,7 +21,7 @@
 #include "gl_analysis.cuh"
 #include "gl_async.cuh"
 #include "gl_fft.cuh"
-#include "gl_fftreg.cuh"
+#include "gl_fftn.cuh"
 
 namespace gl {
 
@@ -139,6 +139,24 @@ GL_D cplx apply_mult(int m, const GeoRef& g, cplx s) {
   return czero();
 }
 
+// The multipliers that divide, as apply_mult forms them.
+GL_D cplx mult_direct(int m, const GeoRef& g, cplx s) {
+  const double nu = g.nu();
+  if (m == M_QX_DIVNU || m == M_QY_DIVNU || m == M_Q2_DIVNU) {
+    const double q = m == M_QX_DIVNU ? g.qx() : m == M_QY_DIVNU ? g.qy() : g.q();
+    const cplx t = cscale(m == M_Q2_DIVNU ? q * q : q, s);
+    const double sn = safe_nu(nu);
+    return cmk(t.x / sn, t.y / sn);
+  }
+  // phi = (-i s)/nu where nu > 0 (M_PSI11), then the vertical derivatives
+  if (!(nu > 0.0)) return czero();
+  const cplx phi = cmk(s.y / nu, -s.x / nu);
+  if (m == M_PSI11) return phi;
+  const double q = g.q();
+  if (m == M_PHI_Q4) return cscale(q * q * q * q, phi);
+  return cmuli(cscale((m == M_PHI_IQXQ2 ? g.qx() : g.qy()) * q * q, phi));
+}
+
 // ---------------------------------------------------------------------------
 // column inverse FFT (spectral box -> banks along y)
 // ---------------------------------------------------------------------------
@@ -163,6 +181,9 @@ struct ColArgs {
   int nbanks;
   int mult[MAX_BANKS];     // multiplier per bank
   int src_of[MAX_BANKS];   // spectrum index per bank (COL_PLAIN / COL_OUTER2)
+  // filled by the launch from mult[]: the factor plane and rotation of rot(f s)
+  signed char fac[MAX_BANKS];
+  unsigned char rot[MAX_BANKS];
   Box box;                 // input box (modes)
   const double* geo;       // geometry planes of the input box
   const cplx* spec;        // input spectra
@@ -268,113 +289,153 @@ GL_D cplx col_base(const ColArgs& a, int job, int i, double nu) {
   return v;
 }
 
-// One block: `cw` box columns of one job.  Each column is one length-n
-// inverse transform along y run by a group of n/16 threads; the damped base
-// spectrum of the columns is computed once and every bank applies its
-// multiplier while the first FFT pass reads it.  Output layout
-// [job][bank][y][column] (rows contiguous for the row kernel).
-template <int MIX>
+// Multipliers that are one rounded product per component, rot(f s) with
+// f a real factor of the bin and rot a multiple of 90 degrees, read their
+// factor from a table behind the geometry planes (column-major, so that a
+// transform group's lanes read it contiguously).  The rest (divisions after
+// or before the product) are formed by apply_mult.
+enum Fac : int {
+  F_A = 0, F_Q2, F_QX, F_QY, F_QXA, F_QYA, F_Q2A, F_NU, F_NU2, F_NU3, F_QX_SNU, F_QY_SNU, F_Q2_SNU, F_NUQX,
+  F_NUQY, F_Q2NU, F_NU4, F_NU2QX, F_NU2QY, F_ANU, N_FAC,
+  F_ONE = -1,      // no factor
+  F_DIRECT = -2,   // apply_mult
+};
+constexpr int GEO_PLANES = 6;
+constexpr int ROT_SWAP = 1, ROT_NEG_RE = 2, ROT_NEG_IM = 4;
+
+// One block: box columns x_first .. x_first + cw - 1 of one job and a slice
+// of its banks.  The damped base spectrum of the columns is computed once into
+// shared memory (column-major); each (bank, column) is then one length-N
+// inverse transform along y by a group of T threads, whose first pass reads
+// base x factor straight into registers -- sixteen independent loads, no
+// staging pass.  Items are dealt to the groups column-fastest, so no group
+// idles when a block has few columns.  Transforms of at most 16 threads need no
+// block barrier between items and write their last pass straight to global
+// memory (two adjacent columns of a warp fill each 32-byte sector); longer ones
+// go back row-major through shared memory, one bank at a time.
+// Output layout [job][bank][y][column] (rows contiguous for the row kernel).
+template <int N>
 __global__ void __launch_bounds__(256, 2) col_ifft_kernel(ColArgs a, const cplx* __restrict__ tw,
                                                          int cw, int banks_per_block) {
   extern __shared__ cplx smem[];
+  constexpr int T = FftLen<N>::T, L = FftLen<N>::COL;
+  constexpr bool direct = T <= 16;
   const int job = blockIdx.y;
   const int x_first = blockIdx.x * cw;
   const int ncol = min(cw, a.box.w - x_first);
   const int k_first = blockIdx.z * banks_per_block;
-  const int k_last = min(a.nbanks, k_first + banks_per_block);
-  const int n = a.n;
-  const int L = padded_len(n);
-  const int h = a.box.h;
-  const int plane = a.box.w * a.box.h;
-  cplx* bufs = smem;                   // cw * L
-  cplx* base = smem + (size_t)cw * L;  // cw * h
+  const int nk = min(a.nbanks - k_first, banks_per_block);
+  const int h = a.box.h, w = a.box.w;
+  const int hp = h | 1;  // odd: no conflicts when consecutive columns are written
+  const int plane = w * h;
+  const int G = blockDim.x / T, g = threadIdx.x / T, t = threadIdx.x % T;
+  const int y0 = mod_n<N>(a.box.y0);
+  cplx* buf = smem + g * L;
+  cplx* base = smem + G * L;  // cw * hp
   const bool shared_base = a.kind != COL_PLAIN && a.kind != COL_OUTER2 && a.kind != COL_FLOORED;
   const int lcw = 31 - __clz(cw);  // cw is a power of two
   if (shared_base) {
-    for (int t = threadIdx.x; t < (h << lcw); t += blockDim.x) {
-      const int c = t & (cw - 1), by = t >> lcw;
+    for (int q = threadIdx.x; q < (h << lcw); q += blockDim.x) {
+      const int c = q & (cw - 1), by = q >> lcw;
       if (c >= ncol) continue;
-      const int i = by * a.box.w + x_first + c;
-      base[c * h + by] = col_base(a, job, i, __ldg(a.geo + 3 * plane + i));
+      const int i = by * w + x_first + c;
+      base[c * hp + by] = col_base(a, job, i, __ldg(a.geo + 3 * plane + i));
     }
+    __syncthreads();
   }
-  __syncthreads();
-  int g, G;
-  const FftGroup f = fft_group(n, a.log2n, g, G);
-  const int iters = (ncol + G - 1) / G;
-  // with at least two columns per warp the last pass writes the columns
-  // straight to global memory (two adjacent columns fill each 32-byte
-  // sector) and the banks need no block-wide barrier; longer columns (one
-  // column per warp or more) are written back row-major through shared memory
-  const bool direct = f.T <= 16;
-  for (int k = k_first; k < k_last; ++k) {
-    const int mult = a.mult[k];
-    const cplx* sk = a.spec + (long long)job * a.spec_job_stride + (long long)a.src_of[k] * a.spec_sub_stride;
+  const int nout = a.twins ? a.nout : a.nbanks;
+  const double scale_im = a.conj_io ? -a.scale : a.scale;
+  const int per = direct ? G : cw;  // (bank, column) items per iteration
+  const int items = direct ? nk * ncol : nk * cw;
+  for (int it = 0; it < items; it += per) {
+    const int item = it + g;
+    const int kk = direct ? item / ncol : it / cw;
+    const int c = direct ? item - kk * ncol : g;
+    const bool active = direct ? item < items : g < ncol;
+    const int k = k_first + (active ? kk : 0);
+    const int x = x_first + (active ? c : 0);
+    const cplx* src = shared_base ? base + (active ? c : 0) * hp
+                                  : a.spec + (long long)job * a.spec_job_stride +
+                                        (long long)a.src_of[k] * a.spec_sub_stride + x;
+    int sstep = shared_base ? 1 : w;
     const bool floor_it = a.floor_max && ((a.kind == COL_OUTER2 && a.src_of[k] == 1) || a.kind == COL_FLOORED);
-    const double floor_abs =
-        !floor_it ? 0.0
-                  : a.floor_rel * as_double(a.kind == COL_FLOORED ? a.floor_max[(size_t)job * a.floor_nsrc + a.src_of[k]]
-                                                                  : a.floor_max[job]);
-    const int nout = a.twins ? a.nout : a.nbanks;
-    const int tb = a.twins ? a.twin[k] : -1;
-    const int tfac = tb >= 0 ? a.twin_fac[k] : 0;
-    cplx* dst = a.out + ((size_t)job * nout + (a.twins ? a.out_of[k] : k)) * n * a.box.w + x_first;
-    cplx* dst2 = tb >= 0 ? a.out + ((size_t)job * nout + tb) * n * a.box.w + x_first : nullptr;
-    for (int it = 0; it < iters; ++it) {
-      const int c = it * G + g;
-      const bool active = c < ncol;
-      cplx* buf = bufs + (size_t)(active ? c : 0) * L;
-      cplx* dcol = dst + (active ? c : 0);
-      cplx* dcol2 = dst2 ? dst2 + (active ? c : 0) : nullptr;
-      const double qxc = (dst2 && active) ? __ldg(a.geo + x_first + c) : 0.0;  // qx plane, row 0
-      // The group first writes its column's multiplied box rows to the front
-      // of the column's buffer (one copy of the multiplier code in a short
-      // loop, all loads independent); the first transform pass reads them
-      // back before it writes the padded column over them.
+    const int fac = a.fac[k];
+    int rot = a.conj_io ? a.rot[k] ^ ROT_NEG_IM : a.rot[k];
+    group_sync<N>(1 + g);  // the row's previous transform has been read
+    if (fac == F_DIRECT || floor_it) {
+      // floored or divided values go through the front of the group's row
       if (active) {
-        for (int by = f.t; by < h; by += f.T) {
-          const int i = by * a.box.w + x_first + c;
-          cplx v;
-          if (shared_base) {
-            v = base[c * h + by];
-          } else {
-            v = sk[i];
-            if (floor_it && abs_below(v, floor_abs)) v = czero();
-          }
-          const cplx mv = apply_mult(mult, GeoRef{a.geo, plane, i}, v);
-          buf[by] = a.conj_io ? cconj(mv) : mv;
+        const double floor_abs =
+            !floor_it ? 0.0
+                      : a.floor_rel * as_double(a.kind == COL_FLOORED
+                                                    ? a.floor_max[(size_t)job * a.floor_nsrc + a.src_of[k]]
+                                                    : a.floor_max[job]);
+#pragma unroll 1
+        for (int by = t; by < h; by += T) {
+          cplx v = src[by * sstep];
+          if (floor_it && abs_below(v, floor_abs)) v = czero();
+          buf[by] = fac == F_DIRECT ? mult_direct(a.mult[k], GeoRef{a.geo, plane, by * w + x}, v) : v;
         }
       }
-      f.sync();
-      auto load = [&](int yb) -> cplx {
-        const int by = wrap_any(yb - a.box.y0, n);
-        return by < h ? buf[by] : czero();
-      };
-      auto store = [&](int yb, cplx v) {
-        if (direct) {
-          const cplx w = cscale(a.scale, a.conj_io ? cconj(v) : v);
-          dcol[(size_t)yb * a.box.w] = w;
-          if (dcol2) {
-            const cplx u = cscale(qxc, w);
-            dcol2[(size_t)yb * a.box.w] = tfac == 2 ? cmuli(u) : u;
-          }
-        } else {
-          buf[phys(yb)] = v;
-        }
-      };
-      fft_row<+1, MIX>(buf, f, active, tw, load, store);
+      src = buf;
+      sstep = 1;
     }
-    if (!direct) {
-      __syncthreads();
-      for (int t = threadIdx.x; t < (n << lcw); t += blockDim.x) {
-        const int y = t >> lcw, c = t & (cw - 1);
-        if (c >= ncol) continue;
-        const cplx v = bufs[(size_t)c * L + phys(y)];
-        const cplx w = cscale(a.scale, a.conj_io ? cconj(v) : v);
-        dst[(size_t)y * a.box.w + c] = w;
+    group_sync<N>(1 + g);
+    const double* f = fac >= 0 ? a.geo + (size_t)(GEO_PLANES + fac) * plane + (size_t)x * h : nullptr;
+    auto load = [&](int yb, int) -> cplx {
+      const int by = wrap_n<N>(yb - y0);
+      cplx z = czero();
+      if (by < h) {
+        const cplx v = src[by * sstep];
+        const double m = f ? __ldg(f + by) : 1.0;
+        z.x = m * (rot & ROT_SWAP ? v.y : v.x);
+        z.y = m * (rot & ROT_SWAP ? v.x : v.y);
+        if (rot & ROT_NEG_RE) z.x = -z.x;
+        if (rot & ROT_NEG_IM) z.y = -z.y;
+      }
+      return z;
+    };
+    const int tb = a.twins ? a.twin[k] : -1;
+    const int tfac = tb >= 0 ? a.twin_fac[k] : 0;
+    cplx* dst = a.out + ((size_t)job * nout + (a.twins ? a.out_of[k] : k)) * N * w + x;
+    cplx* dst2 = tb >= 0 ? a.out + ((size_t)job * nout + tb) * N * w + x : nullptr;
+    auto sink = [&](int o, int step, const cplx* v, int cnt) {
+      if constexpr (direct) {
+        const size_t d = (size_t)step * w;
+        cplx* p = dst + (size_t)o * w;
+#pragma unroll
+        for (int r = 0; r < 16; ++r)
+          if (r < cnt) p[r * d] = cmk(a.scale * v[r].x, scale_im * v[r].y);
         if (dst2) {
-          const cplx u = cscale(__ldg(a.geo + x_first + c), w);
-          dst2[(size_t)y * a.box.w + c] = tfac == 2 ? cmuli(u) : u;
+          const double qx = __ldg(a.geo + x);  // qx plane, row 0
+          cplx* p2 = dst2 + (size_t)o * w;
+#pragma unroll
+          for (int r = 0; r < 16; ++r)
+            if (r < cnt) {
+              const cplx u = cscale(qx, cmk(a.scale * v[r].x, scale_im * v[r].y));
+              p2[r * d] = tfac == 2 ? cmuli(u) : u;
+            }
+        }
+      } else {
+        row_put<N>(buf, o, step, v, cnt);
+      }
+    };
+    fft_n<+1, N>(buf, t, 1 + g, active, tw, load, sink);
+    if constexpr (!direct) {
+      __syncthreads();
+      cplx* d0 = a.out + ((size_t)job * nout + (a.twins ? a.out_of[k_first + kk] : k_first + kk)) * N * w + x_first;
+      const int tb0 = a.twins ? a.twin[k_first + kk] : -1;
+      cplx* d1 = tb0 >= 0 ? a.out + ((size_t)job * nout + tb0) * N * w + x_first : nullptr;
+      const bool turn = tb0 >= 0 && a.twin_fac[k_first + kk] == 2;
+      for (int q = threadIdx.x; q < (N << lcw); q += blockDim.x) {
+        const int y = q >> lcw, cc = q & (cw - 1);
+        if (cc >= ncol) continue;
+        const cplx v = smem[cc * L + pos<N>(y)];
+        const cplx u0 = cmk(a.scale * v.x, scale_im * v.y);
+        d0[(size_t)y * w + cc] = u0;
+        if (d1) {
+          const cplx u = cscale(__ldg(a.geo + x_first + cc), u0);
+          d1[(size_t)y * w + cc] = turn ? cmuli(u) : u;
         }
       }
       __syncthreads();
@@ -771,19 +832,19 @@ GL_D void row_products_adj(int kind, cplx* b, int L, int p) {
 // zero outside the bank's box columns, 16 loads in flight per thread), the
 // stage's products, forward transforms of the outputs, and only the output
 // box's columns are written: [job][out][y][col].
-// One instantiation per row kind, so that each stage's products are compiled
-// (and get registers) on their own.  FAMILY 0: order-2/3 stages, 1: adjoint
-// stages, 2: order-4 stages (their rows are wider than 24 banks and are
-// staged in shared memory first).
-// MIX = m > 0: the row length is the mixed length 16 m (pair stages on a
-// product grid narrower than a power of two); 0: a power of two.  MULTI:
-// several short rows per block (RowArgs::rpb).
+// One instantiation per row kind and length, so that each stage's products
+// are compiled (and get registers) on their own.  FAMILY 0: order-2/3 stages,
+// 1: adjoint stages, 2: order-4 stages.
+// MULTI: rows of fewer than 16 threads per transform (powers of two below
+// 256), several rows per block (RowArgs::rpb).
 // B192: launched with at most 192 threads (the order-3 outer row of 256
 // points: 12 groups of 16, 92 KB of shared memory, 2 blocks per SM), so 2
 // blocks per SM leave it 168 registers instead of the 128 of 2 x 256.
-template <int KIND, int MIX = 0, bool MULTI = false, bool B192 = false>
+template <int KIND, int N, bool B192 = false>
 __global__ void __launch_bounds__(B192 ? 192 : 256, 2) row_kernel_t(RowArgs a, const cplx* __restrict__ tw) {
   constexpr int FAMILY = KIND >= ROW_ADJ_ETA22 ? 1 : (KIND >= ROW_E44_PAIR && KIND <= ROW_E44_ORDER4_PSI ? 2 : 0);
+  constexpr int T = FftLen<N>::T, L = FftLen<N>::ROW;
+  constexpr bool MULTI = T < 16;
   extern __shared__ __align__(128) cplx smem[];
   __shared__ __align__(8) unsigned long long stage_bar;
   // MULTI: a.rpb rows per block, each row with its own team of
@@ -792,39 +853,37 @@ __global__ void __launch_bounds__(B192 ? 192 : 256, 2) row_kernel_t(RowArgs a, c
   const int team = blockDim.x / rpb;
   const int rr = MULTI ? threadIdx.x / team : 0;
   const int tl = MULTI ? threadIdx.x % team : threadIdx.x;
-  const int y0 = blockIdx.x * rpb;
-  const int y = y0 + rr;
+  const int y_first = blockIdx.x * rpb;
+  const int y = y_first + rr;
   const bool row_ok = !MULTI || y < a.ny;
   const int job = blockIdx.y;
-  const int n = a.nx;
-  const int L = padded_len(n);
   int nb = 0;
   for (int q = 0; q < a.ngrp; ++q) nb += a.grp[q].nb;
   cplx* banks = smem + (size_t)rr * nb * L;  // this row's nb * L
   // Stage every bank's box row (w contiguous values) into the front of the
-  // bank's own row buffer with bulk async copies, all issued at block start,
-  // so the later transform rounds find their inputs in shared memory.  The
-  // first pass of a bank's transform reads its staged values into registers
-  // before the group writes the padded row over them.
+  // bank's own row buffer with bulk async copies, all issued at block start by
+  // the lanes of the first warp, so the later transform rounds find their
+  // inputs in shared memory.  The first pass of a bank's transform reads its
+  // staged values into registers before the group writes the padded row over
+  // them.
   const uint32_t bar = smem_u32(&stage_bar);
   if (threadIdx.x == 0) mbar_init(bar, 1);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const int nrows = MULTI ? min(rpb, a.ny - y0) : 1;
-    uint32_t bytes = 0;
-    for (int q = 0; q < a.ngrp; ++q) bytes += (uint32_t)(a.grp[q].nb * a.grp[q].w * sizeof(cplx));
-    mbar_arrive_expect_tx(bar, bytes * (uint32_t)nrows + a.wait_surplus);
-    for (int r = 0; r < nrows; ++r) {
-      cplx* rb = smem + (size_t)r * nb * L;
-      int k0 = 0;
-      for (int q = 0; q < a.ngrp; ++q) {
-        const BankGroup& B = a.grp[q];
-        for (int kk = 0; kk < B.nb; ++kk)
-          bulk_g2s(smem_u32(rb + (size_t)(k0 + kk) * L),
-                   B.data + (((size_t)job * B.nb + kk) * a.ny + y0 + r) * B.w, (uint32_t)(B.w * sizeof(cplx)),
-                   bar);
-        k0 += B.nb;
-      }
+  if (threadIdx.x < 32) {
+    const int nrows = MULTI ? min(rpb, a.ny - y_first) : 1;
+    if (threadIdx.x == 0) {
+      uint32_t bytes = 0;
+      for (int q = 0; q < a.ngrp; ++q) bytes += (uint32_t)(a.grp[q].nb * a.grp[q].w * sizeof(cplx));
+      mbar_arrive_expect_tx(bar, bytes * (uint32_t)nrows + a.wait_surplus);
+    }
+    __syncwarp();
+    for (int q = threadIdx.x; q < nrows * nb; q += 32) {
+      const int r = MULTI ? q / nb : 0, k = MULTI ? q - r * nb : q;
+      int gi = 0, kk = k;
+      while (kk >= a.grp[gi].nb) kk -= a.grp[gi++].nb;
+      const BankGroup& B = a.grp[gi];
+      bulk_g2s(smem_u32(smem + (size_t)(r * nb + k) * L),
+               B.data + (((size_t)job * B.nb + kk) * a.ny + y_first + r) * B.w, (uint32_t)(B.w * sizeof(cplx)), bar);
     }
   }
   {
@@ -843,69 +902,68 @@ __global__ void __launch_bounds__(B192 ? 192 : 256, 2) row_kernel_t(RowArgs a, c
       return;
     }
   }
-  int g, G;
-  const FftGroup f = fft_group_team(n, a.log2nx, tl, team, 1 + rr * (team / (MIX ? 16 : (n >> 4))), g, G);
-  for (int it = 0; it < (nb + G - 1) / G; ++it) {
-    const int k = it * G + g;
+  const int G = team / T, g = tl / T, t = tl % T;
+  for (int it = 0; it < nb; it += G) {
+    const int k = it + g;
     const bool active = k < nb && row_ok;
     cplx* buf = banks + (size_t)(active ? k : 0) * L;
-    bool cj = false;
-    int bx0 = 0, bw = 0;
-    {
-      const int kk0 = active ? k : 0;
-      int k0 = 0;
-      for (int q = 0; q < a.ngrp; ++q) {
-        if (kk0 >= k0 && kk0 < k0 + a.grp[q].nb) {
-          const BankGroup& B = a.grp[q];
-          cj = FAMILY == 1 && B.conj != 0;
-          bx0 = B.x0;
-          bw = B.w;
-        }
-        k0 += a.grp[q].nb;
-      }
-    }
-    auto load = [&](int xb) -> cplx {
-      const int xi = MIX ? wrap_any(xb - bx0, n) : wrap(xb - bx0, n);
+    int gi = 0;
+    for (int kk = active ? k : 0; kk >= a.grp[gi].nb; ++gi) kk -= a.grp[gi].nb;
+    const int bw = a.grp[gi].w, bx0 = mod_n<N>(a.grp[gi].x0);
+    const bool cj = FAMILY == 1 && a.grp[gi].conj != 0;
+    auto load = [&](int xb, int) -> cplx {
+      const int xi = wrap_n<N>(xb - bx0);
       const cplx v = xi < bw ? buf[xi] : czero();  // staged box row
       return cj ? cconj(v) : v;
     };
-    auto store = [&](int xb, cplx v) { buf[phys(xb)] = cj ? cconj(v) : v; };
-    fft_row<+1, MIX>(buf, f, active, tw, load, store);
+    auto sink = [&](int o, int step, cplx* v, int cnt) {
+      if (FAMILY == 1 && cj) {
+#pragma unroll
+        for (int r = 0; r < 16; ++r)
+          if (r < cnt) v[r] = cconj(v[r]);
+      }
+      row_put<N>(buf, o, step, v, cnt);
+    };
+    fft_n<+1, N>(buf, t, 1 + g, active, tw, load, sink);
   }
   __syncthreads();
   if (row_ok) {
     if constexpr (FAMILY == 0) {
       const int chan_count = KIND == ROW_PSI22 ? a.us[job / a.jobs_per_unit].chan_count : 0;
-      for (int p = tl; p < n; p += team) row_products(KIND, banks, L, phys(p), chan_count);
+      for (int p = tl; p < N; p += team) row_products(KIND, banks, L, pos<N>(p), chan_count);
     } else if constexpr (FAMILY == 2) {
-      for (int p = tl; p < n; p += team) row_products_e44(KIND, banks, L, phys(p), a.e44_part);
+      for (int p = tl; p < N; p += team) row_products_e44(KIND, banks, L, pos<N>(p), a.e44_part);
     } else {
-      for (int p = tl; p < n; p += team) row_products_adj(KIND, banks, L, phys(p));
+      for (int p = tl; p < N; p += team) row_products_adj(KIND, banks, L, pos<N>(p));
     }
   }
   __syncthreads();
   const int na = a.nout_a > 0 ? a.nout_a : a.nout;
   const bool oc = FAMILY == 1 && a.out_conj != 0;
-  for (int it = 0; it < (a.nout + G - 1) / G; ++it) {
-    const int o = it * G + g;
+  for (int it = 0; it < a.nout; it += G) {
+    const int o = it + g;
     const bool active = o < a.nout && row_ok;
     const int oo = active ? o : 0;
     cplx* buf = banks + (size_t)oo * L;
     const bool second = oo >= na;
-    const int ox0 = second ? a.out2_x0 : a.out_x0;
+    const int ox0 = mod_n<N>(second ? a.out2_x0 : a.out_x0);
     const int ow = second ? a.out2_w : a.out_w;
     const int yr = row_ok ? y : 0;
     cplx* orow = second ? a.out2 + (((size_t)job * (a.nout - na) + (oo - na)) * a.ny + yr) * ow
                         : a.out + (((size_t)job * na + oo) * a.ny + yr) * ow;
-    auto load = [&](int xb) -> cplx {
-      const cplx v = buf[phys(xb)];
+    auto load = [&](int, int r) -> cplx {
+      const cplx v = buf[pos_in<N>(t, r)];
       return oc ? cconj(v) : v;
     };
-    auto store = [&](int xb, cplx v) {
-      const int xo = MIX ? wrap_any(xb - ox0, n) : wrap(xb - ox0, n);
-      if (xo < ow) orow[xo] = oc ? cconj(v) : v;
+    auto sink = [&](int e, int step, cplx* v, int cnt) {
+#pragma unroll
+      for (int r = 0; r < 16; ++r) {
+        if (r >= cnt) continue;
+        const int xo = wrap_n<N>(e + r * step - ox0);
+        if (xo < ow) orow[xo] = oc ? cconj(v[r]) : v[r];
+      }
     };
-    fft_row<-1, MIX>(buf, f, active, tw, load, store);
+    fft_n<-1, N>(buf, t, 1 + g, active, tw, load, sink);
   }
 }
 
@@ -931,22 +989,21 @@ struct ColFftArgs {
 // input ([js][y][col]) are staged with coalesced loads, each column is one
 // forward transform along y, and only the output box's rows are written
 // (support-masked), with the spectrum's max |.| folded into maxslot.
-template <int MIX>
+template <int N>
 __global__ void __launch_bounds__(256, 2) col_fft_kernel(ColFftArgs a, const cplx* __restrict__ tw, int cw) {
   extern __shared__ cplx smem[];
+  constexpr int T = FftLen<N>::T, L = FftLen<N>::COL;
   const int js = blockIdx.y;
   const int job = js / a.nsrc;
   const int unit = job / a.jobs_per_unit;
   const int x_first = blockIdx.x * cw;
   const int ncol = min(cw, a.box.w - x_first);
-  const int n = a.n;
-  const int L = padded_len(n);
   cplx* bufs = smem;  // cw * L
-  const cplx* src = a.in + (size_t)js * n * a.box.w + x_first;
+  const cplx* src = a.in + (size_t)js * N * a.box.w + x_first;
   // stage the kept columns ([y][col] rows in global memory) with eight
   // independent loads in flight per thread
   const int lcw = 31 - __clz(cw);  // cw is a power of two: (y, c) = (t >> lcw, t & (cw - 1))
-  const int total = n << lcw;
+  const int total = N << lcw;
   for (int t0 = threadIdx.x; t0 < total; t0 += 8 * blockDim.x) {
     cplx v[8];
 #pragma unroll
@@ -958,19 +1015,19 @@ __global__ void __launch_bounds__(256, 2) col_fft_kernel(ColFftArgs a, const cpl
     for (int u = 0; u < 8; ++u) {
       const int t = t0 + u * blockDim.x;
       if (t < total && (t & (cw - 1)) < ncol)
-        bufs[(size_t)(t & (cw - 1)) * L + phys(t >> lcw)] = a.conj_io ? cconj(v[u]) : v[u];
+        bufs[(t & (cw - 1)) * L + pos<N>(t >> lcw)] = a.conj_io ? cconj(v[u]) : v[u];
     }
   }
   __syncthreads();
-  int g, G;
-  const FftGroup f = fft_group(n, a.log2n, g, G);
-  for (int it = 0; it < (ncol + G - 1) / G; ++it) {
-    const int c = it * G + g;
+  const int G = blockDim.x / T, g = threadIdx.x / T, t = threadIdx.x % T;
+  const int y0 = mod_n<N>(a.box.y0);
+  for (int it = 0; it < ncol; it += G) {
+    const int c = it + g;
     const bool active = c < ncol;
-    cplx* buf = bufs + (size_t)(active ? c : 0) * L;
-    auto load = [&](int yb) -> cplx { return buf[phys(yb)]; };
-    auto store = [&](int yb, cplx v) { buf[phys(yb)] = v; };
-    fft_row<-1, MIX>(buf, f, active, tw, load, store);
+    cplx* buf = bufs + (active ? c : 0) * L;
+    auto load = [&](int, int r) -> cplx { return buf[pos_in<N>(t, r)]; };
+    auto sink = [&](int o, int step, const cplx* v, int cnt) { row_put<N>(buf, o, step, v, cnt); };
+    fft_n<-1, N>(buf, t, 1 + g, active, tw, load, sink);
   }
   __syncthreads();
   const unsigned char* mask = a.mask ? a.mask + (size_t)unit * a.box.w * a.box.h : nullptr;
@@ -980,7 +1037,7 @@ __global__ void __launch_bounds__(256, 2) col_fft_kernel(ColFftArgs a, const cpl
     const int c = t & (cw - 1), by = t >> lcw;
     if (c >= ncol) continue;
     const int i = by * a.box.w + x_first + c;
-    const cplx raw = bufs[(size_t)c * L + phys(wrap_any(a.box.y0 + by, n))];
+    const cplx raw = bufs[c * L + pos<N>(wrap_n<N>(y0 + by))];
     cplx v = cscale(a.scale, a.conj_io ? cconj(raw) : raw);
     if (mask && !mask[i]) v = czero();
     dst[i] = v;
@@ -1327,14 +1384,12 @@ struct OutArgs {
 // columns) and writes scaled complex values or (REAL, OutArgs::real_only)
 // real parts; one instantiation per output type keeps one store path per
 // kernel.
-template <bool REAL, bool B192 = false>
-__global__ void __launch_bounds__(B192 ? 192 : 256, 2) out_row_kernel(OutArgs a, const cplx* __restrict__ tw) {
+template <bool REAL, int N>
+__global__ void __launch_bounds__(N <= 1024 ? 192 : 256, 2) out_row_kernel(OutArgs a, const cplx* __restrict__ tw) {
+  constexpr int T = FftLen<N>::T, L = FftLen<N>::ROW;
   extern __shared__ __align__(128) cplx smem[];
   __shared__ __align__(8) unsigned long long stage_bar;
-  const int n = a.nx;
-  const int L = padded_len(n);
-  int g, G;
-  const FftGroup f = fft_group(n, a.log2nx, g, G);
+  const int G = blockDim.x / T, g = threadIdx.x / T, t = threadIdx.x % T;
   const int y0 = blockIdx.x * G;
   const int y = y0 + g;
   const int uc = blockIdx.y;
@@ -1349,11 +1404,12 @@ __global__ void __launch_bounds__(B192 ? 192 : 256, 2) out_row_kernel(OutArgs a,
   const uint32_t bar = smem_u32(&stage_bar);
   if (threadIdx.x == 0) mbar_init(bar, 1);
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
     const int nrows = min(G, a.ny - y0);
     const uint32_t bytes = (uint32_t)(a.w * sizeof(cplx));
-    mbar_arrive_expect_tx(bar, bytes * (uint32_t)nrows);
-    for (int r = 0; r < nrows; ++r)
+    if (threadIdx.x == 0) mbar_arrive_expect_tx(bar, bytes * (uint32_t)nrows);
+    __syncwarp();
+    for (int r = threadIdx.x; r < nrows; r += 32)
       bulk_g2s(smem_u32(smem + (size_t)r * L), a.in + ((size_t)uc * a.ny + y0 + r) * a.w, bytes, bar);
   }
   if (__syncthreads_or(!mbar_wait_bounded(bar, 0, BULK_WAIT_CYCLES))) {
@@ -1364,29 +1420,37 @@ __global__ void __launch_bounds__(B192 ? 192 : 256, 2) out_row_kernel(OutArgs a,
     return;
   }
   const double s = a.comp_scale ? a.comp_scale[comp] : a.scale_value;
-  const size_t base = ((size_t)unit * a.out_ncomp + a.comp_offset + comp) * (size_t)a.ny * n +
-                      (size_t)yy * n;
-  auto load = [&](int xb) -> cplx {
-    const int xi = wrap(xb - a.x0, n);
+  const size_t base = (((size_t)unit * a.out_ncomp + a.comp_offset + comp) * a.ny + yy) * N;
+  const int x0 = mod_n<N>(a.x0);
+  auto load = [&](int xb, int) -> cplx {
+    const int xi = wrap_n<N>(xb - x0);
     return xi < a.w ? buf[xi] : czero();  // staged box row
   };
   bool bad = false;  // the output check of the unit's status, folded into the store
   if constexpr (REAL) {
     double* o = reinterpret_cast<double*>(a.out) + base;
-    auto store = [&](int xb, cplx v) {
-      const double r = s * v.x;
-      bad |= !isfinite(r);
-      o[xb] = r;
+    auto sink = [&](int e, int step, const cplx* v, int cnt) {
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        if (q >= cnt) continue;
+        const double r = s * v[q].x;
+        bad |= !isfinite(r);
+        o[e + q * step] = r;
+      }
     };
-    fft_row<+1>(buf, f, active, tw, load, store);
+    fft_n<+1, N>(buf, t, 1 + g, active, tw, load, sink);
   } else {
     cplx* o = reinterpret_cast<cplx*>(a.out) + base;
-    auto store = [&](int xb, cplx v) {
-      const cplx r = cscale(s, v);
-      bad |= !(isfinite(r.x) && isfinite(r.y));
-      o[xb] = r;
+    auto sink = [&](int e, int step, const cplx* v, int cnt) {
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        if (q >= cnt) continue;
+        const cplx r = cscale(s, v[q]);
+        bad |= !(isfinite(r.x) && isfinite(r.y));
+        o[e + q * step] = r;
+      }
     };
-    fft_row<+1>(buf, f, active, tw, load, store);
+    fft_n<+1, N>(buf, t, 1 + g, active, tw, load, sink);
   }
   if (a.us) {
     const bool any = __any_sync(0xffffffffu, bad);

@@ -35,31 +35,29 @@ struct SFft {
   int tw_log2p;          // w = e^{SIGN 2 pi i / 2^tw_log2p}
 };
 
-template <int SIGN>
+template <int SIGN, int N>
 __global__ void __launch_bounds__(256, 2) strided_fft_kernel(SFft a, const cplx* __restrict__ tw, int cw) {
   extern __shared__ cplx smem[];
   const int o = blockIdx.y;
   const int c0 = blockIdx.x * cw;
   const int nc = min(cw, a.ncount - c0);
-  const int n = a.n;
-  const int L = padded_len(n);
+  constexpr int n = N, T = FftLen<N>::T, L = FftLen<N>::COL;
   cplx* base = a.data + (long long)o * a.ostride + (long long)c0 * a.cstride;
   const bool colwise = a.cstride == 1;  // consecutive transforms adjacent in memory
   for (int t = threadIdx.x; t < n * nc; t += blockDim.x) {
     const int i = colwise ? t / nc : t % n;
     const int c = colwise ? t % nc : t / n;
-    smem[(size_t)c * L + phys(i)] = base[(long long)c * a.cstride + (long long)i * a.stride];
+    smem[(size_t)c * L + pos<N>(i)] = base[(long long)c * a.cstride + (long long)i * a.stride];
   }
   __syncthreads();
-  int g, G;
-  const FftGroup f = fft_group(n, a.log2n, g, G);
-  for (int it = 0; it < (nc + G - 1) / G; ++it) {
-    const int c = it * G + g;
+  const int G = blockDim.x / T, g = threadIdx.x / T, tg = threadIdx.x % T;
+  for (int it = 0; it < nc; it += G) {
+    const int c = it + g;
     const bool active = c < nc;
     cplx* buf = smem + (size_t)(active ? c : 0) * L;
-    auto load = [&](int i) -> cplx { return buf[phys(i)]; };
-    auto store = [&](int i, cplx v) { buf[phys(i)] = v; };
-    fft_row<SIGN>(buf, f, active, tw, load, store);
+    auto load = [&](int, int r) -> cplx { return buf[pos_in<N>(tg, r)]; };
+    auto sink = [&](int e, int step, const cplx* v, int cnt) { row_put<N>(buf, e, step, v, cnt); };
+    fft_n<SIGN, N>(buf, tg, 1 + g, active, tw, load, sink);
   }
   __syncthreads();
   const long long pmask = (1LL << a.tw_log2p) - 1;
@@ -67,7 +65,7 @@ __global__ void __launch_bounds__(256, 2) strided_fft_kernel(SFft a, const cplx*
   for (int t = threadIdx.x; t < n * nc; t += blockDim.x) {
     const int k = colwise ? t / nc : t % n;
     const int c = colwise ? t % nc : t / n;
-    cplx v = cscale(a.scale, smem[(size_t)c * L + phys(k)]);
+    cplx v = cscale(a.scale, smem[(size_t)c * L + pos<N>(k)]);
     if (a.tw_mode) {
       const long long m = a.tw_mode == 1 ? (long long)(c0 + c) / a.tw_div : (long long)o;
       const long long e = ((long long)k * m) & pmask;

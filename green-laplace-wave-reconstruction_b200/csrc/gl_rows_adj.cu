@@ -4,11 +4,11 @@
 
 namespace gl {
 
-bool row_dispatch_adj(const RowArgs& a, dim3 grid, int T, size_t smem, cudaStream_t st, const cplx* tw) {
+bool row_dispatch_adj(const RowArgs& a, int njobs, cudaStream_t st, const cplx* tw) {
   switch (a.kind) {
-    case ROW_ADJ_ETA22: return row_launch_mixed<ROW_ADJ_ETA22>(grid, T, smem, st, a, tw);
-    case ROW_ADJ_INNER: return row_launch_mixed<ROW_ADJ_INNER>(grid, T, smem, st, a, tw);
-    case ROW_ADJ_OUTER: row_launch<ROW_ADJ_OUTER>(grid, T, smem, st, a, tw); return true;
+    case ROW_ADJ_ETA22: return row_launch_len<ROW_ADJ_ETA22, 1024, true>(njobs, st, a, tw);
+    case ROW_ADJ_INNER: return row_launch_len<ROW_ADJ_INNER, 512, true>(njobs, st, a, tw);
+    case ROW_ADJ_OUTER: return row_launch_len<ROW_ADJ_OUTER, 512, false>(njobs, st, a, tw);
   }
   return false;
 }

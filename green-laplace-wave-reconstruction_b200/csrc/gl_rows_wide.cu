@@ -1,17 +1,15 @@
 // Row launches of the power-of-two product rows: the order-3 outer stage and
-// the four order-4 row kinds.
+// the order-4 plans' pair and third-level rows (at most 256 points there).
 #define GL_TRANSFORM_TU
 #include "gl_rows_launch.cuh"
 
 namespace gl {
 
-bool row_dispatch_wide(const RowArgs& a, dim3 grid, int T, size_t smem, cudaStream_t st, const cplx* tw) {
+bool row_dispatch_wide(const RowArgs& a, int njobs, cudaStream_t st, const cplx* tw) {
   switch (a.kind) {
-    case ROW_OUTER: row_launch<ROW_OUTER>(grid, T, smem, st, a, tw); return true;
-    case ROW_E44_PAIR: row_launch<ROW_E44_PAIR>(grid, T, smem, st, a, tw); return true;
-    case ROW_E44_THIRD: row_launch<ROW_E44_THIRD>(grid, T, smem, st, a, tw); return true;
-    case ROW_E44_ORDER4: row_launch<ROW_E44_ORDER4>(grid, T, smem, st, a, tw); return true;
-    case ROW_E44_ORDER4_PSI: row_launch<ROW_E44_ORDER4_PSI>(grid, T, smem, st, a, tw); return true;
+    case ROW_OUTER: return row_launch_len<ROW_OUTER, 512, false>(njobs, st, a, tw);
+    case ROW_E44_PAIR: return row_launch_len<ROW_E44_PAIR, 256, false>(njobs, st, a, tw);
+    case ROW_E44_THIRD: return row_launch_len<ROW_E44_THIRD, 256, false>(njobs, st, a, tw);
   }
   return false;
 }

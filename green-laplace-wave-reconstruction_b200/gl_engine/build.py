@@ -21,7 +21,8 @@ CSRC = PKG.parent / "csrc"
 NATIVE = PKG / "_native"
 LIB = NATIVE / "libgl_b200.so"
 OBJ = PKG.parent.parent / "_build"
-SOURCES = ["gl_engine.cu", "gl_launch_cols.cu", "gl_rows_pair.cu", "gl_rows_wide.cu", "gl_rows_adj.cu"]
+SOURCES = ["gl_engine.cu", "gl_cols_inv.cu", "gl_cols_fwd.cu", "gl_launch_cols.cu", "gl_rows_pair.cu",
+           "gl_rows_inner.cu", "gl_rows_wide.cu", "gl_rows_e44.cu", "gl_rows_adj.cu"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
