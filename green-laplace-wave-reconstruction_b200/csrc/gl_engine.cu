@@ -3570,6 +3570,72 @@ extern "C" gl_status gl_deposit_modes_adjoint(const gl_plan* p, int n_units, int
   return GL_OK;
 }
 
+extern "C" gl_status gl_group_modes(int n, const double* a, const double* b, const double* kx, const double* ky,
+                                    const double* omega, double lx, double ly, int nx, int ny, double tolerance,
+                                    int* box, int* seg_offsets, int* seg_bins, double* ab, double* omega_out,
+                                    long long* index, int* n_live, int* n_segments) {
+  if (n < 1 || !a || !b || !kx || !ky || !omega || !box || !seg_offsets || !seg_bins || !ab || !omega_out ||
+      !n_live || !n_segments || nx < 2 || ny < 2 || !(lx > 0) || !(ly > 0))
+    return fail(GL_ERR_INVALID_ARGUMENT, "bad mode table arguments");
+  try {
+    const double dkx = 6.283185307179586 / lx, dky = 6.283185307179586 / ly;
+    auto round_half_away = [](double v) { return std::copysign(std::floor(std::fabs(v) + 0.5), v); };
+    std::vector<int> mode(2 * (size_t)n), live;
+    live.reserve(n);
+    bool off = false, nyquist = false;
+    for (int i = 0; i < n; ++i) {
+      const double mx = round_half_away(kx[i] / dkx), my = round_half_away(ky[i] / dky);
+      const double tol = tolerance * std::max(1.0, std::hypot(kx[i], ky[i]));
+      off = off || std::fabs(kx[i] - mx * dkx) > tol || std::fabs(ky[i] - my * dky) > tol;
+      const bool over = !(std::fabs(mx) < nx / 2.0) || !(std::fabs(my) < ny / 2.0);
+      nyquist = nyquist || over;
+      mode[2 * i] = over ? 0 : (int)mx;
+      mode[2 * i + 1] = over ? 0 : (int)my;
+      if (std::hypot(a[i], b[i]) > 0) live.push_back(i);
+    }
+    if (off) return fail(GL_ERR_OFF_GRID, "Every component must lie on the requested FFT grid.");
+    if (nyquist) return fail(GL_ERR_NYQUIST, "An input component reaches or exceeds a Nyquist boundary.");
+    if (live.empty()) return fail(GL_ERR_ZERO_INPUT, "At least one input amplitude is required.");
+    int x0 = mode[2 * live[0]], x1 = x0, y0 = mode[2 * live[0] + 1], y1 = y0;
+    for (int i : live) {
+      x0 = std::min(x0, mode[2 * i]);
+      x1 = std::max(x1, mode[2 * i]);
+      y0 = std::min(y0, mode[2 * i + 1]);
+      y1 = std::max(y1, mode[2 * i + 1]);
+    }
+    const int w = x1 - x0 + 1, h = y1 - y0 + 1;
+    box[0] = x0;
+    box[1] = y0;
+    box[2] = w;
+    box[3] = h;
+    // counting sort by bin (stable), then the segments of equal bins
+    std::vector<int> start((size_t)w * h + 1, 0);
+    auto bin_of = [&](int i) { return (mode[2 * i + 1] - y0) * w + (mode[2 * i] - x0); };
+    for (int i : live) ++start[(size_t)bin_of(i) + 1];
+    int segs = 0;
+    for (size_t q = 0; q < (size_t)w * h; ++q) {
+      if (start[q + 1] > 0) {
+        seg_offsets[segs] = start[q];
+        seg_bins[segs++] = (int)q;
+      }
+      start[q + 1] += start[q];
+    }
+    seg_offsets[segs] = (int)live.size();
+    for (int i : live) {
+      const int at = start[bin_of(i)]++;
+      ab[2 * at] = a[i];
+      ab[2 * at + 1] = b[i];
+      omega_out[at] = omega[i];
+      if (index) index[at] = i;
+    }
+    *n_live = (int)live.size();
+    *n_segments = segs;
+  } catch (const std::exception& e) {
+    return fail(GL_ERR_INVALID_ARGUMENT, "mode table: %s", e.what());
+  }
+  return GL_OK;
+}
+
 extern "C" gl_status gl_deposit_modes(const gl_plan* p, int n_units, int n_seg, const int* seg_off,
                                       const int* seg_bin, int n_modes, const double* ab,
                                       const double* omega, const double* times, void* out,

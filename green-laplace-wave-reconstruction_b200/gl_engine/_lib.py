@@ -119,6 +119,8 @@ SIGNATURES = {
     "gl_plan_set_wait_test": (C.c_int, [C.c_void_p, C.c_uint, C.c_longlong]),
     "gl_plan_set_tuning": (C.c_int, [C.c_void_p, C.POINTER(Tuning)]),
     "gl_plan_set_lanes": (C.c_int, [C.c_void_p, C.c_int]),
+    "gl_group_modes": (C.c_int, [C.c_int] + [C.c_void_p] * 5 + [C.c_double, C.c_double, C.c_int, C.c_int,
+                                                                C.c_double] + [C.c_void_p] * 8),
     "gl_deposit_modes": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_int,
                                    C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "gl_execute": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p,

@@ -314,37 +314,37 @@ class ModeDeposit:
     index: np.ndarray | None = None   # deposit order -> input mode index
 
 
-def prepare_deposit(coeffs: GLCoefficients, lx, ly, nx, ny) -> ModeDeposit:
+def _group_modes(coeffs: GLCoefficients, lx, ly, nx, ny, seg_off: int, seg_bin: int, ab: int, om: int,
+                 index: int | None) -> tuple[tuple[int, int, int, int], int, int]:
     """Mode -> bin mapping with the off-grid and Nyquist checks of
-    ``deposit_analytic_input`` (``src/gl_spectral_surface.m:123-149``)."""
-    dkx = 2.0 * np.pi / lx
-    dky = 2.0 * np.pi / ly
-    mx = _matlab_round(coeffs.kx / dkx)
-    my = _matlab_round(coeffs.ky / dky)
-    tol = coeffs.options["grid_tolerance"] * np.maximum(1.0, np.hypot(coeffs.kx, coeffs.ky))
-    if np.any(np.abs(coeffs.kx - mx * dkx) > tol) or np.any(np.abs(coeffs.ky - my * dky) > tol):
-        raise GLError("green_laplace:OffGridComponent",
-                      "Every component must lie on the requested FFT grid.")
-    if np.any(np.abs(mx) >= nx / 2) or np.any(np.abs(my) >= ny / 2):
-        raise GLError("green_laplace:Nyquist",
-                      "An input component reaches or exceeds a Nyquist boundary.")
-    mx = mx.astype(np.int64)
-    my = my.astype(np.int64)
-    live = np.hypot(coeffs.a, coeffs.b) > 0
-    idx = np.flatnonzero(live)
-    x0, x1 = int(mx[idx].min()), int(mx[idx].max())
-    y0, y1 = int(my[idx].min()), int(my[idx].max())
-    box = (x0, y0, x1 - x0 + 1, y1 - y0 + 1)
-    bins = (my[idx] - y0) * box[2] + (mx[idx] - x0)
-    order = np.argsort(bins, kind="stable")
-    sb = bins[order]
-    starts = np.flatnonzero(np.r_[True, sb[1:] != sb[:-1]])
-    seg_offsets = np.r_[starts, sb.size].astype(np.int32)
-    seg_bins = sb[starts].astype(np.int32)
-    sel = idx[order]
-    ab = np.stack([coeffs.a[sel], coeffs.b[sel]], axis=1).astype(np.float64).ravel()
-    return ModeDeposit(box=box, seg_offsets=seg_offsets, seg_bins=seg_bins, ab=ab,
-                       omega=coeffs.omega[sel].astype(np.float64), index=sel.astype(np.int64))
+    ``deposit_analytic_input`` (``src/gl_spectral_surface.m:123-149``) into host
+    buffers at the given addresses (``gl_group_modes``): (box, modes, bins)."""
+    a, b, kx, ky, omega = (np.ascontiguousarray(v, dtype=np.float64)
+                           for v in (coeffs.a, coeffs.b, coeffs.kx, coeffs.ky, coeffs.omega))
+    box = (C.c_int * 4)()
+    counts = (C.c_int * 2)()
+    at = C.addressof(counts)
+    status = _lib.load().gl_group_modes(
+        int(a.size), a.ctypes.data, b.ctypes.data, kx.ctypes.data, ky.ctypes.data, omega.ctypes.data,
+        float(lx), float(ly), int(nx), int(ny), float(coeffs.options["grid_tolerance"]), box, seg_off,
+        seg_bin, ab, om, index, at, at + C.sizeof(C.c_int))
+    if status == 12:
+        raise GLError("green_laplace:OffGridComponent", _lib.last_error())
+    if status == 9:
+        raise GLError("green_laplace:ZeroInput", _lib.last_error())
+    _engine_call(status)
+    return tuple(box), counts[0], counts[1]
+
+
+def prepare_deposit(coeffs: GLCoefficients, lx, ly, nx, ny) -> ModeDeposit:
+    """Mode -> bin mapping of ``coeffs`` on one grid (see :func:`_group_modes`)."""
+    n = int(np.size(coeffs.a))
+    seg_off, seg_bin = np.empty(n + 1, dtype=np.int32), np.empty(n, dtype=np.int32)
+    ab, om, index = np.empty(2 * n), np.empty(n), np.empty(n, dtype=np.int64)
+    box, live, segs = _group_modes(coeffs, lx, ly, nx, ny, seg_off.ctypes.data, seg_bin.ctypes.data,
+                                   ab.ctypes.data, om.ctypes.data, index.ctypes.data)
+    return ModeDeposit(box=box, seg_offsets=seg_off[:segs + 1], seg_bins=seg_bin[:segs], ab=ab[:2 * live],
+                       omega=om[:live], index=index[:live])
 
 
 def _components_for(order: int, components: Sequence[str] | None) -> int:
@@ -411,31 +411,35 @@ def surface_batch_device(coeffs: GLCoefficients, Lx, Ly, Nx, Ny, times, *,
     if device.type != "cuda":
         raise GLError("green_laplace:Device", "the GL engine runs on CUDA devices only")
     mask = _components_for(coeffs.order, components)
-    dep = prepare_deposit(coeffs, Lx, Ly, int(Nx), int(Ny))
     n = int(times.size)
     out_mode = OUT_REAL if output == "real" else OUT_COMPLEX
+    # the mode table and the times go through one pinned buffer and one
+    # asynchronous copy (a pageable source would synchronise the stream first)
+    m = int(np.size(coeffs.a))
+    o_ab = 8 * n
+    o_om, o_off = o_ab + 16 * m, o_ab + 24 * m
+    o_bin = o_off + 4 * (m + 1)
+    host = torch.empty(o_bin + 4 * m, dtype=torch.uint8, pin_memory=True)
+    C.memmove(host.data_ptr(), times.ctypes.data, 8 * n)
+    base = host.data_ptr()
+    box, live, segs = _group_modes(coeffs, Lx, Ly, int(Nx), int(Ny), base + o_off, base + o_bin, base + o_ab,
+                                   base + o_om, None)
     plan = get_plan(nx=int(Nx), ny=int(Ny), lx=float(Lx), ly=float(Ly), depth=coeffs.h,
                     gravity=coeffs.g, order=coeffs.order, components=mask,
                     eta22_rank=int(coeffs.options["eta22_rank"]),
-                    allow_below=coeffs.options["allow_below_model_parent_domain"], box=dep.box,
+                    allow_below=coeffs.options["allow_below_model_parent_domain"], box=box,
                     grid=GRID_REFERENCE if grid == "reference" else GRID_COMPACT,
                     max_units=max_units or min(n, 8), output=out_mode, device=device,
                     inner_rank=int(order3_ranks[0]), outer_rank=int(order3_ranks[1]))
     stream = stream or torch.cuda.current_stream(device)
     with torch.cuda.device(device), torch.cuda.stream(stream):
-        def h2d(arr, dtype):
-            # staged through pinned memory so the copy is asynchronous (a
-            # pageable source would synchronise the stream first)
-            host = torch.from_numpy(np.ascontiguousarray(arr)).to(dtype=dtype).pin_memory()
-            return host.to(device=device, non_blocking=True)
-        seg_off = h2d(dep.seg_offsets, torch.int32)
-        seg_bin = h2d(dep.seg_bins, torch.int32)
-        ab = h2d(dep.ab, torch.float64)
-        om = h2d(dep.omega, torch.float64)
-        tt = h2d(times, torch.float64)
-        w, h = dep.box[2], dep.box[3]
-        box_spec = torch.empty((n, h, w, 2), dtype=torch.float64, device=device)
-        plan.deposit(n, seg_off, seg_bin, ab, om, tt, box_spec, stream.cuda_stream)
+        table = host.to(device=device, non_blocking=True)
+        at = table.data_ptr()
+        box_spec = torch.empty((n, box[3], box[2], 2), dtype=torch.float64, device=device)
+        _engine_call(plan.lib.gl_deposit_modes(
+            plan.handle, n, segs, C.c_void_p(at + o_off), C.c_void_p(at + o_bin), live, C.c_void_p(at + o_ab),
+            C.c_void_p(at + o_om), C.c_void_p(at), C.c_void_p(box_spec.data_ptr()),
+            C.c_void_p(stream.cuda_stream)))
         ncomp = plan.info.n_components
         dtype = torch.float64 if out_mode == OUT_REAL else torch.complex128
         if out is None:
@@ -640,6 +644,18 @@ def _xy(Lx, Ly, Nx, Ny):
     return np.meshgrid(np.arange(Nx) * (Lx / Nx), np.arange(Ny) * (Ly / Ny))
 
 
+def _totals(components: dict, names) -> None:
+    """Adds eta, psi and their analytic fields: the components' sums in order."""
+    for kind in ("eta", "psi"):
+        parts = [components[name + "_plus"] for name in names if name.startswith(kind)]
+        total = parts[0] + parts[1] if len(parts) > 1 else parts[0] + 0.0
+        for part in parts[2:]:
+            total += part
+        components[kind + "_plus"] = total
+    for kind in ("eta", "psi"):
+        components[kind] = np.real(components[kind + "_plus"])
+
+
 def gl_spectral_surface(coeffs: GLCoefficients, Lx, Ly, Nx, Ny, t, *, grid: str = "compact",
                         device=None):
     """Stage 2 of the two-stage API: ``(eta, psi, X, Y, components, audit)``.
@@ -649,19 +665,10 @@ def gl_spectral_surface(coeffs: GLCoefficients, Lx, Ly, Nx, Ny, t, *, grid: str 
     res = surface_batch_device(coeffs, Lx, Ly, Nx, Ny, [t], grid=grid, device=device)
     fields = res.fields[0].cpu().numpy()
     components: dict[str, np.ndarray] = {}
-    eta_plus = np.zeros((int(Ny), int(Nx)), dtype=complex)
-    psi_plus = np.zeros_like(eta_plus)
     for k, name in enumerate(res.names):
         components[name + "_plus"] = fields[k]
         components[name] = np.real(fields[k])
-        if name.startswith("eta"):
-            eta_plus += fields[k]
-        else:
-            psi_plus += fields[k]
-    components["eta_plus"] = eta_plus
-    components["psi_plus"] = psi_plus
-    components["eta"] = np.real(eta_plus)
-    components["psi"] = np.real(psi_plus)
+    _totals(components, res.names)
     X, Y = _xy(Lx, Ly, int(Nx), int(Ny))
     audit = _audit(coeffs, res.plan, res.names, Lx, Ly, Nx, Ny, float(t))
     return components["eta"], components["psi"], X, Y, components, audit
@@ -724,39 +731,43 @@ def reconstruct_directional_field(eta1, *, lx: float, ly: float, depth: float,
         e1 = torch.from_numpy(field_).to(dev)
         raw = fft2_device((e1 / depth).to(torch.complex128))
         mag = raw.abs()
-        scale = max(float(mag.max()), np.finfo(float).tiny)
-        # kx == 0 column (_spectral.py:31-33)
-        if float(mag[:, 0].max()) > tol * scale:
-            raise ValueError("eta1 contains a non-negligible kx=0 component")
         spec = torch.zeros_like(raw)
         spec[:, 1:nx // 2] = 2.0 * raw[:, 1:nx // 2]
         rec = torch.real(depth * fft2_device(spec, inverse=True))
-        err = float(torch.linalg.norm(rec - e1) / max(float(torch.linalg.norm(e1)),
-                                                      np.finfo(float).tiny))
+        amag = spec.abs()
+        sup = amag > 1.0e-13 * amag.max().clamp(min=1.0)
+        # one read back: the input checks' numbers and the support's extents
+        numbers = torch.stack((mag.max(), mag[:, 0].max(), torch.linalg.norm(rec - e1), torch.linalg.norm(e1)))
+        seen = torch.cat((numbers, sup.any(dim=1).double(), sup.any(dim=0).double())).cpu().numpy()
+        tiny = np.finfo(float).tiny
+        # kx == 0 column (_spectral.py:31-33)
+        if seen[1] > tol * max(float(seen[0]), tiny):
+            raise ValueError("eta1 contains a non-negligible kx=0 component")
+        err = float(seen[2] / max(float(seen[3]), tiny))
         if err > tol:
             raise ValueError("eta1 is not consistent with the declared strict-forward x propagation")
-        # time phase exp(-i sqrt(g/h) nu t) (spatial.py:67-72)
-        kx_line = 2.0 * np.pi * np.fft.fftfreq(nx, d=lx / nx)
-        ky_line = 2.0 * np.pi * np.fft.fftfreq(ny, d=ly / ny)
-        kxg, kyg = np.meshgrid(kx_line, ky_line)
-        q = np.hypot(depth * kxg, depth * kyg)
-        nu = np.sqrt(q * np.tanh(q))
-        if time != 0.0:
-            phase = torch.from_numpy(np.exp(-1j * np.sqrt(gravity / depth) * nu * time)).to(dev)
-            spec = spec * phase
-        amag = spec.abs()
-        thr = 1.0e-13 * max(1.0, float(amag.max()))
-        sup = amag > thr
-        if not bool(sup.any()):
+        rows, cols = np.flatnonzero(seen[4:4 + ny]), np.flatnonzero(seen[4 + ny:])
+        if rows.size == 0:
             raise ValueError("eta1 has empty analytic support")
-        rows = torch.nonzero(sup.any(dim=1)).flatten().cpu().numpy()
-        cols = torch.nonzero(sup.any(dim=0)).flatten().cpu().numpy()
         mys = np.where(rows < ny // 2, rows, rows - ny)
         mxs = np.where(cols < nx // 2, cols, cols - nx)
         if np.any(mxs <= 0):
             raise ValueError("strict-forward nonzero analytic eta1 support is required")
         box = (int(mxs.min()), int(mys.min()), int(mxs.max() - mxs.min() + 1),
                int(mys.max() - mys.min() + 1))
+        # time phase exp(-i sqrt(g/h) nu t) (spatial.py:67-72) of the box's bins:
+        # the engine reads no others, and a phase moves no modulus past the
+        # support threshold
+        if time != 0.0:
+            kx_line = 2.0 * np.pi * np.fft.fftfreq(nx, d=lx / nx)
+            ky_line = 2.0 * np.pi * np.fft.fftfreq(ny, d=ly / ny)
+            iy = np.arange(box[1], box[1] + box[3]) % ny
+            kxg, kyg = np.meshgrid(kx_line[box[0]:box[0] + box[2]], ky_line[iy])
+            q = np.hypot(depth * kxg, depth * kyg)
+            nu = np.sqrt(q * np.tanh(q))
+            phase = torch.from_numpy(np.exp(-1j * np.sqrt(gravity / depth) * nu * time)).to(dev)
+            at = torch.from_numpy(iy).to(dev)
+            spec[at, box[0]:box[0] + box[2]] *= phase
         mask = _components_for(order, None)
         try:
             plan = get_plan(nx=nx, ny=ny, lx=float(lx), ly=float(ly), depth=float(depth),
@@ -779,19 +790,10 @@ def reconstruct_directional_field(eta1, *, lx: float, ly: float, depth: float,
         fields = out[0].cpu().numpy()
     names = [COMP_NAMES[c] for c in plan.component_ids]
     components: dict[str, Any] = {}
-    eta_plus = np.zeros((ny, nx), dtype=complex)
-    psi_plus = np.zeros_like(eta_plus)
     for k, name in enumerate(names):
         components[name + "_plus"] = fields[k]
         components[name] = np.real(fields[k])
-        if name.startswith("eta"):
-            eta_plus += fields[k]
-        else:
-            psi_plus += fields[k]
-    components["eta_plus"] = eta_plus
-    components["psi_plus"] = psi_plus
-    components["eta"] = np.real(eta_plus)
-    components["psi"] = np.real(psi_plus)
+    _totals(components, names)
     x, y = _xy(lx, ly, nx, ny)
     audit = {
         "implementation": "gl-b200-cuda-directional-spatial",

@@ -214,6 +214,17 @@ gl_status gl_plan_set_lanes(gl_plan* plan, int lanes);
  * bound; the outputs of a timed-out unit are meaningless. */
 gl_status gl_plan_set_wait_test(gl_plan* plan, unsigned int surplus_bytes, long long wait_cycles);
 
+/* Host mode table of gl_deposit_modes: maps n components (a, b, kx, ky, omega)
+ * to the bins of an nx x ny grid on lx x ly with the off-grid and Nyquist
+ * checks of deposit_analytic_input (src/gl_spectral_surface.m:123-149), drops
+ * those of zero amplitude and groups the rest by bin (stable).  Host buffers:
+ * box[4] (x0, y0, w, h), seg_offsets[n + 1], seg_bins[n], ab[2 n], omega_out[n]
+ * and, unless null, index[n] (grouped order -> component). */
+gl_status gl_group_modes(int n, const double* a, const double* b, const double* kx, const double* ky,
+                         const double* omega, double lx, double ly, int nx, int ny, double tolerance,
+                         int* box, int* seg_offsets, int* seg_bins, double* ab, double* omega_out,
+                         long long* index, int* n_live, int* n_segments);
+
 /* Deposit N^2 (a+ib)/h e^{-i omega t} for n_units time snapshots into box
  * spectra [unit][box_h][box_w].  Modes are grouped by destination bin:
  * segment s covers modes seg_offsets[s] .. seg_offsets[s+1]-1 (summed in
