@@ -106,8 +106,8 @@ gl_status launch_seed_rows(const SeedArgs& a, int nunits, cudaStream_t st, const
 
 gl_status launch_sfft(const SFft& a, int outer, int sign, cudaStream_t st, const cplx* tw) {
   const int cw = std::max(1, 256 / (a.n / 16));
-  dim3 grid((unsigned)((a.ncount + cw - 1) / cw), (unsigned)outer);
-  LaunchScope ls("strided_fft_kernel", st, 2.0 * a.n * (double)a.ncount * outer * sizeof(cplx));
+  dim3 grid((unsigned)((a.ncount + cw - 1) / cw), (unsigned)outer, (unsigned)a.fields);
+  LaunchScope ls("strided_fft_kernel", st, 2.0 * a.n * (double)a.ncount * outer * a.fields * sizeof(cplx));
   switch (a.n) { GL_POW2_CASES(sfft_n, grid, cw, sign, st, a, tw) }
   LAUNCH_CHECK("strided_fft_kernel");
   return GL_OK;
