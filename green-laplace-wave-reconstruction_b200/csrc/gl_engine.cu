@@ -21,6 +21,7 @@
 #include "gl_modal.cuh"
 #include "gl_gen.cuh"
 #include "gl_host.h"
+#include "gl_support.cuh"
 
 using namespace gl;
 
@@ -490,95 +491,10 @@ __global__ void mink_copy_kernel(unsigned char* c, long long plane, int which, U
   }
 }
 
-struct ScalarArgs {
-  const UnitSlots* slots;
-  UnitScalars* us;
-  const double* geo1;
-  Box box;
-  int nx, ny;
-  int order;
-  int want_eta22, want_psi22, want_o3;
-  int allow_below;
-  int full_input;
-  int want_e44;
-  double fixed_peak;  // > 0: peak depth supplied by the caller (order 4)
-};
-
-// Scales, shifts and status per unit (spatial.py:179-189, 246-268;
-// _order3.py:35-52).
+// Scales, shifts and status per unit, for boxes beyond analyse_kernel's reach.
 __global__ void scalars_kernel(ScalarArgs a, int n) {
   const int u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= n) return;
-  const UnitSlots& s = a.slots[u];
-  UnitScalars r;
-  memset(&r, 0, sizeof r);
-  int status = 0;
-  if (s.nonfinite) status = GL_ERR_COMPONENTS;
-  if (!status && s.count == 0) status = GL_ERR_EMPTY_SUPPORT;
-  const double smax = as_double(s.smax);
-  if (!status && a.full_input) {
-    const double thr = 1.0e-13 * (smax > 1.0 ? smax : 1.0);
-    if (as_double(s.pad[1]) > thr) status = GL_ERR_OUTSIDE_PLAN;
-  }
-  const double qmin = as_double(s.pad[0]);
-  if (!status && a.want_o3 && !(qmin > 0.5)) status = GL_ERR_ORDER3_DOMAIN;
-  if (!status && a.want_psi22 && qmin < 0.3 && !a.allow_below) status = GL_ERR_ORDER2_DOMAIN;
-  r.nu_min = as_double(s.nu_min);
-  r.nu_max = as_double(s.nu_max);
-  if (!status) {
-    const unsigned long long flat = s.peak_flat;
-    const int ix = (int)(flat % (unsigned long long)a.nx), iy = (int)(flat / (unsigned long long)a.nx);
-    const int mx = ix < a.nx / 2 ? ix : ix - a.nx;
-    const int my = iy < a.ny / 2 ? iy : iy - a.ny;
-    const int i = (my - a.box.y0) * a.box.w + (mx - a.box.x0);
-    const double qp = a.fixed_peak > 0.0 ? a.fixed_peak : a.geo1[2 * a.box.w * a.box.h + i];
-    r.peak_q = qp;
-    const double pnu = sqrt(qp * tanh(qp));
-    const double sqa2 = as_double(s.sqa_max2);
-    r.shift2 = 0.5 * (r.nu_min + sqa2 / 2.0);
-    if (a.want_eta22) {
-      const double t1 = 2.0 * sqrt(qp * tanh(qp));
-      r.lam22 = sqrt(t1 * t1 - 2.0 * qp * tanh(2.0 * qp));
-      if (!(r.lam22 > 0.0) || !isfinite(r.lam22)) status = GL_ERR_SCALE;
-    }
-    if (a.want_psi22) {
-      const double pout = sqrt(2.0 * qp * tanh(2.0 * qp));
-      r.lam_minus = 2.0 * pnu - pout;
-      r.lam_plus = 2.0 * pnu + pout;
-      if (!(r.lam_minus > 0.0) || !isfinite(r.lam_minus) || !(r.lam_plus > 0.0) ||
-          !isfinite(r.lam_plus))
-        status = GL_ERR_SCALE;
-      int cc = 0;
-      for (int c = 0; c < 2; ++c) {
-        if (s.chan_min[c] != BITS_POS_INF) {
-          r.chan_id[cc] = c;
-          r.chan_shift[cc] = 0.5 * (as_double(s.chan_min[c]) + as_double(s.chan_max[c]));
-          ++cc;
-        }
-      }
-      r.chan_count = cc;
-      const double step = (r.nu_max - r.nu_min) / 2.0;
-      r.edge_mid = step == 0.0 ? r.nu_min : step + r.nu_min;
-    }
-    if (a.want_o3) {
-      const double sqa3 = as_double(s.sqa_max3);
-      r.shift3 = 0.5 * (r.nu_min + sqa3 / 3.0);
-      r.lam2 = 2.0 * pnu - sqrt(2.0 * qp * tanh(2.0 * qp));
-      r.lam3 = 3.0 * pnu - sqrt(3.0 * qp * tanh(3.0 * qp));
-      if (!(r.lam2 > 0.0) || !(r.lam3 > 0.0)) status = GL_ERR_SCALE;
-    }
-    if (a.want_e44) {  // gl_eta44_fftw.cpp:121-128
-      const double sqa3 = as_double(s.sqa_max3), sqa4 = as_double(s.pad[2]);
-      r.shift3 = 0.5 * (r.nu_min + sqa3 / 3.0);
-      r.shift4 = 0.5 * (r.nu_min + sqa4 / 4.0);
-      r.lam2 = 2.0 * pnu - sqrt(2.0 * qp * tanh(2.0 * qp));
-      r.lam3 = 3.0 * pnu - sqrt(3.0 * qp * tanh(3.0 * qp));
-      r.lam4 = 4.0 * pnu - sqrt(4.0 * qp * tanh(4.0 * qp));
-      if (!(r.lam2 > 0.0) || !(r.lam3 > 0.0) || !(r.lam4 > 0.0)) status = GL_ERR_SCALE;
-    }
-  }
-  r.status = status;
-  a.us[u] = r;
+  if (u < n) a.us[u] = unit_scalars(a, a.slots[u]);
 }
 
 // Deposit N^2 (a+ib)/h e^{-i omega t} per bin segment (gl_spectral_surface.m:123-149).
@@ -743,7 +659,8 @@ struct gl_plan {
   // workspace layout (byte offsets), for `group` units
   size_t ws_total;
   size_t o_slots, o_us, o_box, o_s1, o_s1f, o_s1r, o_s2, o_s2f, o_s2r, o_s3, o_ch, o_chf, o_chr,
-      o_pm, o_out22, o_outp22, o_out33, o_scratch;
+      o_pm, o_max, o_out22, o_outp22, o_out33, o_scratch;
+  size_t max_slots;  // 64-bit maxima slots of all stages at o_max, zeroed with the analysis
   size_t scratch_bytes;
   // fourth-order eta44 plans (gl_eta44_plan_create)
   bool e44 = false;
@@ -821,7 +738,6 @@ static size_t stage_scratch(const gl_plan* p, int g) {
     b.take(g * J * 8 * p->b1.w * ncy * c);
     b.take(g * J * 2 * p->b2.w * ncy * c);
     b.take(g * J * 2 * b2 * c);
-    b.take(g * J * 2 * 8);
     upd(b.off);
   }
   if (p->want_psi22) {
@@ -838,13 +754,11 @@ static size_t stage_scratch(const gl_plan* p, int g) {
     const size_t J = p->ranks[3], I = p->ranks[2];
     Bump b;
     b.take(g * J * 4 * b2 * c);  // E
-    b.take(g * J * 8 * 16);      // maxima (E, R_O, F)
     const size_t base = b.off;
     Bump in = b;
     in.take(g * J * I * 12 * p->b1.w * ncy * c);
     in.take(g * J * I * 4 * p->b2.w * ncy * c);
     in.take(g * J * I * 4 * b2 * c);
-    in.take(g * J * I * 4 * 8);
     upd(in.off);
     Bump out = b;
     out.take(g * J * 12 * p->b1.w * ncy * c);
@@ -911,6 +825,11 @@ static size_t layout_units(gl_plan* p, int g) {
   p->o_chf = b.take((size_t)g * 2 * p->b1.h * p->ww1 * 8);
   p->o_chr = b.take((size_t)g * 2 * p->b1.h * p->ww1 * 8);
   p->o_pm = b.take(g * 3 * b2);
+  // maxima of eta22's two spectra per node, of order 3's inner spectra (4 per
+  // job) and of its outer ones (eta_t, 4 forcings, 2 psi forcings, 1 spare)
+  const size_t J3 = p->ranks[3], I3 = p->ranks[2];
+  p->max_slots = (p->want_eta22 ? (size_t)g * p->ranks[0] * 2 : 0) + (p->want_o3 ? g * J3 * (8 + 4 * I3) : 0);
+  p->o_max = b.take(p->max_slots * 8);
   p->o_out22 = b.take(g * b2 * c);
   p->o_outp22 = b.take(g * b2 * c);
   p->o_out33 = b.take(g * 2 * b3 * c);
@@ -1394,6 +1313,31 @@ static int comp_slot(const gl_plan* p, int id) {
 static gl_status run_group_eta44(gl_plan* p, int gu, const void* spectra, int layout,
                                  void* outputs, void* ws, int* status, cudaStream_t st);
 
+// Maxima slots of a group (zeroed by its analysis): eta22's, then order 3's.
+static unsigned long long* eta22_maxima(const gl_plan* p, void* ws) { return at<unsigned long long>(ws, p->o_max); }
+static unsigned long long* order3_maxima(const gl_plan* p, void* ws) {
+  return at<unsigned long long>(ws, p->o_max) + (p->want_eta22 ? (size_t)p->group * p->ranks[0] * 2 : 0);
+}
+
+// Shared memory of analyse_kernel for a box, or 0 when the box is beyond it: a
+// thread holds ANA_PER bins, a row ANA_COLS columns.
+static size_t ana_bytes(const Box& b, int levels, int channels) {
+  if ((long long)b.w * b.h > ANA_BINS || b.w > ANA_COLS) return 0;
+  const size_t bytes = ana_words(b.w, b.h, levels, channels) * sizeof(u32);
+  return bytes <= 200 * 1024 ? bytes : 0;
+}
+
+static gl_status launch_analysis(const AnaArgs& a, int gu, size_t smem, cudaStream_t st) {
+  const cudaError_t e = ensure_smem_attr((const void*)analyse_kernel, 200 * 1024);
+  if (e != cudaSuccess) return fail(GL_ERR_CUDA, "analyse_kernel shared-memory limit: %s", cudaGetErrorString(e));
+  {
+    LaunchScope ls_("analyse_kernel", st, 0.0);
+    analyse_kernel<<<gu * ANA_CLUSTER, ANA_THREADS, smem, st>>>(a);
+  }
+  LAUNCH_CHECK("analyse_kernel");
+  return GL_OK;
+}
+
 // Support analysis of a group of units (spatial.py:160-189, _order3.py:33-52):
 // the parent box spectra (extracted from full spectra when needed), the
 // supports S, S2 = S+S, S3 = S2+S, the psi22 radial channels and the per-unit
@@ -1417,7 +1361,24 @@ static gl_status analyse_group(gl_plan* p, int gu, const void* spectra, int layo
   unsigned long long* chf = at<unsigned long long>(ws, p->o_chf);
   unsigned long long* chr = at<unsigned long long>(ws, p->o_chr);
   unsigned char* pm = at<unsigned char>(ws, p->o_pm);
-  {
+  ScalarArgs sc;
+  std::memset(&sc, 0, sizeof sc);
+  sc.slots = slots;
+  sc.us = us;
+  sc.geo1 = p->geo1;
+  sc.box = B1;
+  sc.nx = p->d.nx;
+  sc.ny = p->d.ny;
+  sc.order = p->d.order;
+  sc.want_eta22 = p->want_eta22;
+  sc.want_psi22 = p->want_psi22;
+  sc.want_o3 = p->want_o3;
+  sc.allow_below = p->d.allow_below_model_parent_domain;
+  sc.full_input = layout == GL_SPECTRA_FULL;
+  const bool need_s2 = p->want_eta22 || p->want_psi22 || p->want_o3;
+  const int levels = p->want_o3 ? 3 : (need_s2 ? 2 : 1);
+  const size_t ana_smem = ana_bytes(B1, levels, p->want_psi22);
+  if (ana_smem == 0 || layout == GL_SPECTRA_FULL) {
     LaunchScope ls_("slots_init_kernel", st, 0.0);
     slots_init_kernel<<<(gu + 63) / 64, 64, 0, st>>>(slots, gu);
   }
@@ -1434,6 +1395,27 @@ static gl_status analyse_group(gl_plan* p, int gu, const void* spectra, int layo
     LAUNCH_CHECK("extract_kernel");
   } else {
     spec = reinterpret_cast<const cplx*>(spectra);
+  }
+  *spec_out = spec;
+  if (ana_smem > 0) {
+    AnaArgs a;
+    std::memset(&a, 0, sizeof a);
+    a.spec = spec;
+    a.slots = layout == GL_SPECTRA_FULL ? slots : nullptr;
+    a.levels = levels;
+    a.geo[0] = p->geo2;
+    a.geo[1] = p->geo3;
+    a.mask[0] = s2;
+    a.mask[1] = s3;
+    a.chan = p->want_psi22 ? ch : nullptr;
+    a.pmask = pm;
+    a.sc = sc;
+    a.zero[0] = at<unsigned long long>(ws, p->o_max);
+    a.n_zero[0] = p->max_slots;
+    return launch_analysis(a, gu, ana_smem, st);
+  }
+  CUDA_TRY(cudaMemsetAsync(at<void>(ws, p->o_max), 0, p->max_slots * 8, st));
+  if (layout != GL_SPECTRA_FULL) {
     dim3 g(grid_for(pl1, T, 64), gu);
     {
       LaunchScope ls_("box_max_kernel", st, 0.0);
@@ -1455,7 +1437,6 @@ static gl_status analyse_group(gl_plan* p, int gu, const void* spectra, int layo
     }
     LAUNCH_CHECK("peak_kernel");
   }
-  const bool need_s2 = p->want_eta22 || p->want_psi22 || p->want_o3;
   if (need_s2) {
     dim3 g(grid_for(B1.h * p->ww1, T, 64), gu);
     {
@@ -1530,28 +1511,10 @@ static gl_status analyse_group(gl_plan* p, int gu, const void* spectra, int layo
     }
   }
   {
-    ScalarArgs a;
-    a.slots = slots;
-    a.us = us;
-    a.geo1 = p->geo1;
-    a.box = B1;
-    a.nx = p->d.nx;
-    a.ny = p->d.ny;
-    a.order = p->d.order;
-    a.want_eta22 = p->want_eta22;
-    a.want_psi22 = p->want_psi22;
-    a.want_o3 = p->want_o3;
-    a.allow_below = p->d.allow_below_model_parent_domain;
-    a.full_input = layout == GL_SPECTRA_FULL;
-    a.want_e44 = 0;
-    a.fixed_peak = 0.0;
-    {
-      LaunchScope ls_("scalars_kernel", st, 0.0);
-      scalars_kernel<<<(gu + 63) / 64, 64, 0, st>>>(a, gu);
-    }
-    LAUNCH_CHECK("scalars_kernel");
+    LaunchScope ls_("scalars_kernel", st, 0.0);
+    scalars_kernel<<<(gu + 63) / 64, 64, 0, st>>>(sc, gu);
   }
-  *spec_out = spec;
+  LAUNCH_CHECK("scalars_kernel");
   return GL_OK;
 }
 
@@ -1588,8 +1551,7 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     cplx* P = reinterpret_cast<cplx*>(scratch + b.take((size_t)njobs * 8 * B1.w * ncy2 * sizeof(cplx)));
     cplx* Q = reinterpret_cast<cplx*>(scratch + b.take((size_t)njobs * 2 * B2.w * ncy2 * sizeof(cplx)));
     cplx* R = reinterpret_cast<cplx*>(scratch + b.take((size_t)njobs * 2 * pl2 * sizeof(cplx)));
-    unsigned long long* mx = reinterpret_cast<unsigned long long*>(scratch + b.take((size_t)njobs * 2 * 8));
-    CUDA_TRY(cudaMemsetAsync(mx, 0, (size_t)njobs * 2 * 8, st));
+    unsigned long long* mx = eta22_maxima(p, ws);
     ColArgs a;
     std::memset(&a, 0, sizeof a);
     a.kind = COL_ETA22;
@@ -1792,18 +1754,15 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     const int njobs = nuj * I;
     Bump b;
     cplx* E = reinterpret_cast<cplx*>(scratch + b.take((size_t)nuj * 4 * pl2 * sizeof(cplx)));
-    unsigned long long* mxs = reinterpret_cast<unsigned long long*>(scratch + b.take((size_t)nuj * 8 * 16));
-    unsigned long long* maxEt = mxs;                 // [nuj]
-    unsigned long long* maxRO = mxs + nuj;           // [nuj][4]
-    unsigned long long* maxF = mxs + 5 * nuj;        // [nuj][2]
-    CUDA_TRY(cudaMemsetAsync(mxs, 0, (size_t)nuj * 8 * 8, st));
+    unsigned long long* maxEt = order3_maxima(p, ws);  // [nuj]
+    unsigned long long* maxRO = maxEt + nuj;           // [nuj][4]
+    unsigned long long* maxF = maxEt + 5 * nuj;        // [nuj][2]
+    unsigned long long* maxRI = maxEt + 8 * nuj;       // [njobs][4]
     // inner stage buffers
     Bump bi = b;
     cplx* PI = reinterpret_cast<cplx*>(scratch + bi.take((size_t)njobs * 12 * B1.w * ncy2 * sizeof(cplx)));
     cplx* QI = reinterpret_cast<cplx*>(scratch + bi.take((size_t)njobs * 4 * B2.w * ncy2 * sizeof(cplx)));
     cplx* RI = reinterpret_cast<cplx*>(scratch + bi.take((size_t)njobs * 4 * pl2 * sizeof(cplx)));
-    unsigned long long* maxRI = reinterpret_cast<unsigned long long*>(scratch + bi.take((size_t)njobs * 4 * 8));
-    CUDA_TRY(cudaMemsetAsync(maxRI, 0, (size_t)njobs * 4 * 8, st));
     {
       ColArgs a;
       std::memset(&a, 0, sizeof a);
@@ -2351,15 +2310,14 @@ static gl_status e44_finalize(gl_plan* p, int gu, const cplx* OUT, unsigned long
 // One group of units over outer nodes [o0, o0 + Ro).  With `partial` set,
 // the accumulated order-4 spectra (before the final floor) are written there
 // and nothing else is produced; otherwise the fields are finished.
-static gl_status e44_run(gl_plan* p, int gu, const void* spectra, int layout, int o0, int Ro,
-                         cplx* partial, void* outputs, void* ws, int* status, cudaStream_t st,
-                         int part = -2) {
-  const int T = 256, R = p->R44;
+// Analysis of an order-4 plan's group whose box is beyond analyse_kernel: one
+// launch per reduction and per Minkowski sum.
+static gl_status e44_analyse_large(gl_plan* p, int gu, const cplx* spec, int layout, void* ws, const ScalarArgs& sc,
+                                   cudaStream_t st) {
+  const int T = 256;
   const Box B1 = p->b1, B2 = p->b2, B3 = p->b3, B4 = p->b4;
   const int pl1 = B1.w * B1.h, pl2 = B2.w * B2.h, pl3 = B3.w * B3.h, pl4 = B4.w * B4.h;
   UnitSlots* slots = at<UnitSlots>(ws, p->o_slots);
-  UnitScalars* us = at<UnitScalars>(ws, p->o_us);
-  cplx* boxv = at<cplx>(ws, p->o_box);
   unsigned char* s1 = at<unsigned char>(ws, p->o_s1);
   unsigned long long* s1f = at<unsigned long long>(ws, p->o_s1f);
   unsigned long long* s1r = at<unsigned long long>(ws, p->o_s1r);
@@ -2370,35 +2328,7 @@ static gl_status e44_run(gl_plan* p, int gu, const void* spectra, int layout, in
   unsigned long long* s3f = at<unsigned long long>(ws, p->o_s3f);
   unsigned long long* s3r = at<unsigned long long>(ws, p->o_s3r);
   unsigned char* s4 = at<unsigned char>(ws, p->o_s4);
-  char* e44 = at<char>(ws, p->o_e44);
-  const E44Layout L = e44_layout(p, p->group);
-  cplx* E = reinterpret_cast<cplx*>(e44 + L.E);
-  unsigned long long* maxE = reinterpret_cast<unsigned long long*>(e44 + L.maxE);
-  cplx* TS = reinterpret_cast<cplx*>(e44 + L.T);
-  unsigned long long* maxT = reinterpret_cast<unsigned long long*>(e44 + L.maxT);
-  cplx* OUT = partial ? partial : reinterpret_cast<cplx*>(e44 + L.OUT);
-  unsigned long long* maxOUT = reinterpret_cast<unsigned long long*>(e44 + L.maxOUT);
-  char* tr = e44 + L.transient;
-  const double* dn = p->nodes;  // nodes, then weights at +MAX_RANK
-  gl_status s;
-
-  // ---- analysis: support, S2..S4, shifts, scales
-  {
-    LaunchScope ls_("slots_init_kernel", st, 0.0);
-    slots_init_kernel<<<(gu + 63) / 64, 64, 0, st>>>(slots, gu);
-  }
-  LAUNCH_CHECK("slots_init_kernel");
-  const cplx* spec = boxv;
-  if (layout == GL_SPECTRA_FULL) {
-    CUDA_TRY(cudaMemsetAsync(boxv, 0, sizeof(cplx) * (size_t)gu * pl1, st));
-    dim3 g(grid_for((size_t)p->d.nx * p->d.ny, T, 1024), gu);
-    {
-      LaunchScope ls_("extract_kernel", st, 0.0);
-      extract_kernel<<<g, T, 0, st>>>(reinterpret_cast<const cplx*>(spectra), boxv, B1, p->d.nx, p->d.ny, slots);
-    }
-    LAUNCH_CHECK("extract_kernel");
-  } else {
-    spec = reinterpret_cast<const cplx*>(spectra);
+  if (layout != GL_SPECTRA_FULL) {
     dim3 g(grid_for(pl1, T, 64), gu);
     {
       LaunchScope ls_("box_max_kernel", st, 0.0);
@@ -2462,23 +2392,99 @@ static gl_status e44_run(gl_plan* p, int gu, const void* spectra, int layout, in
     LAUNCH_CHECK("minkowski_kernel");
   }
   {
-    ScalarArgs a;
-    std::memset(&a, 0, sizeof a);
-    a.slots = slots;
-    a.us = us;
-    a.geo1 = p->geo1;
-    a.box = B1;
-    a.nx = p->d.nx;
-    a.ny = p->d.ny;
-    a.order = 4;
-    a.full_input = layout == GL_SPECTRA_FULL;
-    a.want_e44 = 1;
-    a.fixed_peak = p->peak44;
+    LaunchScope ls_("scalars_kernel", st, 0.0);
+    scalars_kernel<<<(gu + 63) / 64, 64, 0, st>>>(sc, gu);
+  }
+  LAUNCH_CHECK("scalars_kernel");
+  return GL_OK;
+}
+
+static gl_status e44_run(gl_plan* p, int gu, const void* spectra, int layout, int o0, int Ro,
+                         cplx* partial, void* outputs, void* ws, int* status, cudaStream_t st,
+                         int part = -2) {
+  const int T = 256, R = p->R44;
+  const Box B1 = p->b1, B2 = p->b2, B3 = p->b3, B4 = p->b4;
+  const int pl1 = B1.w * B1.h, pl2 = B2.w * B2.h, pl3 = B3.w * B3.h, pl4 = B4.w * B4.h;
+  UnitSlots* slots = at<UnitSlots>(ws, p->o_slots);
+  UnitScalars* us = at<UnitScalars>(ws, p->o_us);
+  cplx* boxv = at<cplx>(ws, p->o_box);
+  unsigned char* s2 = at<unsigned char>(ws, p->o_s2);
+  unsigned char* s3 = at<unsigned char>(ws, p->o_s3);
+  unsigned char* s4 = at<unsigned char>(ws, p->o_s4);
+  char* e44 = at<char>(ws, p->o_e44);
+  const E44Layout L = e44_layout(p, p->group);
+  cplx* E = reinterpret_cast<cplx*>(e44 + L.E);
+  unsigned long long* maxE = reinterpret_cast<unsigned long long*>(e44 + L.maxE);
+  cplx* TS = reinterpret_cast<cplx*>(e44 + L.T);
+  unsigned long long* maxT = reinterpret_cast<unsigned long long*>(e44 + L.maxT);
+  cplx* OUT = partial ? partial : reinterpret_cast<cplx*>(e44 + L.OUT);
+  unsigned long long* maxOUT = reinterpret_cast<unsigned long long*>(e44 + L.maxOUT);
+  char* tr = e44 + L.transient;
+  const double* dn = p->nodes;  // nodes, then weights at +MAX_RANK
+  gl_status s;
+
+  // ---- analysis: support, S2..S4, shifts, scales
+  const int JP = Ro * R * R + Ro * R, GP = Ro * R + Ro;
+  const bool psi = p->e44_psi;
+  const int nts = psi ? 4 : 3;   // third-state spectra: es, ps, pts [, ets]
+  const int nf4 = psi ? 4 : 2;   // order-4 rows: fk, fd [, contact, contact_t]
+  const int nout = psi ? 2 : 1;  // accumulated spectra: eta44 [, psi44]
+  ScalarArgs sc;
+  std::memset(&sc, 0, sizeof sc);
+  sc.slots = slots;
+  sc.us = us;
+  sc.geo1 = p->geo1;
+  sc.box = B1;
+  sc.nx = p->d.nx;
+  sc.ny = p->d.ny;
+  sc.order = 4;
+  sc.full_input = layout == GL_SPECTRA_FULL;
+  sc.want_e44 = 1;
+  sc.fixed_peak = p->peak44;
+  const size_t ana_smem = ana_bytes(B1, 4, 0);
+  if (ana_smem == 0 || layout == GL_SPECTRA_FULL) {
+    LaunchScope ls_("slots_init_kernel", st, 0.0);
+    slots_init_kernel<<<(gu + 63) / 64, 64, 0, st>>>(slots, gu);
+  }
+  LAUNCH_CHECK("slots_init_kernel");
+  const cplx* spec = boxv;
+  if (layout == GL_SPECTRA_FULL) {
+    CUDA_TRY(cudaMemsetAsync(boxv, 0, sizeof(cplx) * (size_t)gu * pl1, st));
+    dim3 g(grid_for((size_t)p->d.nx * p->d.ny, T, 1024), gu);
     {
-      LaunchScope ls_("scalars_kernel", st, 0.0);
-      scalars_kernel<<<(gu + 63) / 64, 64, 0, st>>>(a, gu);
+      LaunchScope ls_("extract_kernel", st, 0.0);
+      extract_kernel<<<g, T, 0, st>>>(reinterpret_cast<const cplx*>(spectra), boxv, B1, p->d.nx, p->d.ny, slots);
     }
-    LAUNCH_CHECK("scalars_kernel");
+    LAUNCH_CHECK("extract_kernel");
+  } else {
+    spec = reinterpret_cast<const cplx*>(spectra);
+  }
+  if (ana_smem > 0) {
+    AnaArgs a;
+    std::memset(&a, 0, sizeof a);
+    a.spec = spec;
+    a.slots = layout == GL_SPECTRA_FULL ? slots : nullptr;
+    a.levels = 4;
+    a.geo[0] = p->geo2;
+    a.geo[1] = p->geo3;
+    a.geo[2] = p->geo4;
+    a.mask[0] = s2;
+    a.mask[1] = s3;
+    a.mask[2] = s4;
+    a.sc = sc;
+    a.zero[0] = maxE;
+    a.n_zero[0] = (size_t)gu * GP * 5;
+    a.zero[1] = maxT;
+    a.n_zero[1] = (size_t)gu * R * nts;
+    a.zero[2] = maxOUT;
+    a.n_zero[2] = (size_t)gu * nout;
+    if ((s = launch_analysis(a, gu, ana_smem, st)) != GL_OK) return s;
+  } else if ((s = e44_analyse_large(p, gu, spec, layout, ws, sc, st)) != GL_OK) {
+    return s;
+  } else {
+    CUDA_TRY(cudaMemsetAsync(maxE, 0, (size_t)gu * GP * 5 * 8, st));
+    CUDA_TRY(cudaMemsetAsync(maxT, 0, (size_t)gu * R * nts * 8, st));
+    CUDA_TRY(cudaMemsetAsync(maxOUT, 0, (size_t)gu * nout * 8, st));
   }
   const double inv_scale = 1.0 / ((double)p->d.nx * (double)p->d.ny);
   // Product grid of each stage: the pair stage only forms products of two
@@ -2494,15 +2500,6 @@ static gl_status e44_run(gl_plan* p, int gu, const void* spectra, int layout, in
                      ((double)p->d.nx * (double)p->d.ny) / ((double)nx * (double)ny)};
   };
   StageGrid cur = stage_grid(p->ncx, p->ncy);
-  const int JP = Ro * R * R + Ro * R, GP = Ro * R + Ro;
-  const bool psi = p->e44_psi;
-  const int nts = psi ? 4 : 3;   // third-state spectra: es, ps, pts [, ets]
-  const int nf4 = psi ? 4 : 2;   // order-4 rows: fk, fd [, contact, contact_t]
-  const int nout = psi ? 2 : 1;  // accumulated spectra: eta44 [, psi44]
-  CUDA_TRY(cudaMemsetAsync(maxE, 0, (size_t)gu * GP * 5 * 8, st));
-  CUDA_TRY(cudaMemsetAsync(maxT, 0, (size_t)gu * R * nts * 8, st));
-  CUDA_TRY(cudaMemsetAsync(maxOUT, 0, (size_t)gu * nout * 8, st));
-
   auto colargs = [&](int kind, int nb, const int* mults, const int* srcs, const Box& box,
                      const double* geo, const cplx* sp, long long job_stride, long long sub_stride,
                      int jobs_per_unit, cplx* outp) {
@@ -2894,10 +2891,10 @@ static bool adj_eta22(const gl_plan* p) { return (p->comps & GL_COMP_ETA22) != 0
 static bool adj_eta33(const gl_plan* p) { return (p->comps & GL_COMP_ETA33) != 0; }
 
 struct AdjStage22 {
-  size_t P, Q, R, mx, RA, QA, end;
+  size_t P, Q, R, RA, QA, end;
 };
 struct AdjStage33 {
-  size_t E, mxs, PI, QI, RI, maxRI, P1, P2, QO, RO, RAo, QA1, QA2, EA, RAi, QAi, end;
+  size_t E, PI, QI, RI, P1, P2, QO, RO, RAo, QA1, QA2, EA, RAi, QAi, end;
 };
 
 static AdjStage22 adj_stage22(const gl_plan* p, size_t base, int g) {
@@ -2909,7 +2906,6 @@ static AdjStage22 adj_stage22(const gl_plan* p, size_t base, int g) {
   s.P = b.take(nj * 8 * p->b1.w * ncy * c);
   s.Q = b.take(nj * 2 * p->b2.w * ncy * c);  // also the adjoint columns
   s.R = b.take(nj * 2 * pl2 * c);
-  s.mx = b.take(nj * 2 * 8);
   s.RA = b.take(nj * 2 * pl2 * c);
   s.QA = b.take(nj * 8 * p->b1.w * ncy * c);
   s.end = b.off;
@@ -2924,11 +2920,9 @@ static AdjStage33 adj_stage33(const gl_plan* p, size_t base, int g) {
   b.off = base;
   AdjStage33 s;
   s.E = b.take(nuj * 4 * pl2 * c);
-  s.mxs = b.take(nuj * 3 * 8);                       // eta_t max [nuj], forcing maxima [nuj][2]
   s.PI = b.take(nj * 12 * p->b1.w * ncy * c);
   s.QI = b.take(nj * 4 * p->b2.w * ncy * c);         // also the inner adjoint columns
   s.RI = b.take(nj * 4 * pl2 * c);
-  s.maxRI = b.take(nj * 4 * 8);
   s.P1 = b.take(nuj * 12 * p->b1.w * ncy * c);
   s.P2 = b.take(nuj * 9 * p->b2.w * ncy * c);
   s.QO = b.take(nuj * 2 * p->b3.w * ncy * c);        // also the outer adjoint columns
@@ -3113,10 +3107,9 @@ static gl_status run_adjoint_group(gl_plan* p, int gu, const void* spectra, int 
     cplx* P = reinterpret_cast<cplx*>(base + S.P);
     cplx* Q = reinterpret_cast<cplx*>(base + S.Q);
     cplx* R = reinterpret_cast<cplx*>(base + S.R);
-    unsigned long long* mx = reinterpret_cast<unsigned long long*>(base + S.mx);
+    unsigned long long* mx = eta22_maxima(p, ws);
     cplx* RA = reinterpret_cast<cplx*>(base + S.RA);
     cplx* QA = reinterpret_cast<cplx*>(base + S.QA);
-    CUDA_TRY(cudaMemsetAsync(mx, 0, (size_t)nj * 2 * 8, st));
     const int m8[8] = {M_ONE, M_NU, M_NU2, M_QX_DIVNU, M_QY_DIVNU, M_Q2_DIVNU, M_QX, M_QY};
     // forward node fields and products (recomputed)
     ColArgs a;
@@ -3215,12 +3208,12 @@ static gl_status run_adjoint_group(gl_plan* p, int gu, const void* spectra, int 
     const int nuj = gu * Jo, nj = nuj * I;
     const AdjStage33 S = adj_stage33(p, L.stage, p->group);
     cplx* E = reinterpret_cast<cplx*>(base + S.E);
-    unsigned long long* maxEt = reinterpret_cast<unsigned long long*>(base + S.mxs);
-    unsigned long long* maxRO = maxEt + nuj;
+    unsigned long long* maxEt = order3_maxima(p, ws);  // [nuj]
+    unsigned long long* maxRO = maxEt + nuj;           // [nuj][2]
+    unsigned long long* maxRI = maxEt + 8 * nuj;       // [nj][4]
     cplx* PI = reinterpret_cast<cplx*>(base + S.PI);
     cplx* QI = reinterpret_cast<cplx*>(base + S.QI);
     cplx* RI = reinterpret_cast<cplx*>(base + S.RI);
-    unsigned long long* maxRI = reinterpret_cast<unsigned long long*>(base + S.maxRI);
     cplx* P1 = reinterpret_cast<cplx*>(base + S.P1);
     cplx* P2 = reinterpret_cast<cplx*>(base + S.P2);
     cplx* QO = reinterpret_cast<cplx*>(base + S.QO);
@@ -3231,8 +3224,6 @@ static gl_status run_adjoint_group(gl_plan* p, int gu, const void* spectra, int 
     cplx* EA = reinterpret_cast<cplx*>(base + S.EA);
     cplx* RAi = reinterpret_cast<cplx*>(base + S.RAi);
     cplx* QAi = reinterpret_cast<cplx*>(base + S.QAi);
-    CUDA_TRY(cudaMemsetAsync(maxEt, 0, (size_t)nuj * 3 * 8, st));
-    CUDA_TRY(cudaMemsetAsync(maxRI, 0, (size_t)nj * 4 * 8, st));
     const int mi[12] = {M_ONE, M_NU, M_NU2, M_NU3, M_QX_SNU, M_QY_SNU,
                         M_QX, M_QY, M_Q2_SNU, M_Q2, M_NUQX, M_NUQY};
     const int m1[12] = {M_ONE, M_IQX, M_IQY, M_QX_SNU, M_QY_SNU, M_MI_NU,
