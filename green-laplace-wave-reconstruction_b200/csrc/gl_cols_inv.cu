@@ -13,6 +13,12 @@ void col_ifft_n(dim3 grid, size_t smem, cudaStream_t st, const ColArgs& a, const
   col_ifft_kernel<N><<<grid, 256, smem, st>>>(a, tw, cw, bpb);
 }
 
+template <int N>
+void final_cols_n(dim3 grid, cudaStream_t st, const FinalCols& a, const cplx* tw, int cw) {
+  ensure_smem_attr((const void*)final_col_kernel<N>, (int)SMEM_LIMIT);
+  final_col_kernel<N><<<grid, 256, (size_t)(256 / FftLen<N>::T) * FftLen<N>::COL * sizeof(cplx), st>>>(a, tw, cw);
+}
+
 // Per-stage names of the column launches in the launch accounting.
 const char* col_ifft_name(int kind) {
   switch (kind) {
@@ -120,6 +126,30 @@ gl_status launch_col_ifft(const ColArgs& a0, int njobs, cudaStream_t st, const c
   LaunchScope ls(col_ifft_name(a.kind), st, bytes);
   GL_LEN_DISPATCH(a.n, col_ifft_n, grid, smem, st, a, tw, best_cw, best_bpb);
   LAUNCH_CHECK("col_ifft_kernel");
+  return GL_OK;
+}
+
+gl_status launch_final_cols(const FinalCols& a0, int ny, int nunits, cudaStream_t st, const cplx* tw) {
+  FinalCols a = a0;
+  const int G = 256 / (ny / 16);
+  auto blocks = [&](int cw) {
+    int n = 0;
+    for (int k = 0; k < a.ncomp; ++k) {
+      a.comp[k].first_block = n;
+      n += (a.comp[k].box.w + cw - 1) / cw;
+    }
+    return n;
+  };
+  // as many columns per block as it has groups, fewer while SMs are idle
+  int cw = G;
+  while (cw > 1 && (long long)blocks(cw / 2) * nunits <= 2 * SM_COUNT) cw /= 2;
+  dim3 grid(blocks(cw), nunits);
+  double bytes = 0.0;
+  for (int k = 0; k < a.ncomp; ++k)
+    bytes += (double)nunits * a.comp[k].box.w * (ny + a.comp[k].box.h) * sizeof(cplx);
+  LaunchScope ls("final_col_kernel", st, bytes);
+  switch (ny) { GL_POW2_CASES(final_cols_n, grid, st, a, tw, cw) }
+  LAUNCH_CHECK("final_col_kernel");
   return GL_OK;
 }
 

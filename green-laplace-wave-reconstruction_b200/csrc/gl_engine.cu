@@ -770,8 +770,10 @@ static size_t stage_scratch(const gl_plan* p, int g) {
   }
   // final column transforms at the reference ny
   {
-    const size_t wmax = std::max({(size_t)p->b1.w, (size_t)p->b2.w, (size_t)p->b3.w});
-    upd((size_t)g * 2 * wmax * p->d.ny * c);
+    size_t widths = 0;
+    for (int k = 0; k < p->ncomp; ++k)
+      widths += p->comp_ids[k] <= GL_COMP_PSI11 ? p->b1.w : (p->comp_ids[k] <= GL_COMP_PSI22 ? p->b2.w : p->b3.w);
+    upd((size_t)g * widths * p->d.ny * c);
   }
   (void)b1;
   return need;
@@ -1219,85 +1221,102 @@ static ColFftArgs tuned(const gl_plan* p, ColFftArgs f) {
   return f;
 }
 
-// Final transform of box spectra `spec` ([unit][nb][box]) to the reference
-// grid, writing output planes comp_offset.. of each unit.
-static gl_status final_output(gl_plan* p, int gu, const Box& box, const double* geo,
-                              const cplx* spec, long long spec_stride, int nb, const int* mults,
-                              const int* srcs, int comp_offset, void* outputs, void* scratch,
-                              cudaStream_t st, const double* comp_scale_dev, UnitScalars* us) {
+// One output component: box spectra of every unit and its slot.
+struct FinalComp {
+  Box box;
+  const double* geo;
+  const cplx* spec;
+  long long spec_stride;
+  int mult;  // M_ONE or M_PSI11
+  int slot;
+};
+
+// Final transforms of `n` components to the reference grid.  The components
+// share launches (a 128^2 call with six: 8 launches of 8 to 22 us became 2) as
+// long as their intermediate columns stay well inside L2.
+static gl_status final_outputs(gl_plan* p, int gu, const FinalComp* f, int n, void* outputs, void* scratch,
+                               cudaStream_t st, UnitScalars* us) {
+  const double scale = 1.0 / ((double)p->d.nx * (double)p->d.ny);
   if (p->gen) {
-    if (nb > 4) return fail(GL_ERR_INVALID_ARGUMENT, "at most 4 final components per launch");
-    GenColArgs a;
-    std::memset(&a, 0, sizeof a);
-    a.nbanks = nb;
-    for (int k = 0; k < nb; ++k) {
-      a.mult[k] = mults[k];
-      a.src_of[k] = srcs[k];
+    for (int k0 = 0, k; k0 < n; k0 = k) {
+      GenColArgs a;
+      std::memset(&a, 0, sizeof a);
+      const long long plane = (long long)f[k0].box.w * f[k0].box.h;
+      // a launch takes up to four components of one box whose spectra are the
+      // same or follow one another
+      for (k = k0; k < n && k - k0 < 4 && f[k].geo == f[k0].geo && f[k].spec_stride == f[k0].spec_stride &&
+                  (f[k].spec == f[k0].spec || f[k].spec == f[k0].spec + plane);
+           ++k) {
+        a.mult[a.nbanks] = f[k].mult;
+        a.src_of[a.nbanks++] = f[k].spec == f[k0].spec ? 0 : 1;
+      }
+      a.box = f[k0].box;
+      a.geo = f[k0].geo;
+      a.spec = f[k0].spec;
+      a.spec_job_stride = f[k0].spec_stride;
+      a.spec_sub_stride = plane;
+      a.out = reinterpret_cast<cplx*>(scratch);
+      a.gp = p->geny;
+      a.twn = p->twy;
+      a.scale = scale;
+      gl_status s = launch_gen_cols(a, gu, st);
+      if (s != GL_OK) return s;
+      GenRowArgs o;
+      std::memset(&o, 0, sizeof o);
+      o.in = reinterpret_cast<cplx*>(scratch);
+      o.w = f[k0].box.w;
+      o.x0 = f[k0].box.x0;
+      o.ny = p->d.ny;
+      o.ncomp = a.nbanks;
+      o.comp_offset = f[k0].slot;
+      o.out_ncomp = p->ncomp;
+      o.comp_scale = p->comp_scale + f[k0].slot;
+      o.out = outputs;
+      o.real_only = p->d.output == GL_OUT_REAL;
+      o.us = us;
+      o.gp = p->genx;
+      o.twn = p->twx;
+      if ((s = launch_gen_rows(o, gu * a.nbanks, st)) != GL_OK) return s;
     }
-    a.box = box;
-    a.geo = geo;
-    a.spec = spec;
-    a.spec_job_stride = spec_stride;
-    a.spec_sub_stride = (long long)box.w * box.h;
-    a.out = reinterpret_cast<cplx*>(scratch);
-    a.gp = p->geny;
-    a.twn = p->twy;
-    a.scale = 1.0 / ((double)p->d.nx * (double)p->d.ny);
-    gl_status s = launch_gen_cols(a, gu, st);
-    if (s != GL_OK) return s;
-    GenRowArgs o;
+    return GL_OK;
+  }
+  constexpr size_t L2_SHARE = 48u << 20;
+  for (int k0 = 0; k0 < n;) {
+    FinalCols a;
+    std::memset(&a, 0, sizeof a);
+    OutArgs o;
     std::memset(&o, 0, sizeof o);
-    o.in = reinterpret_cast<cplx*>(scratch);
-    o.w = box.w;
-    o.x0 = box.x0;
+    size_t off = 0;
+    int k = k0;
+    for (; k < n && k - k0 < MAX_FINAL; ++k) {
+      const size_t cells = (size_t)gu * f[k].box.w * p->d.ny;
+      if (k > k0 && (off + cells) * sizeof(cplx) > L2_SHARE) break;
+      FinalCols::Comp& c = a.comp[a.ncomp];
+      c.spec = f[k].spec;
+      c.spec_stride = f[k].spec_stride;
+      c.box = f[k].box;
+      c.geo = f[k].geo;
+      c.psi11 = f[k].mult == M_PSI11;
+      c.mid = reinterpret_cast<cplx*>(scratch) + off;
+      o.comp[a.ncomp] = OutArgs::Comp{c.mid, (long long)f[k].box.w * p->d.ny, f[k].box.w, f[k].box.x0, f[k].slot};
+      ++a.ncomp;
+      off += cells;
+    }
+    a.scale = scale;
+    gl_status s = launch_final_cols(a, p->d.ny, gu, st, p->tw);
+    if (s != GL_OK) return s;
+    o.nx = p->d.nx;
     o.ny = p->d.ny;
-    o.ncomp = nb;
-    o.comp_offset = comp_offset;
+    o.ncomp = a.ncomp;
     o.out_ncomp = p->ncomp;
-    o.comp_scale = comp_scale_dev + comp_offset;
+    o.comp_scale = p->comp_scale;
     o.out = outputs;
     o.real_only = p->d.output == GL_OUT_REAL;
     o.us = us;
-    o.gp = p->genx;
-    o.twn = p->twx;
-    return launch_gen_rows(o, gu * nb, st);
+    if ((s = launch_out_rows(o, gu, st, p->tw)) != GL_OK) return s;
+    k0 = k;
   }
-  ColArgs a;
-  std::memset(&a, 0, sizeof a);
-  a.kind = COL_PLAIN;
-  a.nbanks = nb;
-  for (int k = 0; k < nb; ++k) {
-    a.mult[k] = mults[k];
-    a.src_of[k] = srcs[k];
-  }
-  a.box = box;
-  a.geo = geo;
-  a.spec = spec;
-  a.spec_job_stride = spec_stride;
-  a.spec_sub_stride = (long long)box.w * box.h;
-  a.jobs_per_unit = 1;
-  a.out = reinterpret_cast<cplx*>(scratch);
-  a.n = p->d.ny;
-  a.log2n = p->lny;
-  a.scale = 1.0 / ((double)p->d.nx * (double)p->d.ny);
-  gl_status s = launch_col_ifft(tuned(p, a), gu, st, p->tw);
-  if (s != GL_OK) return s;
-  OutArgs o;
-  std::memset(&o, 0, sizeof o);
-  o.in = reinterpret_cast<cplx*>(scratch);
-  o.w = box.w;
-  o.x0 = box.x0;
-  o.nx = p->d.nx;
-  o.log2nx = p->lnx;
-  o.ny = p->d.ny;
-  o.ncomp = nb;
-  o.comp_offset = comp_offset;
-  o.out_ncomp = p->ncomp;
-  o.comp_scale = comp_scale_dev + comp_offset;
-  o.out = outputs;
-  o.real_only = p->d.output == GL_OUT_REAL;
-  o.us = us;
-  return launch_out_rows(o, gu * nb, st, p->tw);
+  return GL_OK;
 }
 
 static int comp_slot(const gl_plan* p, int id) {
@@ -1945,46 +1964,20 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
   }
 
   // ---------------- outputs on the reference grid ----------------
-  if (p->want_first) {
-    int mults[2], n = 0, off = -1;
-    if (p->comps & GL_COMP_ETA11) {
-      mults[n++] = M_ONE;
-      off = comp_slot(p, GL_COMP_ETA11);
+  {
+    FinalComp f[MAX_FINAL];
+    int n = 0;
+    for (int k = 0; k < p->ncomp; ++k) {
+      switch (p->comp_ids[k]) {
+        case GL_COMP_ETA11: f[n++] = FinalComp{B1, p->geo1, spec, pl1, M_ONE, k}; break;
+        case GL_COMP_PSI11: f[n++] = FinalComp{B1, p->geo1, spec, pl1, M_PSI11, k}; break;
+        case GL_COMP_ETA22: f[n++] = FinalComp{B2, p->geo2, out22, pl2, M_ONE, k}; break;
+        case GL_COMP_PSI22: f[n++] = FinalComp{B2, p->geo2, outp22, pl2, M_ONE, k}; break;
+        case GL_COMP_ETA33: f[n++] = FinalComp{B3, p->geo3, out33, 2LL * pl3, M_ONE, k}; break;
+        case GL_COMP_PSI33: f[n++] = FinalComp{B3, p->geo3, out33 + pl3, 2LL * pl3, M_ONE, k}; break;
+      }
     }
-    if (p->comps & GL_COMP_PSI11) {
-      mults[n++] = M_PSI11;
-      if (off < 0) off = comp_slot(p, GL_COMP_PSI11);
-    }
-    const int srcs[2] = {0, 0};  // both read the parent spectrum
-    if ((s = final_output(p, gu, B1, p->geo1, spec, pl1, n, mults, srcs, off, outputs, scratch, st,
-                          p->comp_scale, us)) != GL_OK)
-      return s;
-  }
-  if (p->want_eta22) {
-    const int m1[1] = {M_ONE}, z1[1] = {0};
-    if ((s = final_output(p, gu, B2, p->geo2, out22, pl2, 1, m1, z1, comp_slot(p, GL_COMP_ETA22),
-                          outputs, scratch, st, p->comp_scale, us)) != GL_OK)
-      return s;
-  }
-  if (p->want_psi22) {
-    const int m1[1] = {M_ONE}, z1[1] = {0};
-    if ((s = final_output(p, gu, B2, p->geo2, outp22, pl2, 1, m1, z1, comp_slot(p, GL_COMP_PSI22),
-                          outputs, scratch, st, p->comp_scale, us)) != GL_OK)
-      return s;
-  }
-  if (p->want_o3) {
-    const int m2[2] = {M_ONE, M_ONE}, s01[2] = {0, 1};
-    const int ce = comp_slot(p, GL_COMP_ETA33), cp = comp_slot(p, GL_COMP_PSI33);
-    if (ce >= 0 && cp >= 0) {
-      if ((s = final_output(p, gu, B3, p->geo3, out33, 2LL * pl3, 2, m2, s01, ce, outputs, scratch, st,
-                            p->comp_scale, us)) != GL_OK)
-        return s;
-    } else {
-      const int which = ce >= 0 ? 0 : 1;
-      if ((s = final_output(p, gu, B3, p->geo3, out33 + (size_t)which * pl3, 2LL * pl3, 1, m2,
-                            s01, ce >= 0 ? ce : cp, outputs, scratch, st, p->comp_scale, us)) != GL_OK)
-        return s;
-    }
+    if ((s = final_outputs(p, gu, f, n, outputs, scratch, st, us)) != GL_OK) return s;
   }
   // non-finite outputs were flagged by the final transform (out_row_kernel)
   if (status) {
@@ -2281,20 +2274,18 @@ static gl_status e44_finalize(gl_plan* p, int gu, const cplx* OUT, unsigned long
   if ((s = launch_col_ifft(a, gu, st, p->tw)) != GL_OK) return s;
   OutArgs o;
   std::memset(&o, 0, sizeof o);
-  o.in = reinterpret_cast<cplx*>(tr);
-  o.w = B4.w;
-  o.x0 = B4.x0;
+  const long long mid_plane = (long long)B4.w * p->d.ny;
+  for (int k = 0; k < nout; ++k)
+    o.comp[k] = OutArgs::Comp{reinterpret_cast<cplx*>(tr) + k * mid_plane, nout * mid_plane, B4.w, B4.x0, k};
   o.nx = p->d.nx;
-  o.log2nx = p->lnx;
   o.ny = p->d.ny;
   o.ncomp = nout;
-  o.comp_offset = 0;
   o.out_ncomp = nout;
   o.comp_scale = p->comp_scale;
   o.out = outputs;
   o.real_only = p->d.output == GL_OUT_REAL;
   o.us = us;  // non-finite outputs set the unit status inside the transform
-  if ((s = launch_out_rows(o, gu * nout, st, p->tw)) != GL_OK) return s;
+  if ((s = launch_out_rows(o, gu, st, p->tw)) != GL_OK) return s;
   if (us) {
     if (status) {
       {
@@ -4254,14 +4245,10 @@ extern "C" gl_status gl_box_synthesize_noalloc(int n_units, int nx, int ny, int 
   if ((s = launch_col_ifft(a, n_units, st, tw)) != GL_OK) return s;
   OutArgs o;
   std::memset(&o, 0, sizeof o);
-  o.in = mid;
-  o.w = box_w;
-  o.x0 = box_x0;
+  o.comp[0] = OutArgs::Comp{mid, (long long)box_w * ny, box_w, box_x0, 0};
   o.nx = nx;
-  o.log2nx = ilog2(nx);
   o.ny = ny;
   o.ncomp = 1;
-  o.comp_offset = 0;
   o.out_ncomp = 1;
   // the scale travels by value in the launch arguments
   o.comp_scale = nullptr;

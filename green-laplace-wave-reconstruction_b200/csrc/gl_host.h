@@ -140,7 +140,8 @@ gl_status launch_col_ifft(const ColArgs& a, int njobs, cudaStream_t st, const cp
 gl_status launch_col_fft(const ColFftArgs& a, int njs, cudaStream_t st, const cplx* tw,
                          const char* name = "col_fft_kernel");
 gl_status launch_row(const RowArgs& a, int njobs, cudaStream_t st, const cplx* tw);
-gl_status launch_out_rows(const OutArgs& a0, int nuc, cudaStream_t st, const cplx* tw);
+gl_status launch_final_cols(const FinalCols& a, int ny, int nunits, cudaStream_t st, const cplx* tw);
+gl_status launch_out_rows(const OutArgs& a, int nunits, cudaStream_t st, const cplx* tw);
 gl_status launch_seed_rows(const SeedArgs& a, int nunits, cudaStream_t st, const cplx* tw);
 gl_status launch_combine(const CmbArgs& a, int njobs, cudaStream_t st, const cplx* tw);
 gl_status launch_sfft(const SFft& a, int outer, int sign, cudaStream_t st, const cplx* tw);

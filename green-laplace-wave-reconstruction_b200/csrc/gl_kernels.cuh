@@ -1364,23 +1364,98 @@ __global__ void acc_outer_kernel(AccArgs a, const unsigned long long* maxpsi) {
 // final inverse FFT along x on the reference grid
 // ---------------------------------------------------------------------------
 
+constexpr int MAX_FINAL = 6;
+
+// The components of one final pair of launches: box spectra of any of the
+// plan's boxes, transformed along y into `mid` and then along x.
+struct FinalCols {
+  int ncomp;
+  struct Comp {
+    const cplx* spec;       // [unit][box], spec_stride apart
+    long long spec_stride;
+    Box box;
+    const double* geo;      // the box's geometry (psi11 only)
+    int psi11;              // 1: times -i/nu, 0: as it is
+    cplx* mid;              // [unit][ny][w]
+    int first_block;        // first column block of this component
+  } comp[MAX_FINAL];
+  double scale;             // 1/(Nx Ny)
+};
+
+// One block: cw columns of one component of one unit; blockIdx.x runs over the
+// column blocks of all components, so that small boxes share a launch.
+template <int N>
+__global__ void __launch_bounds__(256, 2) final_col_kernel(FinalCols a, const cplx* __restrict__ tw, int cw) {
+  extern __shared__ cplx smem[];
+  constexpr int T = FftLen<N>::T, L = FftLen<N>::COL;
+  constexpr bool direct = T <= 16;
+  int k = 0;
+  while (k + 1 < a.ncomp && (int)blockIdx.x >= a.comp[k + 1].first_block) ++k;
+  const FinalCols::Comp& C = a.comp[k];
+  const int w = C.box.w, h = C.box.h, plane = w * h, unit = blockIdx.y;
+  const int x_first = (blockIdx.x - C.first_block) * cw;
+  const int ncol = min(cw, w - x_first);
+  const int G = blockDim.x / T, g = threadIdx.x / T, t = threadIdx.x % T;
+  const int y0 = mod_n<N>(C.box.y0);
+  cplx* buf = smem + g * L;
+  cplx* mid = C.mid + (size_t)unit * N * w + x_first;
+  const int lcw = 31 - __clz(cw);  // cw is a power of two, at most G
+  const bool active = g < ncol;
+  const cplx* src = C.spec + (long long)unit * C.spec_stride + x_first + (active ? g : 0);
+  int sstep = w;
+  if (C.psi11) {
+    if (active) {
+#pragma unroll 1
+      for (int by = t; by < h; by += T)
+        buf[by] = mult_direct(M_PSI11, GeoRef{C.geo, plane, by * w + x_first + g}, src[by * w]);
+    }
+    src = buf;
+    sstep = 1;
+    group_sync<N>(1 + g);
+  }
+  auto load = [&](int yb, int) -> cplx {
+    const int by = wrap_n<N>(yb - y0);
+    return by < h ? src[by * sstep] : czero();
+  };
+  auto sink = [&](int o, int step, const cplx* v, int cnt) {
+    if constexpr (direct) {
+      cplx* p = mid + (size_t)o * w + g;
+#pragma unroll
+      for (int r = 0; r < 16; ++r)
+        if (r < cnt) p[(size_t)(r * step) * w] = cscale(a.scale, v[r]);
+    } else {
+      row_put<N>(buf, o, step, v, cnt);
+    }
+  };
+  fft_n<+1, N>(buf, t, 1 + g, active, tw, load, sink);
+  if constexpr (!direct) {
+    __syncthreads();
+    for (int q = threadIdx.x; q < (N << lcw); q += blockDim.x) {
+      const int y = q >> lcw, c = q & (cw - 1);
+      if (c < ncol) mid[(size_t)y * w + c] = cscale(a.scale, smem[c * L + pos<N>(y)]);
+    }
+  }
+}
+
 struct OutArgs {
-  const cplx* in;       // [uc][w][ny]  (column-transformed box spectra)
-  int w, x0;            // box columns
-  int nx, log2nx, ny;
+  int nx, ny;
   int ncomp;            // components per unit in this launch
-  int comp_offset;      // first component slot in the output
+  struct Comp {
+    const cplx* in;          // [unit][ny][w] column-transformed box spectra,
+    long long unit_stride;   // unit_stride elements between units
+    int w, x0;               // box columns
+    int slot;                // output component
+  } comp[MAX_FINAL];
   int out_ncomp;        // component slots per unit in the output
-  const double* comp_scale;   // physical scale per component of this launch
+  const double* comp_scale;   // physical scale per output component
   double scale_value;   // the scale of every component when comp_scale is null
   void* out;            // [unit][out_ncomp][ny][nx]
   int real_only;        // write float64 real parts instead of complex
-  int rows;             // rows per block
   UnitScalars* us;      // non-null: a non-finite output sets the unit's status
 };
 
 // Final inverse transform along x on the reference grid: each group of n/16
-// threads takes one output row (inputs [uc][y][col], zero outside the box
+// threads takes one output row (inputs [y][col], zero outside the box
 // columns) and writes scaled complex values or (REAL, OutArgs::real_only)
 // real parts; one instantiation per output type keeps one store path per
 // kernel.
@@ -1392,8 +1467,8 @@ __global__ void __launch_bounds__(N <= 1024 ? 192 : 256, 2) out_row_kernel(OutAr
   const int G = blockDim.x / T, g = threadIdx.x / T, t = threadIdx.x % T;
   const int y0 = blockIdx.x * G;
   const int y = y0 + g;
-  const int uc = blockIdx.y;
-  const int unit = uc / a.ncomp, comp = uc % a.ncomp;
+  const int unit = blockIdx.y / a.ncomp;
+  const OutArgs::Comp& C = a.comp[blockIdx.y % a.ncomp];
   const bool active = y < a.ny;
   const int yy = active ? y : 0;
   cplx* buf = smem + (size_t)g * L;
@@ -1406,11 +1481,12 @@ __global__ void __launch_bounds__(N <= 1024 ? 192 : 256, 2) out_row_kernel(OutAr
   __syncthreads();
   if (threadIdx.x < 32) {
     const int nrows = min(G, a.ny - y0);
-    const uint32_t bytes = (uint32_t)(a.w * sizeof(cplx));
+    const uint32_t bytes = (uint32_t)(C.w * sizeof(cplx));
     if (threadIdx.x == 0) mbar_arrive_expect_tx(bar, bytes * (uint32_t)nrows);
     __syncwarp();
+    const cplx* in = C.in + unit * C.unit_stride + (size_t)y0 * C.w;
     for (int r = threadIdx.x; r < nrows; r += 32)
-      bulk_g2s(smem_u32(smem + (size_t)r * L), a.in + ((size_t)uc * a.ny + y0 + r) * a.w, bytes, bar);
+      bulk_g2s(smem_u32(smem + (size_t)r * L), in + (size_t)r * C.w, bytes, bar);
   }
   if (__syncthreads_or(!mbar_wait_bounded(bar, 0, BULK_WAIT_CYCLES))) {
     // a copy never landed: flag the unit, give the copies one more bounded
@@ -1419,12 +1495,13 @@ __global__ void __launch_bounds__(N <= 1024 ? 192 : 256, 2) out_row_kernel(OutAr
     mbar_wait_bounded(bar, 0, BULK_WAIT_CYCLES);
     return;
   }
-  const double s = a.comp_scale ? a.comp_scale[comp] : a.scale_value;
-  const size_t base = (((size_t)unit * a.out_ncomp + a.comp_offset + comp) * a.ny + yy) * N;
-  const int x0 = mod_n<N>(a.x0);
+  const double s = a.comp_scale ? a.comp_scale[C.slot] : a.scale_value;
+  const size_t base = (((size_t)unit * a.out_ncomp + C.slot) * a.ny + yy) * N;
+  const int x0 = mod_n<N>(C.x0);
+  const int bw = C.w;
   auto load = [&](int xb, int) -> cplx {
     const int xi = wrap_n<N>(xb - x0);
-    return xi < a.w ? buf[xi] : czero();  // staged box row
+    return xi < bw ? buf[xi] : czero();  // staged box row
   };
   bool bad = false;  // the output check of the unit's status, folded into the store
   if constexpr (REAL) {
