@@ -662,6 +662,9 @@ struct gl_plan {
       o_pm, o_max, o_out22, o_outp22, o_out33, o_scratch;
   size_t max_slots;  // 64-bit maxima slots of all stages at o_max, zeroed with the analysis
   size_t scratch_bytes;
+  // the stages' parts of the scratch, and whether their chains may run on branches
+  size_t o_eta22 = 0, o_psi22 = 0, o_first = 0;
+  bool branches = false;
   // fourth-order eta44 plans (gl_eta44_plan_create)
   bool e44 = false;
   bool e44_psi = false;         // psi44 requested with eta44
@@ -694,6 +697,61 @@ struct gl_plan {
   std::mutex lane_mu;
 };
 
+// Side streams for a group's independent stages.  A call takes a set from the
+// device's pool while it queues its work and gives it back joined to the
+// caller's stream, so concurrent calls (other threads, plans, streams) never
+// queue between one call's fork and join; the pool grows to the number of
+// calls that ever queued at once and lives as long as the process.
+constexpr size_t BRANCH_BYTES = 64u << 20;
+struct BranchSet {
+  int device;
+  cudaStream_t st[2];
+  cudaEvent_t ev[5];
+};
+static std::mutex g_branch_mu;
+static std::vector<BranchSet*> g_branch_free;
+
+// A set for work on `st`, or null when the stream is being captured (a pooled
+// stream would stay part of the capture after the call) or none can be made.
+static BranchSet* branch_acquire(cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  int dev = 0;
+  if (cap != cudaStreamCaptureStatusNone || cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  std::lock_guard<std::mutex> lk(g_branch_mu);
+  for (size_t k = 0; k < g_branch_free.size(); ++k)
+    if (g_branch_free[k]->device == dev) {
+      BranchSet* b = g_branch_free[k];
+      g_branch_free.erase(g_branch_free.begin() + k);
+      return b;
+    }
+  BranchSet* b = new (std::nothrow) BranchSet();
+  if (!b) return nullptr;
+  b->device = dev;
+  bool ok = true;
+  for (cudaStream_t& s : b->st) ok = ok && cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess;
+  for (cudaEvent_t& e : b->ev) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+  if (ok) return b;
+  cudaGetLastError();
+  for (cudaStream_t s : b->st)
+    if (s) cudaStreamDestroy(s);
+  for (cudaEvent_t e : b->ev)
+    if (e) cudaEventDestroy(e);
+  delete b;
+  return nullptr;
+}
+
+static void branch_release(BranchSet* b) {
+  std::lock_guard<std::mutex> lk(g_branch_mu);
+  try {
+    g_branch_free.push_back(b);
+  } catch (...) {  // out of memory: the set is lost, its queued work is joined
+  }
+}
+
 // Smallest column-transform length >= v: a power of two (>= 16) or one of the
 // mixed lengths 16 m the column kernels run.
 static int col_len(int v) {
@@ -724,21 +782,21 @@ struct Bump {
   }
 };
 
-// Scratch bytes of each stage, for `g` units.
-static size_t stage_scratch(const gl_plan* p, int g) {
+// Scratch of each stage for `g` units: the main region holds order 3 and the
+// final columns; eta22, psi22 and the outer first-order banks share it when
+// the stages run in turn and follow it when they run on branches.
+static size_t stage_scratch(gl_plan* p, int g, size_t base) {
   const size_t c = sizeof(cplx);
-  const size_t b1 = (size_t)p->b1.w * p->b1.h, b2 = (size_t)p->b2.w * p->b2.h,
-               b3 = (size_t)p->b3.w * p->b3.h;
+  const size_t b2 = (size_t)p->b2.w * p->b2.h, b3 = (size_t)p->b3.w * p->b3.h;
   const size_t ncy = p->ncy;
-  size_t need = 0;
-  auto upd = [&](size_t v) { need = std::max(need, v); };
+  size_t eta = 0, psi = 0, first = 0, main = 0;
   if (p->want_eta22) {
     const size_t J = p->ranks[0];
     Bump b;
     b.take(g * J * 8 * p->b1.w * ncy * c);
     b.take(g * J * 2 * p->b2.w * ncy * c);
     b.take(g * J * 2 * b2 * c);
-    upd(b.off);
+    eta = b.off;
   }
   if (p->want_psi22) {
     Bump b;
@@ -748,35 +806,43 @@ static size_t stage_scratch(const gl_plan* p, int g) {
     b.take((size_t)g * 2 * p->b1.w * ncy * c);       // contact P
     b.take((size_t)g * 1 * p->b2.w * ncy * c);       // contact Q
     b.take((size_t)g * b2 * c);                      // contact R
-    upd(b.off);
+    psi = b.off;
   }
   if (p->want_o3) {
     const size_t J = p->ranks[3], I = p->ranks[2];
     Bump b;
     b.take(g * J * 4 * b2 * c);  // E
-    const size_t base = b.off;
     Bump in = b;
     in.take(g * J * I * 12 * p->b1.w * ncy * c);
     in.take(g * J * I * 4 * p->b2.w * ncy * c);
     in.take(g * J * I * 4 * b2 * c);
-    upd(in.off);
     Bump out = b;
-    out.take(g * J * 12 * p->b1.w * ncy * c);
+    first = out.take(g * J * 12 * p->b1.w * ncy * c);
+    first = out.off - first;
     out.take(g * J * 9 * p->b2.w * ncy * c);
     out.take(g * J * 4 * p->b3.w * ncy * c);
     out.take(g * J * 4 * b3 * c);
-    upd(out.off);
-    (void)base;
+    main = std::max(in.off, out.off);
   }
   // final column transforms at the reference ny
   {
     size_t widths = 0;
     for (int k = 0; k < p->ncomp; ++k)
       widths += p->comp_ids[k] <= GL_COMP_PSI11 ? p->b1.w : (p->comp_ids[k] <= GL_COMP_PSI22 ? p->b2.w : p->b3.w);
-    upd((size_t)g * widths * p->d.ny * c);
+    main = std::max(main, align_up((size_t)g * widths * p->d.ny * c));
   }
-  (void)b1;
-  return need;
+  // Branches pay while the stages' launches leave SMs idle, i.e. while their
+  // buffers are a fraction of L2.
+  const int chains = (p->want_eta22 ? 1 : 0) + (p->want_psi22 ? 1 : 0) + (p->want_o3 ? 2 : 0);
+  p->branches = chains >= 2 && eta + psi + first <= BRANCH_BYTES;
+  if (!p->branches) {
+    p->o_eta22 = p->o_psi22 = p->o_first = base;
+    return std::max({main, eta, psi});
+  }
+  p->o_eta22 = base + main;
+  p->o_psi22 = p->o_eta22 + eta;
+  p->o_first = p->o_psi22 + psi;
+  return main + eta + psi + first;
 }
 
 // The inner accumulation: blocks of 256 threads over (ACC_TILE-bin tiles,
@@ -835,8 +901,9 @@ static size_t layout_units(gl_plan* p, int g) {
   p->o_out22 = b.take(g * b2 * c);
   p->o_outp22 = b.take(g * b2 * c);
   p->o_out33 = b.take(g * 2 * b3 * c);
-  p->scratch_bytes = stage_scratch(p, g);
-  p->o_scratch = b.take(p->scratch_bytes);
+  p->o_scratch = b.off;
+  p->scratch_bytes = stage_scratch(p, g, b.off);
+  b.take(p->scratch_bytes);
   return b.off;
 }
 
@@ -1563,7 +1630,9 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
   const double fwd_scale3 = nn / ((double)p->ncx * (double)ncy3);
 
   // ---------------- eta22 (spatial.py:156-231) ----------------
-  if (p->want_eta22) {
+  auto eta22_stage = [&](cudaStream_t st) -> gl_status {
+    gl_status s;
+    char* scratch = at<char>(ws, p->o_eta22);
     const int J = p->ranks[0];
     const int njobs = gu * J;
     Bump b;
@@ -1637,19 +1706,34 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
       acc_eta22_kernel<<<g, T, 0, st>>>(c);
     }
     LAUNCH_CHECK("acc_eta22_kernel");
-  }
+    return GL_OK;
+  };
 
   // ---------------- psi22 (spatial.py:234-414) ----------------
-  if (p->want_psi22) {
-    const int njobs_c = gu * 2 * 2 * 2;  // (unit, branch, node, channel)
-    const int njobs_r = gu * 2 * 2;      // (unit, branch, node)
-    Bump b;
-    cplx* P = reinterpret_cast<cplx*>(scratch + b.take((size_t)njobs_c * 8 * B1.w * ncy2 * sizeof(cplx)));
-    cplx* Q = reinterpret_cast<cplx*>(scratch + b.take((size_t)njobs_r * 8 * B2.w * ncy2 * sizeof(cplx)));
-    cplx* R = reinterpret_cast<cplx*>(scratch + b.take((size_t)njobs_r * 8 * pl2 * sizeof(cplx)));
-    cplx* Pc = reinterpret_cast<cplx*>(scratch + b.take((size_t)gu * 2 * B1.w * ncy2 * sizeof(cplx)));
-    cplx* Qc = reinterpret_cast<cplx*>(scratch + b.take((size_t)gu * 1 * B2.w * ncy2 * sizeof(cplx)));
-    cplx* Rc = reinterpret_cast<cplx*>(scratch + b.take((size_t)gu * pl2 * sizeof(cplx)));
+  // buffers of the channel products (P, Q, R) and of the Taylor contact
+  const int njobs_c = gu * 2 * 2 * 2;  // (unit, branch, node, channel)
+  const int njobs_r = gu * 2 * 2;      // (unit, branch, node)
+  char* const psi_scratch = at<char>(ws, p->o_psi22);
+  Bump pb;
+  auto psi_take = [&](size_t cells) { return reinterpret_cast<cplx*>(psi_scratch + pb.take(cells * sizeof(cplx))); };
+  cplx* const P22 = psi_take((size_t)njobs_c * 8 * B1.w * ncy2);
+  cplx* const Q22 = psi_take((size_t)njobs_r * 8 * B2.w * ncy2);
+  cplx* const R22 = psi_take((size_t)njobs_r * 8 * pl2);
+  cplx* const Pc = psi_take((size_t)gu * 2 * B1.w * ncy2);
+  cplx* const Qc = psi_take((size_t)gu * 1 * B2.w * ncy2);
+  cplx* const Rc = psi_take((size_t)gu * pl2);
+  auto psi22_fft = [&]() {
+    ColFftArgs f;
+    f.box = B2;
+    f.n = ncy2;
+    f.log2n = p->lncy2;
+    f.mask = nullptr;
+    f.maxslot = nullptr;
+    f.scale = fwd_scale2;
+    return f;
+  };
+  auto psi22_stage = [&](cudaStream_t st) -> gl_status {
+    gl_status s;
     ColArgs a;
     std::memset(&a, 0, sizeof a);
     a.kind = COL_PSI22;
@@ -1665,7 +1749,7 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     a.nodes = dn + 1 * MAX_RANK;
     a.n_inner = 2;
     a.chan_mask = ch;
-    a.out = P;
+    a.out = P22;
     a.n = ncy2;
     a.log2n = p->lncy2;
     a.scale = inv_scale;
@@ -1675,12 +1759,12 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     r.kind = ROW_PSI22;
     // job (unit, branch, node): its two channels are consecutive col jobs,
     // so a row job sees 16 consecutive banks.
-    r.grp[0] = BankGroup{P, 16, B1.x0, B1.w};
+    r.grp[0] = BankGroup{P22, 16, B1.x0, B1.w};
     r.ngrp = 1;
     r.nout = 8;
     r.out_x0 = B2.x0;
     r.out_w = B2.w;
-    r.out = Q;
+    r.out = Q22;
     r.nx = p->ncx2;
     r.log2nx = p->lncx2;
     r.ny = ncy2;
@@ -1690,18 +1774,16 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     r.wait_surplus = p->wait_surplus;
     r.wait_cycles = p->wait_cycles;
     if ((s = launch_row(tuned(p, r), njobs_r, st, p->tw)) != GL_OK) return s;
-    ColFftArgs f;
-    f.in = Q;
-    f.out = R;
-    f.box = B2;
-    f.n = ncy2;
-    f.log2n = p->lncy2;
+    ColFftArgs f = psi22_fft();
+    f.in = Q22;
+    f.out = R22;
     f.nsrc = 8;
     f.jobs_per_unit = 4;
-    f.mask = nullptr;
-    f.maxslot = nullptr;
-    f.scale = fwd_scale2;
     if ((s = launch_col_fft(tuned(p, f), njobs_r * 8, st, p->tw)) != GL_OK) return s;
+    return GL_OK;
+  };
+  auto contact_stage = [&](cudaStream_t st) -> gl_status {
+    gl_status s;
     // Taylor contact 0.5 eta11 phi1z
     ColArgs cc;
     std::memset(&cc, 0, sizeof cc);
@@ -1739,18 +1821,21 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     rc.wait_surplus = p->wait_surplus;
     rc.wait_cycles = p->wait_cycles;
     if ((s = launch_row(tuned(p, rc), gu, st, p->tw)) != GL_OK) return s;
-    ColFftArgs fc = f;
+    ColFftArgs fc = psi22_fft();
     fc.in = Qc;
     fc.out = Rc;
     fc.nsrc = 1;
     fc.jobs_per_unit = 1;
     if ((s = launch_col_fft(tuned(p, fc), gu, st, p->tw)) != GL_OK) return s;
+    return GL_OK;
+  };
+  auto psi22_sum = [&](cudaStream_t st) -> gl_status {
     AccArgs c;
     std::memset(&c, 0, sizeof c);
     c.us = us;
     c.geo = p->geo2;
     c.box = B2;
-    c.in = R;
+    c.in = R22;
     c.out = outp22;
     c.mask = s2;
     c.pmask = pm;
@@ -1764,21 +1849,27 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
       acc_psi22_kernel<<<g, T, 0, st>>>(c);
     }
     LAUNCH_CHECK("acc_psi22_kernel");
-  }
+    return GL_OK;
+  };
 
   // ---------------- order 3 (_order3.py:18-148) ----------------
-  if (p->want_o3) {
-    const int J = p->ranks[3], I = p->ranks[2];
-    const int nuj = gu * J;
-    const int njobs = nuj * I;
-    Bump b;
-    cplx* E = reinterpret_cast<cplx*>(scratch + b.take((size_t)nuj * 4 * pl2 * sizeof(cplx)));
-    unsigned long long* maxEt = order3_maxima(p, ws);  // [nuj]
-    unsigned long long* maxRO = maxEt + nuj;           // [nuj][4]
-    unsigned long long* maxF = maxEt + 5 * nuj;        // [nuj][2]
-    unsigned long long* maxRI = maxEt + 8 * nuj;       // [njobs][4]
-    // inner stage buffers
-    Bump bi = b;
+  const int J = p->ranks[3], I = p->ranks[2];
+  const int nuj = gu * J;
+  const int njobs = nuj * I;
+  Bump b3;
+  cplx* const E = reinterpret_cast<cplx*>(scratch + b3.take((size_t)nuj * 4 * pl2 * sizeof(cplx)));
+  unsigned long long* const maxEt = order3_maxima(p, ws);  // [nuj]
+  unsigned long long* const maxRO = maxEt + nuj;           // [nuj][4]
+  unsigned long long* const maxF = maxEt + 5 * nuj;        // [nuj][2]
+  unsigned long long* const maxRI = maxEt + 8 * nuj;       // [njobs][4]
+  // the outer first-order banks: in the inner stage's region unless the stages
+  // run on branches
+  cplx* const P1 = reinterpret_cast<cplx*>(
+      p->branches ? at<char>(ws, p->o_first)
+                  : scratch + Bump(b3).take((size_t)nuj * 12 * B1.w * ncy3 * sizeof(cplx)));
+  auto inner_stage = [&](cudaStream_t st) -> gl_status {
+    gl_status s;
+    Bump bi = b3;
     cplx* PI = reinterpret_cast<cplx*>(scratch + bi.take((size_t)njobs * 12 * B1.w * ncy2 * sizeof(cplx)));
     cplx* QI = reinterpret_cast<cplx*>(scratch + bi.take((size_t)njobs * 4 * B2.w * ncy2 * sizeof(cplx)));
     cplx* RI = reinterpret_cast<cplx*>(scratch + bi.take((size_t)njobs * 4 * pl2 * sizeof(cplx)));
@@ -1856,111 +1947,173 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
       }
       LAUNCH_CHECK("acc_inner_kernel");
     }
-    // outer stage buffers (reuse the inner region)
-    Bump bo = b;
-    cplx* P1 = reinterpret_cast<cplx*>(scratch + bo.take((size_t)nuj * 12 * B1.w * ncy3 * sizeof(cplx)));
+    return GL_OK;
+  };
+  auto first_stage = [&](cudaStream_t st) -> gl_status {
+    gl_status s;
+    ColArgs a;
+    std::memset(&a, 0, sizeof a);
+    a.kind = COL_OUTER1;
+    const int m12[12] = {M_ONE, M_IQX, M_IQY, M_QX_SNU, M_QY_SNU, M_MI_NU,
+                         M_NUQX, M_NUQY, M_MI_Q2_SNU, M_MI_Q2NU, M_MINUS_A, M_MINUS_Q2};
+    const int z12[12] = {0};
+    set_banks(a, 12, m12, z12);
+    a.box = B1;
+    a.geo = p->geo1;
+    a.spec = spec;
+    a.spec_job_stride = pl1;
+    a.jobs_per_unit = J;
+    a.us = us;
+    a.nodes = dn + 3 * MAX_RANK;
+    a.out = P1;
+    a.n = ncy3;
+    a.log2n = p->lncy3;
+    a.scale = inv_scale;
+    if ((s = launch_col_ifft(tuned(p, a), nuj, st, p->tw)) != GL_OK) return s;
+    return GL_OK;
+  };
+  auto outer_stage = [&](cudaStream_t st, auto&& first_ready) -> gl_status {
+    gl_status s;
+    Bump bo = b3;  // reuses the inner region
+    bo.take((size_t)nuj * 12 * B1.w * ncy3 * sizeof(cplx));  // P1
     cplx* P2 = reinterpret_cast<cplx*>(scratch + bo.take((size_t)nuj * 9 * B2.w * ncy3 * sizeof(cplx)));
     cplx* QO = reinterpret_cast<cplx*>(scratch + bo.take((size_t)nuj * 4 * B3.w * ncy3 * sizeof(cplx)));
     cplx* RO = reinterpret_cast<cplx*>(scratch + bo.take((size_t)nuj * 4 * pl3 * sizeof(cplx)));
+    ColArgs a2;
+    std::memset(&a2, 0, sizeof a2);
+    a2.kind = COL_OUTER2;
+    const int m9[9] = {M_ONE, M_IQX, M_IQY, M_IQX, M_IQY, M_A, M_Q2, M_A, M_ONE};
+    const int src9[9] = {0, 0, 0, 2, 2, 2, 2, 3, 1};
+    set_banks(a2, 9, m9, src9);
+    a2.box = B2;
+    a2.geo = p->geo2;
+    a2.spec = E;
+    a2.spec_job_stride = 4LL * pl2;
+    a2.spec_sub_stride = pl2;
+    a2.jobs_per_unit = J;
+    a2.us = us;
+    a2.floor_max = maxEt;
+    a2.floor_rel = p->floor_rel;
+    a2.out = P2;
+    a2.n = ncy3;
+    a2.log2n = p->lncy3;
+    a2.scale = inv_scale;
+    if ((s = launch_col_ifft(tuned(p, a2), nuj, st, p->tw)) != GL_OK) return s;
+    if ((s = first_ready(st)) != GL_OK) return s;
+    RowArgs r;
+    std::memset(&r, 0, sizeof r);
+    r.kind = ROW_OUTER;
+    r.grp[0] = BankGroup{P1, 12, B1.x0, B1.w};
+    r.grp[1] = BankGroup{P2, 9, B2.x0, B2.w};
+    r.ngrp = 2;
+    r.nout = 4;
+    r.out_x0 = B3.x0;
+    r.out_w = B3.w;
+    r.out = QO;
+    r.nx = p->ncx;
+    r.log2nx = p->lncx;
+    r.ny = ncy3;
+    r.us = us;
+    r.jobs_per_unit = J;
+    r.gmax = ROW_GMAX;
+    r.wait_surplus = p->wait_surplus;
+    r.wait_cycles = p->wait_cycles;
+    if ((s = launch_row(tuned(p, r), nuj, st, p->tw)) != GL_OK) return s;
+    ColFftArgs f;
+    f.in = QO;
+    f.out = RO;
+    f.box = B3;
+    f.n = ncy3;
+    f.log2n = p->lncy3;
+    f.nsrc = 4;
+    f.jobs_per_unit = J;
+    f.mask = s3;
+    f.maxslot = maxRO;
+    f.scale = fwd_scale3;
+    if ((s = launch_col_fft(tuned(p, f), nuj * 4, st, p->tw, "col_fft_kernel[outer]")) != GL_OK) return s;
+    AccArgs c;
+    std::memset(&c, 0, sizeof c);
+    c.us = us;
+    c.geo = p->geo3;
+    c.box = B3;
+    c.in = RO;
+    c.maxin = maxRO;
+    c.maxout = maxF;
+    c.mask = s3;
+    c.floor_rel = p->floor_rel;
+    c.nsub = J;
+    dim3 g(grid_for(pl3, T, 48), nuj);
     {
-      ColArgs a;
-      std::memset(&a, 0, sizeof a);
-      a.kind = COL_OUTER1;
-      const int m12[12] = {M_ONE, M_IQX, M_IQY, M_QX_SNU, M_QY_SNU, M_MI_NU,
-                           M_NUQX, M_NUQY, M_MI_Q2_SNU, M_MI_Q2NU, M_MINUS_A, M_MINUS_Q2};
-      const int z12[12] = {0};
-      set_banks(a, 12, m12, z12);
-      a.box = B1;
-      a.geo = p->geo1;
-      a.spec = spec;
-      a.spec_job_stride = pl1;
-      a.jobs_per_unit = J;
-      a.us = us;
-      a.nodes = dn + 3 * MAX_RANK;
-      a.out = P1;
-      a.n = ncy3;
-      a.log2n = p->lncy3;
-      a.scale = inv_scale;
-      if ((s = launch_col_ifft(tuned(p, a), nuj, st, p->tw)) != GL_OK) return s;
-      ColArgs a2;
-      std::memset(&a2, 0, sizeof a2);
-      a2.kind = COL_OUTER2;
-      const int m9[9] = {M_ONE, M_IQX, M_IQY, M_IQX, M_IQY, M_A, M_Q2, M_A, M_ONE};
-      const int src9[9] = {0, 0, 0, 2, 2, 2, 2, 3, 1};
-      set_banks(a2, 9, m9, src9);
-      a2.box = B2;
-      a2.geo = p->geo2;
-      a2.spec = E;
-      a2.spec_job_stride = 4LL * pl2;
-      a2.spec_sub_stride = pl2;
-      a2.jobs_per_unit = J;
-      a2.us = us;
-      a2.floor_max = maxEt;
-      a2.floor_rel = p->floor_rel;
-      a2.out = P2;
-      a2.n = ncy3;
-      a2.log2n = p->lncy3;
-      a2.scale = inv_scale;
-      if ((s = launch_col_ifft(tuned(p, a2), nuj, st, p->tw)) != GL_OK) return s;
-      RowArgs r;
-      std::memset(&r, 0, sizeof r);
-      r.kind = ROW_OUTER;
-      r.grp[0] = BankGroup{P1, 12, B1.x0, B1.w};
-      r.grp[1] = BankGroup{P2, 9, B2.x0, B2.w};
-      r.ngrp = 2;
-      r.nout = 4;
-      r.out_x0 = B3.x0;
-      r.out_w = B3.w;
-      r.out = QO;
-      r.nx = p->ncx;
-      r.log2nx = p->lncx;
-      r.ny = ncy3;
-      r.us = us;
-      r.jobs_per_unit = J;
-      r.gmax = ROW_GMAX;
-      r.wait_surplus = p->wait_surplus;
-      r.wait_cycles = p->wait_cycles;
-      if ((s = launch_row(tuned(p, r), nuj, st, p->tw)) != GL_OK) return s;
-      ColFftArgs f;
-      f.in = QO;
-      f.out = RO;
-      f.box = B3;
-      f.n = ncy3;
-      f.log2n = p->lncy3;
-      f.nsrc = 4;
-      f.jobs_per_unit = J;
-      f.mask = s3;
-      f.maxslot = maxRO;
-      f.scale = fwd_scale3;
-      if ((s = launch_col_fft(tuned(p, f), nuj * 4, st, p->tw, "col_fft_kernel[outer]")) != GL_OK) return s;
-      AccArgs c;
-      std::memset(&c, 0, sizeof c);
-      c.us = us;
-      c.geo = p->geo3;
-      c.box = B3;
-      c.in = RO;
-      c.maxin = maxRO;
-      c.maxout = maxF;
-      c.mask = s3;
-      c.floor_rel = p->floor_rel;
-      c.nsub = J;
-      dim3 g(grid_for(pl3, T, 48), nuj);
-      {
-        LaunchScope ls_("acc_outer_max_kernel", st, 0.0);
-        acc_outer_max_kernel<<<g, T, 0, st>>>(c);
-      }
-      LAUNCH_CHECK("acc_outer_max_kernel");
-      c.out = out33;
-      c.nodes = dn + 3 * MAX_RANK;
-      c.weights = dn + 7 * MAX_RANK;
-      c.nnodes = J;
-      dim3 g2(grid_for(pl3, T, 256), gu);
-      {
-        LaunchScope ls_("acc_outer_kernel", st, 0.0);
-        acc_outer_kernel<<<g2, T, 0, st>>>(c, maxF);
-      }
-      LAUNCH_CHECK("acc_outer_kernel");
+      LaunchScope ls_("acc_outer_max_kernel", st, 0.0);
+      acc_outer_max_kernel<<<g, T, 0, st>>>(c);
     }
+    LAUNCH_CHECK("acc_outer_max_kernel");
+    c.out = out33;
+    c.nodes = dn + 3 * MAX_RANK;
+    c.weights = dn + 7 * MAX_RANK;
+    c.nnodes = J;
+    dim3 g2(grid_for(pl3, T, 256), gu);
+    {
+      LaunchScope ls_("acc_outer_kernel", st, 0.0);
+      acc_outer_kernel<<<g2, T, 0, st>>>(c, maxF);
+    }
+    LAUNCH_CHECK("acc_outer_kernel");
+    return GL_OK;
+  };
+
+  // ---------------- the stages' order ----------------
+  // psi22's sum needs its contact, the outer rows their first-order banks;
+  // otherwise eta22, psi22 and order 3 are independent until the outputs.
+  // Small groups leave most of the GPU idle in each launch, so their chains run
+  // on two side streams beside the caller's (us per call, chains in turn -> side
+  // by side: 128^2 x4 every component 230 -> 135, 512^2 326 -> 252, 256^2 x8
+  // order 2 170 -> 127); inside a stream capture they stay in turn.
+  BranchSet* br = p->branches && p->lanes <= 1 ? branch_acquire(st) : nullptr;
+  if (!br) {
+    if (p->want_eta22 && (s = eta22_stage(st)) != GL_OK) return s;
+    if (p->want_psi22 && ((s = psi22_stage(st)) != GL_OK || (s = contact_stage(st)) != GL_OK ||
+                          (s = psi22_sum(st)) != GL_OK))
+      return s;
+    if (p->want_o3 && ((s = inner_stage(st)) != GL_OK || (s = first_stage(st)) != GL_OK ||
+                       (s = outer_stage(st, [](cudaStream_t) { return GL_OK; })) != GL_OK))
+      return s;
+  } else {
+    const cudaStream_t side = br->st[0], psi = p->want_o3 ? br->st[1] : st;
+    auto mark = [&](int e, cudaStream_t q) -> gl_status {
+      CUDA_TRY(cudaEventRecord(br->ev[e], q));
+      return GL_OK;
+    };
+    auto after = [&](int e, cudaStream_t q) -> gl_status {
+      CUDA_TRY(cudaStreamWaitEvent(q, br->ev[e], 0));
+      return GL_OK;
+    };
+    auto stages = [&]() -> gl_status {
+      gl_status s;
+      if ((s = mark(0, st)) != GL_OK || (s = after(0, br->st[0])) != GL_OK || (s = after(0, br->st[1])) != GL_OK)
+        return s;
+      if (p->want_o3) {
+        if ((s = first_stage(side)) != GL_OK || (s = mark(1, side)) != GL_OK || (s = inner_stage(st)) != GL_OK)
+          return s;
+      }
+      if (p->want_psi22) {
+        if ((s = psi22_stage(psi)) != GL_OK || (s = contact_stage(side)) != GL_OK || (s = mark(2, side)) != GL_OK ||
+            (s = after(2, psi)) != GL_OK || (s = psi22_sum(psi)) != GL_OK)
+          return s;
+      }
+      if (p->want_eta22 && (s = eta22_stage(side)) != GL_OK) return s;
+      if (p->want_o3 && (s = outer_stage(st, [&](cudaStream_t q) { return after(1, q); })) != GL_OK) return s;
+      return GL_OK;
+    };
+    s = stages();
+    // joined even after a failed launch, so that the caller's stream never runs
+    // ahead of work already queued
+    for (int l = 0; l < 2; ++l) {
+      const cudaError_t e1 = cudaEventRecord(br->ev[3 + l], br->st[l]);
+      const cudaError_t e2 = e1 == cudaSuccess ? cudaStreamWaitEvent(st, br->ev[3 + l], 0) : e1;
+      if (e2 != cudaSuccess && s == GL_OK) s = fail(GL_ERR_CUDA, "branch join: %s", cudaGetErrorString(e2));
+    }
+    branch_release(br);
+    if (s != GL_OK) return s;
   }
 
   // ---------------- outputs on the reference grid ----------------
