@@ -836,12 +836,13 @@ GL_D void row_products_adj(int kind, cplx* b, int L, int p) {
 // are compiled (and get registers) on their own.  FAMILY 0: order-2/3 stages,
 // 1: adjoint stages, 2: order-4 stages.
 // MULTI: rows of fewer than 16 threads per transform (powers of two below
-// 256), several rows per block (RowArgs::rpb).
-// B192: launched with at most 192 threads (the order-3 outer row of 256
-// points: 12 groups of 16, 92 KB of shared memory, 2 blocks per SM), so 2
-// blocks per SM leave it 168 registers instead of the 128 of 2 x 256.
-template <int KIND, int N, bool B192 = false>
-__global__ void __launch_bounds__(B192 ? 192 : 256, 2) row_kernel_t(RowArgs a, const cplx* __restrict__ tw) {
+// 256), possibly several rows per block (RowArgs::rpb).
+// 384 resident threads per SM leave each 168 registers: the radix-16 passes
+// run without spills (at 2 blocks of 256 threads and 128 registers they spilled
+// 80 to 220 bytes; the adjoint's 1024-point rows keep 96).
+constexpr int ROW_THREADS = 192;
+template <int KIND, int N>
+__global__ void __launch_bounds__(ROW_THREADS, 2) row_kernel_t(RowArgs a, const cplx* __restrict__ tw) {
   constexpr int FAMILY = KIND >= ROW_ADJ_ETA22 ? 1 : (KIND >= ROW_E44_PAIR && KIND <= ROW_E44_ORDER4_PSI ? 2 : 0);
   constexpr int T = FftLen<N>::T, L = FftLen<N>::ROW;
   constexpr bool MULTI = T < 16;

@@ -1,5 +1,5 @@
-// The row-stage launch shape shared by the row translation units: groups per
-// block, several short rows per block, and the 192-thread outer-row variant.
+// The row-stage launch shape shared by the row translation units: threads per
+// block and, for the shortest rows, several rows per block.
 #pragma once
 #include "gl_host.h"
 
@@ -11,51 +11,29 @@ void row_launch(int njobs, cudaStream_t st, const RowArgs& a, const cplx* tw) {
   int nb = 0;
   for (int g = 0; g < a.ngrp; ++g) nb += a.grp[g].nb;
   const size_t smem = (size_t)nb * FftLen<N>::ROW * sizeof(cplx);
-  const bool few = (long long)a.ny * njobs <= 2 * SM_COUNT;
-  // 8 transform groups per block when the row has at most 12 banks (4
-  // blocks fit per SM), 16 for wider rows (2 per SM by shared memory); a
-  // forward row with more than 16 banks (the order-3 outer row: 21) gets the
-  // fewest whole-warp groups that keep its rounds (12: the same rounds with
-  // fewer idle groups measured 6 % faster; more resident blocks for the
-  // 12-bank rows measured slower).  A launch of few rows has SMs to spare and
-  // takes a group per bank.
-  int G = nb <= 12 ? 8 : 16;
-  if (K == ROW_OUTER && nb > 16) {
-    const int rounds = (nb + 15) / 16;
-    G = (nb + rounds - 1) / rounds;
-    while ((G * T) % 32 != 0) ++G;
-  } else if (few && nb > G) {
-    G = nb;
-    while ((G * T) % 32 != 0) ++G;
-  }
-  if (a.groups > 0) G = a.groups;  // a plan's tuning
-  G = std::max(1, std::min(G, 256 / T));
-  // Short rows (fewer than 16 threads per transform) carry little work per
-  // block, so a block takes several rows (one team of G groups each) while it
-  // stays within 256 threads and ~76 KB of shared memory (3 blocks per SM),
-  // and while the launch still has two blocks for every SM.
-  const int team = G * T;
+  // 384 threads per SM (168 registers each), in as many blocks as
+  // shared memory holds of the row's banks: small blocks keep their groups busy
+  // (a block's last round and its forward transforms use few of them) and meet
+  // at cheap barriers.  A launch of fewer rows than those blocks takes fewer,
+  // larger ones.  Same-box, device us, 8 or 16 groups of 16 threads -> this:
+  // inner rows of 160 points (12 banks, 33 KB: 6 blocks of 64), 16 records
+  // of a 1024 grid: 525 -> 422;
+  // the three order-4 row stages, 64 points (pair rows: 16 banks, 17 KB, 12
+  // blocks of 32): 882 -> 705;
+  // the 256-point outer rows (21 banks, 91 KB) had 2 blocks of 192 already.
+  const int fit = std::max(1, (int)(SMEM_LIMIT / (smem + 1024)));
+  const long long rows = (long long)a.ny * njobs;
+  const int blocks = (int)std::min<long long>(fit, (rows + SM_COUNT - 1) / SM_COUNT);
+  int threads = std::max(std::max(32, T), std::min(ROW_THREADS, 2 * ROW_THREADS / blocks / 32 * 32));
+  if (a.groups > 0) threads = std::max(32, std::min(ROW_THREADS / T, a.groups) * T);  // a plan's tuning
+  threads = std::max(T, threads / T * T);
+  // rows so short that one row's banks leave lanes of a single warp idle share it
   int rpb = 1;
-  if (T < 16) {
-    auto whole_warps = [&](int r) {
-      while (r > 1 && (team * r) % 32 != 0) --r;
-      return r;
-    };
-    rpb = whole_warps(std::min(256 / std::max(1, team), (int)((76 * 1024) / smem)));
-    while (rpb > 1 && (long long)((a.ny + rpb - 1) / rpb) * njobs < 2 * SM_COUNT) rpb = whole_warps(rpb / 2);
-    rpb = std::max(1, rpb);
-  }
-  const int threads = rpb > 1 ? team * rpb : std::max(32, std::min(256, team));
+  if (T < 16)
+    while (threads == 32 && nb * T * rpb * 2 <= 32) rpb *= 2;
   RowArgs b = a;
   b.rpb = rpb;
   dim3 grid((a.ny + rpb - 1) / rpb, njobs);
-  if constexpr (K == ROW_OUTER && N == 256) {
-    if (threads <= 192) {
-      ensure_smem_attr((const void*)row_kernel_t<K, N, true>, (int)ROW_SMEM_LIMIT);
-      row_kernel_t<K, N, true><<<grid, threads, smem, st>>>(b, tw);
-      return;
-    }
-  }
   // a failed attribute call surfaces as the launch's own error
   ensure_smem_attr((const void*)row_kernel_t<K, N>, (int)ROW_SMEM_LIMIT);
   row_kernel_t<K, N><<<grid, threads, smem * rpb, st>>>(b, tw);
