@@ -9,9 +9,16 @@ namespace gl {
 namespace {
 
 template <int N>
-void col_fft_n(dim3 grid, int cw, cudaStream_t st, const ColFftArgs& a, const cplx* tw) {
+void col_fft_n(int cw, int njs, cudaStream_t st, const ColFftArgs& a, const cplx* tw) {
+  constexpr int T = FftLen<N>::T;
+  int threads = 256;
+  if constexpr (T <= 16) {  // a group per column: blocks of whole warps
+    threads = std::min(COL_THREADS, std::max(32, cw * T));
+    cw = threads / T;
+  }
+  dim3 grid((a.box.w + cw - 1) / cw, njs);
   ensure_smem_attr((const void*)col_fft_kernel<N>, (int)SMEM_LIMIT);
-  col_fft_kernel<N><<<grid, 256, (size_t)cw * FftLen<N>::COL * sizeof(cplx), st>>>(a, tw, cw);
+  col_fft_kernel<N><<<grid, threads, (size_t)cw * FftLen<N>::COL * sizeof(cplx), st>>>(a, tw, cw);
 }
 
 template <int N>
@@ -30,10 +37,9 @@ gl_status launch_col_fft(const ColFftArgs& a, int njs, cudaStream_t st, const cp
   // and write-back loops shorten and the transforms spread over more SMs
   else
     while (cw > 2 && (long long)((a.box.w + cw / 2 - 1) / (cw / 2)) * njs <= 2 * SM_COUNT) cw /= 2;
-  dim3 grid((a.box.w + cw - 1) / cw, njs);
   const double bytes = (double)njs * a.box.w * (a.n + a.box.h) * sizeof(cplx);
   LaunchScope ls(name, st, bytes);
-  GL_LEN_DISPATCH(a.n, col_fft_n, grid, cw, st, a, tw);
+  GL_LEN_DISPATCH(a.n, col_fft_n, cw, njs, st, a, tw);
   LAUNCH_CHECK("col_fft_kernel");
   return GL_OK;
 }

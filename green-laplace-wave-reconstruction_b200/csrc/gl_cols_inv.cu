@@ -8,9 +8,9 @@ namespace gl {
 namespace {
 
 template <int N>
-void col_ifft_n(dim3 grid, size_t smem, cudaStream_t st, const ColArgs& a, const cplx* tw, int cw, int bpb) {
+void col_ifft_n(dim3 grid, int threads, size_t smem, cudaStream_t st, const ColArgs& a, const cplx* tw, int cw, int bpb) {
   ensure_smem_attr((const void*)col_ifft_kernel<N>, (int)SMEM_LIMIT);
-  col_ifft_kernel<N><<<grid, 256, smem, st>>>(a, tw, cw, bpb);
+  col_ifft_kernel<N><<<grid, threads, smem, st>>>(a, tw, cw, bpb);
 }
 
 template <int N>
@@ -78,8 +78,10 @@ gl_status launch_col_ifft(const ColArgs& a0, int njobs, cudaStream_t st, const c
   ColArgs a = a0;
   if (!is_pow2(a.n) && !mixed_len(a.n)) return fail(GL_ERR_UNSUPPORTED, "column length %d has no transform", a.n);
   for (int k = 0; k < a.nbanks; ++k) factor_of(a.mult[k], a.fac[k], a.rot[k]);
-  const int T = is_pow2(a.n) ? a.n / 16 : 16, G = 256 / T;
+  const int T = is_pow2(a.n) ? a.n / 16 : 16;
   const bool direct = T <= 16;
+  const int threads = direct ? COL_THREADS : 256;
+  const int G = threads / T;
   // the damped base spectrum of the block's columns is formed only for the
   // kinds that share one base across their banks (col_ifft_kernel)
   const bool shared_base = a.kind != COL_PLAIN && a.kind != COL_OUTER2 && a.kind != COL_FLOORED;
@@ -92,22 +94,23 @@ gl_status launch_col_ifft(const ColArgs& a0, int njobs, cudaStream_t st, const c
   // damped base (about a third of a round per element and thread) and half a
   // round of prologue; blocks run in waves of the resident ones.  Splitting the
   // banks repeats the base but fills the GPU when a launch has few columns and
-  // jobs (one 128^2 unit: 24 blocks of four serial rounds became 192 of one),
-  // and trims the last wave of large ones (16 units of the 1024^2 order-3
-  // workload: 640 blocks in 3 waves).
-  const int cw_top = fft_cols_per_block(a.n, w);
+  // jobs, and trims the last wave of large ones.  Of short transforms a block
+  // takes two columns, which fill a sector; more only lengthen the base's
+  // prologue (64-point order-4 banks 331 us with 2 columns, 364 with 16).
+  const int cw_top = std::min(direct ? (a.cw_max > 0 ? G : 2) : G, next_pow2(w));
   int best_cw = cw_top, best_bpb = a.nbanks;
   double best = 1e30;
   for (int cw = a.cw_max > 0 ? std::min(a.cw_max, cw_top) : cw_top; cw >= 1; cw /= 2) {
     const size_t sm = smem_of(cw);
     if (sm > SMEM_LIMIT) continue;
-    const double slots = (double)SM_COUNT * (2 * (sm + 1024) <= SMEM_LIMIT + 1024 ? 2 : 1);
+    const size_t resident = std::min<size_t>(direct ? 6 : 2, (SMEM_LIMIT + 1024) / (sm + 1024));
+    const double slots = (double)SM_COUNT * std::max<size_t>(1, resident);
     for (int nz = 1; nz <= a.nbanks; ++nz) {
       const int bpb = (a.nbanks + nz - 1) / nz;
       const double blocks = (double)((w + cw - 1) / cw) * njobs * ((a.nbanks + bpb - 1) / bpb);
       const int cols = std::min(cw, w);
       const int rounds = direct ? (bpb * cols + G - 1) / G : bpb;
-      const int base_iters = shared_base ? (cw * a.box.h + 255) / 256 : 0;
+      const int base_iters = shared_base ? (cw * a.box.h + threads - 1) / threads : 0;
       const double q = blocks / slots;
       const double waves = q <= 4.0 ? std::ceil(q) : q + 0.5;
       const double cost = waves * (0.5 + 0.35 * base_iters + rounds) * (blocks <= SM_COUNT ? 0.7 : 1.0);
@@ -124,7 +127,7 @@ gl_status launch_col_ifft(const ColArgs& a0, int njobs, cudaStream_t st, const c
   const double bytes = (double)njobs * (a.twins ? a.nout : a.nbanks) * w * a.n * sizeof(cplx) +
                        (double)njobs * w * a.box.h * sizeof(cplx);
   LaunchScope ls(col_ifft_name(a.kind), st, bytes);
-  GL_LEN_DISPATCH(a.n, col_ifft_n, grid, smem, st, a, tw, best_cw, best_bpb);
+  GL_LEN_DISPATCH(a.n, col_ifft_n, grid, threads, smem, st, a, tw, best_cw, best_bpb);
   LAUNCH_CHECK("col_ifft_kernel");
   return GL_OK;
 }

@@ -87,8 +87,9 @@ GL_D void group_sync(int id) {
 
 // One Stockham pass of radix R over sub-transforms of NS points: LAST hands its
 // butterflies to sink(o, step, v, R) -- element r of v is output o + r * step.
-template <int SIGN, int N, int R, int NS, bool LAST, class Load, class Sink>
-GL_D void pass_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__ tw, Load& load, Sink& sink) {
+template <int SIGN, int N, int R, int NS, bool LAST, class Load, class Sink, class After>
+GL_D void pass_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__ tw, Load& load, Sink& sink,
+                 After& after) {
   constexpr int T = FftLen<N>::T, B = 16 / R, stride = N / R;
   constexpr int twstep = TW_N / (NS * R);
   if constexpr (NS == 1) {
@@ -96,6 +97,7 @@ GL_D void pass_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__
     if (active) {
 #pragma unroll
       for (int r = 0; r < 16; ++r) v[r] = load(t + r * stride, r);
+      after(v);
     }
     group_sync<N>(id);
     if (active) {
@@ -152,10 +154,16 @@ GL_D void pass_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__
 // group makes the same call; `id` names the group's barrier when T > 32.
 // The first pass has read all its inputs before it writes `buf`, and the last
 // one has read element i when it hands it to the sink, so load may read `buf`
-// and sink may write each element back to its own place.  Other lanes may
+// and sink may write each element back to its own place.  after(v) changes a
+// thread's inputs once all of them are on their way (a branch inside load would
+// wait for each before the next is asked for).  Other lanes may
 // still be reading `buf` when a thread returns.
-template <int SIGN, int N, class Load, class Sink>
-GL_D void fft_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__ tw, Load& load, Sink& sink) {
+struct AsLoaded {
+  GL_D void operator()(cplx*) const {}
+};
+template <int SIGN, int N, class Load, class Sink, class After = const AsLoaded>
+GL_D void fft_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__ tw, Load& load, Sink& sink,
+                After& after = AsLoaded{}) {
   if constexpr (FftLen<N>::mixed) {
     constexpr int M = FftLen<N>::M, MP = FftLen<N>::MP;
     {
@@ -163,6 +171,7 @@ GL_D void fft_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__ 
       if (active) {
 #pragma unroll
         for (int r = 0; r < M; ++r) v[r] = load(t + 16 * r, r);
+        after(v);
       }
       group_sync<N>(id);
       if (active) {
@@ -183,13 +192,13 @@ GL_D void fft_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__ 
       sink(t, M, v, 16);
     }
   } else {
-    pass_n<SIGN, N, 16, 1, N == 16>(buf, t, id, active, tw, load, sink);
+    pass_n<SIGN, N, 16, 1, N == 16>(buf, t, id, active, tw, load, sink, after);
     if constexpr (N >= 256) {
-      pass_n<SIGN, N, 16, 16, N == 256>(buf, t, id, active, tw, load, sink);
-      if constexpr (N == 4096) pass_n<SIGN, N, 16, 256, true>(buf, t, id, active, tw, load, sink);
-      else if constexpr (N > 256) pass_n<SIGN, N, N / 256, 256, true>(buf, t, id, active, tw, load, sink);
+      pass_n<SIGN, N, 16, 16, N == 256>(buf, t, id, active, tw, load, sink, after);
+      if constexpr (N == 4096) pass_n<SIGN, N, 16, 256, true>(buf, t, id, active, tw, load, sink, after);
+      else if constexpr (N > 256) pass_n<SIGN, N, N / 256, 256, true>(buf, t, id, active, tw, load, sink, after);
     } else if constexpr (N > 16) {
-      pass_n<SIGN, N, N / 16, 16, true>(buf, t, id, active, tw, load, sink);
+      pass_n<SIGN, N, N / 16, 16, true>(buf, t, id, active, tw, load, sink, after);
     }
   }
 }

@@ -308,14 +308,23 @@ constexpr int ROT_SWAP = 1, ROT_NEG_RE = 2, ROT_NEG_IM = 4;
 // shared memory (column-major); each (bank, column) is then one length-N
 // inverse transform along y by a group of T threads, whose first pass reads
 // base x factor straight into registers -- sixteen independent loads, no
-// staging pass.  Items are dealt to the groups column-fastest, so no group
+// staging pass, and no branch among them: a floor test inside the load waited
+// for each value before asking for the next (outer banks of 16 records of a
+// 1024 grid, 9 of 240 points from 4 spectra: 281 us, now 173; the 12 damped
+// ones 159, now 124; inner banks of 144 points 293, now 243).  Items are dealt to the groups column-fastest, so no group
 // idles when a block has few columns.  Transforms of at most 16 threads need no
 // block barrier between items and write their last pass straight to global
 // memory (two adjacent columns of a warp fill each 32-byte sector); longer ones
 // go back row-major through shared memory, one bank at a time.
 // Output layout [job][bank][y][column] (rows contiguous for the row kernel).
+// Blocks of the column kernels: transforms of at most 16 threads run in blocks
+// of COL_THREADS, six per SM (168 registers: no spills up to 192 points, 56
+// bytes at 240).  Eight or ten blocks (128 or 102 registers) spilled 260 to 600
+// bytes and measured slower (inner banks of 16 records 289 and 347 us against
+// 243).
+constexpr int COL_THREADS = 64;
 template <int N>
-__global__ void __launch_bounds__(256, 2) col_ifft_kernel(ColArgs a, const cplx* __restrict__ tw,
+__global__ void __launch_bounds__(FftLen<N>::T <= 16 ? COL_THREADS : 256, FftLen<N>::T <= 16 ? 6 : 2) col_ifft_kernel(ColArgs a, const cplx* __restrict__ tw,
                                                          int cw, int banks_per_block) {
   extern __shared__ cplx smem[];
   constexpr int T = FftLen<N>::T, L = FftLen<N>::COL;
@@ -362,38 +371,55 @@ __global__ void __launch_bounds__(256, 2) col_ifft_kernel(ColArgs a, const cplx*
     const int fac = a.fac[k];
     int rot = a.conj_io ? a.rot[k] ^ ROT_NEG_IM : a.rot[k];
     group_sync<N>(1 + g);  // the row's previous transform has been read
-    if (fac == F_DIRECT || floor_it) {
-      // floored or divided values go through the front of the group's row
+    const double floor_abs =
+        !floor_it ? 0.0
+                  : a.floor_rel * as_double(a.kind == COL_FLOORED
+                                                ? a.floor_max[(size_t)job * a.floor_nsrc + a.src_of[k]]
+                                                : a.floor_max[job]);
+    if (fac == F_DIRECT) {
+      // divided values go through the front of the group's row
       if (active) {
-        const double floor_abs =
-            !floor_it ? 0.0
-                      : a.floor_rel * as_double(a.kind == COL_FLOORED
-                                                    ? a.floor_max[(size_t)job * a.floor_nsrc + a.src_of[k]]
-                                                    : a.floor_max[job]);
 #pragma unroll 1
         for (int by = t; by < h; by += T) {
           cplx v = src[by * sstep];
           if (floor_it && abs_below(v, floor_abs)) v = czero();
-          buf[by] = fac == F_DIRECT ? mult_direct(a.mult[k], GeoRef{a.geo, plane, by * w + x}, v) : v;
+          buf[by] = mult_direct(a.mult[k], GeoRef{a.geo, plane, by * w + x}, v);
         }
       }
       src = buf;
       sstep = 1;
     }
+    const bool floor_load = floor_it && fac != F_DIRECT;
     group_sync<N>(1 + g);
     const double* f = fac >= 0 ? a.geo + (size_t)(GEO_PLANES + fac) * plane + (size_t)x * h : nullptr;
     auto load = [&](int yb, int) -> cplx {
       const int by = wrap_n<N>(yb - y0);
-      cplx z = czero();
-      if (by < h) {
-        const cplx v = src[by * sstep];
-        const double m = f ? __ldg(f + by) : 1.0;
-        z.x = m * (rot & ROT_SWAP ? v.y : v.x);
-        z.y = m * (rot & ROT_SWAP ? v.x : v.y);
+      cplx v = czero();
+      if (by < h) v = src[by * sstep];
+      return v;
+    };
+    auto after = [&](cplx* v) {
+      constexpr int C = FftLen<N>::mixed ? FftLen<N>::M : 16, S = FftLen<N>::mixed ? 16 : N / 16;
+      if (floor_load) {
+#pragma unroll
+        for (int r = 0; r < C; ++r)
+          if (abs_below(v[r], floor_abs)) v[r] = czero();
+      }
+      double m[C];
+#pragma unroll
+      for (int r = 0; r < C; ++r) {
+        const int by = wrap_n<N>(t + r * S - y0);
+        m[r] = 1.0;
+        if (f && by < h) m[r] = __ldg(f + by);
+      }
+#pragma unroll
+      for (int r = 0; r < C; ++r) {
+        const bool in = wrap_n<N>(t + r * S - y0) < h;
+        cplx z = cmk(m[r] * (rot & ROT_SWAP ? v[r].y : v[r].x), m[r] * (rot & ROT_SWAP ? v[r].x : v[r].y));
         if (rot & ROT_NEG_RE) z.x = -z.x;
         if (rot & ROT_NEG_IM) z.y = -z.y;
+        v[r] = in ? z : czero();
       }
-      return z;
     };
     const int tb = a.twins ? a.twin[k] : -1;
     const int tfac = tb >= 0 ? a.twin_fac[k] : 0;
@@ -420,7 +446,7 @@ __global__ void __launch_bounds__(256, 2) col_ifft_kernel(ColArgs a, const cplx*
         row_put<N>(buf, o, step, v, cnt);
       }
     };
-    fft_n<+1, N>(buf, t, 1 + g, active, tw, load, sink);
+    fft_n<+1, N>(buf, t, 1 + g, active, tw, load, sink, after);
     if constexpr (!direct) {
       __syncthreads();
       cplx* d0 = a.out + ((size_t)job * nout + (a.twins ? a.out_of[k_first + kk] : k_first + kk)) * N * w + x_first;
@@ -986,63 +1012,104 @@ struct ColFftArgs {
   int cw_max = 0;          // > 0: at most this many columns per block (a power of two; tuning)
 };
 
-// One block: `cw` kept columns of one (job, source) spectrum.  Rows of the
-// input ([js][y][col]) are staged with coalesced loads, each column is one
-// forward transform along y, and only the output box's rows are written
-// (support-masked), with the spectrum's max |.| folded into maxslot.
+// One block: `cw` kept columns of one (job, source) spectrum ([js][y][col]).
+// Each column is one forward transform along y; only the output box's rows are
+// written (support-masked), with the spectrum's max |.| folded into maxslot.
+// Transforms of at most 16 threads (cw = groups of the block) read their first
+// pass from global memory into registers and write their last pass from
+// registers, with no block barrier: two or more adjacent columns of a warp use
+// every 32-byte sector.  All loads of a thread are on their way before the
+// first is used.  Staged through shared memory in 256-thread blocks at 128
+// registers, with the mask and hypot in one loop, the inner stage of 16 records
+// (145 x 145 of 144 points, 2048 spectra) took 329 us; this takes 277.
+// Longer columns are staged with coalesced loads.
 template <int N>
-__global__ void __launch_bounds__(256, 2) col_fft_kernel(ColFftArgs a, const cplx* __restrict__ tw, int cw) {
+__global__ void __launch_bounds__(FftLen<N>::T <= 16 ? COL_THREADS : 256, FftLen<N>::T <= 16 ? 6 : 2) col_fft_kernel(ColFftArgs a, const cplx* __restrict__ tw, int cw) {
   extern __shared__ cplx smem[];
   constexpr int T = FftLen<N>::T, L = FftLen<N>::COL;
+  constexpr bool direct = T <= 16;
   const int js = blockIdx.y;
   const int job = js / a.nsrc;
   const int unit = job / a.jobs_per_unit;
   const int x_first = blockIdx.x * cw;
   const int ncol = min(cw, a.box.w - x_first);
-  cplx* bufs = smem;  // cw * L
   const cplx* src = a.in + (size_t)js * N * a.box.w + x_first;
-  // stage the kept columns ([y][col] rows in global memory) with eight
-  // independent loads in flight per thread
-  const int lcw = 31 - __clz(cw);  // cw is a power of two: (y, c) = (t >> lcw, t & (cw - 1))
-  const int total = N << lcw;
-  for (int t0 = threadIdx.x; t0 < total; t0 += 8 * blockDim.x) {
-    cplx v[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int t = t0 + u * blockDim.x;
-      if (t < total && (t & (cw - 1)) < ncol) v[u] = src[(size_t)(t >> lcw) * a.box.w + (t & (cw - 1))];
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int t = t0 + u * blockDim.x;
-      if (t < total && (t & (cw - 1)) < ncol)
-        bufs[(t & (cw - 1)) * L + pos<N>(t >> lcw)] = a.conj_io ? cconj(v[u]) : v[u];
-    }
-  }
-  __syncthreads();
-  const int G = blockDim.x / T, g = threadIdx.x / T, t = threadIdx.x % T;
-  const int y0 = mod_n<N>(a.box.y0);
-  for (int it = 0; it < ncol; it += G) {
-    const int c = it + g;
-    const bool active = c < ncol;
-    cplx* buf = bufs + (active ? c : 0) * L;
-    auto load = [&](int, int r) -> cplx { return buf[pos_in<N>(t, r)]; };
-    auto sink = [&](int o, int step, const cplx* v, int cnt) { row_put<N>(buf, o, step, v, cnt); };
-    fft_n<-1, N>(buf, t, 1 + g, active, tw, load, sink);
-  }
-  __syncthreads();
   const unsigned char* mask = a.mask ? a.mask + (size_t)unit * a.box.w * a.box.h : nullptr;
   cplx* dst = a.out + (size_t)js * a.box.w * a.box.h;
+  const int G = blockDim.x / T, g = threadIdx.x / T, t = threadIdx.x % T;
+  const int y0 = mod_n<N>(a.box.y0);
   double local = 0.0;
-  for (int t = threadIdx.x; t < (a.box.h << lcw); t += blockDim.x) {
-    const int c = t & (cw - 1), by = t >> lcw;
-    if (c >= ncol) continue;
-    const int i = by * a.box.w + x_first + c;
-    const cplx raw = bufs[c * L + pos<N>(wrap_n<N>(y0 + by))];
+  auto put = [&](int i, const cplx& raw) {
     cplx v = cscale(a.scale, a.conj_io ? cconj(raw) : raw);
     if (mask && !mask[i]) v = czero();
     dst[i] = v;
-    local = keep_max_abs(local, v);
+    return v;
+  };
+  if constexpr (direct) {
+    const bool active = g < ncol;
+    const int c = active ? g : 0;
+    auto load = [&](int y, int) -> cplx {
+      const cplx v = src[(size_t)y * a.box.w + c];
+      return a.conj_io ? cconj(v) : v;
+    };
+    auto sink = [&](int o, int step, cplx* v, int cnt) {
+      unsigned char keep[16];
+#pragma unroll
+      for (int r = 0; r < 16; ++r) {  // all mask bytes on their way before the first is used
+        if (r >= cnt) continue;
+        const int by = wrap_n<N>(o + r * step - y0);
+        keep[r] = by < a.box.h;
+        if (mask && by < a.box.h) keep[r] = __ldg(mask + by * a.box.w + x_first + c);
+      }
+#pragma unroll
+      for (int r = 0; r < 16; ++r) {
+        if (r >= cnt) continue;
+        const int by = wrap_n<N>(o + r * step - y0);
+        cplx z = cscale(a.scale, a.conj_io ? cconj(v[r]) : v[r]);
+        if (!keep[r]) z = czero();
+        v[r] = z;
+        if (by < a.box.h) dst[by * a.box.w + x_first + c] = z;
+      }
+#pragma unroll
+      for (int r = 0; r < 16; ++r)
+        if (r < cnt) local = keep_max_abs(local, v[r]);
+    };
+    fft_n<-1, N>(smem + g * L, t, 1 + g, active, tw, load, sink);
+  } else {
+    cplx* bufs = smem;  // cw * L
+    // stage the kept columns ([y][col] rows in global memory) with eight
+    // independent loads in flight per thread
+    const int lcw = 31 - __clz(cw);  // cw is a power of two: (y, c) = (q >> lcw, q & (cw - 1))
+    const int total = N << lcw;
+    for (int q0 = threadIdx.x; q0 < total; q0 += 8 * blockDim.x) {
+      cplx v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int q = q0 + u * blockDim.x;
+        if (q < total && (q & (cw - 1)) < ncol) v[u] = src[(size_t)(q >> lcw) * a.box.w + (q & (cw - 1))];
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int q = q0 + u * blockDim.x;
+        if (q < total && (q & (cw - 1)) < ncol)
+          bufs[(q & (cw - 1)) * L + pos<N>(q >> lcw)] = a.conj_io ? cconj(v[u]) : v[u];
+      }
+    }
+    __syncthreads();
+    for (int it = 0; it < ncol; it += G) {
+      const int c = it + g;
+      const bool active = c < ncol;
+      cplx* buf = bufs + (active ? c : 0) * L;
+      auto load = [&](int, int r) -> cplx { return buf[pos_in<N>(t, r)]; };
+      auto sink = [&](int o, int step, const cplx* v, int cnt) { row_put<N>(buf, o, step, v, cnt); };
+      fft_n<-1, N>(buf, t, 1 + g, active, tw, load, sink);
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < (a.box.h << lcw); q += blockDim.x) {
+      const int c = q & (cw - 1), by = q >> lcw;
+      if (c < ncol)
+        local = keep_max_abs(local, put(by * a.box.w + x_first + c, bufs[c * L + pos<N>(wrap_n<N>(y0 + by))]));
+    }
   }
   if (a.maxslot) {
     for (int o = 16; o > 0; o >>= 1) {
