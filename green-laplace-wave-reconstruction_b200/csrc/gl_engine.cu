@@ -3904,51 +3904,63 @@ struct Fields {
   long long stride;
 };
 
-static SFft sfft(const Fields& d, int n, long long stride, long long cstride, int ncount, long long ostride,
-                 double scale) {
+// A launch over the columns [grp * gpitch + w], w < cols, elements `stride` apart.
+static SFft sfft(const Fields& d, int n, long long stride, int cols, int groups, long long gpitch, double scale,
+                 const int* live) {
   SFft a;
   std::memset(&a, 0, sizeof a);
   a.data = d.data;
   a.fields = d.count;
   a.fstride = d.stride;
   a.n = n;
-  a.log2n = ilog2(n);
   a.stride = stride;
-  a.cstride = cstride;
-  a.ncount = ncount;
-  a.ostride = ostride;
+  a.cols = cols;
+  a.groups = groups;
+  a.gpitch = gpitch;
   a.scale = scale;
+  a.live = live;
   return a;
 }
 
-// Transform along axis 0 of a [P][M] array (length P, power of two).  sign > 0:
-// natural input, output rows permuted when P > 4096; sign < 0: the inverse
-// ordering (permuted input, natural output).  Four-step split P = P1 P2.
-static gl_status axis0_transform(const Fields& d, int P, int M, int sign, double scale, cudaStream_t st,
-                                 const cplx* tw) {
-  if (P <= TW_N) return launch_sfft(sfft(d, P, M, 1, M, 0, scale), 1, sign, st, tw);
+// Transform along axis 0 of the first `cols` columns (and *live of them) of a
+// [P][M] array (length P, power of two).  sign > 0: natural input, output rows
+// permuted when P > 4096; sign < 0: the inverse ordering (permuted input,
+// natural output).  Four-step split P = P1 P2.  `banks`: the fields are the
+// multiplier banks of another array.
+static gl_status axis0_transform(const Fields& d, int P, int M, int cols, const int* live, int sign, double scale,
+                                 cudaStream_t st, const cplx* tw, const ModalBank* banks = nullptr,
+                                 const ModalGeo* geo = nullptr) {
+  auto with_banks = [&](SFft a, int row_step) {
+    if (banks) {
+      a.nbanks = d.count;
+      for (int k = 0; k < d.count; ++k) a.bank[k] = banks[k];
+      a.geo = *geo;
+      a.row_step = row_step;
+    }
+    return a;
+  };
+  if (P <= TW_N) return launch_sfft(with_banks(sfft(d, P, M, cols, 1, 0, scale, live), 1), sign, st, tw);
   const int p = ilog2(P);
   const int P1 = 1 << (p - p / 2), P2 = 1 << (p / 2);
+  const long long row = (long long)P1 * M;
   gl_status s;
   if (sign > 0) {
-    SFft a = sfft(d, P2, (long long)P1 * M, 1, P1 * M, 0, 1.0);
-    a.tw_mode = 1;
-    a.tw_div = M;
+    SFft a = with_banks(sfft(d, P2, row, cols, P1, M, 1.0, live), P1);
     a.tw_log2p = p;
-    if ((s = launch_sfft(a, 1, +1, st, tw)) != GL_OK) return s;
-    return launch_sfft(sfft(d, P1, M, 1, M, (long long)P1 * M, scale), P2, +1, st, tw);
+    if ((s = launch_sfft(a, +1, st, tw)) != GL_OK) return s;
+    return launch_sfft(sfft(d, P1, M, cols, P2, row, scale, live), +1, st, tw);
   }
-  SFft a = sfft(d, P1, M, 1, M, (long long)P1 * M, 1.0);
-  a.tw_mode = 2;
+  SFft a = sfft(d, P1, M, cols, P2, row, 1.0, live);
   a.tw_log2p = p;
-  if ((s = launch_sfft(a, P2, -1, st, tw)) != GL_OK) return s;
-  return launch_sfft(sfft(d, P2, (long long)P1 * M, 1, P1 * M, 0, scale), 1, -1, st, tw);
+  if ((s = launch_sfft(a, -1, st, tw)) != GL_OK) return s;
+  return launch_sfft(sfft(d, P2, row, cols, P1, M, scale, live), -1, st, tw);
 }
 
-// Transform along the contiguous last axis of [rows][M].
-static gl_status axis_last_transform(const Fields& d, long long rows, int M, int sign, double scale,
-                                     cudaStream_t st, const cplx* tw) {
-  return launch_sfft(sfft(d, M, 1, M, (int)rows, 0, scale), 1, sign, st, tw);
+// Transform along the contiguous last axis of [rows][M]: inputs at and past
+// live_max (or *live) are zero, outputs at and past `keep` are not written.
+static gl_status axis_last_transform(const Fields& d, long long rows, int M, int live_max, const int* live, int keep,
+                                     int sign, double scale, cudaStream_t st, const cplx* tw) {
+  return launch_lfft(LFft{d.data, M, rows, live, live_max, keep, scale, d.count, d.stride}, sign, st, tw);
 }
 
 static int modal_pad(int w) { return std::max(16, next_pow2(w)); }
@@ -4001,6 +4013,8 @@ extern "C" gl_status gl_modal_level(const gl_modal_desc* d, int nnz, const long 
   const size_t plane = align_up((size_t)total * sizeof(cplx));
   char* base = reinterpret_cast<char*>(d_ws);
   double* dn = reinterpret_cast<double*>(base);  // nodes then weights
+  int* live = reinterpret_cast<int*>(dn + 2 * MAX_RANK);  // columns of the joint array that hold values
+  static_assert(2 * MAX_RANK * sizeof(double) + sizeof(int) <= 4096, "workspace head");
   char* bufs = base + align_up(4096);
   auto buf = [&](int k) { return reinterpret_cast<cplx*>(bufs + (size_t)k * plane); };
   char* small = bufs + modal_buffers(d->order) * plane;
@@ -4029,42 +4043,33 @@ extern "C" gl_status gl_modal_level(const gl_modal_desc* d, int nnz, const long 
   const int eb = grid_for((size_t)total, T, 8192);
   cplx* joint = buf(0);
   CUDA_TRY(cudaMemsetAsync(joint, 0, (size_t)total * sizeof(cplx), st));
+  CUDA_TRY(cudaMemsetAsync(live, 0, sizeof(int), st));
   if (nnz) {
     // indices arrive in [P][W]; the joint is [P][M]
     LaunchScope ls_("modal_scatter_kernel", st, 0.0);
-    modal_scatter_kernel<<<grid_for(nnz, T, 1024), T, 0, st>>>(d_idx, d_val, nnz, joint, W, M);
+    modal_scatter_kernel<<<grid_for(nnz, T, 1024), T, 0, st>>>(d_idx, d_val, nnz, joint, W, M, live);
   }
   LAUNCH_CHECK("modal_scatter_kernel");
   const long long step = (long long)(plane / sizeof(cplx));
-  auto to_spectrum = [&](const Fields& b) -> gl_status {
-    gl_status r = axis_last_transform(b, P, M, +1, 1.0 / M, st, tw);
+  // the first n bins of a field's spectrum
+  auto to_spectrum = [&](const Fields& b, int n) -> gl_status {
+    gl_status r = axis_last_transform(b, P, M, M, nullptr, n, +1, 1.0 / M, st, tw);
     if (r != GL_OK) return r;
-    return axis0_transform(b, P, M, -1, 1.0 / P, st, tw);
+    return axis0_transform(b, P, M, n, nullptr, -1, 1.0 / P, st, tw);
   };
-  // banks first .. first + n - 1: src x mult, transformed to fields
-  auto bank_fields = [&](int first, int n, const cplx* const* src, const int* mult) -> gl_status {
-    ModalBanks a;
-    a.g = g;
-    for (int k = 0; k < n; ++k) {
-      a.src[k] = src[k];
-      a.mult[k] = mult[k];
-    }
-    a.out = buf(first);
-    a.stride = step;
-    {
-      LaunchScope ls_("modal_bank_kernel", st, 0.0);
-      modal_bank_kernel<<<dim3(eb, n), T, 0, st>>>(a);
-    }
-    LAUNCH_CHECK("modal_bank_kernel");
+  // banks first .. first + n - 1 of arrays that are zero from column `cols`
+  // (or *nz) on, transformed to fields
+  auto bank_fields = [&](int first, int n, const ModalBank* banks, int cols, const int* nz) -> gl_status {
     const Fields b{buf(first), n, step};
-    gl_status r = axis0_transform(b, P, M, +1, 1.0, st, tw);
+    gl_status r = axis0_transform(b, P, M, cols, nz, +1, 1.0, st, tw, banks, &g);
     if (r != GL_OK) return r;
-    return axis_last_transform(b, P, M, -1, 1.0, st, tw);
+    return axis_last_transform(b, P, M, cols, nz, M, -1, 1.0, st, tw);
   };
-  // order-2 banks: 1 v, 2 vn, 3 vn2, 4 hx, 5 jx, 6 radial
-  const int m6[6] = {MM_ONE, MM_NU, MM_NU2, MM_Q_SNU, MM_Q, MM_Q2_SNU};
-  const cplx* src6[6] = {joint, joint, joint, joint, joint, joint};
-  if ((s = bank_fields(1, 6, src6, m6)) != GL_OK) return s;
+  // order-2 banks: 1 v, 2 vn, 3 vn2, 4 hx, 5 jx, 6 radial (multipliers of modal_time.py:240-246)
+  const ModalBank m6[6] = {{joint, 0, MC_ONE, 0, false},     {joint, 0, MC_NU, 0, false},
+                           {joint, 0, MC_NU2, 0, false},     {joint, 1, MC_OVER_NU, 0, false},
+                           {joint, 1, MC_ONE, 0, false},     {joint, 2, MC_OVER_NU, 0, false}};
+  if ((s = bank_fields(1, 6, m6, W, live)) != GL_OK) return s;
   {
     LaunchScope ls_("modal_sources_kernel", st, 0.0);
     modal_sources_kernel<<<eb, T, 0, st>>>(total, buf(1), buf(2), buf(3), buf(4), buf(5), buf(6));
@@ -4072,7 +4077,8 @@ extern "C" gl_status gl_modal_level(const gl_modal_desc* d, int nnz, const long 
   LAUNCH_CHECK("modal_sources_kernel");
   cplx* SD = buf(3);
   cplx* SK = buf(6);
-  if ((s = to_spectrum(Fields{SD, 2, 3 * step})) != GL_OK) return s;  // and SK
+  const int n2 = 2 * wmax + 1, n3 = 3 * wmax + 1;
+  if ((s = to_spectrum(Fields{SD, 2, 3 * step}, n2)) != GL_OK) return s;  // and SK
   ModalResp r;
   std::memset(&r, 0, sizeof r);
   r.g = g;
@@ -4089,7 +4095,7 @@ extern "C" gl_status gl_modal_level(const gl_modal_desc* d, int nnz, const long 
   r.scale = d->scale22;
   {
     LaunchScope ls_("modal_response_kernel", st, 0.0);
-    modal_response_kernel<<<r.nbins, 256, 0, st>>>(r);
+    modal_response_kernel<<<r.nbins, RESPONSE_THREADS, 0, st>>>(r);
   }
   LAUNCH_CHECK("modal_response_kernel");
   {
@@ -4113,10 +4119,15 @@ extern "C" gl_status gl_modal_level(const gl_modal_desc* d, int nnz, const long 
   LAUNCH_CHECK("modal_pair_kernel");
   // first-order fields: v (1) and hx (4) are eta and phix; the others in 9..15;
   // pair fields 16..21: eta, etax (from e2); phix, phiz, phizz, phitz (from p2)
-  const int m13[13] = {MM_IQ,     MM_MI_NU,   MM_NU_Q,    MM_MI_Q2_SNU, MM_MI_Q2_NU, MM_MINUS_NU2, MM_MINUS_Q2,
-                       MM_PAIR_E, MM_PAIR_EX, MM_PAIR_PX, MM_PAIR_PZ,   MM_PAIR_PZZ, MM_PAIR_PTZ};
-  const cplx* src13[13] = {joint, joint, joint, joint, joint, joint, joint, E2, E2, P2, P2, P2, P2};
-  if ((s = bank_fields(9, 13, src13, m13)) != GL_OK) return s;
+  // (multipliers of modal_time.py:302-317)
+  const ModalBank first7[7] = {{joint, 1, MC_ONE, 1, false},  {joint, 0, MC_NU, -1, false},
+                               {joint, 1, MC_NU, 0, false},   {joint, 2, MC_OVER_NU, -1, false},
+                               {joint, 2, MC_NU, -1, false},  {joint, 0, MC_NU2, 0, true},
+                               {joint, 2, MC_ONE, 0, true}};
+  const ModalBank pair6[6] = {{E2, 0, MC_ONE, 0, false},  {E2, 1, MC_ONE, 1, false}, {P2, 1, MC_ONE, 1, false},
+                              {P2, -1, MC_ONE, 0, false}, {P2, 2, MC_ONE, 0, false}, {P2, -1, MC_INNER, -1, false}};
+  if ((s = bank_fields(9, 7, first7, W, live)) != GL_OK) return s;
+  if ((s = bank_fields(16, 6, pair6, n2, nullptr)) != GL_OK) return s;
   ModalForcing fo;
   fo.fe = buf(1);
   fo.fex = buf(9);
@@ -4141,7 +4152,7 @@ extern "C" gl_status gl_modal_level(const gl_modal_desc* d, int nnz, const long 
     modal_forcing_kernel<<<eb, T, 0, st>>>(fo);
   }
   LAUNCH_CHECK("modal_forcing_kernel");
-  if ((s = to_spectrum(Fields{fo.fk, 2, 3 * step})) != GL_OK) return s;  // and fd
+  if ((s = to_spectrum(Fields{fo.fk, 2, 3 * step}, n3)) != GL_OK) return s;  // and fd
   ModalResp r3 = r;
   r3.sd = fo.fd;
   r3.sk = fo.fk;
@@ -4152,7 +4163,7 @@ extern "C" gl_status gl_modal_level(const gl_modal_desc* d, int nnz, const long 
   r3.scale = d->lambda3;
   {
     LaunchScope ls_("modal_response_kernel", st, 0.0);
-    modal_response_kernel<<<r3.nbins, 256, 0, st>>>(r3);
+    modal_response_kernel<<<r3.nbins, RESPONSE_THREADS, 0, st>>>(r3);
   }
   LAUNCH_CHECK("modal_response_kernel");
   {
@@ -4206,6 +4217,7 @@ extern "C" gl_status gl_eta20_level(const gl_eta20_desc* d, int nnz, const long 
   const size_t plane = align_up((size_t)total * sizeof(cplx));
   char* base = reinterpret_cast<char*>(d_ws);
   double* dn = reinterpret_cast<double*>(base);
+  int* live = reinterpret_cast<int*>(dn + 2 * MAX_RANK);  // columns of the joint array that hold values
   {
     double host[2 * MAX_RANK] = {0};
     std::memcpy(host, d->nodes, sizeof(double) * d->rank);
@@ -4226,30 +4238,31 @@ extern "C" gl_status gl_eta20_level(const gl_eta20_desc* d, int nnz, const long 
   const int eb = grid_for((size_t)total, T, 8192);
   cplx* joint = buf(0);
   CUDA_TRY(cudaMemsetAsync(joint, 0, (size_t)total * sizeof(cplx), st));
+  CUDA_TRY(cudaMemsetAsync(live, 0, sizeof(int), st));
   if (nnz) {
     LaunchScope ls_("modal_scatter_kernel", st, 0.0);
-    modal_scatter_kernel<<<grid_for(nnz, T, 1024), T, 0, st>>>(d_idx, d_val, nnz, joint, W, M);
+    modal_scatter_kernel<<<grid_for(nnz, T, 1024), T, 0, st>>>(d_idx, d_val, nnz, joint, W, M, live);
   }
   LAUNCH_CHECK("modal_scatter_kernel");
   // joint fields: inverse along y and x (unnormalised), forward along the bins
   const long long step = (long long)(plane / sizeof(cplx));
   auto to_field = [&](const Fields& b) -> gl_status {
-    gl_status r = launch_sfft(sfft(b, ny, (long long)nx * M, 1, nx * M, 0, 1.0), 1, +1, st, tw);
+    gl_status r = launch_sfft(sfft(b, ny, (long long)nx * M, W, nx, M, 1.0, live), +1, st, tw);
     if (r != GL_OK) return r;
-    r = launch_sfft(sfft(b, nx, M, 1, M, (long long)nx * M, 1.0), ny, +1, st, tw);
+    r = launch_sfft(sfft(b, nx, M, W, ny, (long long)nx * M, 1.0, live), +1, st, tw);
     if (r != GL_OK) return r;
-    return axis_last_transform(b, (long long)ny * nx, M, -1, 1.0, st, tw);
+    return axis_last_transform(b, (long long)ny * nx, M, W, live, M, -1, 1.0, st, tw);
   };
   auto to_spectrum = [&](const Fields& b) -> gl_status {
-    gl_status r = axis_last_transform(b, (long long)ny * nx, M, +1, 1.0 / M, st, tw);
+    gl_status r = axis_last_transform(b, (long long)ny * nx, M, M, nullptr, M, +1, 1.0 / M, st, tw);
     if (r != GL_OK) return r;
-    r = launch_sfft(sfft(b, ny, (long long)nx * M, 1, nx * M, 0, 1.0), 1, -1, st, tw);
+    r = launch_sfft(sfft(b, ny, (long long)nx * M, M, nx, M, 1.0, nullptr), -1, st, tw);
     if (r != GL_OK) return r;
-    return launch_sfft(sfft(b, nx, M, 1, M, (long long)nx * M, 1.0 / ((double)nx * ny)), ny, -1, st, tw);
+    return launch_sfft(sfft(b, nx, M, M, ny, (long long)nx * M, 1.0 / ((double)nx * ny), nullptr), -1, st, tw);
   };
   {
     LaunchScope ls_("e20_bank_kernel", st, 0.0);
-    e20_bank_kernel<<<dim3(eb, 8), T, 0, st>>>(g, joint, buf(1), step);
+    e20_bank_kernel<<<dim3(eb, 8), T, 0, st>>>(g, joint, buf(1), step, live);
   }
   LAUNCH_CHECK("e20_bank_kernel");
   if ((s = to_field(Fields{buf(1), 8, step})) != GL_OK) return s;
@@ -4284,7 +4297,7 @@ extern "C" gl_status gl_eta20_level(const gl_eta20_desc* d, int nnz, const long 
   r.rank = d->rank;
   {
     LaunchScope ls_("e20_response_kernel", st, 0.0);
-    e20_response_kernel<<<W, 256, 0, st>>>(r);
+    e20_response_kernel<<<W, RESPONSE_THREADS, 0, st>>>(r);
   }
   LAUNCH_CHECK("e20_response_kernel");
   return GL_OK;

@@ -78,16 +78,18 @@ GL_D int mod_n(int m) {
   return r < 0 ? r + N : r;
 }
 
-template <int N>
+// BLOCK: the block's groups are interleaved over its threads and meet together.
+template <int N, bool BLOCK = false>
 GL_D void group_sync(int id) {
   constexpr int T = FftLen<N>::T;
-  if constexpr (T <= 32) __syncwarp();
+  if constexpr (BLOCK) __syncthreads();
+  else if constexpr (T <= 32) __syncwarp();
   else asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(T) : "memory");
 }
 
 // One Stockham pass of radix R over sub-transforms of NS points: LAST hands its
 // butterflies to sink(o, step, v, R) -- element r of v is output o + r * step.
-template <int SIGN, int N, int R, int NS, bool LAST, class Load, class Sink, class After>
+template <int SIGN, int N, int R, int NS, bool LAST, bool BLOCK, class Load, class Sink, class After>
 GL_D void pass_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__ tw, Load& load, Sink& sink,
                  After& after) {
   constexpr int T = FftLen<N>::T, B = 16 / R, stride = N / R;
@@ -99,7 +101,7 @@ GL_D void pass_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__
       for (int r = 0; r < 16; ++r) v[r] = load(t + r * stride, r);
       after(v);
     }
-    group_sync<N>(id);
+    group_sync<N, BLOCK>(id);
     if (active) {
       dft16<SIGN>(v);
       if constexpr (LAST) {
@@ -136,7 +138,7 @@ GL_D void pass_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__
 #pragma unroll
       for (int r = 0; r < 16; ++r) v[r] = p[r * (stride + stride / 16)];
     }
-    group_sync<N>(id);
+    group_sync<N, BLOCK>(id);
     if (active) {
       apply_twiddles<SIGN, 16>(v, k * twstep, tw);
       dft16<SIGN>(v);
@@ -145,7 +147,7 @@ GL_D void pass_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__
       for (int r = 0; r < 16; ++r) p[r * (NS + NS / 16)] = v[r];
     }
   }
-  if constexpr (!LAST) group_sync<N>(id);
+  if constexpr (!LAST) group_sync<N, BLOCK>(id);
 }
 
 // Full transform of one row by its group's T threads (thread t): inputs from
@@ -161,7 +163,7 @@ GL_D void pass_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__
 struct AsLoaded {
   GL_D void operator()(cplx*) const {}
 };
-template <int SIGN, int N, class Load, class Sink, class After = const AsLoaded>
+template <int SIGN, int N, bool BLOCK = false, class Load, class Sink, class After = const AsLoaded>
 GL_D void fft_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__ tw, Load& load, Sink& sink,
                 After& after = AsLoaded{}) {
   if constexpr (FftLen<N>::mixed) {
@@ -173,7 +175,7 @@ GL_D void fft_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__ 
         for (int r = 0; r < M; ++r) v[r] = load(t + 16 * r, r);
         after(v);
       }
-      group_sync<N>(id);
+      group_sync<N, BLOCK>(id);
       if (active) {
         dft_mixed<SIGN, M>(v);
         cplx* p = buf + t * MP;
@@ -181,7 +183,7 @@ GL_D void fft_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__ 
         for (int r = 0; r < M; ++r) p[r] = v[r];
       }
     }
-    group_sync<N>(id);
+    group_sync<N, BLOCK>(id);
     const bool act = active && t < M;
     cplx v[16];
     if (act) {
@@ -192,13 +194,13 @@ GL_D void fft_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__ 
       sink(t, M, v, 16);
     }
   } else {
-    pass_n<SIGN, N, 16, 1, N == 16>(buf, t, id, active, tw, load, sink, after);
+    pass_n<SIGN, N, 16, 1, N == 16, BLOCK>(buf, t, id, active, tw, load, sink, after);
     if constexpr (N >= 256) {
-      pass_n<SIGN, N, 16, 16, N == 256>(buf, t, id, active, tw, load, sink, after);
-      if constexpr (N == 4096) pass_n<SIGN, N, 16, 256, true>(buf, t, id, active, tw, load, sink, after);
-      else if constexpr (N > 256) pass_n<SIGN, N, N / 256, 256, true>(buf, t, id, active, tw, load, sink, after);
+      pass_n<SIGN, N, 16, 16, N == 256, BLOCK>(buf, t, id, active, tw, load, sink, after);
+      if constexpr (N == 4096) pass_n<SIGN, N, 16, 256, true, BLOCK>(buf, t, id, active, tw, load, sink, after);
+      else if constexpr (N > 256) pass_n<SIGN, N, N / 256, 256, true, BLOCK>(buf, t, id, active, tw, load, sink, after);
     } else if constexpr (N > 16) {
-      pass_n<SIGN, N, N / 16, 16, true>(buf, t, id, active, tw, load, sink, after);
+      pass_n<SIGN, N, N / 16, 16, true, BLOCK>(buf, t, id, active, tw, load, sink, after);
     }
   }
 }

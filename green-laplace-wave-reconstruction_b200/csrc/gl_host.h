@@ -24,6 +24,7 @@ namespace gl {
 struct SeedArgs;
 struct CmbArgs;
 struct SFft;
+struct LFft;
 
 // ---------------------------------------------------------------------------
 // errors: a thread-local message plus the returned status
@@ -144,7 +145,8 @@ gl_status launch_final_cols(const FinalCols& a, int ny, int nunits, cudaStream_t
 gl_status launch_out_rows(const OutArgs& a, int nunits, cudaStream_t st, const cplx* tw);
 gl_status launch_seed_rows(const SeedArgs& a, int nunits, cudaStream_t st, const cplx* tw);
 gl_status launch_combine(const CmbArgs& a, int njobs, cudaStream_t st, const cplx* tw);
-gl_status launch_sfft(const SFft& a, int outer, int sign, cudaStream_t st, const cplx* tw);
+gl_status launch_sfft(const SFft& a, int sign, cudaStream_t st, const cplx* tw);
+gl_status launch_lfft(const LFft& a, int sign, cudaStream_t st, const cplx* tw);
 // Final transforms of reference grids that are not powers of two (gl_gen.cuh).
 struct GenColArgs;
 struct GenRowArgs;

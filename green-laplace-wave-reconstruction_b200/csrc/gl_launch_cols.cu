@@ -33,15 +33,23 @@ void seed_rows_n(dim3 grid, int G, cudaStream_t st, const SeedArgs& a, const cpl
 }
 
 template <int N>
-void sfft_n(dim3 grid, int cw, int sign, cudaStream_t st, const SFft& a, const cplx* tw) {
-  const size_t smem = (size_t)cw * FftLen<N>::COL * sizeof(cplx);
-  if (sign > 0) {
-    ensure_smem_attr((const void*)strided_fft_kernel<+1, N>, (int)SMEM_LIMIT);
-    strided_fft_kernel<+1, N><<<grid, 256, smem, st>>>(a, tw, cw);
-  } else {
-    ensure_smem_attr((const void*)strided_fft_kernel<-1, N>, (int)SMEM_LIMIT);
-    strided_fft_kernel<-1, N><<<grid, 256, smem, st>>>(a, tw, cw);
-  }
+void sfft_n(int sign, cudaStream_t st, const SFft& a, const cplx* tw) {
+  using S = StridedLen<N>;
+  const size_t smem = (size_t)S::CW * S::L * sizeof(cplx);
+  dim3 grid((unsigned)(((long long)a.cols * a.groups + S::CW - 1) / S::CW), (unsigned)a.fields);
+  auto* k = sign > 0 ? strided_fft_kernel<+1, N> : strided_fft_kernel<-1, N>;
+  ensure_smem_attr((const void*)k, (int)SMEM_LIMIT);
+  k<<<grid, S::THREADS, smem, st>>>(a, tw);
+}
+
+template <int N>
+void lfft_n(int sign, cudaStream_t st, const LFft& a, const cplx* tw) {
+  constexpr int T = FftLen<N>::T, G = line_threads(T) / T;
+  const size_t smem = (size_t)G * FftLen<N>::COL * sizeof(cplx);
+  dim3 grid((unsigned)((a.rows + G - 1) / G), (unsigned)a.fields);
+  auto* k = sign > 0 ? line_fft_kernel<+1, N> : line_fft_kernel<-1, N>;
+  ensure_smem_attr((const void*)k, (int)SMEM_LIMIT);
+  k<<<grid, line_threads(T), smem, st>>>(a, tw);
 }
 
 }  // namespace
@@ -102,12 +110,18 @@ gl_status launch_seed_rows(const SeedArgs& a, int nunits, cudaStream_t st, const
   return GL_OK;
 }
 
-gl_status launch_sfft(const SFft& a, int outer, int sign, cudaStream_t st, const cplx* tw) {
-  const int cw = std::max(1, 256 / (a.n / 16));
-  dim3 grid((unsigned)((a.ncount + cw - 1) / cw), (unsigned)outer, (unsigned)a.fields);
-  LaunchScope ls("strided_fft_kernel", st, 2.0 * a.n * (double)a.ncount * outer * a.fields * sizeof(cplx));
-  switch (a.n) { GL_POW2_CASES(sfft_n, grid, cw, sign, st, a, tw) }
+gl_status launch_sfft(const SFft& a, int sign, cudaStream_t st, const cplx* tw) {
+  LaunchScope ls("strided_fft_kernel", st, 2.0 * a.n * (double)a.cols * a.groups * a.fields * sizeof(cplx));
+  switch (a.n) { GL_POW2_CASES(sfft_n, sign, st, a, tw) }
   LAUNCH_CHECK("strided_fft_kernel");
+  return GL_OK;
+}
+
+gl_status launch_lfft(const LFft& a, int sign, cudaStream_t st, const cplx* tw) {
+  LaunchScope ls("line_fft_kernel", st,
+                 (double)a.rows * a.fields * (std::min(a.live_max, a.n) + std::min(a.keep, a.n)) * sizeof(cplx));
+  switch (a.n) { GL_POW2_CASES(lfft_n, sign, st, a, tw) }
+  LAUNCH_CHECK("line_fft_kernel");
   return GL_OK;
 }
 

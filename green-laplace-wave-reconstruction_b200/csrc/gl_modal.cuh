@@ -21,62 +21,157 @@
 
 namespace gl {
 
+struct ModalGeo {
+  int P, M, W;           // q nodes, padded bins, work bins
+  double q_step;         // q-axis spacing
+  double fstep;          // dimensionless frequency of one bin
+  int b0;                // first retained bin
+};
+
+// A multiplier bank: src x q^p (or A = |q| tanh |q|) x the column's factor,
+// turned by 1, i or -i.
+enum ModalCol : int { MC_ONE = 0, MC_NU, MC_NU2, MC_OVER_NU, MC_INNER };  // MC_INNER: the (2 b0 + w) bin
+struct ModalBank {
+  const cplx* src;
+  signed char p;         // power of q; -1: A
+  signed char col;       // ModalCol
+  signed char turn;      // 0: 1, 1: i, -1: -i
+  bool neg;
+};
+constexpr int MODAL_BANKS = 13;
+
+// signed q of row j in numpy's ifftshift order
+GL_D double modal_q(const ModalGeo& g, int j) {
+  const int s = (j + g.P / 2) & (g.P - 1);
+  return (double)(s - g.P / 2) * g.q_step;
+}
+
+// Transforms along a strided axis: column w < cols of group `grp` starts at
+// grp * gpitch + w, its elements `stride` apart.
 struct SFft {
   cplx* data;
-  int n, log2n;          // transform length (16..4096)
+  int n;                 // transform length (16..4096)
   long long stride;      // element step inside one transform
-  long long cstride;     // step between consecutive transforms
-  int ncount;            // transforms per outer index
-  long long ostride;     // step between outer indices
+  int cols;              // columns per group
+  int groups;
+  long long gpitch;      // elements between groups
+  const int* live;       // non-null: columns *live and up hold zeros, and are left alone
   double scale;          // applied to the outputs
-  int tw_mode;           // 0 none; 1: output k of transform c times w^(k (c / tw_div));
-                         // 2: output k of outer index o times w^(k o)
-  long long tw_div;
-  int tw_log2p;          // w = e^{SIGN 2 pi i / 2^tw_log2p}
+  int tw_log2p;          // > 0: output k times w^(k grp), w = e^{SIGN 2 pi i / 2^tw_log2p}
   int fields;            // arrays transformed alike (grid z), fstride elements apart
   long long fstride;
+  int nbanks;            // > 0: field z is read from bank z
+  ModalBank bank[MODAL_BANKS];
+  ModalGeo geo;
+  int row_step;          // bank: element i of group grp is row i * row_step + grp
+};
+
+// One block: CW adjacent columns, a thread of each in turn, so a warp's loads
+// and stores take whole sectors (32 to 128 bytes of a row); both ends go
+// straight between global memory and registers, 16 loads of a thread in flight.
+// Staged element by element through shared memory, with divisions by the
+// column count, the 22 launches of a 1024-sample record took 1408 us (and the
+// multiplier banks 164 in kernels of their own); these and the
+// line transforms, banks included, take 622.
+template <int N>
+struct StridedLen {
+  static constexpr int T = FftLen<N>::T;
+  static constexpr int CW = T >= 128 ? 512 / T : (T >= 4 ? 8 : 32 / T);
+  static constexpr int THREADS = CW * T;
+  // columns offset so that eight consecutive lanes hit different banks
+  static constexpr int L = (N + N / 16 + 7) / 8 * 8 + (CW < 8 ? 8 / CW : 1);
 };
 
 template <int SIGN, int N>
-__global__ void __launch_bounds__(256, 2) strided_fft_kernel(SFft a, const cplx* __restrict__ tw, int cw) {
+__global__ void __launch_bounds__(StridedLen<N>::THREADS, StridedLen<N>::THREADS >= 512 ? 1 : 384 / StridedLen<N>::THREADS)
+    strided_fft_kernel(SFft a, const cplx* __restrict__ tw) {
   extern __shared__ cplx smem[];
-  const int o = blockIdx.y;
-  const int c0 = blockIdx.x * cw;
-  const int nc = min(cw, a.ncount - c0);
-  constexpr int n = N, T = FftLen<N>::T, L = FftLen<N>::COL;
-  cplx* base = a.data + blockIdx.z * a.fstride + (long long)o * a.ostride + (long long)c0 * a.cstride;
-  const bool colwise = a.cstride == 1;  // consecutive transforms adjacent in memory
-  for (int t = threadIdx.x; t < n * nc; t += blockDim.x) {
-    const int i = colwise ? t / nc : t % n;
-    const int c = colwise ? t % nc : t / n;
-    smem[(size_t)c * L + pos<N>(i)] = base[(long long)c * a.cstride + (long long)i * a.stride];
-  }
-  __syncthreads();
-  const int G = blockDim.x / T, g = threadIdx.x / T, tg = threadIdx.x % T;
-  for (int it = 0; it < nc; it += G) {
-    const int c = it + g;
-    const bool active = c < nc;
-    cplx* buf = smem + (size_t)(active ? c : 0) * L;
-    auto load = [&](int, int r) -> cplx { return buf[pos_in<N>(tg, r)]; };
-    auto sink = [&](int e, int step, const cplx* v, int cnt) { row_put<N>(buf, e, step, v, cnt); };
-    fft_n<SIGN, N>(buf, tg, 1 + g, active, tw, load, sink);
-  }
-  __syncthreads();
-  const long long pmask = (1LL << a.tw_log2p) - 1;
-  const double pinv = a.tw_mode ? 2.0 / (double)(1LL << a.tw_log2p) : 0.0;
-  for (int t = threadIdx.x; t < n * nc; t += blockDim.x) {
-    const int k = colwise ? t / nc : t % n;
-    const int c = colwise ? t % nc : t / n;
-    cplx v = cscale(a.scale, smem[(size_t)c * L + pos<N>(k)]);
-    if (a.tw_mode) {
-      const long long m = a.tw_mode == 1 ? (long long)(c0 + c) / a.tw_div : (long long)o;
-      const long long e = ((long long)k * m) & pmask;
-      double sn, cs;
-      sincospi((double)SIGN * pinv * (double)e, &sn, &cs);
-      v = cmul(v, cmk(cs, sn));
+  constexpr int T = FftLen<N>::T, CW = StridedLen<N>::CW;
+  const int c = threadIdx.x % CW, t = threadIdx.x / CW;
+  const int cc = blockIdx.x * CW + c;
+  const int grp = cc / a.cols, w = cc - grp * a.cols;
+  const bool active = grp < a.groups && (!a.live || w < *a.live);
+  if (!__syncthreads_or(active)) return;
+  const long long at = active ? grp * a.gpitch + w : 0;
+  cplx* data = a.data + blockIdx.y * a.fstride + at;
+  const cplx* src = a.nbanks ? a.bank[blockIdx.y].src + at : data;
+  auto load = [&](int i, int) -> cplx { return src[i * a.stride]; };
+  auto after = [&](cplx* v) {
+    if (!a.nbanks) return;
+    const ModalBank& b = a.bank[blockIdx.y];
+    const double nu = (a.geo.b0 + w) * a.geo.fstep;
+    const double g = b.col == MC_NU    ? nu
+                     : b.col == MC_NU2 ? nu * nu
+                     : b.col == MC_INNER ? (2 * a.geo.b0 + w) * a.geo.fstep
+                     : b.col == MC_OVER_NU ? (nu > 2.2250738585072014e-308 ? nu : 2.2250738585072014e-308) : 1.0;
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      const double q = modal_q(a.geo, (t + r * T) * a.row_step + grp), qa = fabs(q);
+      double f = b.p == 0 ? 1.0 : b.p == 1 ? q : b.p == 2 ? q * q : qa * tanh(qa);
+      f = b.col == MC_OVER_NU ? f / g : f * g;
+      if (b.neg) f = -f;
+      const cplx z = cscale(f, v[r]);
+      v[r] = b.turn == 0 ? z : b.turn > 0 ? cmuli(z) : cmulmi(z);
     }
-    base[(long long)c * a.cstride + (long long)k * a.stride] = v;
-  }
+  };
+  const long long pmask = (1LL << a.tw_log2p) - 1;
+  const double pinv = 2.0 / (double)(1LL << a.tw_log2p);
+  auto sink = [&](int o, int step, const cplx* v, int cnt) {
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      if (r >= cnt) continue;
+      const int k = o + r * step;
+      cplx z = cscale(a.scale, v[r]);
+      if (a.tw_log2p > 0) {
+        const long long e = ((long long)k * grp) & pmask;
+        double sn, cs;
+        sincospi((double)SIGN * pinv * (double)e, &sn, &cs);
+        z = cmul(z, cmk(cs, sn));
+      }
+      data[k * a.stride] = z;
+    }
+  };
+  fft_n<SIGN, N, true>(smem + c * StridedLen<N>::L, t, 1, active, tw, load, sink, after);
+}
+
+// Transforms along the contiguous axis of [rows][N], in place.
+struct LFft {
+  cplx* data;
+  int n;
+  long long rows;
+  const int* live;       // non-null: elements *live and up of a row are zero and are not read
+  int live_max;          // and so are elements live_max and up
+  int keep;              // outputs keep and up are not wanted
+  double scale;
+  int fields;
+  long long fstride;
+};
+
+constexpr int line_threads(int T) { return T > 64 ? 256 : 64; }
+
+template <int SIGN, int N>
+__global__ void __launch_bounds__(line_threads(FftLen<N>::T), FftLen<N>::T > 64 ? 2 : 6)
+    line_fft_kernel(LFft a, const cplx* __restrict__ tw) {
+  extern __shared__ cplx smem[];
+  constexpr int T = FftLen<N>::T, L = FftLen<N>::COL, G = line_threads(T) / T;
+  const int g = threadIdx.x / T, t = threadIdx.x % T;
+  const long long row = (long long)blockIdx.x * G + g;
+  const bool active = row < a.rows;
+  const int live = a.live ? min(*a.live, a.live_max) : a.live_max;
+  cplx* data = a.data + blockIdx.y * a.fstride + (active ? row : 0) * N;
+  auto load = [&](int i, int) -> cplx {
+    cplx v = czero();
+    if (i < live) v = data[i];
+    return v;
+  };
+  auto sink = [&](int o, int step, const cplx* v, int cnt) {
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      const int k = o + r * step;
+      if (r < cnt && k < a.keep) data[k] = cscale(a.scale, v[r]);
+    }
+  };
+  fft_n<SIGN, N>(smem + g * L, t, 1 + g, active, tw, load, sink);
 }
 
 // ---------------------------------------------------------------------------
@@ -85,87 +180,14 @@ __global__ void __launch_bounds__(256, 2) strided_fft_kernel(SFft a, const cplx*
 
 #ifndef GL_TRANSFORM_TU  // elementwise kernels: compiled by gl_engine.cu only
 // joint[row][col] = val for idx = row * W + col (distinct indices; the joint
-// [rows][M] is zeroed first by the caller).
+// [rows][M] and *live are zeroed first by the caller); *live becomes one past
+// the last column that holds a value.
 __global__ void modal_scatter_kernel(const long long* idx, const double* val, int nnz, cplx* joint,
-                                     int W, int M) {
+                                     int W, int M, int* live) {
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nnz; t += gridDim.x * blockDim.x) {
     const long long row = idx[t] / W, col = idx[t] % W;
     joint[row * M + col] = cmk(val[2 * t], val[2 * t + 1]);
-  }
-}
-
-enum ModalMult : int {
-  MM_ONE = 0, MM_NU, MM_NU2, MM_Q_SNU, MM_Q, MM_Q2_SNU,           // order-2 banks
-  MM_IQ, MM_MI_NU, MM_NU_Q, MM_MI_Q2_SNU, MM_MI_Q2_NU, MM_MINUS_NU2, MM_MINUS_Q2,  // first order
-  MM_PAIR_E, MM_PAIR_EX, MM_PAIR_PX, MM_PAIR_PZ, MM_PAIR_PZZ, MM_PAIR_PTZ,        // pair fields
-};
-
-struct ModalGeo {
-  int P, M, W;           // q nodes, padded bins, work bins
-  double q_step;         // q-axis spacing
-  double fstep;          // dimensionless frequency of one bin
-  int b0;                // first retained bin
-};
-
-// signed q of row j in numpy's ifftshift order
-GL_D double modal_q(const ModalGeo& g, int j) {
-  const int s = (j + g.P / 2) & (g.P - 1);
-  return (double)(s - g.P / 2) * g.q_step;
-}
-
-constexpr int MODAL_BANKS = 13;
-struct ModalBanks {
-  ModalGeo g;
-  const cplx* src[MODAL_BANKS];
-  int mult[MODAL_BANKS];
-  cplx* out;             // bank k at out + k * stride
-  long long stride;
-};
-
-// bank blockIdx.y: out = src * multiplier(row, column) (evaluation order of modal_time.py:240-246, 302-317)
-__global__ void modal_bank_kernel(ModalBanks a) {
-  const ModalGeo& g = a.g;
-  const long long total = (long long)g.P * g.M;
-  const cplx* src = a.src[blockIdx.y];
-  cplx* out = a.out + blockIdx.y * a.stride;
-  const int mult = a.mult[blockIdx.y];
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int j = (int)(t / g.M), w = (int)(t % g.M);
-    const cplx s = src[t];
-    const double q = modal_q(g, j);
-    const double nu = (g.b0 + w) * g.fstep;
-    const double snu = nu > 2.2250738585072014e-308 ? nu : 2.2250738585072014e-308;
-    const double qa = fabs(q);
-    cplx v;
-    switch (mult) {
-      case MM_ONE: v = s; break;
-      case MM_NU: v = cscale(nu, s); break;
-      case MM_NU2: v = cscale(nu * nu, s); break;
-      case MM_Q_SNU: v = cscale(q / snu, s); break;
-      case MM_Q: v = cscale(q, s); break;
-      case MM_Q2_SNU: v = cscale((q * q) / snu, s); break;
-      case MM_IQ: v = cmul(s, cmk(0.0, q)); break;
-      case MM_MI_NU: v = cmul(s, cmk(0.0, -nu)); break;
-      case MM_NU_Q: v = cscale(nu * q, s); break;
-      case MM_MI_Q2_SNU: v = cmul(s, cmk(0.0, -(q * q) / snu)); break;
-      case MM_MI_Q2_NU: v = cmul(s, cmk(0.0, -(q * q) * nu)); break;
-      case MM_MINUS_NU2: v = cscale(-(nu * nu), s); break;
-      case MM_MINUS_Q2: v = cscale(-(q * q), s); break;
-      // pair spectra: columns are the inner (2 b0 + w) bins, A = |q| tanh |q|
-      case MM_PAIR_E: v = s; break;
-      case MM_PAIR_EX: v = cmul(s, cmk(0.0, q)); break;
-      case MM_PAIR_PX: v = cmul(s, cmk(0.0, q)); break;
-      case MM_PAIR_PZ: v = cscale(qa * tanh(qa), s); break;
-      case MM_PAIR_PZZ: v = cscale(q * q, s); break;
-      case MM_PAIR_PTZ: {
-        const double inner = (2 * g.b0 + w) * g.fstep;
-        v = cscale(qa * tanh(qa), cmul(s, cmk(0.0, -inner)));
-        break;
-      }
-      default: v = czero();
-    }
-    out[t] = v;
+    atomicMax(live, (int)col + 1);
   }
 }
 
@@ -247,10 +269,14 @@ GL_D void modal_node_sums(double s, double ra, double scale, const double* nodes
   }
 }
 
+// A few hundred bins give about one block per SM, so a block takes as many
+// threads as its registers allow (256: 149 us a record, 512: 135).
+constexpr int RESPONSE_THREADS = 512;
+
 // One block per output work bin: the q-axis sum of the node responses,
 // reduced in a fixed order (modal_time.py:268-279, 339-351).
-__global__ void modal_response_kernel(ModalResp a) {
-  __shared__ double2 part[256];
+__global__ void __launch_bounds__(RESPONSE_THREADS) modal_response_kernel(ModalResp a) {
+  __shared__ double2 part[RESPONSE_THREADS];
   const int w = blockIdx.x;
   const double s = (double)(a.mult_b0 * a.g.b0 + w) * a.g.fstep;
   cplx acc = czero();
@@ -328,15 +354,18 @@ GL_D void e20_q(const E20Geo& g, int iy, int ix, double& qx, double& qy) {
 
 enum E20Mult : int { E20_ONE = 0, E20_NU2, E20_NU, E20_BX, E20_BY, E20_QX, E20_QY, E20_RAD };
 
-// bank blockIdx.y (an E20Mult) of the eight at out + blockIdx.y * stride
-__global__ void e20_bank_kernel(E20Geo g, const cplx* src, cplx* out0, long long stride) {
+// bank blockIdx.y (an E20Mult) of the eight at out + blockIdx.y * stride, of
+// the columns that hold values
+__global__ void e20_bank_kernel(E20Geo g, const cplx* src, cplx* out0, long long stride, const int* live) {
   const int mult = blockIdx.y;
   cplx* out = out0 + mult * stride;
-  const long long total = (long long)g.ny * g.nx * g.M;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int w = (int)(t % g.M);
-    const long long r = t / g.M;
+  const int cols = *live;
+  const long long total = (long long)g.ny * g.nx * cols;
+  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < total;
+       q += (long long)gridDim.x * blockDim.x) {
+    const long long r = q / cols;
+    const int w = (int)(q - r * cols);
+    const long long t = r * g.M + w;
     const int ix = (int)(r % g.nx), iy = (int)(r / g.nx);
     double qx, qy;
     e20_q(g, iy, ix, qx, qy);
@@ -401,8 +430,8 @@ struct E20Resp {
 
 // One block per signed bin: the grid sum of the eta20 node responses
 // (_eta20.py:120-143), reduced in a fixed order.
-__global__ void e20_response_kernel(E20Resp a) {
-  __shared__ double2 part[256];
+__global__ void __launch_bounds__(RESPONSE_THREADS) e20_response_kernel(E20Resp a) {
+  __shared__ double2 part[RESPONSE_THREADS];
   const int k = blockIdx.x;
   const int sb = k <= a.span ? k : k - (2 * a.span + 1);
   const int col = sb >= 0 ? sb : sb + a.g.M;  // padded-period index of the signed bin
