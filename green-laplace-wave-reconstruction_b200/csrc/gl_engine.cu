@@ -181,23 +181,27 @@ __global__ void factor_kernel(double* geo, Box box, int nfac) {
   }
 }
 
-// tw[m] = exp(-2 pi i m/TW_N) for m < TW_N; with count = TW_ALLOC also the
-// tables of the mixed lengths n = 16 m after it (W_n^e, e < n).
-__global__ void twiddle_kernel(cplx* tw, int count) {
-  for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < count; m += gridDim.x * blockDim.x) {
-    int n = TW_N, e = m;
-    if (m >= TW_N) {
-      const int lens[7] = {48, 80, 96, 144, 160, 192, 240};
-      for (int k = 0; k < 7; ++k) {
-        const int off = TW_N + mixed_tw_offset(lens[k]);
-        if (m >= off && m < off + lens[k]) {
-          n = lens[k];
-          e = m - off;
-        }
-      }
-    }
+// tw[m] = exp(-2 pi i m/TW_N), m < TW_N: the table of gl_fft2's transforms.
+__global__ void twiddle_kernel(cplx* tw) {
+  for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < TW_N; m += gridDim.x * blockDim.x) {
     double s, c;
-    sincospi(2.0 * (double)e / (double)n, &s, &c);
+    sincospi(2.0 * (double)m / (double)TW_N, &s, &c);
+    tw[m] = cmk(c, -s);
+  }
+}
+
+// The pass tables of every transform length (pass_tw_offset).
+__global__ void pass_twiddle_kernel(cplx* tw) {
+  const int lens[15] = {32, 64, 128, 256, 512, 1024, 2048, 4096, 48, 80, 96, 144, 160, 192, 240};
+  for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < PASS_TW; m += gridDim.x * blockDim.x) {
+    int i = 14;
+    while (pass_tw_offset(lens[i]) > m) --i;
+    const int len = lens[i], e = m - pass_tw_offset(len);
+    const int ns = mixed_len(len) ? len / 16 : (len <= 256 ? 16 : 256), R = len / ns;
+    const int j = e / ns, k = e % ns;
+    const int power = R == 4 ? j + 1 : 1 << j;
+    double s, c;
+    sincospi(2.0 * (double)(power * k) / (double)len, &s, &c);
     tw[m] = cmk(c, -s);
   }
 }
@@ -1056,9 +1060,9 @@ extern "C" gl_status gl_plan_create(gl_plan** out, const gl_plan_desc* desc) {
   geo_alloc(&p->geo1, p->b1, o3 ? F_Q2NU + 1 : (o2 ? F_NU2 + 1 : 0));
   geo_alloc(&p->geo2, p->b2, o3 ? F_QY + 1 : 0);
   geo_alloc(&p->geo3, p->b3, 0);
-  if (e == cudaSuccess) e = cudaMalloc(&p->tw, sizeof(cplx) * TW_ALLOC);
+  if (e == cudaSuccess) e = cudaMalloc(&p->tw, sizeof(cplx) * PASS_TW);
   if (e == cudaSuccess) {
-    twiddle_kernel<<<TW_ALLOC / 256 + 1, 256>>>(p->tw, TW_ALLOC);
+    pass_twiddle_kernel<<<PASS_TW / 256 + 1, 256>>>(p->tw);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMalloc(&p->nodes, sizeof(double) * 8 * MAX_RANK);
@@ -2323,9 +2327,9 @@ extern "C" gl_status gl_eta44_plan_create(gl_plan** out, const gl_eta44_desc* de
   geo_alloc(&p->geo2, p->b2, F_Q2A + 1);
   geo_alloc(&p->geo3, p->b3, F_QY + 1);
   geo_alloc(&p->geo4, p->b4, 0);
-  if (err == cudaSuccess) err = cudaMalloc(&p->tw, sizeof(cplx) * TW_ALLOC);
+  if (err == cudaSuccess) err = cudaMalloc(&p->tw, sizeof(cplx) * PASS_TW);
   if (err == cudaSuccess) {
-    twiddle_kernel<<<TW_ALLOC / 256 + 1, 256>>>(p->tw, TW_ALLOC);
+    pass_twiddle_kernel<<<PASS_TW / 256 + 1, 256>>>(p->tw);
     err = cudaGetLastError();
   }
   if (err == cudaSuccess) err = cudaMalloc(&p->nodes, sizeof(double) * 2 * MAX_RANK);
@@ -3839,14 +3843,16 @@ __global__ void fft2_cols_kernel(cplx* data, int nx, int ny, int log2ny, int cw,
 
 static cplx* g_tw_global[64] = {nullptr};
 
+// The device's tables: TW_N entries for gl_fft2, then the pass tables.
 static gl_status device_twiddles(cplx** out) {
   int dev = 0;
   CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return fail(GL_ERR_CUDA, "device index out of range");
   if (!g_tw_global[dev]) {
     cplx* tw = nullptr;
-    CUDA_TRY(cudaMalloc(&tw, sizeof(cplx) * TW_N));
-    twiddle_kernel<<<TW_N / 256, 256>>>(tw, TW_N);
+    CUDA_TRY(cudaMalloc(&tw, sizeof(cplx) * (TW_N + PASS_TW)));
+    twiddle_kernel<<<TW_N / 256, 256>>>(tw);
+    pass_twiddle_kernel<<<PASS_TW / 256 + 1, 256>>>(tw + TW_N);
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaDeviceSynchronize());
     g_tw_global[dev] = tw;
@@ -4007,6 +4013,7 @@ extern "C" gl_status gl_modal_level(const gl_modal_desc* d, int nnz, const long 
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   cplx* tw = nullptr;
   if ((s = device_twiddles(&tw)) != GL_OK) return s;
+  tw += TW_N;  // the pass tables
   const int P = d->points, W = d->width, M = modal_pad(W);
   const int wmax = (W - 1) / d->order;
   const long long total = (long long)P * M;
@@ -4212,6 +4219,7 @@ extern "C" gl_status gl_eta20_level(const gl_eta20_desc* d, int nnz, const long 
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   cplx* tw = nullptr;
   if ((s = device_twiddles(&tw)) != GL_OK) return s;
+  tw += TW_N;  // the pass tables
   const int W = 2 * d->span + 1, M = modal_pad(W), nx = d->nx, ny = d->ny;
   const long long total = (long long)ny * nx * M;
   const size_t plane = align_up((size_t)total * sizeof(cplx));
@@ -4350,7 +4358,7 @@ static gl_status noalloc_scratch(cudaStream_t st, unsigned char** out) {
     if (e != cudaSuccess || !ptr)
       return fail(GL_ERR_CUDA, "cudaGetSymbolAddress of the no-alloc scratch failed: %s",
                   cudaGetErrorString(e));
-    twiddle_kernel<<<TW_N / 256, 256, 0, st>>>(reinterpret_cast<cplx*>(ptr), TW_N);
+    pass_twiddle_kernel<<<PASS_TW / 256 + 1, 256, 0, st>>>(reinterpret_cast<cplx*>(ptr));
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaStreamSynchronize(st));
     g_noalloc_base[dev] = reinterpret_cast<unsigned char*>(ptr);
@@ -4370,6 +4378,7 @@ extern "C" gl_status gl_box_synthesize_noalloc(int n_units, int nx, int ny, int 
   if (box_w > nx || box_h > ny || std::abs(box_x0) >= nx || std::abs(box_y0) >= ny ||
       std::abs(box_x0 + box_w - 1) >= nx || std::abs(box_y0 + box_h - 1) >= ny)
     return fail(GL_ERR_INVALID_ARGUMENT, "box does not fit the grid");
+  static_assert(PASS_TW <= TW_N, "the static array's head");
   const size_t tw_bytes = align_up(sizeof(cplx) * TW_N);
   const size_t geo_bytes = align_up(sizeof(double) * 6 * (size_t)box_w * box_h);
   const size_t mid_bytes = align_up(sizeof(cplx) * (size_t)n_units * box_w * ny);

@@ -93,7 +93,7 @@ template <int SIGN, int N, int R, int NS, bool LAST, bool BLOCK, class Load, cla
 GL_D void pass_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__ tw, Load& load, Sink& sink,
                  After& after) {
   constexpr int T = FftLen<N>::T, B = 16 / R, stride = N / R;
-  constexpr int twstep = TW_N / (NS * R);
+  constexpr int tab = pass_tw_offset(NS * R);
   if constexpr (NS == 1) {
     cplx v[16];
     if (active) {
@@ -125,7 +125,7 @@ GL_D void pass_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__
 #pragma unroll
         for (int r = 0; r < R; ++r) v[r] = p[r * (NS + NS / 16)];
         const int j = t + T * b;
-        apply_twiddles<SIGN, R>(v, j * twstep, tw);
+        apply_twiddles<SIGN, R, NS>(v, j, tw + tab);
         dftR<SIGN, R>(v);
         sink(j, NS, v, R);
       }
@@ -140,7 +140,7 @@ GL_D void pass_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__
     }
     group_sync<N, BLOCK>(id);
     if (active) {
-      apply_twiddles<SIGN, 16>(v, k * twstep, tw);
+      apply_twiddles<SIGN, 16, NS>(v, k, tw + tab);
       dft16<SIGN>(v);
       cplx* p = buf + o + (o >> 4);
 #pragma unroll
@@ -189,7 +189,7 @@ GL_D void fft_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__ 
     if (act) {
 #pragma unroll
       for (int r = 0; r < 16; ++r) v[r] = buf[t + MP * r];
-      if (t > 0) apply_twiddles<SIGN, 16>(v, t, tw + TW_N + mixed_tw_offset(N));
+      if (t > 0) apply_twiddles<SIGN, 16, M>(v, t, tw + pass_tw_offset(N));
       dft16<SIGN>(v);
       sink(t, M, v, 16);
     }

