@@ -150,6 +150,42 @@ GL_D void pass_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__
   if constexpr (!LAST) group_sync<N, BLOCK>(id);
 }
 
+struct AsLoaded {
+  GL_D void operator()(cplx*) const {}
+};
+
+// The two passes of a mixed length 16 M: a butterfly of M points by each of a
+// group's 16 threads, then M butterflies of 16 points (t < M; `active` ones).
+template <int SIGN, int N, bool BLOCK, class Load, class After>
+GL_D void mixed_first(cplx* buf, int t, int id, bool active, Load& load, After& after) {
+  constexpr int M = FftLen<N>::M, MP = FftLen<N>::MP;
+  cplx v[M];
+  if (active) {
+#pragma unroll
+    for (int r = 0; r < M; ++r) v[r] = load(t + 16 * r, r);
+    after(v);
+  }
+  group_sync<N, BLOCK>(id);
+  if (active) {
+    dft_mixed<SIGN, M>(v);
+    cplx* p = buf + t * MP;
+#pragma unroll
+    for (int r = 0; r < M; ++r) p[r] = v[r];
+  }
+}
+
+template <int SIGN, int N, class Sink>
+GL_D void mixed_last(const cplx* buf, int t, bool active, const cplx* __restrict__ tw, Sink& sink) {
+  constexpr int M = FftLen<N>::M, MP = FftLen<N>::MP;
+  if (!active) return;
+  cplx v[16];
+#pragma unroll
+  for (int r = 0; r < 16; ++r) v[r] = buf[t + MP * r];
+  if (t > 0) apply_twiddles<SIGN, 16, M>(v, t, tw + pass_tw_offset(N));
+  dft16<SIGN>(v);
+  sink(t, M, v, 16);
+}
+
 // Full transform of one row by its group's T threads (thread t): inputs from
 // load(i, r) (element i, the thread's r-th), outputs to sink(o, step, v, count) (elements o + r * step); the
 // passes between them go through the padded row `buf`.  Every thread of the
@@ -160,39 +196,13 @@ GL_D void pass_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__
 // thread's inputs once all of them are on their way (a branch inside load would
 // wait for each before the next is asked for).  Other lanes may
 // still be reading `buf` when a thread returns.
-struct AsLoaded {
-  GL_D void operator()(cplx*) const {}
-};
 template <int SIGN, int N, bool BLOCK = false, class Load, class Sink, class After = const AsLoaded>
 GL_D void fft_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__ tw, Load& load, Sink& sink,
                 After& after = AsLoaded{}) {
   if constexpr (FftLen<N>::mixed) {
-    constexpr int M = FftLen<N>::M, MP = FftLen<N>::MP;
-    {
-      cplx v[M];
-      if (active) {
-#pragma unroll
-        for (int r = 0; r < M; ++r) v[r] = load(t + 16 * r, r);
-        after(v);
-      }
-      group_sync<N, BLOCK>(id);
-      if (active) {
-        dft_mixed<SIGN, M>(v);
-        cplx* p = buf + t * MP;
-#pragma unroll
-        for (int r = 0; r < M; ++r) p[r] = v[r];
-      }
-    }
+    mixed_first<SIGN, N, BLOCK>(buf, t, id, active, load, after);
     group_sync<N, BLOCK>(id);
-    const bool act = active && t < M;
-    cplx v[16];
-    if (act) {
-#pragma unroll
-      for (int r = 0; r < 16; ++r) v[r] = buf[t + MP * r];
-      if (t > 0) apply_twiddles<SIGN, 16, M>(v, t, tw + pass_tw_offset(N));
-      dft16<SIGN>(v);
-      sink(t, M, v, 16);
-    }
+    mixed_last<SIGN, N>(buf, t, active && t < FftLen<N>::M, tw, sink);
   } else {
     pass_n<SIGN, N, 16, 1, N == 16, BLOCK>(buf, t, id, active, tw, load, sink, after);
     if constexpr (N >= 256) {

@@ -951,7 +951,36 @@ __global__ void __launch_bounds__(ROW_THREADS, 2) row_kernel_t(RowArgs a, const 
       }
       row_put<N>(buf, o, step, v, cnt);
     };
-    fft_n<+1, N>(buf, t, 1 + g, active, tw, load, sink);
+    if constexpr (FftLen<N>::mixed) {
+      constexpr AsLoaded none;
+      mixed_first<+1, N, false>(buf, t, 1 + g, active, load, none);
+    } else {
+      fft_n<+1, N>(buf, t, 1 + g, active, tw, load, sink);
+    }
+  }
+  if constexpr (FftLen<N>::mixed) {
+    // The second pass has M butterflies a row, fewer than a group's threads:
+    // they are dealt to the block's threads without regard to groups (160
+    // points: 12 banks in two rounds of 64 threads for three of 40;
+    // the inner rows of 16 records 414 -> 404 us, of one 512 grid 31 -> 25).
+    constexpr int M = FftLen<N>::M;
+    __syncthreads();
+    for (int q = threadIdx.x; q < nb * M; q += blockDim.x) {
+      const int k = q / M;
+      cplx* buf = banks + (size_t)k * L;
+      int gi = 0;
+      if (FAMILY == 1)
+        for (int kk = k; kk >= a.grp[gi].nb; ++gi) kk -= a.grp[gi].nb;
+      const bool cj = FAMILY == 1 && a.grp[gi].conj != 0;
+      auto sink = [&](int o, int step, cplx* v, int cnt) {
+        if (FAMILY == 1 && cj) {
+#pragma unroll
+          for (int r = 0; r < 16; ++r) v[r] = cconj(v[r]);
+        }
+        row_put<N>(buf, o, step, v, cnt);
+      };
+      mixed_last<+1, N>(buf, q - k * M, true, tw, sink);
+    }
   }
   __syncthreads();
   if (row_ok) {
@@ -967,30 +996,53 @@ __global__ void __launch_bounds__(ROW_THREADS, 2) row_kernel_t(RowArgs a, const 
   __syncthreads();
   const int na = a.nout_a > 0 ? a.nout_a : a.nout;
   const bool oc = FAMILY == 1 && a.out_conj != 0;
+  // output o of the row: where its kept columns start, and how many
+  struct Out {
+    cplx* row;
+    int x0, w;
+  };
+  auto output = [&](int o) -> Out {
+    const bool second = o >= na;
+    const int w = second ? a.out2_w : a.out_w;
+    const int yr = row_ok ? y : 0;
+    return {second ? a.out2 + (((size_t)job * (a.nout - na) + (o - na)) * a.ny + yr) * w
+                   : a.out + (((size_t)job * na + o) * a.ny + yr) * w,
+            mod_n<N>(second ? a.out2_x0 : a.out_x0), w};
+  };
+  auto store = [&](const Out& out, int e, int step, const cplx* v, int cnt) {
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      if (r >= cnt) continue;
+      const int xo = wrap_n<N>(e + r * step - out.x0);
+      if (xo < out.w) out.row[xo] = oc ? cconj(v[r]) : v[r];
+    }
+  };
   for (int it = 0; it < a.nout; it += G) {
     const int o = it + g;
     const bool active = o < a.nout && row_ok;
-    const int oo = active ? o : 0;
-    cplx* buf = banks + (size_t)oo * L;
-    const bool second = oo >= na;
-    const int ox0 = mod_n<N>(second ? a.out2_x0 : a.out_x0);
-    const int ow = second ? a.out2_w : a.out_w;
-    const int yr = row_ok ? y : 0;
-    cplx* orow = second ? a.out2 + (((size_t)job * (a.nout - na) + (oo - na)) * a.ny + yr) * ow
-                        : a.out + (((size_t)job * na + oo) * a.ny + yr) * ow;
+    cplx* buf = banks + (size_t)(active ? o : 0) * L;
     auto load = [&](int, int r) -> cplx {
       const cplx v = buf[pos_in<N>(t, r)];
       return oc ? cconj(v) : v;
     };
-    auto sink = [&](int e, int step, cplx* v, int cnt) {
-#pragma unroll
-      for (int r = 0; r < 16; ++r) {
-        if (r >= cnt) continue;
-        const int xo = wrap_n<N>(e + r * step - ox0);
-        if (xo < ow) orow[xo] = oc ? cconj(v[r]) : v[r];
-      }
-    };
-    fft_n<-1, N>(buf, t, 1 + g, active, tw, load, sink);
+    if constexpr (FftLen<N>::mixed) {
+      constexpr AsLoaded none;
+      mixed_first<-1, N, false>(buf, t, 1 + g, active, load, none);
+    } else {
+      const Out out = output(active ? o : 0);
+      auto sink = [&](int e, int step, const cplx* v, int cnt) { store(out, e, step, v, cnt); };
+      fft_n<-1, N>(buf, t, 1 + g, active, tw, load, sink);
+    }
+  }
+  if constexpr (FftLen<N>::mixed) {
+    constexpr int M = FftLen<N>::M;
+    __syncthreads();
+    for (int q = threadIdx.x; q < a.nout * M; q += blockDim.x) {
+      const int o = q / M;
+      const Out out = output(o);
+      auto sink = [&](int e, int step, const cplx* v, int cnt) { store(out, e, step, v, cnt); };
+      mixed_last<-1, N>(banks + (size_t)o * L, q - o * M, true, tw, sink);
+    }
   }
 }
 
