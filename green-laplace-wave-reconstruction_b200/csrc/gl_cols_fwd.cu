@@ -9,16 +9,20 @@ namespace gl {
 namespace {
 
 template <int N>
-void col_fft_n(int cw, int njs, cudaStream_t st, const ColFftArgs& a, const cplx* tw) {
-  constexpr int T = FftLen<N>::T;
-  int threads = 256;
-  if constexpr (T <= 16) {  // a group per column: blocks of whole warps
-    threads = std::min(COL_THREADS, std::max(32, cw * T));
-    cw = threads / T;
-  }
+void col_fft_n(int cw_max, int njs, cudaStream_t st, const ColFftArgs& a, const cplx* tw) {
+  constexpr bool tile = FftLen<N>::T <= 16;
+  constexpr int L = tile ? ColTile<N>::L : FftLen<N>::COL;
+  int cw = tile ? ColTile<N>::C : 256 / FftLen<N>::T;
+  cw = std::min(cw, FftLen<N>::mixed ? a.box.w : next_pow2(a.box.w));
+  if (cw_max > 0) cw = std::min(cw, cw_max);
+  // a launch that leaves SMs idle takes fewer columns per block: its passes
+  // spread over more SMs
+  else
+    while (cw > 2 && (long long)((a.box.w + cw / 2 - 1) / (cw / 2)) * njs <= 2 * SM_COUNT) cw /= 2;
+  const int threads = tile ? TILE_THREADS : 256;
   dim3 grid((a.box.w + cw - 1) / cw, njs);
   ensure_smem_attr((const void*)col_fft_kernel<N>, (int)SMEM_LIMIT);
-  col_fft_kernel<N><<<grid, threads, (size_t)cw * FftLen<N>::COL * sizeof(cplx), st>>>(a, tw, cw);
+  col_fft_kernel<N><<<grid, threads, (size_t)cw * L * sizeof(cplx), st>>>(a, tw, cw);
 }
 
 template <int N>
@@ -31,15 +35,9 @@ void combine_n(dim3 grid, int cw, cudaStream_t st, const CmbArgs& a, const cplx*
 
 gl_status launch_col_fft(const ColFftArgs& a, int njs, cudaStream_t st, const cplx* tw, const char* name) {
   if (!is_pow2(a.n) && !mixed_len(a.n)) return fail(GL_ERR_UNSUPPORTED, "column length %d has no transform", a.n);
-  int cw = fft_cols_per_block(a.n, a.box.w);
-  if (a.cw_max > 0) cw = std::min(a.cw_max, cw);
-  // a launch that leaves SMs idle takes fewer columns per block: the staging
-  // and write-back loops shorten and the transforms spread over more SMs
-  else
-    while (cw > 2 && (long long)((a.box.w + cw / 2 - 1) / (cw / 2)) * njs <= 2 * SM_COUNT) cw /= 2;
   const double bytes = (double)njs * a.box.w * (a.n + a.box.h) * sizeof(cplx);
   LaunchScope ls(name, st, bytes);
-  GL_LEN_DISPATCH(a.n, col_fft_n, cw, njs, st, a, tw);
+  GL_LEN_DISPATCH(a.n, col_fft_n, a.cw_max, njs, st, a, tw);
   LAUNCH_CHECK("col_fft_kernel");
   return GL_OK;
 }

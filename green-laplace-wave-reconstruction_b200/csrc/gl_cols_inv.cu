@@ -31,6 +31,29 @@ const char* col_ifft_name(int kind) {
   return "col_ifft_kernel";
 }
 
+// What a launch needs to know of a length's transforms.
+struct ColShape {
+  bool tile;         // tiles of adjacent columns (at most 16 threads a transform)
+  int columns, row;  // columns a block can take, elements of a column's row
+  int m;             // second-pass butterflies of a mixed length, 0: a power of two
+  int pad;
+  int pitch(int len) const { return (len + 7) / 8 * 8 + pad; }
+};
+template <int N>
+void col_shape_n(ColShape& s) {
+  using F = FftLen<N>;
+  s.tile = F::T <= 16;
+  s.columns = s.tile ? ColTile<N>::C : 256 / F::T;
+  s.row = s.tile ? ColTile<N>::L : F::COL;
+  s.m = F::M;
+  s.pad = ColTile<N>::PAD;
+}
+ColShape col_shape(int n) {
+  ColShape s{};
+  GL_LEN_DISPATCH(n, col_shape_n, s);
+  return s;
+}
+
 // A multiplier as rot(f s): its factor plane and rotation.
 void factor_of(int mult, signed char& fac, unsigned char& rot) {
   constexpr int I = ROT_SWAP | ROT_NEG_RE, MI = ROT_SWAP | ROT_NEG_IM, NEG = ROT_NEG_RE | ROT_NEG_IM;
@@ -78,42 +101,42 @@ gl_status launch_col_ifft(const ColArgs& a0, int njobs, cudaStream_t st, const c
   ColArgs a = a0;
   if (!is_pow2(a.n) && !mixed_len(a.n)) return fail(GL_ERR_UNSUPPORTED, "column length %d has no transform", a.n);
   for (int k = 0; k < a.nbanks; ++k) factor_of(a.mult[k], a.fac[k], a.rot[k]);
-  const int T = is_pow2(a.n) ? a.n / 16 : 16;
-  const bool direct = T <= 16;
-  const int threads = direct ? COL_THREADS : 256;
-  const int G = threads / T;
+  const ColShape F = col_shape(a.n);
+  const int threads = F.tile ? TILE_THREADS : 256;
   // the damped base spectrum of the block's columns is formed only for the
   // kinds that share one base across their banks (col_ifft_kernel)
   const bool shared_base = a.kind != COL_PLAIN && a.kind != COL_OUTER2 && a.kind != COL_FLOORED;
-  const int hp = a.box.h | 1, w = a.box.w;
+  bool divides = false;
+  for (int k = 0; k < a.nbanks; ++k) divides |= a.fac[k] == F_DIRECT;
+  const int w = a.box.w, hp = F.tile ? F.pitch(a.box.h) : a.box.h | 1;
   auto smem_of = [&](int cw) {
-    return ((size_t)G * columns_row_len(a.n) + (shared_base ? (size_t)cw * hp : 0)) * sizeof(cplx);
+    const size_t rows = (size_t)(F.tile ? cw : F.columns) * F.row;
+    return (rows + (size_t)cw * hp * ((shared_base ? 1 : 0) + (F.tile && divides ? 1 : 0))) * sizeof(cplx);
   };
   // Columns per block and banks per block by a small cost model, in units of
-  // one transform round of a block's G groups: a block costs its rounds, the
-  // damped base (about a third of a round per element and thread) and half a
-  // round of prologue; blocks run in waves of the resident ones.  Splitting the
-  // banks repeats the base but fills the GPU when a launch has few columns and
-  // jobs, and trims the last wave of large ones.  Of short transforms a block
-  // takes two columns, which fill a sector; more only lengthen the base's
-  // prologue (64-point order-4 banks 331 us with 2 columns, 364 with 16).
-  const int cw_top = std::min(direct ? (a.cw_max > 0 ? G : 2) : G, next_pow2(w));
+  // one transform of a block: a block costs its banks, the damped base (about
+  // a third of a transform per element and thread) and half a transform of
+  // prologue; blocks run in waves of the resident ones.  Splitting the banks
+  // repeats the base but fills the GPU when a launch has few columns and jobs,
+  // and trims the last wave of large ones.
+  const int cw_top = std::min(F.columns, F.m ? w : next_pow2(w));
   int best_cw = cw_top, best_bpb = a.nbanks;
   double best = 1e30;
   for (int cw = a.cw_max > 0 ? std::min(a.cw_max, cw_top) : cw_top; cw >= 1; cw /= 2) {
     const size_t sm = smem_of(cw);
     if (sm > SMEM_LIMIT) continue;
-    const size_t resident = std::min<size_t>(direct ? 6 : 2, (SMEM_LIMIT + 1024) / (sm + 1024));
+    const size_t resident = std::min<size_t>(F.tile ? 6 : 2, (SMEM_LIMIT + 1024) / (sm + 1024));
     const double slots = (double)SM_COUNT * std::max<size_t>(1, resident);
+    // a mixed length's passes cover the block's threads one by one
+    const double round = F.m ? 0.3 * ((16 * cw + threads - 1) / threads) + 0.7 * ((F.m * cw + threads - 1) / threads)
+                             : 1.0;
     for (int nz = 1; nz <= a.nbanks; ++nz) {
       const int bpb = (a.nbanks + nz - 1) / nz;
       const double blocks = (double)((w + cw - 1) / cw) * njobs * ((a.nbanks + bpb - 1) / bpb);
-      const int cols = std::min(cw, w);
-      const int rounds = direct ? (bpb * cols + G - 1) / G : bpb;
       const int base_iters = shared_base ? (cw * a.box.h + threads - 1) / threads : 0;
       const double q = blocks / slots;
       const double waves = q <= 4.0 ? std::ceil(q) : q + 0.5;
-      const double cost = waves * (0.5 + 0.35 * base_iters + rounds) * (blocks <= SM_COUNT ? 0.7 : 1.0);
+      const double cost = waves * (0.5 + 0.35 * base_iters + bpb * round) * (blocks <= SM_COUNT ? 0.7 : 1.0);
       if (cost < best - 1e-9) {
         best = cost;
         best_cw = cw;

@@ -215,6 +215,58 @@ GL_D void fft_n(cplx* buf, int t, int id, bool active, const cplx* __restrict__ 
   }
 }
 
+// A tile of adjacent columns transformed together, interleaved over the block's
+// threads (column fastest), so that a warp's global accesses run along whole
+// stretches of a row.  A mixed length takes as many columns as its M second-pass
+// butterflies fill TILE_THREADS threads; a power of two one column per group.
+constexpr int TILE_THREADS = 64;
+template <int N>
+struct ColTile {
+  static constexpr bool mixed = FftLen<N>::mixed;
+  static constexpr int C = mixed ? TILE_THREADS / FftLen<N>::M
+                                 : (FftLen<N>::T < TILE_THREADS ? TILE_THREADS / FftLen<N>::T : 1);
+  // column pitch: eight consecutive lanes hit different banks
+  static constexpr int PAD = !mixed && C < 8 ? 8 / C : 1;
+  static constexpr int pitch(int len) { return (len + 7) / 8 * 8 + PAD; }
+  static constexpr int L = pitch(FftLen<N>::ROW);
+};
+
+// Transforms of columns 0 .. C - 1 of a tile (`buf`: C rows, ColTile<N>::L
+// apart) by all of the block's threads: load(c, y, r), after(c, t, v) and
+// sink(c, o, step, v, count) as for fft_n.  C is a power of two for those lengths.
+// `buf` may still be read when a thread returns.
+template <int SIGN, int N, class Load, class After, class Sink>
+GL_D void fft_tile(cplx* buf, int C, const cplx* __restrict__ tw, Load& load, After& after, Sink& sink) {
+  if constexpr (FftLen<N>::mixed) {
+    constexpr int M = FftLen<N>::M, MP = FftLen<N>::MP, L = ColTile<N>::L;
+    const int rc = (65536 + C - 1) / C;  // q / C = q rc >> 16 for q < 1024
+    __syncthreads();
+    for (int q = threadIdx.x; q < 16 * C; q += TILE_THREADS) {
+      const int t = q * rc >> 16, c = q - t * C;
+      cplx v[M];
+#pragma unroll
+      for (int r = 0; r < M; ++r) v[r] = load(c, t + 16 * r, r);
+      after(c, t, v);
+      dft_mixed<SIGN, M>(v);
+      cplx* p = buf + c * L + t * MP;
+#pragma unroll
+      for (int r = 0; r < M; ++r) p[r] = v[r];
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < M * C; q += TILE_THREADS) {
+      const int t = q * rc >> 16, c = q - t * C;
+      auto out = [&](int o, int step, cplx* v, int cnt) { sink(c, o, step, v, cnt); };
+      mixed_last<SIGN, N>(buf + c * L, t, true, tw, out);
+    }
+  } else {
+    const int c = threadIdx.x & (C - 1), t = threadIdx.x >> (31 - __clz(C));
+    auto in = [&](int y, int r) { return load(c, y, r); };
+    auto change = [&](cplx* v) { after(c, t, v); };
+    auto out = [&](int o, int step, cplx* v, int cnt) { sink(c, o, step, v, cnt); };
+    fft_n<SIGN, N, true>(buf + c * ColTile<N>::L, t, 1, t < FftLen<N>::T, tw, in, out, change);
+  }
+}
+
 // Sink that writes a pass's outputs back to a padded row.
 template <int N>
 GL_D void row_put(cplx* buf, int o, int step, const cplx* v, int cnt) {

@@ -124,12 +124,6 @@ inline int grid_for(size_t n, int threads, int cap = 4096) {
   return (int)b;
 }
 
-inline int fft_cols_per_block(int n, int w) {
-  const int T = is_pow2(n) ? n / 16 : 16;  // threads per column transform
-  // a power of two (the kernels split thread indices with shifts)
-  return std::max(1, std::min(256 / T, next_pow2(w)));
-}
-
 // SMs of a B200 (launch shapes weigh their waves against it).
 constexpr int SM_COUNT = 148;
 

@@ -304,27 +304,23 @@ constexpr int GEO_PLANES = 6;
 constexpr int ROT_SWAP = 1, ROT_NEG_RE = 2, ROT_NEG_IM = 4;
 
 // One block: box columns x_first .. x_first + cw - 1 of one job and a slice
-// of its banks.  The damped base spectrum of the columns is computed once into
-// shared memory (column-major); each (bank, column) is then one length-N
-// inverse transform along y by a group of T threads, whose first pass reads
+// of its banks, one bank after another.  The damped base spectrum of the
+// columns is computed once into shared memory (column-major); each column is
+// then one length-N inverse transform along y, whose first pass reads
 // base x factor straight into registers -- sixteen independent loads, no
 // staging pass, and no branch among them: a floor test inside the load waited
-// for each value before asking for the next (outer banks of 16 records of a
-// 1024 grid, 9 of 240 points from 4 spectra: 281 us, now 173; the 12 damped
-// ones 159, now 124; inner banks of 144 points 293, now 243).  Items are dealt to the groups column-fastest, so no group
-// idles when a block has few columns.  Transforms of at most 16 threads need no
-// block barrier between items and write their last pass straight to global
-// memory (two adjacent columns of a warp fill each 32-byte sector); longer ones
-// go back row-major through shared memory, one bank at a time.
+// for each value before asking for the next (16 records of a 1024 grid, outer
+// banks, 9 of 240 points from 4 spectra: 281 us, without 173).  Transforms of at
+// most 16 threads go in tiles of adjacent columns (ColTile) and write their last
+// pass straight to global memory; longer ones go back row-major through shared
+// memory.  Tiles against two columns to a warp: order-4 banks of 64 and 128
+// points 331 -> 275 us, inner and outer banks 538 -> 527.
 // Output layout [job][bank][y][column] (rows contiguous for the row kernel).
-// Blocks of the column kernels: transforms of at most 16 threads run in blocks
-// of COL_THREADS, six per SM (168 registers: no spills up to 192 points, 56
-// bytes at 240).  Eight or ten blocks (128 or 102 registers) spilled 260 to 600
-// bytes and measured slower (inner banks of 16 records 289 and 347 us against
-// 243).
-constexpr int COL_THREADS = 64;
+// Tiles run six blocks to an SM (168 registers).  Eight or ten (128 or
+// 102 registers) spilled 260 to 600 bytes and measured slower (inner banks of
+// 16 records 289 and 347 us against 243).
 template <int N>
-__global__ void __launch_bounds__(FftLen<N>::T <= 16 ? COL_THREADS : 256, FftLen<N>::T <= 16 ? 6 : 2) col_ifft_kernel(ColArgs a, const cplx* __restrict__ tw,
+__global__ void __launch_bounds__(FftLen<N>::T <= 16 ? TILE_THREADS : 256, FftLen<N>::T <= 16 ? 6 : 2) col_ifft_kernel(ColArgs a, const cplx* __restrict__ tw,
                                                          int cw, int banks_per_block) {
   extern __shared__ cplx smem[];
   constexpr int T = FftLen<N>::T, L = FftLen<N>::COL;
@@ -335,70 +331,77 @@ __global__ void __launch_bounds__(FftLen<N>::T <= 16 ? COL_THREADS : 256, FftLen
   const int k_first = blockIdx.z * banks_per_block;
   const int nk = min(a.nbanks - k_first, banks_per_block);
   const int h = a.box.h, w = a.box.w;
-  const int hp = h | 1;  // odd: no conflicts when consecutive columns are written
   const int plane = w * h;
-  const int G = blockDim.x / T, g = threadIdx.x / T, t = threadIdx.x % T;
   const int y0 = mod_n<N>(a.box.y0);
-  cplx* buf = smem + g * L;
-  cplx* base = smem + G * L;  // cw * hp
   const bool shared_base = a.kind != COL_PLAIN && a.kind != COL_OUTER2 && a.kind != COL_FLOORED;
-  const int lcw = 31 - __clz(cw);  // cw is a power of two
+  // column pitch of box columns in shared memory: consecutive columns are
+  // written and read together
+  const int hp = direct ? ColTile<N>::pitch(h) : h | 1;
+  cplx* base = smem + (direct ? cw * ColTile<N>::L : blockDim.x / T * L);  // cw * hp
+  cplx* divided = base + (shared_base ? cw * hp : 0);                      // short columns: cw * hp if any bank divides
+  // the box's (row, column) elements of this block, columns fastest
+  auto each = [&](auto&& body) {
+    const int dy = blockDim.x / cw, dc = blockDim.x - dy * cw;
+    for (int by = threadIdx.x / cw, c = threadIdx.x - by * cw; by < h; by += dy, c += dc) {
+      if (c >= cw) c -= cw, ++by;
+      if (by < h && c < ncol) body(by, c);
+    }
+  };
   if (shared_base) {
-    for (int q = threadIdx.x; q < (h << lcw); q += blockDim.x) {
-      const int c = q & (cw - 1), by = q >> lcw;
-      if (c >= ncol) continue;
+    each([&](int by, int c) {
       const int i = by * w + x_first + c;
       base[c * hp + by] = col_base(a, job, i, __ldg(a.geo + 3 * plane + i));
-    }
+    });
     __syncthreads();
   }
   const int nout = a.twins ? a.nout : a.nbanks;
   const double scale_im = a.conj_io ? -a.scale : a.scale;
-  const int per = direct ? G : cw;  // (bank, column) items per iteration
-  const int items = direct ? nk * ncol : nk * cw;
-  for (int it = 0; it < items; it += per) {
-    const int item = it + g;
-    const int kk = direct ? item / ncol : it / cw;
-    const int c = direct ? item - kk * ncol : g;
-    const bool active = direct ? item < items : g < ncol;
-    const int k = k_first + (active ? kk : 0);
-    const int x = x_first + (active ? c : 0);
-    const cplx* src = shared_base ? base + (active ? c : 0) * hp
-                                  : a.spec + (long long)job * a.spec_job_stride +
-                                        (long long)a.src_of[k] * a.spec_sub_stride + x;
-    int sstep = shared_base ? 1 : w;
+  // One bank after another: the columns of a block share its multiplier.
+  for (int k = k_first; k < k_first + nk; ++k) {
+    const cplx* src = a.spec + (long long)job * a.spec_job_stride + (long long)a.src_of[k] * a.spec_sub_stride + x_first;
+    int cstep = 1, ystep = w;  // steps between the source's columns and rows
+    if (shared_base) {
+      src = base;
+      cstep = hp;
+      ystep = 1;
+    }
     const bool floor_it = a.floor_max && ((a.kind == COL_OUTER2 && a.src_of[k] == 1) || a.kind == COL_FLOORED);
     const int fac = a.fac[k];
-    int rot = a.conj_io ? a.rot[k] ^ ROT_NEG_IM : a.rot[k];
-    group_sync<N>(1 + g);  // the row's previous transform has been read
+    const int rot = a.conj_io ? a.rot[k] ^ ROT_NEG_IM : a.rot[k];
     const double floor_abs =
         !floor_it ? 0.0
                   : a.floor_rel * as_double(a.kind == COL_FLOORED
                                                 ? a.floor_max[(size_t)job * a.floor_nsrc + a.src_of[k]]
                                                 : a.floor_max[job]);
+    const double* f = fac >= 0 ? a.geo + (size_t)(GEO_PLANES + fac) * plane + (size_t)x_first * h : nullptr;
+    const int tb = a.twins ? a.twin[k] : -1;
+    const bool turn = tb >= 0 && a.twin_fac[k] == 2;
+    cplx* dst = a.out + ((size_t)job * nout + (a.twins ? a.out_of[k] : k)) * N * w + x_first;
+    cplx* dst2 = tb >= 0 ? a.out + ((size_t)job * nout + tb) * N * w + x_first : nullptr;
     if (fac == F_DIRECT) {
-      // divided values go through the front of the group's row
-      if (active) {
-#pragma unroll 1
-        for (int by = t; by < h; by += T) {
-          cplx v = src[by * sstep];
-          if (floor_it && abs_below(v, floor_abs)) v = czero();
-          buf[by] = mult_direct(a.mult[k], GeoRef{a.geo, plane, by * w + x}, v);
-        }
-      }
-      src = buf;
-      sstep = 1;
+      // divided values are formed first: into `divided`, or into the front of a
+      // long column's own row
+      __syncthreads();
+      const int cp = direct ? hp : L;
+      cplx* into = direct ? divided : smem;
+      each([&](int by, int c) {
+        cplx v = src[c * cstep + by * ystep];
+        if (floor_it && abs_below(v, floor_abs)) v = czero();
+        into[c * cp + by] = mult_direct(a.mult[k], GeoRef{a.geo, plane, by * w + x_first + c}, v);
+      });
+      __syncthreads();
+      src = into;
+      cstep = cp;
+      ystep = 1;
     }
     const bool floor_load = floor_it && fac != F_DIRECT;
-    group_sync<N>(1 + g);
-    const double* f = fac >= 0 ? a.geo + (size_t)(GEO_PLANES + fac) * plane + (size_t)x * h : nullptr;
-    auto load = [&](int yb, int) -> cplx {
+    auto load = [&](int c, int yb, int) -> cplx {
       const int by = wrap_n<N>(yb - y0);
       cplx v = czero();
-      if (by < h) v = src[by * sstep];
+      if (by < h && c < ncol) v = src[c * cstep + by * ystep];
       return v;
     };
-    auto after = [&](cplx* v) {
+    auto after = [&](int c, int t, cplx* v) {
       constexpr int C = FftLen<N>::mixed ? FftLen<N>::M : 16, S = FftLen<N>::mixed ? 16 : N / 16;
       if (floor_load) {
 #pragma unroll
@@ -410,7 +413,7 @@ __global__ void __launch_bounds__(FftLen<N>::T <= 16 ? COL_THREADS : 256, FftLen
       for (int r = 0; r < C; ++r) {
         const int by = wrap_n<N>(t + r * S - y0);
         m[r] = 1.0;
-        if (f && by < h) m[r] = __ldg(f + by);
+        if (f && by < h && c < ncol) m[r] = __ldg(f + c * h + by);
       }
 #pragma unroll
       for (int r = 0; r < C; ++r) {
@@ -421,47 +424,44 @@ __global__ void __launch_bounds__(FftLen<N>::T <= 16 ? COL_THREADS : 256, FftLen
         v[r] = in ? z : czero();
       }
     };
-    const int tb = a.twins ? a.twin[k] : -1;
-    const int tfac = tb >= 0 ? a.twin_fac[k] : 0;
-    cplx* dst = a.out + ((size_t)job * nout + (a.twins ? a.out_of[k] : k)) * N * w + x;
-    cplx* dst2 = tb >= 0 ? a.out + ((size_t)job * nout + tb) * N * w + x : nullptr;
-    auto sink = [&](int o, int step, const cplx* v, int cnt) {
-      if constexpr (direct) {
+    if constexpr (direct) {
+      auto sink = [&](int c, int o, int step, const cplx* v, int cnt) {
+        if (c >= ncol) return;
         const size_t d = (size_t)step * w;
-        cplx* p = dst + (size_t)o * w;
+        cplx* p = dst + (size_t)o * w + c;
 #pragma unroll
         for (int r = 0; r < 16; ++r)
           if (r < cnt) p[r * d] = cmk(a.scale * v[r].x, scale_im * v[r].y);
         if (dst2) {
-          const double qx = __ldg(a.geo + x);  // qx plane, row 0
-          cplx* p2 = dst2 + (size_t)o * w;
+          const double qx = __ldg(a.geo + x_first + c);  // qx plane, row 0
+          cplx* p2 = dst2 + (size_t)o * w + c;
 #pragma unroll
           for (int r = 0; r < 16; ++r)
             if (r < cnt) {
               const cplx u = cscale(qx, cmk(a.scale * v[r].x, scale_im * v[r].y));
-              p2[r * d] = tfac == 2 ? cmuli(u) : u;
+              p2[r * d] = turn ? cmuli(u) : u;
             }
         }
-      } else {
-        row_put<N>(buf, o, step, v, cnt);
-      }
-    };
-    fft_n<+1, N>(buf, t, 1 + g, active, tw, load, sink, after);
-    if constexpr (!direct) {
+      };
+      fft_tile<+1, N>(smem, cw, tw, load, after, sink);
+    } else {
+      const int lcw = 31 - __clz(cw);  // cw is a power of two
+      const int c = threadIdx.x / T, t = threadIdx.x % T;
+      cplx* buf = smem + c * L;
+      auto in = [&](int y, int r) { return load(c, y, r); };
+      auto change = [&](cplx* v) { after(c, t, v); };
+      auto sink = [&](int o, int step, const cplx* v, int cnt) { row_put<N>(buf, o, step, v, cnt); };
+      fft_n<+1, N>(buf, t, 1 + c, c < ncol, tw, in, sink, change);
       __syncthreads();
-      cplx* d0 = a.out + ((size_t)job * nout + (a.twins ? a.out_of[k_first + kk] : k_first + kk)) * N * w + x_first;
-      const int tb0 = a.twins ? a.twin[k_first + kk] : -1;
-      cplx* d1 = tb0 >= 0 ? a.out + ((size_t)job * nout + tb0) * N * w + x_first : nullptr;
-      const bool turn = tb0 >= 0 && a.twin_fac[k_first + kk] == 2;
       for (int q = threadIdx.x; q < (N << lcw); q += blockDim.x) {
         const int y = q >> lcw, cc = q & (cw - 1);
         if (cc >= ncol) continue;
         const cplx v = smem[cc * L + pos<N>(y)];
         const cplx u0 = cmk(a.scale * v.x, scale_im * v.y);
-        d0[(size_t)y * w + cc] = u0;
-        if (d1) {
+        dst[(size_t)y * w + cc] = u0;
+        if (dst2) {
           const cplx u = cscale(__ldg(a.geo + x_first + cc), u0);
-          d1[(size_t)y * w + cc] = turn ? cmuli(u) : u;
+          dst2[(size_t)y * w + cc] = turn ? cmuli(u) : u;
         }
       }
       __syncthreads();
@@ -1067,16 +1067,15 @@ struct ColFftArgs {
 // One block: `cw` kept columns of one (job, source) spectrum ([js][y][col]).
 // Each column is one forward transform along y; only the output box's rows are
 // written (support-masked), with the spectrum's max |.| folded into maxslot.
-// Transforms of at most 16 threads (cw = groups of the block) read their first
-// pass from global memory into registers and write their last pass from
-// registers, with no block barrier: two or more adjacent columns of a warp use
-// every 32-byte sector.  All loads of a thread are on their way before the
-// first is used.  Staged through shared memory in 256-thread blocks at 128
-// registers, with the mask and hypot in one loop, the inner stage of 16 records
-// (145 x 145 of 144 points, 2048 spectra) took 329 us; this takes 277.
+// Transforms of at most 16 threads go in tiles (ColTile): the first pass reads
+// global memory into registers, the last writes from registers, and all loads
+// of a thread, mask bytes too, are on their way before the first is used.
+// Staged through shared memory in 256-thread blocks at 128 registers the inner
+// stage of 16 records (145 x 145 of 144 points, 2048 spectra) took 329 us;
+// straight to registers, two columns to a warp, 277; in tiles of seven, 231.
 // Longer columns are staged with coalesced loads.
 template <int N>
-__global__ void __launch_bounds__(FftLen<N>::T <= 16 ? COL_THREADS : 256, FftLen<N>::T <= 16 ? 6 : 2) col_fft_kernel(ColFftArgs a, const cplx* __restrict__ tw, int cw) {
+__global__ void __launch_bounds__(FftLen<N>::T <= 16 ? TILE_THREADS : 256, FftLen<N>::T <= 16 ? 6 : 2) col_fft_kernel(ColFftArgs a, const cplx* __restrict__ tw, int cw) {
   extern __shared__ cplx smem[];
   constexpr int T = FftLen<N>::T, L = FftLen<N>::COL;
   constexpr bool direct = T <= 16;
@@ -1088,7 +1087,6 @@ __global__ void __launch_bounds__(FftLen<N>::T <= 16 ? COL_THREADS : 256, FftLen
   const cplx* src = a.in + (size_t)js * N * a.box.w + x_first;
   const unsigned char* mask = a.mask ? a.mask + (size_t)unit * a.box.w * a.box.h : nullptr;
   cplx* dst = a.out + (size_t)js * a.box.w * a.box.h;
-  const int G = blockDim.x / T, g = threadIdx.x / T, t = threadIdx.x % T;
   const int y0 = mod_n<N>(a.box.y0);
   double local = 0.0;
   auto put = [&](int i, const cplx& raw) {
@@ -1098,20 +1096,22 @@ __global__ void __launch_bounds__(FftLen<N>::T <= 16 ? COL_THREADS : 256, FftLen
     return v;
   };
   if constexpr (direct) {
-    const bool active = g < ncol;
-    const int c = active ? g : 0;
-    auto load = [&](int y, int) -> cplx {
-      const cplx v = src[(size_t)y * a.box.w + c];
+    auto load = [&](int c, int y, int) -> cplx {
+      cplx v = czero();
+      if (c < ncol) v = src[(size_t)y * a.box.w + c];
       return a.conj_io ? cconj(v) : v;
     };
-    auto sink = [&](int o, int step, cplx* v, int cnt) {
+    auto after = [](int, int, cplx*) {};
+    auto sink = [&](int c, int o, int step, cplx* v, int cnt) {
+      const int i0 = x_first + c;
       unsigned char keep[16];
 #pragma unroll
       for (int r = 0; r < 16; ++r) {  // all mask bytes on their way before the first is used
         if (r >= cnt) continue;
         const int by = wrap_n<N>(o + r * step - y0);
-        keep[r] = by < a.box.h;
-        if (mask && by < a.box.h) keep[r] = __ldg(mask + by * a.box.w + x_first + c);
+        const bool in = by < a.box.h && c < ncol;
+        keep[r] = in;
+        if (mask && in) keep[r] = __ldg(mask + by * a.box.w + i0);
       }
 #pragma unroll
       for (int r = 0; r < 16; ++r) {
@@ -1120,14 +1120,15 @@ __global__ void __launch_bounds__(FftLen<N>::T <= 16 ? COL_THREADS : 256, FftLen
         cplx z = cscale(a.scale, a.conj_io ? cconj(v[r]) : v[r]);
         if (!keep[r]) z = czero();
         v[r] = z;
-        if (by < a.box.h) dst[by * a.box.w + x_first + c] = z;
+        if (by < a.box.h && c < ncol) dst[by * a.box.w + i0] = z;
       }
 #pragma unroll
       for (int r = 0; r < 16; ++r)
         if (r < cnt) local = keep_max_abs(local, v[r]);
     };
-    fft_n<-1, N>(smem + g * L, t, 1 + g, active, tw, load, sink);
+    fft_tile<-1, N>(smem, cw, tw, load, after, sink);
   } else {
+    const int G = blockDim.x / T, g = threadIdx.x / T, t = threadIdx.x % T;
     cplx* bufs = smem;  // cw * L
     // stage the kept columns ([y][col] rows in global memory) with eight
     // independent loads in flight per thread
