@@ -1704,10 +1704,10 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     c.weights = dn + 4 * MAX_RANK;
     c.nnodes = J;
     c.floor_rel = p->floor_rel;
-    dim3 g(grid_for(pl2, T, 256), gu);
+    dim3 g(std::max(1, (pl2 + ACC_BINS - 1) / ACC_BINS), gu);
     {
       LaunchScope ls_("acc_eta22_kernel", st, 0.0);
-      acc_eta22_kernel<<<g, T, 0, st>>>(c);
+      acc_eta22_kernel<<<g, acc_threads(c.nnodes), 0, st>>>(c);
     }
     LAUNCH_CHECK("acc_eta22_kernel");
     return GL_OK;
@@ -1847,10 +1847,10 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     c.nodes = dn + 1 * MAX_RANK;
     c.weights = dn + 5 * MAX_RANK;
     c.nnodes = 2;
-    dim3 g(grid_for(pl2, T, 256), gu);
+    dim3 g(std::max(1, (pl2 + ACC_BINS - 1) / ACC_BINS), gu);
     {
       LaunchScope ls_("acc_psi22_kernel", st, 0.0);
-      acc_psi22_kernel<<<g, T, 0, st>>>(c);
+      acc_psi22_kernel<<<g, acc_threads(2 * c.nnodes), 0, st>>>(c);
     }
     LAUNCH_CHECK("acc_psi22_kernel");
     return GL_OK;
@@ -2056,10 +2056,10 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     c.nodes = dn + 3 * MAX_RANK;
     c.weights = dn + 7 * MAX_RANK;
     c.nnodes = J;
-    dim3 g2(grid_for(pl3, T, 256), gu);
+    dim3 g2(std::max(1, (pl3 + ACC_BINS - 1) / ACC_BINS), gu);
     {
       LaunchScope ls_("acc_outer_kernel", st, 0.0);
-      acc_outer_kernel<<<g2, T, 0, st>>>(c, maxF);
+      acc_outer_kernel<<<g2, acc_threads(c.nnodes), 0, st>>>(c, maxF);
     }
     LAUNCH_CHECK("acc_outer_kernel");
     return GL_OK;
@@ -2741,7 +2741,8 @@ static gl_status e44_run(gl_plan* p, int gu, const void* spectra, int layout, in
     c.Ro = Ro;
     c.outer0 = o0;
     c.floor_rel = p->floor_rel;
-    dim3 g(grid_for(pl2, T, 64), gu * GP);
+    c.mask = s2;
+    dim3 g(std::max(1, (pl2 + E44_TILE - 1) / E44_TILE), gu * ((GP + E44_GROUPS - 1) / E44_GROUPS));
     {
       LaunchScope ls_("acc_e44_pair_kernel", st, 0.0);
       acc_e44_pair_kernel<<<g, T, 0, st>>>(c);
@@ -2799,10 +2800,12 @@ static gl_status e44_run(gl_plan* p, int gu, const void* spectra, int layout, in
     c.floor_rel = p->floor_rel;
     c.nspec = nts;
     c.only_t1 = part >= 0 ? part + 1 : 0;
-    dim3 g(grid_for(pl3, T, 64), gu * Ro);
+    c.mask = s3;
+    // 64-thread blocks: a few units' bins spread over more SMs
+    dim3 g(grid_for(pl3, 64, 256), gu * Ro);
     {
       LaunchScope ls_("acc_e44_third_kernel", st, 0.0);
-      acc_e44_third_kernel<<<g, T, 0, st>>>(c);
+      acc_e44_third_kernel<<<g, 64, 0, st>>>(c);
     }
     LAUNCH_CHECK("acc_e44_third_kernel");
   }
@@ -2859,10 +2862,10 @@ static gl_status e44_run(gl_plan* p, int gu, const void* spectra, int layout, in
     c.outer0 = o0;
     c.floor_rel = p->floor_rel;
     c.nspec = nf4;
-    dim3 g(grid_for(pl4, T, 64), gu);
+    dim3 g(grid_for(pl4, 64, 512), gu);
     {
       LaunchScope ls_("acc_e44_order4_kernel", st, 0.0);
-      acc_e44_order4_kernel<<<g, T, 0, st>>>(c);
+      acc_e44_order4_kernel<<<g, 64, 0, st>>>(c);
     }
     LAUNCH_CHECK("acc_e44_order4_kernel");
   }

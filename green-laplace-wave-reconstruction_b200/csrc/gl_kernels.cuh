@@ -1181,6 +1181,12 @@ GL_D cplx floored(cplx v, double rel, unsigned long long peak_bits) {
   return abs_below(v, rel * as_double(peak_bits)) ? czero() : v;
 }
 
+// The accumulation kernels ask for a node's values while they sum the previous
+// one's: `floored` compares magnitudes, and a thread that loads each value just
+// before its comparison waits for every one in turn.  The floors of a block's
+// nodes are formed once, in shared memory.
+GL_D cplx above(cplx v, double floor_abs) { return abs_below(v, floor_abs) ? czero() : v; }
+
 struct AccArgs {
   const UnitScalars* us;
   const double* geo;        // geometry planes of the output box
@@ -1202,79 +1208,111 @@ struct AccArgs {
 constexpr int ACC_TILE = 64;  // a multiple of 32: each warp's items share one outer node
 
 #ifndef GL_TRANSFORM_TU  // elementwise kernels: compiled by gl_engine.cu only
+// The node sums below are short (up to 16 or 32 terms of a few thousand bins) but
+// each term is a chain of exponentials and comparisons, so a block takes
+// ACC_BINS bins and gives each warp its own nodes; the terms meet in shared
+// memory, where one warp adds them in node order -- the sum a single thread would form.
+// One thread per bin and all its nodes left most SMs idle: one 512 x 512
+// order-3 snapshot, psi22 / eta22 / outer @AC@.
+constexpr int ACC_BINS = 32, ACC_WARPS = 8;  // at most ACC_WARPS, no more than there are terms
+inline int acc_threads(int terms) { return 32 * (terms < 2 ? 2 : terms < ACC_WARPS ? terms : ACC_WARPS); }
+
 // eta22: sum_n coef_n (-A sh_n sd_n + ch_n sk_n)   (spatial.py:206-221)
-__global__ void acc_eta22_kernel(AccArgs a) {
+__global__ void __launch_bounds__(32 * ACC_WARPS) acc_eta22_kernel(AccArgs a) {
   const int unit = blockIdx.y;
   const int plane = a.box.w * a.box.h;
   const UnitScalars& u = a.us[unit];
-  // per-node times and coefficients, once per block
-  __shared__ double s_tau[MAX_RANK], s_coef[MAX_RANK];
-  if (threadIdx.x < a.nnodes) {
-    const double x = a.nodes[threadIdx.x], w = a.weights[threadIdx.x];
-    const double tau = x / u.lam22;
-    s_tau[threadIdx.x] = tau;
-    s_coef[threadIdx.x] = w * exp(x) / u.lam22 / 4.0 * exp(-2.0 * u.shift2 * tau);
+  const int b = threadIdx.x % ACC_BINS, warp = threadIdx.x / ACC_BINS;
+  const int i = blockIdx.x * ACC_BINS + b;
+  __shared__ cplx s_term[MAX_RANK][ACC_BINS];
+  __shared__ double s_coef[MAX_RANK];
+  if (i < plane) {
+    const double sqa = __ldg(a.geo + 5 * plane + i), ga = __ldg(a.geo + 4 * plane + i);
+    for (int nn = warp; nn < a.nnodes; nn += blockDim.x / 32) {
+      const int js = unit * a.nnodes + nn;
+      const cplx vd = a.in[((size_t)js * 2 + 0) * plane + i], vk = a.in[((size_t)js * 2 + 1) * plane + i];
+      const double x = a.nodes[nn], w = a.weights[nn];
+      const double tau = x / u.lam22;
+      if (b == 0) s_coef[nn] = w * exp(x) / u.lam22 / 4.0 * exp(-2.0 * u.shift2 * tau);
+      const double sh = sinh_over_root(sqa, tau);
+      const double ch = cosh(sqa * tau);
+      const cplx sd = floored(vd, a.floor_rel, a.maxin[js * 2 + 0]);
+      const cplx sk = floored(vk, a.floor_rel, a.maxin[js * 2 + 1]);
+      s_term[nn][b] = cadd(cscale(-ga * sh, sd), cscale(ch, sk));
+    }
   }
   __syncthreads();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < plane; i += gridDim.x * blockDim.x) {
-    BinGeo g = load_geo(a.geo, plane, i);
+  if (warp == 0 && i < plane) {
     cplx acc = czero();
-    for (int nn = 0; nn < a.nnodes; ++nn) {
-      const int js = unit * a.nnodes + nn;
-      const double tau = s_tau[nn];
-      const double coef = s_coef[nn];
-      const double sh = sinh_over_root(g.sqa, tau);
-      const double ch = cosh(g.sqa * tau);
-      cplx sd = floored(a.in[((size_t)js * 2 + 0) * plane + i], a.floor_rel, a.maxin[js * 2 + 0]);
-      cplx sk = floored(a.in[((size_t)js * 2 + 1) * plane + i], a.floor_rel, a.maxin[js * 2 + 1]);
-      cplx term = cadd(cscale(-g.a * sh, sd), cscale(ch, sk));
-      acc = cadd(acc, cscale(coef, term));
-    }
+    for (int nn = 0; nn < a.nnodes; ++nn) acc = cadd(acc, cscale(s_coef[nn], s_term[nn][b]));
     a.out[(size_t)unit * plane + i] = acc;
   }
 }
 
 // psi22 dual-branch resolvent + Taylor contact, masked to the pair support
 // (spatial.py:276-308, 384-393).
-__global__ void acc_psi22_kernel(AccArgs a) {
+__global__ void __launch_bounds__(32 * ACC_WARPS) acc_psi22_kernel(AccArgs a) {
   const int unit = blockIdx.y;
   const int plane = a.box.w * a.box.h;
   const UnitScalars& u = a.us[unit];
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < plane; i += gridDim.x * blockDim.x) {
-    BinGeo g = load_geo(a.geo, plane, i);
-    cplx res = czero();
-    for (int branch = 0; branch < 2; ++branch) {
-      const double lam = branch == 0 ? u.lam_minus : u.lam_plus;
-      const double ksign = branch == 0 ? -1.0 : 1.0;
-      for (int nn = 0; nn < a.nnodes; ++nn) {
-        const double x = a.nodes[nn], w = a.weights[nn];
-        const double tau = x / lam;
-        const double coef = w * exp(x) / lam / 8.0;
-        const int js = (unit * 2 + branch) * a.nnodes + nn;
-        cplx resp = czero();
-        for (int ci = 0; ci < u.chan_count; ++ci) {
-          for (int cj = 0; cj < u.chan_count; ++cj) {
-            const int o = 2 * (2 * ci + cj);
-            const cplx sd = a.in[((size_t)js * 8 + o) * plane + i];
-            const cplx sk = a.in[((size_t)js * 8 + o + 1) * plane + i];
-            const double ssum = u.chan_shift[ci] + u.chan_shift[cj];
-            const double factor =
-                branch == 0 ? exp((g.sqa - ssum) * tau) : exp(-(g.sqa + ssum) * tau);
-            const cplx ks = cscale(ksign, sk);
-            const double sa = safe_nu(g.sqa);
-            cplx part = cscale(factor, cadd(sd, cmk(ks.x / sa, ks.y / sa)));
-            // pair support of the physical channel pair
-            const int pi = u.chan_id[ci] + u.chan_id[cj];  // 0: (0,0) 1: (0,1)/(1,0) 2: (1,1)
-            const int pidx = (u.chan_count == 1) ? (u.chan_id[0] == 0 ? 0 : 2) : pi;
-            if (!a.pmask[((size_t)unit * 3 + pidx) * plane + i]) part = czero();
-            resp = cadd(resp, part);
+  const int b = threadIdx.x % ACC_BINS, warp = threadIdx.x / ACC_BINS;
+  const int i = blockIdx.x * ACC_BINS + b;
+  __shared__ cplx s_term[2 * MAX_RANK][ACC_BINS];  // [branch][node]
+  const int nc = u.chan_count;
+  const bool on = i < plane && a.mask[(size_t)unit * plane + i];
+  if (on) {
+    const double sqa = __ldg(a.geo + 5 * plane + i);
+    const double sa = safe_nu(sqa);
+    // pair supports of the physical channel pairs (0,0), (0,1) and (1,1)
+    bool in[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) in[k] = a.pmask[((size_t)unit * 3 + k) * plane + i];
+    for (int q = warp; q < 2 * a.nnodes; q += blockDim.x / 32) {
+      const int branch = q >= a.nnodes, nn = q - branch * a.nnodes;
+      const cplx* src = a.in + ((size_t)(unit * 2 + branch) * a.nnodes + nn) * 8 * plane + i;
+      cplx v[8];
+#pragma unroll
+      for (int ci = 0; ci < 2; ++ci)
+#pragma unroll
+        for (int cj = 0; cj < 2; ++cj) {
+          const int o = 2 * (2 * ci + cj);
+          if (ci < nc && cj < nc) {
+            v[o] = src[(size_t)o * plane];
+            v[o + 1] = src[(size_t)(o + 1) * plane];
           }
         }
-        res = cadd(res, cmul(cmk(0.0, coef), resp));
-      }
+      const double lam = branch == 0 ? u.lam_minus : u.lam_plus;
+      const double ksign = branch == 0 ? -1.0 : 1.0;
+      const double x = a.nodes[nn], w = a.weights[nn];
+      const double tau = x / lam;
+      const double coef = w * exp(x) / lam / 8.0;
+      cplx resp = czero();
+#pragma unroll
+      for (int ci = 0; ci < 2; ++ci)
+#pragma unroll
+        for (int cj = 0; cj < 2; ++cj) {
+          if (ci >= nc || cj >= nc) continue;
+          const int o = 2 * (2 * ci + cj);
+          const double ssum = u.chan_shift[ci] + u.chan_shift[cj];
+          const double factor = branch == 0 ? exp((sqa - ssum) * tau) : exp(-(sqa + ssum) * tau);
+          const cplx ks = cscale(ksign, v[o + 1]);
+          cplx part = cscale(factor, cadd(v[o], cmk(ks.x / sa, ks.y / sa)));
+          const int pi = u.chan_id[ci] + u.chan_id[cj];
+          const int pidx = nc == 1 ? (u.chan_id[0] == 0 ? 0 : 2) : pi;
+          if (!(pidx == 0 ? in[0] : pidx == 1 ? in[1] : in[2])) part = czero();
+          resp = cadd(resp, part);
+        }
+      s_term[q][b] = cmul(cmk(0.0, coef), resp);
     }
-    cplx total = cadd(res, a.extra[(size_t)unit * plane + i]);
-    if (!a.mask[(size_t)unit * plane + i]) total = czero();
+  }
+  __syncthreads();
+  if (warp == 0 && i < plane) {
+    cplx total = czero();
+    if (on) {
+      cplx res = czero();
+      for (int q = 0; q < 2 * a.nnodes; ++q) res = cadd(res, s_term[q][b]);
+      total = cadd(res, a.extra[(size_t)unit * plane + i]);
+    }
     a.out[(size_t)unit * plane + i] = total;
   }
 }
@@ -1285,8 +1323,10 @@ __global__ void acc_psi22_kernel(AccArgs a) {
 // (AccArgs::nsub of them).  The node responses sinh(sqrt(A) tau)/sqrt(A) and
 // cosh(sqrt(A) tau) depend on the unit, the inner node and the bin only, so
 // each is evaluated once per block into shared memory; the block's threads
-// then accumulate the (outer node, bin) items from there.
-__global__ void __launch_bounds__(256, 4) acc_inner_kernel(AccArgs a) {
+// then accumulate the (outer node, bin) items from there, a node's four values
+// on their way while the previous node's are summed (16 records 135 us without,
+// 115 with; at 64 and at 128 registers 140 and 148).
+__global__ void __launch_bounds__(256, 3) acc_inner_kernel(AccArgs a) {
   const int unit = blockIdx.y;
   const int J = a.nsub, I = a.nnodes;
   const int plane = a.box.w * a.box.h;
@@ -1299,6 +1339,9 @@ __global__ void __launch_bounds__(256, 4) acc_inner_kernel(AccArgs a) {
     s_tau[threadIdx.x] = tau;
     s_coef[threadIdx.x] = w * exp(x) / u.lam2 * exp(-2.0 * u.shift2 * tau) / 4.0;
   }
+  __shared__ double s_floor[4 * MAX_RANK * MAX_RANK];
+  for (int k = threadIdx.x; k < 4 * J * I; k += blockDim.x)
+    s_floor[k] = a.floor_rel * as_double(a.maxin[(size_t)unit * J * I * 4 + k]);
   const int ntiles = (plane + ACC_TILE - 1) / ACC_TILE;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int i0 = tile * ACC_TILE;
@@ -1325,18 +1368,29 @@ __global__ void __launch_bounds__(256, 4) acc_inner_kernel(AccArgs a) {
         dst[2 * plane + i] = czero();
         dst[3 * plane + i] = czero();
       } else if (i < plane) {
+        const cplx* src = a.in + (size_t)uj * I * 4 * plane + i;
+        cplx v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = src[(size_t)k * plane];
         const double ga = a.geo[4 * plane + i];
         cplx e = czero(), et = czero(), p = czero(), pt = czero();
         for (int ii = 0; ii < I; ++ii) {
-          const int js = uj * I + ii;
+          cplx n[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) n[k] = v[k];
+          if (ii + 1 < I) {
+            src += 4 * (size_t)plane;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[k] = src[(size_t)k * plane];
+          }
+          const double* fl = s_floor + 4 * (j * I + ii);
           const double coef = s_coef[ii];
           const double sh = s_sh[ii][b];
           const double ch = s_ch[ii][b];
-          const cplx* src = a.in + (size_t)js * 4 * plane;
-          cplx sd = floored(src[i], a.floor_rel, a.maxin[js * 4 + 0]);
-          cplx sk = floored(src[plane + i], a.floor_rel, a.maxin[js * 4 + 1]);
-          cplx sdt = floored(src[2 * plane + i], a.floor_rel, a.maxin[js * 4 + 2]);
-          cplx skt = floored(src[3 * plane + i], a.floor_rel, a.maxin[js * 4 + 3]);
+          cplx sd = above(n[0], fl[0]);
+          cplx sk = above(n[1], fl[1]);
+          cplx sdt = above(n[2], fl[2]);
+          cplx skt = above(n[3], fl[3]);
           const double mash = -ga * sh;
           e = cadd(e, cscale(coef, cadd(cscale(mash, sd), cscale(ch, sk))));
           et = csub(et, cmul(cmk(0.0, coef), cadd(cscale(mash, sdt), cscale(ch, skt))));
@@ -1381,12 +1435,6 @@ GL_D OuterForcing outer_forcing_of(const cplx* v, double ga, double floor_rel,
   o.kpsi = cmk(__fma_rn(ga, c.x, o.fk.x), __fma_rn(ga, c.y, o.fk.y));
   o.dpsi = csub(o.fd, ct);
   return o;
-}
-
-GL_D OuterForcing outer_forcing(const cplx* src, int plane, int i, double ga, double floor_rel,
-                                const unsigned long long* mx) {
-  const cplx v[4] = {src[i], src[plane + i], src[2 * plane + i], src[3 * plane + i]};
-  return outer_forcing_of(v, ga, floor_rel, mx);
 }
 
 // order-3 outer forcing maxima: the maxima of |fk + A c| and |fd - c_t| over
@@ -1438,45 +1486,47 @@ __global__ void acc_outer_max_kernel(AccArgs a) {
 // order-3 outer accumulation into eta33 / psi33 spectra (_order3.py:124-138):
 // `in` holds the four forcing spectra of each outer node, `maxin` their
 // maxima and `maxpsi` the psi forcings' maxima (acc_outer_max_kernel).
-__global__ void acc_outer_kernel(AccArgs a, const unsigned long long* maxpsi) {
+__global__ void __launch_bounds__(32 * ACC_WARPS) acc_outer_kernel(AccArgs a, const unsigned long long* maxpsi) {
   const int unit = blockIdx.y;
   const int plane = a.box.w * a.box.h;
   const UnitScalars& u = a.us[unit];
-  __shared__ double s_tau[MAX_RANK], s_coef[MAX_RANK];
+  const int b = threadIdx.x % ACC_BINS, warp = threadIdx.x / ACC_BINS;
+  const int i = blockIdx.x * ACC_BINS + b;
+  __shared__ cplx s_eta[MAX_RANK][ACC_BINS], s_psi[MAX_RANK][ACC_BINS];
+  __shared__ double s_coef[MAX_RANK];
   if (threadIdx.x < a.nnodes) {
     const double x = a.nodes[threadIdx.x], w = a.weights[threadIdx.x];
     const double tau = x / u.lam3;
-    s_tau[threadIdx.x] = tau;
     s_coef[threadIdx.x] = w * exp(x) / u.lam3 * exp(-3.0 * u.shift3 * tau);
   }
-  __syncthreads();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < plane; i += gridDim.x * blockDim.x) {
-    // off the triple support the output is zero: the bin skips its loads
-    // and node responses
-    if (!a.mask[(size_t)unit * plane + i]) {
-      a.out[((size_t)unit * 2 + 0) * plane + i] = czero();
-      a.out[((size_t)unit * 2 + 1) * plane + i] = czero();
-      continue;
-    }
-    BinGeo g = load_geo(a.geo, plane, i);
-    cplx eta = czero(), psi = czero();
-    for (int j = 0; j < a.nnodes; ++j) {
+  // off the triple support the output is zero: the bin skips its loads
+  // and node responses
+  const bool on = i < plane && a.mask[(size_t)unit * plane + i];
+  if (on) {
+    const double sqa = __ldg(a.geo + 5 * plane + i), ga = __ldg(a.geo + 4 * plane + i);
+    for (int j = warp; j < a.nnodes; j += blockDim.x / 32) {
       const int uj = unit * a.nnodes + j;
-      const double tau = s_tau[j];
-      const double sh = sinh_over_root(g.sqa, tau);
-      const double ch = cosh(g.sqa * tau);
-      const double coef = s_coef[j];
-      const OuterForcing o = outer_forcing(a.in + (size_t)uj * 4 * plane, plane, i, g.a,
-                                           a.floor_rel, a.maxin + uj * 4);
+      const cplx* src = a.in + (size_t)uj * 4 * plane + i;
+      cplx v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = src[(size_t)k * plane];
+      const double tau = a.nodes[j] / u.lam3;
+      const double sh = sinh_over_root(sqa, tau);
+      const double ch = cosh(sqa * tau);
+      const OuterForcing o = outer_forcing_of(v, ga, a.floor_rel, a.maxin + uj * 4);
       const cplx kpsi = floored(o.kpsi, a.floor_rel, maxpsi[uj * 2 + 0]);
       const cplx dpsi = floored(o.dpsi, a.floor_rel, maxpsi[uj * 2 + 1]);
-      cplx te = csub(cscale(g.a * sh, o.fd), cmul(cmk(0.0, ch), o.fk));
-      cplx tp = csub(cmul(cmk(0.0, -ch), dpsi), cscale(sh, kpsi));
-      eta = cadd(eta, cscale(coef, te));
-      psi = cadd(psi, cscale(coef, tp));
+      s_eta[j][b] = csub(cscale(ga * sh, o.fd), cmul(cmk(0.0, ch), o.fk));
+      s_psi[j][b] = csub(cmul(cmk(0.0, -ch), dpsi), cscale(sh, kpsi));
     }
-    a.out[((size_t)unit * 2 + 0) * plane + i] = eta;
-    a.out[((size_t)unit * 2 + 1) * plane + i] = psi;
+  }
+  __syncthreads();
+  // one warp sums eta, another psi
+  if (warp < 2 && i < plane) {
+    cplx acc = czero();
+    if (on)
+      for (int j = 0; j < a.nnodes; ++j) acc = cadd(acc, cscale(s_coef[j], warp == 0 ? s_eta[j][b] : s_psi[j][b]));
+    a.out[((size_t)unit * 2 + warp) * plane + i] = acc;
   }
 }
 #endif  // GL_TRANSFORM_TU
