@@ -498,7 +498,11 @@ __global__ void mink_copy_kernel(unsigned char* c, long long plane, int which, U
 // Scales, shifts and status per unit, for boxes beyond analyse_kernel's reach.
 __global__ void scalars_kernel(ScalarArgs a, int n) {
   const int u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u < n) a.us[u] = unit_scalars(a, a.slots[u]);
+  if (u >= n) return;
+  const double qp = peak_depth(a, a.slots[u]);
+  double th[4];
+  for (int k = 0; k < 4; ++k) th[k] = tanh((k + 1.0) * qp);
+  a.us[u] = unit_scalars(a, a.slots[u], qp, th);
 }
 
 // Deposit N^2 (a+ib)/h e^{-i omega t} per bin segment (gl_spectral_surface.m:123-149).
@@ -1409,8 +1413,8 @@ static unsigned long long* order3_maxima(const gl_plan* p, void* ws) {
   return at<unsigned long long>(ws, p->o_max) + (p->want_eta22 ? (size_t)p->group * p->ranks[0] * 2 : 0);
 }
 
-// Shared memory of analyse_kernel for a box, or 0 when the box is beyond it: a
-// thread holds ANA_PER bins, a row ANA_COLS columns.
+// Shared memory of analyse_kernel for a box, or 0 when the box is beyond it
+// (ANA_BINS bins, ANA_COLS columns).
 static size_t ana_bytes(const Box& b, int levels, int channels) {
   if ((long long)b.w * b.h > ANA_BINS || b.w > ANA_COLS) return 0;
   const size_t bytes = ana_words(b.w, b.h, levels, channels) * sizeof(u32);

@@ -7,16 +7,17 @@
 // 20 us, each a barrier for the whole batch (about 110 us of a 128^2
 // third-order call with every component, 150 us per group of eight 1024^2
 // units).
-// Its data are a few thousand bins per unit: every block of the cluster holds
-// them in registers and the supports as bit rows in shared memory, the blocks
-// share out the rows of the Minkowski sums, and a sum's rows travel to the
-// other blocks through distributed shared memory.  A row of a sum is the OR
+// Its data are a few thousand bins per unit: the blocks share out the rows of
+// the box and of the Minkowski sums, every block holds the supports as bit rows
+// in shared memory, and the rows, like the sums and extrema over the box, travel
+// to the other blocks through distributed shared memory.  A row of a sum is the OR
 // over row pairs of one row dilated by the other's runs of set bits; the
 // dilations by powers of two are tabulated, so a run costs two shifted ORs
-// whatever its length.  What bounds it is the latency of the phases
-// (26 us, 44 us with 51 x 49 bins and every component, 60 us for eight
-// units of 73 x 69).  Larger boxes keep the
-// separate kernels, which spread over the GPU.
+// whatever its length.  What bounds it is the latency of the phases: 22 us,
+// 39 with 51 x 49 bins and every component, 41 for eight units of 73 x 69 (50
+// and 60 when every block scanned the whole box by itself, and one thread
+// computed every hyperbolic tangent of the scalars at the end).  Larger boxes
+// keep the separate kernels, which spread over the GPU.
 #pragma once
 #include <cooperative_groups.h>
 
@@ -27,7 +28,7 @@ namespace gl {
 typedef unsigned long long u64;
 typedef unsigned int u32;
 
-constexpr int ANA_CLUSTER = 8, ANA_THREADS = 512, ANA_PER = 16, ANA_BINS = ANA_THREADS * ANA_PER, ANA_COLS = 128;
+constexpr int ANA_CLUSTER = 8, ANA_THREADS = 512, ANA_BINS = 8192, ANA_COLS = 128;
 // 32-bit words of a row of S, S+S, S+S+S and S+S+S+S
 constexpr int ANA_W1 = 4, ANA_W2 = 8, ANA_W3 = 12, ANA_W4 = 16;
 
@@ -47,7 +48,18 @@ struct ScalarArgs {
 
 // Scales, shifts and status of one unit (spatial.py:179-189, 246-268;
 // _order3.py:35-52).
-GL_D UnitScalars unit_scalars(const ScalarArgs& a, const UnitSlots& s) {
+// The peak's depth, and tanh of one to four times it, are the caller's.
+GL_D double peak_depth(const ScalarArgs& a, const UnitSlots& s) {
+  if (a.fixed_peak > 0.0) return a.fixed_peak;
+  if (s.count == 0 || s.peak_flat == ~0ull) return 0.0;
+  const unsigned long long flat = s.peak_flat;
+  const int ix = (int)(flat % (unsigned long long)a.nx), iy = (int)(flat / (unsigned long long)a.nx);
+  const int mx = ix < a.nx / 2 ? ix : ix - a.nx;
+  const int my = iy < a.ny / 2 ? iy : iy - a.ny;
+  return a.geo1[2 * a.box.w * a.box.h + (my - a.box.y0) * a.box.w + (mx - a.box.x0)];
+}
+
+GL_D UnitScalars unit_scalars(const ScalarArgs& a, const UnitSlots& s, double qp, const double* th) {
   UnitScalars r;
   memset(&r, 0, sizeof r);
   int status = 0;
@@ -64,23 +76,17 @@ GL_D UnitScalars unit_scalars(const ScalarArgs& a, const UnitSlots& s) {
   r.nu_min = as_double(s.nu_min);
   r.nu_max = as_double(s.nu_max);
   if (!status) {
-    const unsigned long long flat = s.peak_flat;
-    const int ix = (int)(flat % (unsigned long long)a.nx), iy = (int)(flat / (unsigned long long)a.nx);
-    const int mx = ix < a.nx / 2 ? ix : ix - a.nx;
-    const int my = iy < a.ny / 2 ? iy : iy - a.ny;
-    const int i = (my - a.box.y0) * a.box.w + (mx - a.box.x0);
-    const double qp = a.fixed_peak > 0.0 ? a.fixed_peak : a.geo1[2 * a.box.w * a.box.h + i];
     r.peak_q = qp;
-    const double pnu = sqrt(qp * tanh(qp));
+    const double pnu = sqrt(qp * th[0]);
     const double sqa2 = as_double(s.sqa_max2);
     r.shift2 = 0.5 * (r.nu_min + sqa2 / 2.0);
     if (a.want_eta22) {
-      const double t1 = 2.0 * sqrt(qp * tanh(qp));
-      r.lam22 = sqrt(t1 * t1 - 2.0 * qp * tanh(2.0 * qp));
+      const double t1 = 2.0 * sqrt(qp * th[0]);
+      r.lam22 = sqrt(t1 * t1 - 2.0 * qp * th[1]);
       if (!(r.lam22 > 0.0) || !isfinite(r.lam22)) status = GL_ERR_SCALE;
     }
     if (a.want_psi22) {
-      const double pout = sqrt(2.0 * qp * tanh(2.0 * qp));
+      const double pout = sqrt(2.0 * qp * th[1]);
       r.lam_minus = 2.0 * pnu - pout;
       r.lam_plus = 2.0 * pnu + pout;
       if (!(r.lam_minus > 0.0) || !isfinite(r.lam_minus) || !(r.lam_plus > 0.0) ||
@@ -101,17 +107,17 @@ GL_D UnitScalars unit_scalars(const ScalarArgs& a, const UnitSlots& s) {
     if (a.want_o3) {
       const double sqa3 = as_double(s.sqa_max3);
       r.shift3 = 0.5 * (r.nu_min + sqa3 / 3.0);
-      r.lam2 = 2.0 * pnu - sqrt(2.0 * qp * tanh(2.0 * qp));
-      r.lam3 = 3.0 * pnu - sqrt(3.0 * qp * tanh(3.0 * qp));
+      r.lam2 = 2.0 * pnu - sqrt(2.0 * qp * th[1]);
+      r.lam3 = 3.0 * pnu - sqrt(3.0 * qp * th[2]);
       if (!(r.lam2 > 0.0) || !(r.lam3 > 0.0)) status = GL_ERR_SCALE;
     }
     if (a.want_e44) {  // gl_eta44_fftw.cpp:121-128
       const double sqa3 = as_double(s.sqa_max3), sqa4 = as_double(s.pad[2]);
       r.shift3 = 0.5 * (r.nu_min + sqa3 / 3.0);
       r.shift4 = 0.5 * (r.nu_min + sqa4 / 4.0);
-      r.lam2 = 2.0 * pnu - sqrt(2.0 * qp * tanh(2.0 * qp));
-      r.lam3 = 3.0 * pnu - sqrt(3.0 * qp * tanh(3.0 * qp));
-      r.lam4 = 4.0 * pnu - sqrt(4.0 * qp * tanh(4.0 * qp));
+      r.lam2 = 2.0 * pnu - sqrt(2.0 * qp * th[1]);
+      r.lam3 = 3.0 * pnu - sqrt(3.0 * qp * th[2]);
+      r.lam4 = 4.0 * pnu - sqrt(4.0 * qp * th[3]);
       if (!(r.lam2 > 0.0) || !(r.lam3 > 0.0) || !(r.lam4 > 0.0)) status = GL_ERR_SCALE;
     }
   }
@@ -283,6 +289,8 @@ GL_D void ana_level(cooperative_groups::cluster_group& cl, const u32* tab, int h
 __global__ void __cluster_dims__(ANA_CLUSTER) __launch_bounds__(ANA_THREADS) analyse_kernel(AnaArgs a) {
   extern __shared__ __align__(16) u32 sh[];
   __shared__ UnitSlots S;
+  __shared__ UnitSlots parts[3][ANA_CLUSTER];  // of each gathering, so that none is overwritten while it is read
+  __shared__ double s_th[5];
   cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
   const int u = blockIdx.x / ANA_CLUSTER, rank = cl.block_rank(), tid = threadIdx.x, lane = tid & 31;
   const Box box = a.sc.box;
@@ -307,69 +315,91 @@ __global__ void __cluster_dims__(ANA_CLUSTER) __launch_bounds__(ANA_THREADS) ana
       S.pad[1] = a.slots[u].pad[1];
     }
   }
-  for (int i = tid; i < h * ANA_W1 * (a.chan ? 3 : 1); i += ANA_THREADS) r1[i] = 0u;
-  // moduli of the thread's bins, and their maximum
+  // The cluster's warps share out the rows of the box.  The bit rows (a ballot
+  // per 32 bins) go to every block; sums and extrema gather in the block's slots,
+  // which are then sent to every block and merged there.
   const cplx* spec = a.spec + (size_t)u * plane;
-  double m[ANA_PER], lmax = 0.0;
-#pragma unroll
-  for (int j = 0; j < ANA_PER; ++j) {
-    const int i = tid + j * ANA_THREADS;
-    m[j] = i < plane ? cabs_(spec[i]) : 0.0;
-    lmax = (m[j] > lmax || m[j] != m[j]) ? m[j] : lmax;
-  }
-  __syncthreads();
+  const int first = (tid >> 5) * ANA_CLUSTER + rank, step_y = (ANA_THREADS / 32) * ANA_CLUSTER;
+  const bool to = lane < ANA_CLUSTER;
+  auto gather = [&](int phase, auto&& merge) {
+    __syncthreads();
+    if (tid < ANA_CLUSTER) *cl.map_shared_rank(&parts[phase][rank], tid) = S;
+    cl.sync();
+    if (tid == 0)
+      for (int b = 0; b < ANA_CLUSTER; ++b)
+        if (b != rank) merge(parts[phase][b]);
+    __syncthreads();
+  };
+  cl.sync();  // the blocks' memory may be written by the others
   if (!a.slots) {
+    double lmax = 0.0;
+    for (int y = first; y < h; y += step_y)
+#pragma unroll 1
+      for (int x = lane; x < w; x += 32) {
+        const double m = cabs_(spec[y * w + x]);
+        lmax = (m > lmax || m != m) ? m : lmax;
+      }
     for (int o = 16; o > 0; o >>= 1) {
       const double v = __shfl_xor_sync(0xffffffffu, lmax, o);
       lmax = (v > lmax || v != v) ? v : lmax;
     }
     if (lane == 0) atomic_max_nonneg(&S.smax, lmax);
-    __syncthreads();
+    gather(0, [&](const UnitSlots& o) { S.smax = o.smax > S.smax ? o.smax : S.smax; });
   }
   // the support and its reductions
+  const double smax = as_double(S.smax);
+  const double thr = 1.0e-13 * (smax > 1.0 ? smax : 1.0);
   {
-    const double smax = as_double(S.smax);
-    const double thr = 1.0e-13 * (smax > 1.0 ? smax : 1.0);
     double numin = INFINITY, numax = 0.0, amax = 0.0, qmin = INFINITY;
-    u64 cnt = 0, bad = 0;
-#pragma unroll
-    for (int j = 0; j < ANA_PER; ++j) {
-      const int i = tid + j * ANA_THREADS;
-      if (i >= plane) continue;
-      if (!(m[j] == m[j]) || m[j] == INFINITY) bad = 1;
-      if (m[j] > thr) {
-        const double nu = a.sc.geo1[3 * plane + i], q = a.sc.geo1[2 * plane + i];
-        numin = fmin(numin, nu);
-        numax = fmax(numax, nu);
-        qmin = fmin(qmin, q);
-        amax = fmax(amax, m[j] * m[j]);
-        ++cnt;
-        const int y = i / w, x = i - y * w;
-        atomicOr(r1 + y * ANA_W1 + (x >> 5), 1u << (x & 31));
-      } else {
-        m[j] = -1.0;  // off the support
+    unsigned cnt = 0, bad = 0;
+    for (int y = first; y < h; y += step_y)
+#pragma unroll 1
+      for (int q = 0; q < ANA_W1; ++q) {
+        const int x = 32 * q + lane, i = y * w + x;
+        bool on = false;
+        if (x < w) {
+          const double m = cabs_(spec[i]);
+          if (!(m == m) || m == INFINITY) bad = 1;
+          on = m > thr;
+          if (on) {
+            const double nu = a.sc.geo1[3 * plane + i];
+            numin = fmin(numin, nu);
+            numax = fmax(numax, nu);
+            qmin = fmin(qmin, a.sc.geo1[2 * plane + i]);
+            amax = fmax(amax, m * m);
+            ++cnt;
+          }
+        }
+        const u32 word = __ballot_sync(0xffffffffu, on);
+        if (to) cl.map_shared_rank(r1, lane)[y * ANA_W1 + q] = word;
       }
-    }
     for (int o = 16; o > 0; o >>= 1) {
       numin = fmin(numin, __shfl_xor_sync(0xffffffffu, numin, o));
       numax = fmax(numax, __shfl_xor_sync(0xffffffffu, numax, o));
       qmin = fmin(qmin, __shfl_xor_sync(0xffffffffu, qmin, o));
       amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-      cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-      bad |= __shfl_xor_sync(0xffffffffu, bad, o);
     }
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    bad = __reduce_or_sync(0xffffffffu, bad);
     if (lane == 0) {
       if (cnt) {
         atomicMin(&S.nu_min, (u64)__double_as_longlong(numin));
         atomicMin(&S.pad[0], (u64)__double_as_longlong(qmin));
         atomic_max_nonneg(&S.nu_max, numax);
         atomic_max_nonneg(&S.amp2_max, amax);
-        atomicAdd(&S.count, cnt);
+        atomicAdd(&S.count, (u64)cnt);
       }
       if (bad) atomicOr(&S.nonfinite, 1ull);
     }
   }
-  __syncthreads();
+  gather(1, [&](const UnitSlots& o) {
+    S.nu_min = o.nu_min < S.nu_min ? o.nu_min : S.nu_min;
+    S.pad[0] = o.pad[0] < S.pad[0] ? o.pad[0] : S.pad[0];
+    S.nu_max = o.nu_max > S.nu_max ? o.nu_max : S.nu_max;
+    S.amp2_max = o.amp2_max > S.amp2_max ? o.amp2_max : S.amp2_max;
+    S.count += o.count;
+    S.nonfinite |= o.nonfinite;
+  });
   // first argmax in reference flat order; radial channels and their nu ranges
   {
     const double amax = as_double(S.amp2_max);
@@ -378,58 +408,72 @@ __global__ void __cluster_dims__(ANA_CLUSTER) __launch_bounds__(ANA_THREADS) ana
     const double mid = step == 0.0 ? lo : step + lo;
     u64 best = ~0ull;
     double cmin[2] = {INFINITY, INFINITY}, cmax[2] = {0.0, 0.0};
+    for (int y = first; y < h; y += step_y)
+#pragma unroll 1
+      for (int q = 0; q < ANA_W1; ++q) {
+        const int x = 32 * q + lane, i = y * w + x;
+        bool c[2] = {false, false};
+        if ((r1[y * ANA_W1 + q] >> lane) & 1u) {
+          const double m = cabs_(spec[i]);
+          if (m * m == amax) {
+            const u64 flat = (u64)wrap_any(box.y0 + y, a.sc.ny) * (u64)a.sc.nx + (u64)wrap_any(box.x0 + x, a.sc.nx);
+            best = flat < best ? flat : best;
+          }
+          if (a.chan) {
+            const double nu = a.sc.geo1[3 * plane + i];
+            c[0] = nu >= lo && nu < mid;
+            c[1] = nu >= mid && nu <= hi;
 #pragma unroll
-    for (int j = 0; j < ANA_PER; ++j) {
-      const int i = tid + j * ANA_THREADS;
-      if (i >= plane) continue;
-      const int y = i / w, x = i - y * w;
-      unsigned char c[2] = {0, 0};
-      if (m[j] >= 0.0) {
-        if (m[j] * m[j] == amax) {
-          const u64 flat = (u64)wrap_any(box.y0 + y, a.sc.ny) * (u64)a.sc.nx + (u64)wrap_any(box.x0 + x, a.sc.nx);
-          best = flat < best ? flat : best;
+            for (int b = 0; b < 2; ++b)
+              if (c[b]) {
+                cmin[b] = fmin(cmin[b], nu);
+                cmax[b] = fmax(cmax[b], nu);
+              }
+          }
         }
         if (a.chan) {
-          const double nu = a.sc.geo1[3 * plane + i];
-          c[0] = nu >= lo && nu < mid;
-          c[1] = nu >= mid && nu <= hi;
 #pragma unroll
-          for (int q = 0; q < 2; ++q)
-            if (c[q]) {
-              cmin[q] = fmin(cmin[q], nu);
-              cmax[q] = fmax(cmax[q], nu);
-              atomicOr(rc + (q * h + y) * ANA_W1 + (x >> 5), 1u << (x & 31));
-            }
+          for (int b = 0; b < 2; ++b) {
+            const u32 word = __ballot_sync(0xffffffffu, c[b]);
+            if (to) cl.map_shared_rank(rc, lane)[(b * h + y) * ANA_W1 + q] = word;
+            if (x < w) a.chan[((size_t)u * 2 + b) * plane + i] = c[b];
+          }
         }
       }
-      if (a.chan && j % ANA_CLUSTER == rank) {
-        a.chan[((size_t)u * 2 + 0) * plane + i] = c[0];
-        a.chan[((size_t)u * 2 + 1) * plane + i] = c[1];
-      }
-    }
     for (int o = 16; o > 0; o >>= 1) {
       const u64 ob = __shfl_xor_sync(0xffffffffu, best, o);
       best = ob < best ? ob : best;
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        cmin[q] = fmin(cmin[q], __shfl_xor_sync(0xffffffffu, cmin[q], o));
-        cmax[q] = fmax(cmax[q], __shfl_xor_sync(0xffffffffu, cmax[q], o));
+    }
+    if (lane == 0 && best != ~0ull) atomicMin(&S.peak_flat, best);
+    if (a.chan) {
+#pragma unroll 1
+      for (int b = 0; b < 2; ++b) {
+        double mn = cmin[b], mxv = cmax[b];
+        for (int o = 16; o > 0; o >>= 1) {
+          mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+          mxv = fmax(mxv, __shfl_xor_sync(0xffffffffu, mxv, o));
+        }
+        if (lane == 0 && mn != INFINITY) {
+          atomicMin(&S.chan_min[b], (u64)__double_as_longlong(mn));
+          atomic_max_nonneg(&S.chan_max[b], mxv);
+        }
       }
     }
-    if (lane == 0) {
-      atomicMin(&S.peak_flat, best);
-#pragma unroll
-      for (int q = 0; q < 2; ++q)
-        if (a.chan && cmin[q] != INFINITY) {
-          atomicMin(&S.chan_min[q], (u64)__double_as_longlong(cmin[q]));
-          atomic_max_nonneg(&S.chan_max[q], cmax[q]);
-        }
-    }
   }
-  __syncthreads();
-  // supports of the products; the cluster's blocks meet before the first write
-  // into another block's rows and after each level that sends rows
-  if (a.levels >= 3) cl.sync();
+  gather(2, [&](const UnitSlots& o) {
+    S.peak_flat = o.peak_flat < S.peak_flat ? o.peak_flat : S.peak_flat;
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      S.chan_min[b] = o.chan_min[b] < S.chan_min[b] ? o.chan_min[b] : S.chan_min[b];
+      S.chan_max[b] = o.chan_max[b] > S.chan_max[b] ? o.chan_max[b] : S.chan_max[b];
+    }
+  });
+  // the peak's depth and its hyperbolic tangents, beside the sums
+  if (rank == 0 && tid >= ANA_THREADS - 32) {
+    const double qp = peak_depth(a.sc, S);
+    if (lane < 4) s_th[lane] = tanh((lane + 1.0) * qp);
+    if (lane == 0) s_th[4] = qp;
+  }
   if (a.levels >= 2) {
     const size_t pl2 = (size_t)w2 * h2, tn = (size_t)h * (k * ANA_W2 + 1);
     ana_dilate<ANA_W1, ANA_W2>(r1, h, k, tab);
@@ -473,7 +517,7 @@ __global__ void __cluster_dims__(ANA_CLUSTER) __launch_bounds__(ANA_THREADS) ana
     ana_fold(m2, &S.sqa_max2);
     ana_fold(m3, &S.sqa_max3);
     ana_fold(m4, &S.pad[2]);
-    if (lane == 0) a.sc.us[u] = unit_scalars(a.sc, S);
+    if (lane == 0) a.sc.us[u] = unit_scalars(a.sc, S, s_th[4], s_th);
   }
   cl.sync();
 }
