@@ -298,6 +298,22 @@ def get_plan(*, nx, ny, lx, ly, depth, gravity, order, components, eta22_rank, a
     return plan
 
 
+GROUP_BYTES = 2 << 30
+
+
+def _plan_for(n: int, max_units: int | None, **spec) -> Plan:
+    """The plan that evaluates ``n`` units in groups of ``max_units``.  Left to
+    the library, a group is 16 units while its workspace stays within
+    GROUP_BYTES, else 8: larger launches have fewer nearly empty last waves (16
+    order-3 records at 1024 x 1024 in one group of 16 instead of two of 8: 2278 -> 2082 us)."""
+    if max_units:
+        return get_plan(max_units=max_units, **spec)
+    plan = get_plan(max_units=min(n, 16), **spec)
+    if n > 8 and plan.workspace_bytes > GROUP_BYTES:
+        plan = get_plan(max_units=8, **spec)
+    return plan
+
+
 def _matlab_round(v: np.ndarray) -> np.ndarray:
     return np.sign(v) * np.floor(np.abs(v) + 0.5)
 
@@ -424,13 +440,13 @@ def surface_batch_device(coeffs: GLCoefficients, Lx, Ly, Nx, Ny, times, *,
     base = host.data_ptr()
     box, live, segs = _group_modes(coeffs, Lx, Ly, int(Nx), int(Ny), base + o_off, base + o_bin, base + o_ab,
                                    base + o_om, None)
-    plan = get_plan(nx=int(Nx), ny=int(Ny), lx=float(Lx), ly=float(Ly), depth=coeffs.h,
-                    gravity=coeffs.g, order=coeffs.order, components=mask,
-                    eta22_rank=int(coeffs.options["eta22_rank"]),
-                    allow_below=coeffs.options["allow_below_model_parent_domain"], box=box,
-                    grid=GRID_REFERENCE if grid == "reference" else GRID_COMPACT,
-                    max_units=max_units or min(n, 8), output=out_mode, device=device,
-                    inner_rank=int(order3_ranks[0]), outer_rank=int(order3_ranks[1]))
+    plan = _plan_for(n, max_units, nx=int(Nx), ny=int(Ny), lx=float(Lx), ly=float(Ly), depth=coeffs.h,
+                     gravity=coeffs.g, order=coeffs.order, components=mask,
+                     eta22_rank=int(coeffs.options["eta22_rank"]),
+                     allow_below=coeffs.options["allow_below_model_parent_domain"], box=box,
+                     grid=GRID_REFERENCE if grid == "reference" else GRID_COMPACT,
+                     output=out_mode, device=device,
+                     inner_rank=int(order3_ranks[0]), outer_rank=int(order3_ranks[1]))
     stream = stream or torch.cuda.current_stream(device)
     with torch.cuda.device(device), torch.cuda.stream(stream):
         table = host.to(device=device, non_blocking=True)
@@ -504,15 +520,15 @@ class SurfaceStream:
         dev = self.device
         mask = _components_for(coeffs.order, kw["components"])
         out_mode = OUT_REAL if kw["output"] == "real" else OUT_COMPLEX
-        plan = get_plan(nx=int(Nx), ny=int(Ny), lx=float(Lx), ly=float(Ly), depth=coeffs.h,
-                        gravity=coeffs.g, order=coeffs.order, components=mask,
-                        eta22_rank=int(coeffs.options["eta22_rank"]),
-                        allow_below=coeffs.options["allow_below_model_parent_domain"],
-                        box=dep.box,
-                        grid=GRID_REFERENCE if kw["grid"] == "reference" else GRID_COMPACT,
-                        max_units=kw["max_units"] or min(n, 8), output=out_mode, device=dev,
-                        inner_rank=int(kw["order3_ranks"][0]),
-                        outer_rank=int(kw["order3_ranks"][1]))
+        plan = _plan_for(n, kw["max_units"], nx=int(Nx), ny=int(Ny), lx=float(Lx), ly=float(Ly), depth=coeffs.h,
+                         gravity=coeffs.g, order=coeffs.order, components=mask,
+                         eta22_rank=int(coeffs.options["eta22_rank"]),
+                         allow_below=coeffs.options["allow_below_model_parent_domain"],
+                         box=dep.box,
+                         grid=GRID_REFERENCE if kw["grid"] == "reference" else GRID_COMPACT,
+                         output=out_mode, device=dev,
+                         inner_rank=int(kw["order3_ranks"][0]),
+                         outer_rank=int(kw["order3_ranks"][1]))
         pin = lambda a, dt: torch.from_numpy(np.ascontiguousarray(a)).to(dtype=dt).pin_memory()  # noqa: E731
         st = {
             "plan": plan,
