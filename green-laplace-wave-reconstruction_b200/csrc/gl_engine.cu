@@ -3040,6 +3040,8 @@ extern "C" gl_status gl_execute(gl_plan* p, int n_units, const void* d_spectra, 
 
 struct AdjLayout {
   size_t e1, e2, e3, da22, da1, dai, stage, total;  // offsets from the scratch base
+  size_t side;  // seed rows, then eta22's stage: `stage` itself, or their own region
+  bool split;   // their own region: they may run beside order 3
 };
 
 static bool adj_eta22(const gl_plan* p) { return (p->comps & GL_COMP_ETA22) != 0; }
@@ -3107,10 +3109,12 @@ static AdjLayout adj_layout(const gl_plan* p, int g) {
   L.dai = b.take(e33 ? (size_t)g * p->ranks[3] * p->ranks[2] * pl1 * c : 0);
   L.stage = b.off;
   const size_t wmax = std::max({(size_t)p->b1.w, (size_t)p->b2.w, (size_t)p->b3.w});
-  size_t end = L.stage + align_up((size_t)g * p->d.ny * wmax * c);  // seed rows
-  if (e22) end = std::max(end, adj_stage22(p, L.stage, g).end);
-  if (e33) end = std::max(end, adj_stage33(p, L.stage, g).end);
-  L.total = end;
+  const size_t rows = align_up((size_t)g * p->d.ny * wmax * c);
+  auto side_end = [&](size_t base) { return std::max(base + rows, e22 ? adj_stage22(p, base, g).end : base); };
+  const size_t end33 = e33 ? adj_stage33(p, L.stage, g).end : L.stage;
+  L.split = e33 && side_end(0) <= BRANCH_BYTES;
+  L.side = L.split ? end33 : L.stage;
+  L.total = std::max(end33, side_end(L.side));
   return L;
 }
 
@@ -3248,17 +3252,15 @@ static gl_status run_adjoint_group(gl_plan* p, int gu, const void* spectra, int 
   if ((s = analyse_group(p, gu, spectra, layout, ws, st, &spec)) != GL_OK) return s;
 
   // seeds: Ebar on each differentiated component's box
-  cplx* rows = reinterpret_cast<cplx*>(base + L.stage);
+  cplx* rows = reinterpret_cast<cplx*>(base + L.side);
   const bool e11 = p->comps & GL_COMP_ETA11, e22 = adj_eta22(p), e33 = adj_eta33(p);
-  if (e11 && (s = adj_seed(p, gu, resid, B1, rows, E1, st)) != GL_OK) return s;
-  if (e22 && (s = adj_seed(p, gu, resid, B2, rows, E2, st)) != GL_OK) return s;
-  if (e33 && (s = adj_seed(p, gu, resid, B3, rows, E3, st)) != GL_OK) return s;
 
   // ---------------- eta22 (spatial.py:156-231), transposed ----------------
-  if (e22) {
+  auto eta22_chain = [&](cudaStream_t st) -> gl_status {
+    gl_status s;
     const int J = p->ranks[0];
     const int nj = gu * J;
-    const AdjStage22 S = adj_stage22(p, L.stage, p->group);
+    const AdjStage22 S = adj_stage22(p, L.side, p->group);
     cplx* P = reinterpret_cast<cplx*>(base + S.P);
     cplx* Q = reinterpret_cast<cplx*>(base + S.Q);
     cplx* R = reinterpret_cast<cplx*>(base + S.R);
@@ -3354,11 +3356,12 @@ static gl_status run_adjoint_group(gl_plan* p, int gu, const void* spectra, int 
     if ((s = launch_row(ra, nj, st, p->tw)) != GL_OK) return s;
     CmbArgs c = cmb_args(p, G2, CMB_ETA22, 8, m8, nullptr, 1, B1, p->geo1, QA, DA22, us, J);
     c.nodes = dn + 0 * MAX_RANK;
-    if ((s = launch_combine(c, nj, st, p->tw)) != GL_OK) return s;
-  }
+    return launch_combine(c, nj, st, p->tw);
+  };
 
   // ---------------- order 3 (_order3.py:18-148), eta33 transposed ----------------
-  if (e33) {
+  // `seeded` makes the stream wait for the seed E3
+  auto order3_chain = [&](auto&& seeded) -> gl_status {
     const int Jo = p->ranks[3], I = p->ranks[2];
     const int nuj = gu * Jo, nj = nuj * I;
     const AdjStage33 S = adj_stage33(p, L.stage, p->group);
@@ -3531,6 +3534,7 @@ static gl_status run_adjoint_group(gl_plan* p, int gu, const void* spectra, int 
       aa.us = us;
       aa.geo = p->geo3;
       aa.box = B3;
+      if ((s = seeded()) != GL_OK) return s;
       aa.seed = E3;
       aa.fwd = RO;
       aa.fwdmax = maxRO;
@@ -3623,8 +3627,43 @@ static gl_status run_adjoint_group(gl_plan* p, int gu, const void* spectra, int 
       c.nodes = dn + 3 * MAX_RANK;
       c.nodes2 = dn + 2 * MAX_RANK;
       c.n_inner = I;
-      if ((s = launch_combine(c, nj, st, p->tw)) != GL_OK) return s;
+      return launch_combine(c, nj, st, p->tw);
     }
+  };
+
+  // The seeds and eta22 on a side stream beside order 3's long chain, as
+  // run_group's branches (a 512^2 gradient with all components 1157 -> 1124 us).
+  BranchSet* br = L.split ? branch_acquire(st) : nullptr;
+  if (!br) {
+    if (e11 && (s = adj_seed(p, gu, resid, B1, rows, E1, st)) != GL_OK) return s;
+    if (e22 && (s = adj_seed(p, gu, resid, B2, rows, E2, st)) != GL_OK) return s;
+    if (e33 && (s = adj_seed(p, gu, resid, B3, rows, E3, st)) != GL_OK) return s;
+    if (e22 && (s = eta22_chain(st)) != GL_OK) return s;
+    if (e33 && (s = order3_chain([] { return GL_OK; })) != GL_OK) return s;
+  } else {
+    const cudaStream_t side = br->st[0];
+    auto chains = [&]() -> gl_status {
+      gl_status s;
+      CUDA_TRY(cudaEventRecord(br->ev[0], st));
+      CUDA_TRY(cudaStreamWaitEvent(side, br->ev[0], 0));
+      if ((s = adj_seed(p, gu, resid, B3, rows, E3, side)) != GL_OK) return s;
+      CUDA_TRY(cudaEventRecord(br->ev[1], side));
+      if (e11 && (s = adj_seed(p, gu, resid, B1, rows, E1, side)) != GL_OK) return s;
+      if (e22 && (s = adj_seed(p, gu, resid, B2, rows, E2, side)) != GL_OK) return s;
+      if (e22 && (s = eta22_chain(side)) != GL_OK) return s;
+      return order3_chain([&]() -> gl_status {
+        CUDA_TRY(cudaStreamWaitEvent(st, br->ev[1], 0));
+        return GL_OK;
+      });
+    };
+    s = chains();
+    // joined even after a failed launch, so that the caller's stream never runs
+    // ahead of work already queued
+    const cudaError_t e1 = cudaEventRecord(br->ev[3], side);
+    const cudaError_t e2 = e1 == cudaSuccess ? cudaStreamWaitEvent(st, br->ev[3], 0) : e1;
+    if (e2 != cudaSuccess && s == GL_OK) s = fail(GL_ERR_CUDA, "branch join: %s", cudaGetErrorString(e2));
+    branch_release(br);
+    if (s != GL_OK) return s;
   }
 
   // ---------------- gradient on the parent box ----------------

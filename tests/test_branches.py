@@ -76,3 +76,39 @@ def test_eager_lanes_and_their_graph_agree():
     runner.replay()
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, (_, _, b) in zip(eager, runner.outputs()))
+
+
+def test_gradients_from_threads_beside_each_other():
+    """The seeds and the second order run beside the third order's chain; calls
+    from several threads and streams take their own side streams."""
+    import torch
+
+    from gl_engine import adjoint
+
+    n, units = 128, 2
+    _, s = _coeffs(n, 3)
+    times = np.linspace(0.0, 10.0, units)
+    a, b = (torch.from_numpy(v).cuda() for v in (s.a, s.b))
+    resid = torch.from_numpy(np.random.default_rng(5).standard_normal((units, n, n))).cuda()
+
+    def gradient():
+        model = adjoint.EtaSurfaceModel(s.kx, s.ky, depth=s.depth, lx=s.lx, ly=s.ly, nx=n, ny=n, times=times)
+        return [model.vjp(a, b, resid) for _ in range(5)]
+
+    want = gradient()[0]
+    torch.cuda.synchronize()
+    got = [None] * 4
+
+    def work(k):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            got[k] = gradient()
+            torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for each in got:
+        for g in each:
+            assert torch.equal(g[0], want[0]) and torch.equal(g[1], want[1])
