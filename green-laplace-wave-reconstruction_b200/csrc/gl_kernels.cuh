@@ -870,7 +870,7 @@ constexpr int ROW_THREADS = 192;
 template <int KIND, int N>
 __global__ void __launch_bounds__(ROW_THREADS, 2) row_kernel_t(RowArgs a, const cplx* __restrict__ tw) {
   constexpr int FAMILY = KIND >= ROW_ADJ_ETA22 ? 1 : (KIND >= ROW_E44_PAIR && KIND <= ROW_E44_ORDER4_PSI ? 2 : 0);
-  constexpr int T = FftLen<N>::T, L = FftLen<N>::ROW;
+  constexpr int T = FftLen<N>::T, L = FftLen<N>::PITCH;
   constexpr bool MULTI = T < 16;
   extern __shared__ __align__(128) cplx smem[];
   __shared__ __align__(8) unsigned long long stage_bar;

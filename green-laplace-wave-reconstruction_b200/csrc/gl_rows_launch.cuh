@@ -10,7 +10,7 @@ void row_launch(int njobs, cudaStream_t st, const RowArgs& a, const cplx* tw) {
   constexpr int T = FftLen<N>::T;
   int nb = 0;
   for (int g = 0; g < a.ngrp; ++g) nb += a.grp[g].nb;
-  const size_t smem = (size_t)nb * FftLen<N>::ROW * sizeof(cplx);
+  const size_t smem = (size_t)nb * FftLen<N>::PITCH * sizeof(cplx);
   // 384 threads per SM (168 registers each), in as many blocks as
   // shared memory holds of the row's banks: small blocks keep their groups busy
   // (a block's last round and its forward transforms use few of them) and meet
