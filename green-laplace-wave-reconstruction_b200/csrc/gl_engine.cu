@@ -4649,7 +4649,7 @@ extern "C" gl_status gl_wit_sector_range(int sector, int n_modes, const int* d_m
   const unsigned long long count = q_end - q_begin;
   if (sector == 44 && n_modes <= WIT44_PAIR_MODES) {
     // Real arithmetic over tabulated pair and triple states; 100 modes (4.4 M
-    // quartets): 13.4 ms by the general kernel below, 0.34 ms.  The
+    // quartets): 13.4 ms by the general kernel below, 0.37 so.  The
     // triple table is built when the call's candidates outnumber its entries
     // (a rank's small share forms its triples per quartet, by the same
     // function).  Sectors 40 and 42 mix signs, and their intermediate sums

@@ -10,7 +10,7 @@ leaving them idle.  Every input is staged on the device before capture, and
 the whole batch -- one deposit and one gl_execute per sea state, the lanes as
 parallel branches between one fork and one join -- is captured once and
 replayed.  Replays skip the host entirely: no Python, no argument marshalling,
-no launch latency between the ~40 kernels of each sea state.
+no launch latency between the ten to thirty kernels of each sea state.
 
 ``autotune_group`` times the units-per-launch group size of a plan on the
 device, ``autotune_tiles`` the launch shapes of its transform kernels
