@@ -23,7 +23,8 @@
 // Rows in shared memory keep the first pass's stores free of bank conflicts:
 // powers of two pad one element every 16, mixed lengths with even m one every
 // m, odd m none.  Groups of at most 32 threads synchronise with __syncwarp;
-// larger ones use one named barrier per group.
+// larger ones use one named barrier per group; tiles of interleaved columns
+// (fft_tile) meet as a block.
 #pragma once
 #include "gl_fftreg.cuh"
 

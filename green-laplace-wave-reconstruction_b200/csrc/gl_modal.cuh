@@ -10,9 +10,9 @@
 // output bin then sums its GL node responses over the q-axis.
 //
 // Transforms: strided_fft_kernel runs batched power-of-two transforms of up to
-// 4096 points along any axis of a row-major array (loads and stores staged
-// through shared memory, coalesced along whichever index is contiguous).
-// q-axes longer than 4096 use two such passes (four-step: P = P1 P2 with a
+// 4096 points along a strided axis, adjacent columns interleaved over a block's
+// threads, line_fft_kernel along the contiguous one; both read and write global
+// memory from registers.  q-axes longer than 4096 use two such passes (four-step: P = P1 P2 with a
 // twiddle between the passes); their x-space rows then come out in a
 // permuted order, which the pointwise products do not see and the inverse
 // pass undoes.
