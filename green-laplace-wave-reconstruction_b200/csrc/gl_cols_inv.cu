@@ -157,7 +157,7 @@ gl_status launch_col_ifft(const ColArgs& a0, int njobs, cudaStream_t st, const c
 
 gl_status launch_final_cols(const FinalCols& a0, int ny, int nunits, cudaStream_t st, const cplx* tw) {
   FinalCols a = a0;
-  const int G = 256 / (ny / 16);
+  const int G = 256 / (is_pow2(ny) ? ny / 16 : 16);
   auto blocks = [&](int cw) {
     int n = 0;
     for (int k = 0; k < a.ncomp; ++k) {
@@ -174,7 +174,7 @@ gl_status launch_final_cols(const FinalCols& a0, int ny, int nunits, cudaStream_
   for (int k = 0; k < a.ncomp; ++k)
     bytes += (double)nunits * a.comp[k].box.w * (ny + a.comp[k].box.h) * sizeof(cplx);
   LaunchScope ls("final_col_kernel", st, bytes);
-  switch (ny) { GL_POW2_CASES(final_cols_n, grid, st, a, tw, cw) }
+  GL_LEN_DISPATCH(ny, final_cols_n, grid, st, a, tw, cw);
   LAUNCH_CHECK("final_col_kernel");
   return GL_OK;
 }

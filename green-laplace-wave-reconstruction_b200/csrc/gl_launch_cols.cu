@@ -88,14 +88,14 @@ gl_status launch_out_rows(const OutArgs& a, int nunits, cudaStream_t st, const c
   // SM leave each thread 168 registers (the 256-thread form is held to 128
   // and spills), for 12 instead of 16 resident warps (same-box A/B at 1024^2:
   // the kernel 7 % faster)
-  const int T = a.nx / 16;
+  const int T = is_pow2(a.nx) ? a.nx / 16 : 16;
   const int G = (T <= 64 ? 192 : 256) / T;
   dim3 grid((a.ny + G - 1) / G, nunits * a.ncomp);
   double bytes = (double)nunits * a.ncomp * a.nx * a.ny * (a.real_only ? sizeof(double) : sizeof(cplx));
   for (int k = 0; k < a.ncomp; ++k) bytes += (double)nunits * a.comp[k].w * a.ny * sizeof(cplx);
   LaunchScope ls("out_row_kernel", st, bytes);
   // a failed attribute call surfaces as the launch's own error
-  switch (a.nx) { GL_POW2_CASES(out_rows_n, grid, G, st, a, tw) }
+  GL_LEN_DISPATCH(a.nx, out_rows_n, grid, G, st, a, tw);
   LAUNCH_CHECK("out_row_kernel");
   return GL_OK;
 }
