@@ -280,24 +280,30 @@ __global__ void __launch_bounds__(RESPONSE_THREADS) modal_response_kernel(ModalR
   const int w = blockIdx.x;
   const double s = (double)(a.mult_b0 * a.g.b0 + w) * a.g.fstep;
   cplx acc = czero();
-  for (int j = threadIdx.x; j < a.g.P; j += blockDim.x) {
+  // rows j and P - j hold q and -q: their node sums, exponentials most of this
+  // kernel's work, are the same (the four launches of a record 135 -> 111 us)
+  for (int j = threadIdx.x; j <= a.g.P / 2; j += blockDim.x) {
     const double qa = fabs(modal_q(a.g, j));
     const double ra = sqrt(qa * tanh(qa));
     if (!(s > ra)) continue;
     const double aq = qa * tanh(qa);
     double S, C;
     modal_node_sums(s, ra, a.scale, a.nodes, a.weights, a.rank, S, C);
-    const cplx d = a.sd[(long long)j * a.g.M + w], k = a.sk[(long long)j * a.g.M + w];
-    cplx r;
-    if (a.kind == 2) {
-      r = cadd(cscale(-aq * S, d), cscale(C, k));
-      r = cmk(r.x / (4.0 * a.depth), r.y / (4.0 * a.depth));
-    } else {
-      r = csub(cscale(aq * S, d), cmul(cmk(0.0, C), k));
-      const double d2 = a.depth * a.depth;
-      r = cmk(r.x / d2, r.y / d2);
+    for (int side = 0; side < 2; ++side) {
+      const int row = side ? a.g.P - j : j;
+      if (side && (row == a.g.P || row == j)) break;
+      const cplx d = a.sd[(long long)row * a.g.M + w], k = a.sk[(long long)row * a.g.M + w];
+      cplx r;
+      if (a.kind == 2) {
+        r = cadd(cscale(-aq * S, d), cscale(C, k));
+        r = cmk(r.x / (4.0 * a.depth), r.y / (4.0 * a.depth));
+      } else {
+        r = csub(cscale(aq * S, d), cmul(cmk(0.0, C), k));
+        const double d2 = a.depth * a.depth;
+        r = cmk(r.x / d2, r.y / d2);
+      }
+      acc = cadd(acc, r);
     }
-    acc = cadd(acc, r);
   }
   part[threadIdx.x] = acc;
   __syncthreads();
@@ -311,28 +317,32 @@ __global__ void __launch_bounds__(RESPONSE_THREADS) modal_response_kernel(ModalR
 // Inner pair spectra e2, p2 at every (q, inner bin) (modal_time.py:290-299):
 // e2 = (-A S sd + C sk)/4, p2 = i (C sd - S sk)/4 with the lambda2 scale.
 __global__ void modal_pair_kernel(ModalResp a, cplx* e2, cplx* p2) {
-  const long long total = (long long)a.g.P * a.g.M;
+  const long long total = (long long)(a.g.P / 2 + 1) * a.g.M;  // rows j and P - j together
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
     const int j = (int)(t / a.g.M), w = (int)(t % a.g.M);
-    cplx ev = czero(), pv = czero();
-    if (w < a.nbins) {
-      const double s = (double)(2 * a.g.b0 + w) * a.g.fstep;
-      const double qa = fabs(modal_q(a.g, j));
-      const double ra = sqrt(qa * tanh(qa));
-      if (s > ra) {
-        const double aq = qa * tanh(qa);
-        double S, C;
-        modal_node_sums(s, ra, a.scale, a.nodes, a.weights, a.rank, S, C);
-        const cplx d = a.sd[t], k = a.sk[t];
+    const double s = (double)(2 * a.g.b0 + w) * a.g.fstep;
+    const double qa = fabs(modal_q(a.g, j));
+    const double ra = sqrt(qa * tanh(qa));
+    const bool on = w < a.nbins && s > ra;
+    const double aq = qa * tanh(qa);
+    double S = 0.0, C = 0.0;
+    if (on) modal_node_sums(s, ra, a.scale, a.nodes, a.weights, a.rank, S, C);
+    for (int side = 0; side < 2; ++side) {
+      const int row = side ? a.g.P - j : j;
+      if (side && (row == a.g.P || row == j)) break;
+      const long long i = (long long)row * a.g.M + w;
+      cplx ev = czero(), pv = czero();
+      if (on) {
+        const cplx d = a.sd[i], k = a.sk[i];
         ev = cadd(cscale(-aq * S, d), cscale(C, k));
         ev = cmk(ev.x / 4.0, ev.y / 4.0);
         pv = cmuli(csub(cscale(C, d), cscale(S, k)));
         pv = cmk(pv.x / 4.0, pv.y / 4.0);
       }
+      e2[i] = ev;
+      p2[i] = pv;
     }
-    e2[t] = ev;
-    p2[t] = pv;
   }
 }
 
