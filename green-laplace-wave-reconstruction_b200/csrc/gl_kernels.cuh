@@ -1567,11 +1567,11 @@ __global__ void __launch_bounds__(256, 2) final_col_kernel(FinalCols a, const cp
   const int w = C.box.w, h = C.box.h, plane = w * h, unit = blockIdx.y;
   const int x_first = (blockIdx.x - C.first_block) * cw;
   const int ncol = min(cw, w - x_first);
-  const int G = blockDim.x / T, g = threadIdx.x / T, t = threadIdx.x % T;
+  const int g = threadIdx.x / T, t = threadIdx.x % T;
   const int y0 = mod_n<N>(C.box.y0);
   cplx* buf = smem + g * L;
   cplx* mid = C.mid + (size_t)unit * N * w + x_first;
-  const int lcw = 31 - __clz(cw);  // cw is a power of two, at most G
+  const int lcw = 31 - __clz(cw);  // cw is a power of two, at most the groups of the block
   const bool active = g < ncol;
   const cplx* src = C.spec + (long long)unit * C.spec_stride + x_first + (active ? g : 0);
   int sstep = w;
