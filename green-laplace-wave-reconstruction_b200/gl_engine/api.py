@@ -420,7 +420,7 @@ def surface_batch_device(coeffs: GLCoefficients, Lx, Ly, Nx, Ny, times, *,
     for name, value in (("Nx", Nx), ("Ny", Ny)):
         if not (isinstance(value, (int, np.integer)) and value > 0 and value % 2 == 0):
             raise GLError("green_laplace:Grid", f"{name} must be a positive even integer")
-    times = np.atleast_1d(np.asarray(times, dtype=np.float64))
+    times = np.ascontiguousarray(times, dtype=np.float64)  # any view's values in order: copied by address below
     if not np.all(np.isfinite(times)):
         raise GLError("green_laplace:Grid", "t must be finite")
     device = torch.device(device if device is not None else "cuda")
