@@ -335,13 +335,19 @@ def _group_modes(coeffs: GLCoefficients, lx, ly, nx, ny, seg_off: int, seg_bin: 
     """Mode -> bin mapping with the off-grid and Nyquist checks of
     ``deposit_analytic_input`` (``src/gl_spectral_surface.m:123-149``) into host
     buffers at the given addresses (``gl_group_modes``): (box, modes, bins)."""
-    a, b, kx, ky, omega = (np.ascontiguousarray(v, dtype=np.float64)
-                           for v in (coeffs.a, coeffs.b, coeffs.kx, coeffs.ky, coeffs.omega))
+    fields = (coeffs.a, coeffs.b, coeffs.kx, coeffs.ky, coeffs.omega)
+    n = int(np.size(coeffs.a))
+    # the table reads n values of each by its address
+    if n == 0 or not all(isinstance(v, np.ndarray) and v.ndim == 1 for v in fields) or \
+            any(v.size != n or v.dtype.kind not in "biuf" for v in fields[:4]) or coeffs.omega.size < n:
+        raise GLError("green_laplace:ComponentSize",
+                      "a, b, kx, ky, and omega must be nonempty real vectors of equal length.")
+    a, b, kx, ky, omega = (np.ascontiguousarray(v, dtype=np.float64) for v in fields)
     box = (C.c_int * 4)()
     counts = (C.c_int * 2)()
     at = C.addressof(counts)
     status = _lib.load().gl_group_modes(
-        int(a.size), a.ctypes.data, b.ctypes.data, kx.ctypes.data, ky.ctypes.data, omega.ctypes.data,
+        n, a.ctypes.data, b.ctypes.data, kx.ctypes.data, ky.ctypes.data, omega.ctypes.data,
         float(lx), float(ly), int(nx), int(ny), float(coeffs.options["grid_tolerance"]), box, seg_off,
         seg_bin, ab, om, index, at, at + C.sizeof(C.c_int))
     if status == 12:
