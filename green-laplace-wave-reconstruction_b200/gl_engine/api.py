@@ -342,6 +342,15 @@ def _group_modes(coeffs: GLCoefficients, lx, ly, nx, ny, seg_off: int, seg_bin: 
             any(v.size != n or v.dtype.kind not in "biuf" for v in fields[:4]) or coeffs.omega.size < n:
         raise GLError("green_laplace:ComponentSize",
                       "a, b, kx, ky, and omega must be nonempty real vectors of equal length.")
+    if any(v.dtype.kind == "f" and v.dtype != np.float64 for v in fields[2:4]):
+        # compared with the grid in their own precision, then the grid's wavenumbers
+        dkx, dky = 2.0 * np.pi / lx, 2.0 * np.pi / ly
+        mx, my = _matlab_round(coeffs.kx / dkx), _matlab_round(coeffs.ky / dky)
+        tol = coeffs.options["grid_tolerance"] * np.maximum(1.0, np.hypot(coeffs.kx, coeffs.ky))
+        if np.any(np.abs(coeffs.kx - mx * dkx) > tol) or np.any(np.abs(coeffs.ky - my * dky) > tol):
+            raise GLError("green_laplace:OffGridComponent",
+                          "Every component must lie on the requested FFT grid.")
+        fields = (*fields[:2], mx.astype(np.float64) * dkx, my.astype(np.float64) * dky, coeffs.omega)
     a, b, kx, ky, omega = (np.ascontiguousarray(v, dtype=np.float64) for v in fields)
     box = (C.c_int * 4)()
     counts = (C.c_int * 2)()
