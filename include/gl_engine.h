@@ -217,7 +217,8 @@ gl_status gl_plan_set_wait_test(gl_plan* plan, unsigned int surplus_bytes, long 
 /* Host mode table of gl_deposit_modes: maps n components (a, b, kx, ky, omega)
  * to the bins of an nx x ny grid on lx x ly with the off-grid and Nyquist
  * checks of deposit_analytic_input (src/gl_spectral_surface.m:123-149), drops
- * those of zero amplitude and groups the rest by bin (stable).  Host buffers:
+ * those of zero amplitude and groups the rest by bin (stable).  A box of more
+ * than 2^31 - 1 bins is GL_ERR_UNSUPPORTED.  Host buffers:
  * box[4] (x0, y0, w, h), seg_offsets[n + 1], seg_bins[n], ab[2 n], omega_out[n]
  * and, unless null, index[n] (grouped order -> component). */
 gl_status gl_group_modes(int n, const double* a, const double* b, const double* kx, const double* ky,
