@@ -330,14 +330,15 @@ class ModeDeposit:
     index: np.ndarray | None = None   # deposit order -> input mode index
 
 
-def _group_modes(coeffs: GLCoefficients, lx, ly, nx, ny, seg_off: int, seg_bin: int, ab: int, om: int,
-                 index: int | None) -> tuple[tuple[int, int, int, int], int, int]:
-    """Mode -> bin mapping with the off-grid and Nyquist checks of
-    ``deposit_analytic_input`` (``src/gl_spectral_surface.m:123-149``) into host
-    buffers at the given addresses (``gl_group_modes``): (box, modes, bins)."""
+_F64 = np.dtype(np.float64)
+
+
+def _component_fields(coeffs: GLCoefficients, lx, ly) -> tuple[np.ndarray, ...]:
+    """(a, b, kx, ky, omega) of components that are not all float64 vectors of
+    one length: refused where the table, which reads as many values of each as
+    ``a`` has by its address, could not take them."""
     fields = (coeffs.a, coeffs.b, coeffs.kx, coeffs.ky, coeffs.omega)
     n = int(np.size(coeffs.a))
-    # the table reads n values of each by its address
     if n == 0 or not all(isinstance(v, np.ndarray) and v.ndim == 1 for v in fields) or \
             any(v.size != n or v.dtype.kind not in "biuf" for v in fields[:4]) or coeffs.omega.size < n:
         raise GLError("green_laplace:ComponentSize",
@@ -351,12 +352,26 @@ def _group_modes(coeffs: GLCoefficients, lx, ly, nx, ny, seg_off: int, seg_bin: 
             raise GLError("green_laplace:OffGridComponent",
                           "Every component must lie on the requested FFT grid.")
         fields = (*fields[:2], mx.astype(np.float64) * dkx, my.astype(np.float64) * dky, coeffs.omega)
-    a, b, kx, ky, omega = (np.ascontiguousarray(v, dtype=np.float64) for v in fields)
+    return tuple(v.astype(np.float64) for v in fields)
+
+
+def _group_modes(coeffs: GLCoefficients, lx, ly, nx, ny, seg_off: int, seg_bin: int, ab: int, om: int,
+                 index: int | None) -> tuple[tuple[int, int, int, int], int, int]:
+    """Mode -> bin mapping with the off-grid and Nyquist checks of
+    ``deposit_analytic_input`` (``src/gl_spectral_surface.m:123-149``) into host
+    buffers at the given addresses (``gl_group_modes``): (box, modes, bins)."""
+    fields = (coeffs.a, coeffs.b, coeffs.kx, coeffs.ky, coeffs.omega)
+    shape = np.shape(coeffs.a)
+    for v in fields:
+        if type(v) is not np.ndarray or v.dtype is not _F64 or v.shape != shape or shape == (0,) or len(shape) != 1:
+            fields = _component_fields(coeffs, lx, ly)
+            break
+    a, b, kx, ky, omega = map(np.ascontiguousarray, fields)
     box = (C.c_int * 4)()
     counts = (C.c_int * 2)()
     at = C.addressof(counts)
     status = _lib.load().gl_group_modes(
-        n, a.ctypes.data, b.ctypes.data, kx.ctypes.data, ky.ctypes.data, omega.ctypes.data,
+        int(a.size), a.ctypes.data, b.ctypes.data, kx.ctypes.data, ky.ctypes.data, omega.ctypes.data,
         float(lx), float(ly), int(nx), int(ny), float(coeffs.options["grid_tolerance"]), box, seg_off,
         seg_bin, ab, om, index, at, at + C.sizeof(C.c_int))
     if status == 12:
