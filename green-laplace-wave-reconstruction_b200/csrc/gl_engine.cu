@@ -3766,7 +3766,7 @@ extern "C" gl_status gl_group_modes(int n, const double* a, const double* b, con
                                     int* box, int* seg_offsets, int* seg_bins, double* ab, double* omega_out,
                                     long long* index, int* n_live, int* n_segments) {
   if (n < 1 || !a || !b || !kx || !ky || !omega || !box || !seg_offsets || !seg_bins || !ab || !omega_out ||
-      !n_live || !n_segments || nx < 2 || ny < 2 || !(lx > 0) || !(ly > 0))
+      !n_live || !n_segments || !(lx > 0) || !(ly > 0))
     return fail(GL_ERR_INVALID_ARGUMENT, "bad mode table arguments");
   try {
     const double dkx = 6.283185307179586 / lx, dky = 6.283185307179586 / ly;
