@@ -710,34 +710,24 @@ struct gl_plan {
 // Side streams for a group's independent stages.  A call takes a set from the
 // device's pool while it queues its work and gives it back joined to the
 // caller's stream, so concurrent calls (other threads, plans, streams) never
-// queue between one call's fork and join; the pool grows to the number of
-// calls that ever queued at once and lives as long as the process.
+// queue between one call's fork and join.  A set that still runs a call's work
+// goes to later calls on the same stream only, which that work precedes anyway:
+// independent streams never wait for one another through it.  The pool holds
+// up to BRANCH_SETS sets a device for the life of the process; a call that finds
+// none runs its stages in turn.
 constexpr size_t BRANCH_BYTES = 64u << 20;
+constexpr int BRANCH_SETS = 16;
 struct BranchSet {
   int device;
+  unsigned long long owner;  // id of the stream it was last joined to
   cudaStream_t st[2];
-  cudaEvent_t ev[5];
+  cudaEvent_t ev[5];         // the last two: the joins
 };
 static std::mutex g_branch_mu;
 static std::vector<BranchSet*> g_branch_free;
+static int g_branch_count[64] = {0};
 
-// A set for work on `st`, or null when the stream is being captured (a pooled
-// stream would stay part of the capture after the call) or none can be made.
-static BranchSet* branch_acquire(cudaStream_t st) {
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
-  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  int dev = 0;
-  if (cap != cudaStreamCaptureStatusNone || cudaGetDevice(&dev) != cudaSuccess) return nullptr;
-  std::lock_guard<std::mutex> lk(g_branch_mu);
-  for (size_t k = 0; k < g_branch_free.size(); ++k)
-    if (g_branch_free[k]->device == dev) {
-      BranchSet* b = g_branch_free[k];
-      g_branch_free.erase(g_branch_free.begin() + k);
-      return b;
-    }
+static BranchSet* branch_create(int dev) {
   BranchSet* b = new (std::nothrow) BranchSet();
   if (!b) return nullptr;
   b->device = dev;
@@ -752,6 +742,54 @@ static BranchSet* branch_acquire(cudaStream_t st) {
     if (e) cudaEventDestroy(e);
   delete b;
   return nullptr;
+}
+
+// Whether a set's last work has ended (its events record nothing before the first).
+static bool branch_idle(const BranchSet* b) {
+  for (int k = 3; k < 5; ++k) {
+    const cudaError_t e = cudaEventQuery(b->ev[k]);
+    if (e == cudaErrorNotReady) cudaGetLastError();
+    if (e != cudaSuccess) return false;
+  }
+  return true;
+}
+
+// A set for work on `st`, or null when the stream is being captured (a pooled
+// stream would stay part of the capture after the call) or none can be had.
+static BranchSet* branch_acquire(cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  int dev = 0;
+  if (cap != cudaStreamCaptureStatusNone || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  // queries and new streams are no part of a capture that another thread runs
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return nullptr;
+  BranchSet* b = nullptr;
+  unsigned long long id = 0;
+  if (cudaStreamGetId(st, &id) == cudaSuccess) {
+    std::lock_guard<std::mutex> lk(g_branch_mu);
+    const size_t n = g_branch_free.size();
+    size_t pick = 0;
+    while (pick < n && !(g_branch_free[pick]->device == dev && g_branch_free[pick]->owner == id)) ++pick;
+    if (pick == n) {
+      pick = 0;
+      while (pick < n && !(g_branch_free[pick]->device == dev && branch_idle(g_branch_free[pick]))) ++pick;
+    }
+    if (pick < n) {
+      b = g_branch_free[pick];
+      g_branch_free.erase(g_branch_free.begin() + pick);
+    } else if (g_branch_count[dev] < BRANCH_SETS && (b = branch_create(dev))) {
+      ++g_branch_count[dev];
+    }
+    if (b) b->owner = id;
+  } else {
+    cudaGetLastError();
+  }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return b;
 }
 
 static void branch_release(BranchSet* b) {
