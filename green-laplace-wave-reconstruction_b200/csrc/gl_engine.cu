@@ -4597,20 +4597,50 @@ static gl_status wit_upload_tables() {
 
 static size_t wit_binom_stride(int n_modes) { return (size_t)n_modes + 4; }
 
-// Table sizes of the sector-44 sum.  Pair states cost 24 M^2 bytes (0.4 GB at
-// the limit of 4096 modes, far beyond any sum that ends); triple states 8 M^3
+// Tables of the sector-44 sum.  Pair states cost 24 M^2 bytes (0.4 GB at the
+// limit of 4096 modes, far beyond any sum that ends); triple states 8 M^3
 // (1 GB at 500 modes) and are formed per quartet above that.
 constexpr int WIT44_PAIR_MODES = 4096, WIT44_TRIPLE_MODES = 500;
+constexpr unsigned long long WIT44_CHEAP_PAIRS = 1u << 22;
 static size_t wit_pairs(int n) { return n <= WIT44_PAIR_MODES ? (size_t)n * (n + 1) / 2 : 0; }
 static size_t wit_triples(int n) { return n <= WIT44_TRIPLE_MODES ? (size_t)n * (n + 1) * (n + 2) / 6 : 0; }
 static size_t wit_head_bytes(int n_modes) {
   return align_up(sizeof(WitStats)) + 5 * wit_binom_stride(n_modes) * sizeof(unsigned long long);
 }
+static size_t wit_table_bytes(size_t states) { return states ? 256 + 3 * states * sizeof(double2) : 0; }  // 256: alignment
+
+// Which tables a call of `count` candidates forms.  Of the pairs: all calls but
+// small shares of many modes, where the table is the whole cost (4000 modes, 8 M
+// pairs: 207 us with 1 to 1000 candidates, the general kernel 137 to 156; with
+// 125000 candidates 233 and 481; 1000 modes, 0.5 M pairs: 58 and 129 with one).  Of the
+// triples: calls whose candidates outnumber them (a rank's small share forms
+// its triples per quartet, by the same function).  Sectors 40 and 42 mix signs,
+// and their intermediate sums resonate, so they keep the general recursion.
+struct Wit44Path {
+  bool pairs, triples;
+};
+static Wit44Path wit44_path(int sector, int n, unsigned long long count) {
+  Wit44Path p{false, false};
+  if (sector != 44 || n > WIT44_PAIR_MODES || count == 0) return p;
+  p.pairs = wit_pairs(n) <= WIT44_CHEAP_PAIRS || count >= wit_pairs(n) / 256;
+  p.triples = p.pairs && n <= WIT44_TRIPLE_MODES && count >= wit_triples(n);
+  return p;
+}
+static size_t wit_range_bytes(int sector, int n, unsigned long long count) {
+  const Wit44Path p = wit44_path(sector, n, count);
+  return wit_head_bytes(n) + wit_table_bytes(p.pairs ? n + wit_pairs(n) + (p.triples ? wit_triples(n) : 0) : 0);
+}
 
 extern "C" size_t gl_wit_workspace_size(int n_modes) {
   if (n_modes < 1) return 0;
-  const size_t subs = (n_modes <= WIT44_PAIR_MODES ? (size_t)n_modes : 0) + wit_pairs(n_modes) + wit_triples(n_modes);
-  return wit_head_bytes(n_modes) + (subs ? 256 + 3 * subs * sizeof(double2) : 0);  // 256: table alignment
+  return wit_head_bytes(n_modes) +
+         wit_table_bytes(n_modes <= WIT44_PAIR_MODES ? n_modes + wit_pairs(n_modes) + wit_triples(n_modes) : 0);
+}
+
+extern "C" size_t gl_wit_range_workspace_size(int sector, int n_modes, unsigned long long q_begin,
+                                              unsigned long long q_end) {
+  if (n_modes < 1 || q_end < q_begin) return 0;
+  return wit_range_bytes(sector, n_modes, q_end - q_begin);
 }
 
 extern "C" gl_status gl_wit_read_sector_stats(int sector, const void* d_work, int n_modes,
@@ -4666,11 +4696,11 @@ extern "C" gl_status gl_wit_sector_range(int sector, int n_modes, const int* d_m
     return fail(GL_ERR_INVALID_ARGUMENT, "WIT grid sizes must be positive and even");
   if (!(gravity > 0) || !(depth > 0) || !(dkx > 0) || !(dky > 0) || !(threshold > 0))
     return fail(GL_ERR_INVALID_ARGUMENT, "gravity, depth, dk and the resonance threshold must be positive");
-  if (work_bytes < gl_wit_workspace_size(n_modes))
-    return fail(GL_ERR_WORKSPACE, "WIT workspace needs %zu bytes", gl_wit_workspace_size(n_modes));
   if (q_begin > q_end || q_end > wit_candidates(sector, (unsigned long long)n_modes))
     return fail(GL_ERR_INVALID_ARGUMENT, "quartet range [%llu, %llu) outside the sector's %llu candidates",
                 q_begin, q_end, wit_candidates(sector, (unsigned long long)n_modes));
+  const size_t need = wit_range_bytes(sector, n_modes, q_end - q_begin);
+  if (work_bytes < need) return fail(GL_ERR_WORKSPACE, "WIT workspace needs %zu bytes", need);
   gl_status s = wit_upload_tables();
   if (s != GL_OK) return s;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -4711,17 +4741,14 @@ extern "C" gl_status gl_wit_sector_range(int sector, int n_modes, const int* d_m
   a.sector = sector;
   if (q_end == q_begin) return GL_OK;  // an empty share: zero fields, zero counts
   const unsigned long long count = q_end - q_begin;
-  if (sector == 44 && n_modes <= WIT44_PAIR_MODES) {
+  const Wit44Path path = wit44_path(sector, n_modes, count);
+  if (path.pairs) {
     // Real arithmetic over tabulated pair and triple states; 100 modes (4.4 M
-    // quartets): 13.4 ms by the general kernel below, 0.37 so.  The
-    // triple table is built when the call's candidates outnumber its entries
-    // (a rank's small share forms its triples per quartet, by the same
-    // function).  Sectors 40 and 42 mix signs, and their intermediate sums
-    // resonate, so they keep the general recursion.
+    // quartets): 13.4 ms by the general kernel below, 0.37 so.
     Wit44Tables t;
     t.n_modes = n_modes;
     t.n_pairs = wit_pairs(n_modes);
-    t.n_triples = count >= wit_triples(n_modes) ? wit_triples(n_modes) : 0;
+    t.n_triples = path.triples ? wit_triples(n_modes) : 0;
     double2* base = reinterpret_cast<double2*>(
         (reinterpret_cast<uintptr_t>(work) + wit_head_bytes(n_modes) + 255) & ~(uintptr_t)255);
     t.single = base;

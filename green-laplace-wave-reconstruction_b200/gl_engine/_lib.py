@@ -144,6 +144,7 @@ SIGNATURES = {
                                             C.c_int, C.c_void_p, C.c_double, C.c_void_p, C.c_int,
                                             C.c_void_p]),
     "gl_wit_workspace_size": (C.c_size_t, [C.c_int]),
+    "gl_wit_range_workspace_size": (C.c_size_t, [C.c_int, C.c_int, C.c_ulonglong, C.c_ulonglong]),
     "gl_wit_eta44": (C.c_int, [C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_int,
                                C.c_double, C.c_double, C.c_double, C.c_double, C.c_double,
                                C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]),

@@ -170,7 +170,8 @@ def wit_sector(inp: WitInput, sector: int = 44, *, device=None, as_numpy: bool =
         d_modes = torch.from_numpy(modes).to(dev)
         d_amp = torch.from_numpy(amps).to(dev)
         out = torch.empty((5, cases, inp.ny, inp.nx), dtype=torch.complex128, device=dev)
-        work = torch.empty(int(lib.gl_wit_workspace_size(m)) + 256, dtype=torch.uint8, device=dev)
+        work = torch.empty(int(lib.gl_wit_range_workspace_size(int(sector), m, q0, q1)) + 256, dtype=torch.uint8,
+                           device=dev)
         stream = torch.cuda.current_stream(dev).cuda_stream
         _lib.check(lib.gl_wit_sector_range(int(sector), m, C.c_void_p(d_modes.data_ptr()), cases,
                                            C.c_void_p(d_amp.data_ptr()), inp.nx, inp.ny,

@@ -359,13 +359,18 @@ gl_status gl_box_synthesize_noalloc(int n_units, int nx, int ny, int box_x0, int
  * :747-773).  d_modes: (mx, my) int32 pairs; d_amp: [case][mode] complex128;
  * d_out: 5 planes [field][case][ny][nx] complex128 (eta, psi, etaCoordinate,
  * psiCoordinate, retained), zeroed and accumulated by the call; d_work:
- * gl_wit_workspace_size(n_modes) device bytes (statistics, binomial table, sector-44 pair and triple states). */
+ * gl_wit_workspace_size(n_modes) device bytes (statistics, binomial table and
+ * the pair and triple states of a whole sector-44 sum), which serve every sector
+ * and range; gl_wit_range_workspace_size gives what one call needs: sectors 40
+ * and 42 and small shares of sector 44 form fewer tables or none. */
 typedef struct gl_wit_stats {
   unsigned long long candidates, kept, near, strict_zero_output, strict_zero_intermediate;
   double max_residual, min_detuning, max_strict_zero_source;
 } gl_wit_stats;
 
 size_t gl_wit_workspace_size(int n_modes);
+size_t gl_wit_range_workspace_size(int sector, int n_modes, unsigned long long q_begin,
+                                   unsigned long long q_end);
 gl_status gl_wit_eta44(int n_modes, const int* d_modes, int n_cases, const void* d_amp, int nx,
                        int ny, double gravity, double depth, double dkx, double dky,
                        double threshold, void* d_out, void* d_work, size_t work_bytes,
