@@ -36,6 +36,13 @@ GL_HD constexpr int padded_row_len(int n) {
   return n == 96 || n == 160 || n == 192 ? n + 16 : (n == 48 || n == 80 || n == 144 || n == 240 ? n : n + n / 16);
 }
 GL_HD constexpr int columns_row_len(int n) { return padded_row_len(n) | 1; }
+// Pitch of a block's rows: a mixed length's second-pass butterflies (of m = n / 16
+// points), dealt to the threads row after row, go on at the bank where the
+// previous row's end (inner rows of 160 points, 16 records: 386 -> 363 us).
+GL_HD constexpr int row_pitch(int n) {
+  const bool mixed = n == 48 || n == 80 || n == 96 || n == 144 || n == 160 || n == 192 || n == 240;
+  return padded_row_len(n) + (mixed ? (n / 16 + 8 - padded_row_len(n) % 8) % 8 : 0);
+}
 
 template <int N>
 struct FftLen {
@@ -46,10 +53,7 @@ struct FftLen {
   static constexpr int MP = M + (M % 2 == 0 ? 1 : 0);      // padded run of m elements
   static constexpr int ROW = padded_row_len(N), COL = columns_row_len(N);
   static_assert(!mixed || ROW == 16 * MP, "one pad element per run of an even m");
-  // pitch of a block's rows: a mixed length's second-pass butterflies, dealt to
-  // the threads row after row, go on at the bank where the previous row's end
-  // (inner rows of 160 points, 16 records: 386 -> 363 us)
-  static constexpr int PITCH = mixed ? ROW + (M + 8 - ROW % 8) % 8 : ROW;
+  static constexpr int PITCH = row_pitch(N);
 };
 
 // Position of element i in a padded row.

@@ -113,9 +113,11 @@ constexpr size_t SMEM_LIMIT = 227 * 1024;
 // row kernels also hold a static mbarrier: their dynamic budget leaves 1 KB
 constexpr size_t ROW_SMEM_LIMIT = SMEM_LIMIT - 1024;
 
-// Shared-memory budget of a row of `nbanks` banks, as plans are accepted by it
-// (padded_row_len plus one element of slack).
-inline size_t row_smem(int nbanks, int ncx) { return (size_t)nbanks * (ncx + ncx / 16 + 1) * sizeof(cplx); }
+// Shared memory that a row of `nbanks` banks may take, by which plans and
+// launches are accepted: one element a bank above the padded row, or the pitch
+// of the launch where that is more.
+constexpr int row_budget(int ncx) { return ncx + ncx / 16 + 1 > row_pitch(ncx) ? ncx + ncx / 16 + 1 : row_pitch(ncx); }
+inline size_t row_smem(int nbanks, int ncx) { return (size_t)nbanks * row_budget(ncx) * sizeof(cplx); }
 
 inline int grid_for(size_t n, int threads, int cap = 4096) {
   size_t b = (n + threads - 1) / threads;

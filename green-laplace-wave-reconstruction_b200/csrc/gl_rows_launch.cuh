@@ -8,6 +8,7 @@ namespace gl {
 template <int K, int N>
 void row_launch(int njobs, cudaStream_t st, const RowArgs& a, const cplx* tw) {
   constexpr int T = FftLen<N>::T;
+  static_assert(FftLen<N>::PITCH <= row_budget(N), "a row's banks fit the memory its plan was accepted by");
   int nb = 0;
   for (int g = 0; g < a.ngrp; ++g) nb += a.grp[g].nb;
   const size_t smem = (size_t)nb * FftLen<N>::PITCH * sizeof(cplx);
