@@ -655,6 +655,7 @@ struct gl_plan {
   Box b1, b2, b3;
   int ww1, ww2;                 // bitset words per row (S1, S2)
   bool want_eta22, want_psi22, want_o3, want_first;
+  void* tables = nullptr;       // the device tables below, one allocation (alloc_tables)
   double* geo1 = nullptr;
   double* geo2 = nullptr;
   double* geo3 = nullptr;
@@ -901,17 +902,40 @@ static void launch_acc_inner(const AccArgs& c, size_t plane, int units, cudaStre
   acc_inner_kernel<<<dim3(std::max(1, std::min(ntiles, 4096)), units), 256, 0, st>>>(c);
 }
 
+// The plan's device tables in one allocation: geometry planes with `nfac` factor
+// planes behind each box's, pass twiddles, nodes, scales and the general
+// transforms' tables.  The driver maps memory in steps of 2 MB, 0.3 ms each to
+// make and again to free, and separate tables met that several times (us to make
+// and free a plan, separate -> one: order 3 at 1024^2 1860 -> 700, order 4 at 256^2
+// with 27 x 40 bins 1270 -> 700, the least of any plan 690).
+static cudaError_t alloc_tables(gl_plan* p, std::initializer_list<int> nfac, int node_count) {
+  const Box* box[4] = {&p->b1, &p->b2, &p->b3, &p->b4};
+  size_t geo[4];
+  Bump t;
+  int k = 0;
+  for (int n : nfac) {
+    geo[k] = t.take(sizeof(double) * (size_t)(GEO_PLANES + n) * box[k]->w * box[k]->h);
+    ++k;
+  }
+  const size_t tw = t.take(sizeof(cplx) * PASS_TW), nodes = t.take(sizeof(double) * node_count),
+               scale = t.take(sizeof(double) * 6), twx = t.take(p->gen ? sizeof(cplx) * p->d.nx : 0),
+               twy = t.take(p->gen ? sizeof(cplx) * p->d.ny : 0);
+  const cudaError_t e = cudaMalloc(&p->tables, t.off);
+  if (e != cudaSuccess) return e;
+  char* base = reinterpret_cast<char*>(p->tables);
+  double** to[4] = {&p->geo1, &p->geo2, &p->geo3, &p->geo4};
+  for (int i = 0; i < k; ++i) *to[i] = reinterpret_cast<double*>(base + geo[i]);
+  p->tw = reinterpret_cast<cplx*>(base + tw);
+  p->nodes = reinterpret_cast<double*>(base + nodes);
+  p->comp_scale = reinterpret_cast<double*>(base + scale);
+  p->twx = reinterpret_cast<cplx*>(base + twx);
+  p->twy = reinterpret_cast<cplx*>(base + twy);
+  return cudaSuccess;
+}
+
 static void plan_free(gl_plan* p) {
   if (!p) return;
-  cudaFree(p->geo4);
-  cudaFree(p->geo1);
-  cudaFree(p->geo2);
-  cudaFree(p->geo3);
-  cudaFree(p->tw);
-  cudaFree(p->nodes);
-  cudaFree(p->comp_scale);
-  cudaFree(p->twx);
-  cudaFree(p->twy);
+  cudaFree(p->tables);
   for (int l = 0; l < GL_MAX_LANES; ++l) {
     if (p->lane_st[l]) cudaStreamDestroy(p->lane_st[l]);
     if (p->lane_ev[l]) cudaEventDestroy(p->lane_ev[l]);
@@ -1087,29 +1111,23 @@ extern "C" gl_status gl_plan_create(gl_plan** out, const gl_plan_desc* desc) {
     const int id = p->comp_ids[c];
     p->h_comp_scale[c] = (id == GL_COMP_ETA11 || id == GL_COMP_ETA22 || id == GL_COMP_ETA33) ? d.depth : pscale;
   }
-  // device tables
-  cudaError_t e = cudaSuccess;
-  // geometry planes, and behind them the factor planes of the box's column
-  // banks: eta22 and psi22 read the parent box's up to nu^2, order 3 its up to
-  // q^2 nu and the pair box's first four
-  auto geo_alloc = [&](double** g, const Box& b, int nfac) {
-    if (e == cudaSuccess) e = cudaMalloc(g, sizeof(double) * (GEO_PLANES + nfac) * b.w * b.h);
-    if (e == cudaSuccess) {
-      const int plane = b.w * b.h, blocks = std::min(1024, (plane + 255) / 256);
-      geo_kernel<<<blocks, 256>>>(*g, b, d.nx, d.ny, d.lx, d.ly, d.depth, 0.0);
-      if (nfac) factor_kernel<<<blocks, 256>>>(*g, b, nfac);
-      e = cudaGetLastError();
-    }
+  // device tables: geometry planes, and behind them the factor planes of the
+  // box's column banks: eta22 and psi22 read the parent box's up to nu^2, order 3
+  // its up to q^2 nu and the pair box's first four
+  const int nfac1 = o3 ? F_Q2NU + 1 : (o2 ? F_NU2 + 1 : 0), nfac2 = o3 ? F_QY + 1 : 0;
+  cudaError_t e = alloc_tables(p, {nfac1, nfac2, 0}, 8 * MAX_RANK);
+  auto fill_geo = [&](double* g, const Box& b, int nfac) {
+    const int plane = b.w * b.h, blocks = std::min(1024, (plane + 255) / 256);
+    geo_kernel<<<blocks, 256>>>(g, b, d.nx, d.ny, d.lx, d.ly, d.depth, 0.0);
+    if (nfac) factor_kernel<<<blocks, 256>>>(g, b, nfac);
   };
-  geo_alloc(&p->geo1, p->b1, o3 ? F_Q2NU + 1 : (o2 ? F_NU2 + 1 : 0));
-  geo_alloc(&p->geo2, p->b2, o3 ? F_QY + 1 : 0);
-  geo_alloc(&p->geo3, p->b3, 0);
-  if (e == cudaSuccess) e = cudaMalloc(&p->tw, sizeof(cplx) * PASS_TW);
   if (e == cudaSuccess) {
+    fill_geo(p->geo1, p->b1, nfac1);
+    fill_geo(p->geo2, p->b2, nfac2);
+    fill_geo(p->geo3, p->b3, 0);
     pass_twiddle_kernel<<<PASS_TW / 256 + 1, 256>>>(p->tw);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaMalloc(&p->nodes, sizeof(double) * 8 * MAX_RANK);
   if (e == cudaSuccess) {
     double host[8 * MAX_RANK];
     for (int k = 0; k < 4; ++k) {
@@ -1118,16 +1136,11 @@ extern "C" gl_status gl_plan_create(gl_plan** out, const gl_plan_desc* desc) {
     }
     e = cudaMemcpy(p->nodes, host, sizeof host, cudaMemcpyHostToDevice);
   }
-  if (gen) {
-    if (e == cudaSuccess) e = cudaMalloc(&p->twx, sizeof(cplx) * d.nx);
-    if (e == cudaSuccess) e = cudaMalloc(&p->twy, sizeof(cplx) * d.ny);
-    if (e == cudaSuccess) {
-      gen_twiddle_kernel<<<(d.nx + 255) / 256, 256>>>(p->twx, d.nx);
-      gen_twiddle_kernel<<<(d.ny + 255) / 256, 256>>>(p->twy, d.ny);
-      e = cudaGetLastError();
-    }
+  if (gen && e == cudaSuccess) {
+    gen_twiddle_kernel<<<(d.nx + 255) / 256, 256>>>(p->twx, d.nx);
+    gen_twiddle_kernel<<<(d.ny + 255) / 256, 256>>>(p->twy, d.ny);
+    e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaMalloc(&p->comp_scale, sizeof(double) * 6);
   if (e == cudaSuccess)
     e = cudaMemcpy(p->comp_scale, p->h_comp_scale, sizeof(double) * 6, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
@@ -2360,34 +2373,26 @@ extern "C" gl_status gl_eta44_plan_create(gl_plan** out, const gl_eta44_desc* de
   p->h_comp_scale[0] = e.depth;
   p->h_comp_scale[1] = want_psi ? e.depth * std::sqrt(e.gravity * e.depth) : 0.0;
   if (want_psi) p->d.gravity = e.gravity;
-  cudaError_t err = cudaSuccess;
   // geometry planes and the factor planes of each box's column banks
-  auto geo_alloc = [&](double** g, const Box& b, int nfac) {
-    if (err == cudaSuccess) err = cudaMalloc(g, sizeof(double) * (GEO_PLANES + nfac) * b.w * b.h);
-    if (err == cudaSuccess) {
-      const int plane = b.w * b.h, blocks = std::min(1024, (plane + 255) / 256);
-      geo_kernel<<<blocks, 256>>>(*g, b, e.n, e.n, p->d.lx, p->d.ly, e.depth, e.dk);
-      if (nfac) factor_kernel<<<blocks, 256>>>(*g, b, nfac);
-      err = cudaGetLastError();
-    }
-  };
-  geo_alloc(&p->geo1, p->b1, N_FAC);
-  geo_alloc(&p->geo2, p->b2, F_Q2A + 1);
-  geo_alloc(&p->geo3, p->b3, F_QY + 1);
-  geo_alloc(&p->geo4, p->b4, 0);
-  if (err == cudaSuccess) err = cudaMalloc(&p->tw, sizeof(cplx) * PASS_TW);
+  const int nfac[4] = {N_FAC, F_Q2A + 1, F_QY + 1, 0};
+  cudaError_t err = alloc_tables(p, {nfac[0], nfac[1], nfac[2], nfac[3]}, 2 * MAX_RANK);
   if (err == cudaSuccess) {
+    const Box* box[4] = {&p->b1, &p->b2, &p->b3, &p->b4};
+    double* geo[4] = {p->geo1, p->geo2, p->geo3, p->geo4};
+    for (int k = 0; k < 4; ++k) {
+      const int plane = box[k]->w * box[k]->h, blocks = std::min(1024, (plane + 255) / 256);
+      geo_kernel<<<blocks, 256>>>(geo[k], *box[k], e.n, e.n, p->d.lx, p->d.ly, e.depth, e.dk);
+      if (nfac[k]) factor_kernel<<<blocks, 256>>>(geo[k], *box[k], nfac[k]);
+    }
     pass_twiddle_kernel<<<PASS_TW / 256 + 1, 256>>>(p->tw);
     err = cudaGetLastError();
   }
-  if (err == cudaSuccess) err = cudaMalloc(&p->nodes, sizeof(double) * 2 * MAX_RANK);
   if (err == cudaSuccess) {
     double host[2 * MAX_RANK] = {0};
     std::memcpy(host, p->h_nodes[0], sizeof(double) * MAX_RANK);
     std::memcpy(host + MAX_RANK, p->h_weights[0], sizeof(double) * MAX_RANK);
     err = cudaMemcpy(p->nodes, host, sizeof host, cudaMemcpyHostToDevice);
   }
-  if (err == cudaSuccess) err = cudaMalloc(&p->comp_scale, sizeof(double) * 6);
   if (err == cudaSuccess) err = cudaMemcpy(p->comp_scale, p->h_comp_scale, sizeof(double) * 6, cudaMemcpyHostToDevice);
   if (err == cudaSuccess) err = cudaDeviceSynchronize();
   if (err != cudaSuccess) {
