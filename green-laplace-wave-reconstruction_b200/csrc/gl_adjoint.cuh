@@ -30,7 +30,7 @@ namespace gl {
 
 struct SeedArgs {
   const double* r;   // [unit][ny][nx] dL/deta
-  int nx, log2nx, ny;
+  int nx, ny;
   int x0, w;         // kept columns (modes)
   cplx* out;         // [unit][ny][w]
 };
@@ -89,7 +89,7 @@ struct CmbArgs {
   const double* geo;
   const cplx* in;          // [job][bank][n][box.w] (row-transformed adjoint fields)
   cplx* out;               // [job][nout][box.h][box.w]
-  int n, log2n;            // compact grid along y
+  int n;                   // compact grid along y
   double scale;            // the forward inverse transform's 1/(Nx Ny)
   const UnitScalars* us;
   const double* nodes;     // eta22 nodes (ETA22) or outer nodes (FIRST3, INNER)

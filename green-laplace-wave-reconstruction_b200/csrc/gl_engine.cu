@@ -642,19 +642,19 @@ struct gl_plan {
   int comps;                    // GL_COMP_* actually produced
   int ncomp;
   int comp_ids[6];
-  int ncx, ncy, lncx, lncy, lnx, lny;
+  int ncx, ncy;
   // forward column grids of the pair (eta22, psi22, inner order-3) and triple
   // (outer order-3) stages: the smallest column lengths >= the box heights,
   // mixed lengths 16 m allowed (log2 0 for those); ncy (a power of two) is
   // the adjoint's grid and bounds both
-  int ncy2, lncy2, ncy3, lncy3;
+  int ncy2, ncy3;
   // forward row length of the pair stages (power of two or 144/160/192/240,
   // <= ncx: their products need a period covering only the pair box)
-  int ncx2, lncx2;
+  int ncx2;
   int ncx3 = 0;  // eta44 third-level row length (power of two covering B3)
   Box b1, b2, b3;
   int ww1, ww2;                 // bitset words per row (S1, S2)
-  bool want_eta22, want_psi22, want_o3, want_first;
+  bool want_eta22, want_psi22, want_o3;
   void* tables = nullptr;       // the device tables below, one allocation (alloc_tables)
   double* geo1 = nullptr;
   double* geo2 = nullptr;
@@ -810,7 +810,6 @@ static int col_len(int v) {
     if (mixed[k] >= v && mixed[k] < best) best = mixed[k];
   return best;
 }
-static int col_log2(int n) { return is_pow2(n) ? ilog2(n) : 0; }
 
 // Smallest row-transform length >= v: a power of two (>= 16) or one of the
 // mixed lengths the pair-stage row kernels are instantiated for.
@@ -1038,7 +1037,6 @@ extern "C" gl_status gl_plan_create(gl_plan** out, const gl_plan_desc* desc) {
   p->ncomp = 0;
   for (int b = 0; b < 6; ++b)
     if (comps & (1 << b)) p->comp_ids[p->ncomp++] = 1 << b;
-  p->want_first = comps & (GL_COMP_ETA11 | GL_COMP_PSI11);
   p->want_eta22 = comps & GL_COMP_ETA22;
   p->want_psi22 = comps & GL_COMP_PSI22;
   p->want_o3 = o3;
@@ -1065,8 +1063,6 @@ extern "C" gl_status gl_plan_create(gl_plan** out, const gl_plan_desc* desc) {
     if (is_pow2(d.nx)) p->ncx = std::min(d.nx, p->ncx);
     if (is_pow2(d.ny)) p->ncy = std::min(d.ny, p->ncy);
   }
-  p->lncx = ilog2(p->ncx);
-  p->lncy = ilog2(p->ncy);
   p->ncy2 = p->ncy3 = p->ncy;
   p->ncx2 = p->ncx;
   if (d.grid != GL_GRID_REFERENCE && deg > 1) {
@@ -1074,11 +1070,6 @@ extern "C" gl_status gl_plan_create(gl_plan** out, const gl_plan_desc* desc) {
     if (deg == 3) p->ncy3 = std::min(p->ncy, col_len(p->b3.h));
     p->ncx2 = std::min(p->ncx, row_len(p->b2.w));
   }
-  p->lncx2 = col_log2(p->ncx2);
-  p->lncy2 = col_log2(p->ncy2);
-  p->lncy3 = col_log2(p->ncy3);
-  p->lnx = ilog2(d.nx);
-  p->lny = ilog2(d.ny);
   const int max_banks = o3 ? 21 : (p->want_psi22 ? 16 : 8);
   if (deg > 1 && row_smem(max_banks, p->ncx) > ROW_SMEM_LIMIT) {
     plan_free(p);
@@ -1451,12 +1442,6 @@ static gl_status final_outputs(gl_plan* p, int gu, const FinalComp* f, int n, vo
   return GL_OK;
 }
 
-static int comp_slot(const gl_plan* p, int id) {
-  for (int k = 0; k < p->ncomp; ++k)
-    if (p->comp_ids[k] == id) return k;
-  return -1;
-}
-
 // ---------------------------------------------------------------------------
 // one group of units
 // ---------------------------------------------------------------------------
@@ -1720,7 +1705,6 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     a.nodes = dn + 0 * MAX_RANK;
     a.out = P;
     a.n = ncy2;
-    a.log2n = p->lncy2;
     a.scale = inv_scale;
     if ((s = launch_col_ifft(tuned(p, a), njobs, st, p->tw)) != GL_OK) return s;
     RowArgs r;
@@ -1733,11 +1717,9 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     r.out_w = B2.w;
     r.out = Q;
     r.nx = p->ncx2;
-    r.log2nx = p->lncx2;
     r.ny = ncy2;
     r.us = us;
     r.jobs_per_unit = J;
-    r.gmax = ROW_GMAX;
     r.wait_surplus = p->wait_surplus;
     r.wait_cycles = p->wait_cycles;
     if ((s = launch_row(tuned(p, r), njobs, st, p->tw)) != GL_OK) return s;
@@ -1746,7 +1728,6 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     f.out = R;
     f.box = B2;
     f.n = ncy2;
-    f.log2n = p->lncy2;
     f.nsrc = 2;
     f.jobs_per_unit = J;
     f.mask = s2;
@@ -1791,7 +1772,6 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     ColFftArgs f;
     f.box = B2;
     f.n = ncy2;
-    f.log2n = p->lncy2;
     f.mask = nullptr;
     f.maxslot = nullptr;
     f.scale = fwd_scale2;
@@ -1816,7 +1796,6 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     a.chan_mask = ch;
     a.out = P22;
     a.n = ncy2;
-    a.log2n = p->lncy2;
     a.scale = inv_scale;
     if ((s = launch_col_ifft(tuned(p, a), njobs_c, st, p->tw)) != GL_OK) return s;
     RowArgs r;
@@ -1831,11 +1810,9 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     r.out_w = B2.w;
     r.out = Q22;
     r.nx = p->ncx2;
-    r.log2nx = p->lncx2;
     r.ny = ncy2;
     r.us = us;
     r.jobs_per_unit = 4;
-    r.gmax = ROW_GMAX;
     r.wait_surplus = p->wait_surplus;
     r.wait_cycles = p->wait_cycles;
     if ((s = launch_row(tuned(p, r), njobs_r, st, p->tw)) != GL_OK) return s;
@@ -1865,7 +1842,6 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     cc.jobs_per_unit = 1;
     cc.out = Pc;
     cc.n = ncy2;
-    cc.log2n = p->lncy2;
     cc.scale = inv_scale;
     if ((s = launch_col_ifft(tuned(p, cc), gu, st, p->tw)) != GL_OK) return s;
     RowArgs rc;
@@ -1878,11 +1854,9 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     rc.out_w = B2.w;
     rc.out = Qc;
     rc.nx = p->ncx2;
-    rc.log2nx = p->lncx2;
     rc.ny = ncy2;
     rc.us = us;
     rc.jobs_per_unit = 1;
-    rc.gmax = ROW_GMAX;
     rc.wait_surplus = p->wait_surplus;
     rc.wait_cycles = p->wait_cycles;
     if ((s = launch_row(tuned(p, rc), gu, st, p->tw)) != GL_OK) return s;
@@ -1958,7 +1932,6 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
       a.n_outer = J;
       a.out = PI;
       a.n = ncy2;
-      a.log2n = p->lncy2;
       a.scale = inv_scale;
       if ((s = launch_col_ifft(tuned(p, a), njobs, st, p->tw)) != GL_OK) return s;
       RowArgs r;
@@ -1971,11 +1944,9 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
       r.out_w = B2.w;
       r.out = QI;
       r.nx = p->ncx2;
-      r.log2nx = p->lncx2;
       r.ny = ncy2;
       r.us = us;
       r.jobs_per_unit = J * I;
-      r.gmax = ROW_GMAX;
       r.wait_surplus = p->wait_surplus;
       r.wait_cycles = p->wait_cycles;
       if ((s = launch_row(tuned(p, r), njobs, st, p->tw)) != GL_OK) return s;
@@ -1984,7 +1955,6 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
       f.out = RI;
       f.box = B2;
       f.n = ncy2;
-      f.log2n = p->lncy2;
       f.nsrc = 4;
       f.jobs_per_unit = J * I;
       f.mask = s2;
@@ -2032,7 +2002,6 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     a.nodes = dn + 3 * MAX_RANK;
     a.out = P1;
     a.n = ncy3;
-    a.log2n = p->lncy3;
     a.scale = inv_scale;
     if ((s = launch_col_ifft(tuned(p, a), nuj, st, p->tw)) != GL_OK) return s;
     return GL_OK;
@@ -2061,7 +2030,6 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     a2.floor_rel = p->floor_rel;
     a2.out = P2;
     a2.n = ncy3;
-    a2.log2n = p->lncy3;
     a2.scale = inv_scale;
     if ((s = launch_col_ifft(tuned(p, a2), nuj, st, p->tw)) != GL_OK) return s;
     if ((s = first_ready(st)) != GL_OK) return s;
@@ -2076,11 +2044,9 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     r.out_w = B3.w;
     r.out = QO;
     r.nx = p->ncx;
-    r.log2nx = p->lncx;
     r.ny = ncy3;
     r.us = us;
     r.jobs_per_unit = J;
-    r.gmax = ROW_GMAX;
     r.wait_surplus = p->wait_surplus;
     r.wait_cycles = p->wait_cycles;
     if ((s = launch_row(tuned(p, r), nuj, st, p->tw)) != GL_OK) return s;
@@ -2089,7 +2055,6 @@ static gl_status run_group(gl_plan* p, int gu, const void* spectra, int layout, 
     f.out = RO;
     f.box = B3;
     f.n = ncy3;
-    f.log2n = p->lncy3;
     f.nsrc = 4;
     f.jobs_per_unit = J;
     f.mask = s3;
@@ -2337,9 +2302,6 @@ extern "C" gl_status gl_eta44_plan_create(gl_plan** out, const gl_eta44_desc* de
   p->ww3 = (p->b3.w + 63) / 64;
   p->ncx = std::min(e.n, std::max(16, next_pow2(p->b4.w)));
   p->ncy = std::min(e.n, std::max(16, next_pow2(p->b4.h)));
-  p->lncx = ilog2(p->ncx);
-  p->lncy = ilog2(p->ncy);
-  p->lnx = p->lny = ilog2(e.n);
   // pair and third stages: rows a power of two covering B2 / B3 (the order-4
   // row kernels run powers of two), columns the shortest length covering
   // B2 / B3 that the column kernels run
@@ -2347,9 +2309,6 @@ extern "C" gl_status gl_eta44_plan_create(gl_plan** out, const gl_eta44_desc* de
   p->ncy2 = std::min(p->ncy, col_len(p->b2.h));
   p->ncx3 = std::min(p->ncx, std::max(16, next_pow2(p->b3.w)));
   p->ncy3 = std::min(p->ncy, col_len(p->b3.h));
-  p->lncx2 = col_log2(p->ncx2);
-  p->lncy2 = col_log2(p->ncy2);
-  p->lncy3 = col_log2(p->ncy3);
   const int row_banks = want_psi ? 46 : 45;
   if (row_smem(row_banks, p->ncx) > ROW_SMEM_LIMIT) {
     plan_free(p);
@@ -2479,7 +2438,6 @@ static gl_status e44_finalize(gl_plan* p, int gu, const cplx* OUT, unsigned long
   a.floor_rel = p->floor_rel;
   a.out = reinterpret_cast<cplx*>(tr);
   a.n = p->d.ny;
-  a.log2n = p->lny;
   a.scale = 1.0 / ((double)p->d.nx * (double)p->d.ny);
   if ((s = launch_col_ifft(a, gu, st, p->tw)) != GL_OK) return s;
   OutArgs o;
@@ -2508,9 +2466,6 @@ static gl_status e44_finalize(gl_plan* p, int gu, const cplx* OUT, unsigned long
   return GL_OK;
 }
 
-// One group of units over outer nodes [o0, o0 + Ro).  With `partial` set,
-// the accumulated order-4 spectra (before the final floor) are written there
-// and nothing else is produced; otherwise the fields are finished.
 // Analysis of an order-4 plan's group whose box is beyond analyse_kernel: one
 // launch per reduction and per Minkowski sum.
 static gl_status e44_analyse_large(gl_plan* p, int gu, const cplx* spec, int layout, void* ws, const ScalarArgs& sc,
@@ -2600,6 +2555,9 @@ static gl_status e44_analyse_large(gl_plan* p, int gu, const cplx* spec, int lay
   return GL_OK;
 }
 
+// One group of units over outer nodes [o0, o0 + Ro).  With `partial` set,
+// the accumulated order-4 spectra (before the final floor) are written there
+// and nothing else is produced; otherwise the fields are finished.
 static gl_status e44_run(gl_plan* p, int gu, const void* spectra, int layout, int o0, int Ro,
                          cplx* partial, void* outputs, void* ws, int* status, cudaStream_t st,
                          int part = -2) {
@@ -2693,11 +2651,11 @@ static gl_status e44_run(gl_plan* p, int gu, const void* spectra, int layout, in
   // covering B2 and B3 (rows a power of two, columns a power of two or a
   // mixed length 16 m); the order-4 stage on the plan's grid covering B4.
   struct StageGrid {
-    int nx, lnx, ny, lny;
+    int nx, ny;
     double fwd;  // (Nx Ny)/(nx ny): forward-transform scale
   };
   auto stage_grid = [&](int nx, int ny) {
-    return StageGrid{nx, col_log2(nx), ny, col_log2(ny),
+    return StageGrid{nx, ny,
                      ((double)p->d.nx * (double)p->d.ny) / ((double)nx * (double)ny)};
   };
   StageGrid cur = stage_grid(p->ncx, p->ncy);
@@ -2724,7 +2682,6 @@ static gl_status e44_run(gl_plan* p, int gu, const void* spectra, int layout, in
     a.floor_rel = p->floor_rel;
     a.out = outp;
     a.n = cur.ny;
-    a.log2n = cur.lny;
     a.scale = inv_scale;
     return a;
   };
@@ -2737,11 +2694,9 @@ static gl_status e44_run(gl_plan* p, int gu, const void* spectra, int layout, in
     r.out_w = outbox.w;
     r.out = outp;
     r.nx = cur.nx;
-    r.log2nx = cur.lnx;
     r.ny = cur.ny;
     r.us = us;
     r.jobs_per_unit = 1;
-    r.gmax = ROW_GMAX;
     return r;
   };
   auto colfft = [&](const cplx* in, cplx* outp, const Box& box, int nsrc, const unsigned char* mask,
@@ -2751,7 +2706,6 @@ static gl_status e44_run(gl_plan* p, int gu, const void* spectra, int layout, in
     f.out = outp;
     f.box = box;
     f.n = cur.ny;
-    f.log2n = cur.lny;
     f.nsrc = nsrc;
     f.jobs_per_unit = jobs_per_unit;
     f.mask = mask;
@@ -3193,7 +3147,6 @@ static gl_status adj_seed(gl_plan* p, int gu, const double* resid, const Box& bo
   SeedArgs sa;
   sa.r = resid;
   sa.nx = p->d.nx;
-  sa.log2nx = p->lnx;
   sa.ny = p->d.ny;
   sa.x0 = box.x0;
   sa.w = box.w;
@@ -3205,7 +3158,6 @@ static gl_status adj_seed(gl_plan* p, int gu, const double* resid, const Box& bo
   f.out = out;
   f.box = box;
   f.n = p->d.ny;
-  f.log2n = p->lny;
   f.nsrc = 1;
   f.jobs_per_unit = 1;
   f.mask = nullptr;
@@ -3221,7 +3173,7 @@ static gl_status adj_seed(gl_plan* p, int gu, const double* resid, const Box& bo
 // combine): the pair stages run on (ncx2, ncy2), the triple stage on
 // (ncx, ncy3), like the forward stages they transpose.
 struct AdjGrid {
-  int nx, lnx, ny, lny;
+  int nx, ny;
 };
 
 static gl_status adj_cols(gl_plan* p, const AdjGrid& gr, const Box& box, const double* geo,
@@ -3242,7 +3194,6 @@ static gl_status adj_cols(gl_plan* p, const AdjGrid& gr, const Box& box, const d
   a.jobs_per_unit = 1;
   a.out = out;
   a.n = gr.ny;
-  a.log2n = gr.lny;
   a.scale = ((double)p->d.nx * (double)p->d.ny) / ((double)gr.nx * (double)gr.ny);
   a.conj_io = 1;
   return launch_col_ifft(a, njobs, st, p->tw);
@@ -3265,7 +3216,6 @@ static CmbArgs cmb_args(gl_plan* p, const AdjGrid& gr, int kind, int nb, const i
   a.in = in;
   a.out = out;
   a.n = gr.ny;
-  a.log2n = gr.lny;
   a.scale = 1.0 / ((double)p->d.nx * (double)p->d.ny);
   a.us = us;
   a.jobs_per_unit = jobs_per_unit;
@@ -3285,8 +3235,8 @@ static gl_status run_adjoint_group(gl_plan* p, int gu, const void* spectra, int 
   const double* dn = p->nodes;
   const double inv_scale = 1.0 / ((double)p->d.nx * (double)p->d.ny);
   // pair segments on (ncx2, ncy2), the triple segment on (ncx, ncy3)
-  const AdjGrid G2{p->ncx2, p->lncx2, p->ncy2, p->lncy2};
-  const AdjGrid G3{p->ncx, p->lncx, p->ncy3, p->lncy3};
+  const AdjGrid G2{p->ncx2, p->ncy2};
+  const AdjGrid G3{p->ncx, p->ncy3};
   const double fwd2 = ((double)p->d.nx * (double)p->d.ny) / ((double)G2.nx * (double)G2.ny);
   const double fwd3 = ((double)p->d.nx * (double)p->d.ny) / ((double)G3.nx * (double)G3.ny);
   const AdjLayout L = adj_layout(p, p->group);
@@ -3332,7 +3282,6 @@ static gl_status run_adjoint_group(gl_plan* p, int gu, const void* spectra, int 
     a.nodes = dn + 0 * MAX_RANK;
     a.out = P;
     a.n = G2.ny;
-    a.log2n = G2.lny;
     a.scale = inv_scale;
     if ((s = launch_col_ifft(a, nj, st, p->tw)) != GL_OK) return s;
     RowArgs r;
@@ -3345,18 +3294,15 @@ static gl_status run_adjoint_group(gl_plan* p, int gu, const void* spectra, int 
     r.out_w = B2.w;
     r.out = Q;
     r.nx = G2.nx;
-    r.log2nx = G2.lnx;
     r.ny = G2.ny;
     r.us = us;
     r.jobs_per_unit = J;
-    r.gmax = ROW_GMAX;
     if ((s = launch_row(r, nj, st, p->tw)) != GL_OK) return s;
     ColFftArgs f;
     f.in = Q;
     f.out = R;
     f.box = B2;
     f.n = G2.ny;
-    f.log2n = G2.lny;
     f.nsrc = 2;
     f.jobs_per_unit = J;
     f.mask = s2;
@@ -3397,11 +3343,9 @@ static gl_status run_adjoint_group(gl_plan* p, int gu, const void* spectra, int 
     ra.out = QA;
     ra.out_conj = 1;
     ra.nx = G2.nx;
-    ra.log2nx = G2.lnx;
     ra.ny = G2.ny;
     ra.us = us;
     ra.jobs_per_unit = J;
-    ra.gmax = ROW_GMAX;
     if ((s = launch_row(ra, nj, st, p->tw)) != GL_OK) return s;
     CmbArgs c = cmb_args(p, G2, CMB_ETA22, 8, m8, nullptr, 1, B1, p->geo1, QA, DA22, us, J);
     c.nodes = dn + 0 * MAX_RANK;
@@ -3456,7 +3400,6 @@ static gl_status run_adjoint_group(gl_plan* p, int gu, const void* spectra, int 
       a.n_outer = Jo;
       a.out = PI;
       a.n = G2.ny;
-      a.log2n = G2.lny;
       a.scale = inv_scale;
       if ((s = launch_col_ifft(a, nj, st, p->tw)) != GL_OK) return s;
       RowArgs r;
@@ -3469,18 +3412,15 @@ static gl_status run_adjoint_group(gl_plan* p, int gu, const void* spectra, int 
       r.out_w = B2.w;
       r.out = QI;
       r.nx = G2.nx;
-      r.log2nx = G2.lnx;
       r.ny = G2.ny;
       r.us = us;
       r.jobs_per_unit = Jo * I;
-      r.gmax = ROW_GMAX;
       if ((s = launch_row(r, nj, st, p->tw)) != GL_OK) return s;
       ColFftArgs f;
       f.in = QI;
       f.out = RI;
       f.box = B2;
       f.n = G2.ny;
-      f.log2n = G2.lny;
       f.nsrc = 4;
       f.jobs_per_unit = Jo * I;
       f.mask = s2;
@@ -3525,7 +3465,6 @@ static gl_status run_adjoint_group(gl_plan* p, int gu, const void* spectra, int 
       a.nodes = dn + 3 * MAX_RANK;
       a.out = P1;
       a.n = G3.ny;
-      a.log2n = G3.lny;
       a.scale = inv_scale;
       if ((s = launch_col_ifft(a, nuj, st, p->tw)) != GL_OK) return s;
       ColArgs a2;
@@ -3543,7 +3482,6 @@ static gl_status run_adjoint_group(gl_plan* p, int gu, const void* spectra, int 
       a2.floor_rel = p->floor_rel;
       a2.out = P2;
       a2.n = G3.ny;
-      a2.log2n = G3.lny;
       a2.scale = inv_scale;
       if ((s = launch_col_ifft(a2, nuj, st, p->tw)) != GL_OK) return s;
       RowArgs r;
@@ -3557,18 +3495,15 @@ static gl_status run_adjoint_group(gl_plan* p, int gu, const void* spectra, int 
       r.out_w = B3.w;
       r.out = QO;
       r.nx = G3.nx;
-      r.log2nx = G3.lnx;
       r.ny = G3.ny;
       r.us = us;
       r.jobs_per_unit = Jo;
-      r.gmax = ROW_GMAX;
       if ((s = launch_row(r, nuj, st, p->tw)) != GL_OK) return s;
       ColFftArgs f;
       f.in = QO;
       f.out = RO;
       f.box = B3;
       f.n = G3.ny;
-      f.log2n = G3.lny;
       f.nsrc = 2;
       f.jobs_per_unit = Jo;
       f.mask = s3;
@@ -3617,11 +3552,9 @@ static gl_status run_adjoint_group(gl_plan* p, int gu, const void* spectra, int 
       ra.out2 = QA2;
       ra.out_conj = 1;
       ra.nx = G3.nx;
-      ra.log2nx = G3.lnx;
       ra.ny = G3.ny;
       ra.us = us;
       ra.jobs_per_unit = Jo;
-      ra.gmax = ROW_GMAX;
       if ((s = launch_row(ra, nuj, st, p->tw)) != GL_OK) return s;
       CmbArgs c1 = cmb_args(p, G3, CMB_FIRST3, 12, m1, nullptr, 1, B1, p->geo1, QA1, DA1, us, Jo);
       c1.nodes = dn + 3 * MAX_RANK;
@@ -3666,11 +3599,9 @@ static gl_status run_adjoint_group(gl_plan* p, int gu, const void* spectra, int 
       ra.out = QAi;
       ra.out_conj = 1;
       ra.nx = G2.nx;
-      ra.log2nx = G2.lnx;
       ra.ny = G2.ny;
       ra.us = us;
       ra.jobs_per_unit = Jo * I;
-      ra.gmax = ROW_GMAX;
       if ((s = launch_row(ra, nj, st, p->tw)) != GL_OK) return s;
       CmbArgs c = cmb_args(p, G2, CMB_INNER, 12, mi, nullptr, 1, B1, p->geo1, QAi, DAI, us, Jo * I);
       c.nodes = dn + 3 * MAX_RANK;
@@ -4530,7 +4461,6 @@ extern "C" gl_status gl_box_synthesize_noalloc(int n_units, int nx, int ny, int 
   a.jobs_per_unit = 1;
   a.out = mid;
   a.n = ny;
-  a.log2n = ilog2(ny);
   a.scale = 1.0 / ((double)nx * (double)ny);
   if ((s = launch_col_ifft(a, n_units, st, tw)) != GL_OK) return s;
   OutArgs o;

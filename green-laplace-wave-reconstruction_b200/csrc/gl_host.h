@@ -108,7 +108,6 @@ inline int next_pow2(int v) {
 }
 inline size_t align_up(size_t v) { return (v + 255) & ~(size_t)255; }
 
-constexpr int ROW_GMAX = 4;
 constexpr size_t SMEM_LIMIT = 227 * 1024;
 // row kernels also hold a static mbarrier: their dynamic budget leaves 1 KB
 constexpr size_t ROW_SMEM_LIMIT = SMEM_LIMIT - 1024;

@@ -203,7 +203,7 @@ struct ColArgs {
   double floor_rel;
   // output
   cplx* out;               // [job][bank][w][n]
-  int n, log2n;            // transform length along y
+  int n;                   // transform length along y
   double scale;            // applied to the inverse transform (1/(Nx Ny))
   // 1: run the transform with the opposite exponent sign, through
   // conj(F(conj x)) -- the transpose of a forward transform, used by the
@@ -492,11 +492,10 @@ struct RowArgs {
   int nout;
   int out_x0, out_w;       // kept output columns (modes)
   cplx* out;               // [job][nout][out_w][n_y]
-  int nx, log2nx;          // compact grid along x
+  int nx;                  // compact grid along x
   int ny;                  // compact grid along y (column length of inputs)
   UnitScalars* us;         // per-unit scalars; status word flagged on a timed-out copy
   int jobs_per_unit;
-  int gmax;                // FFT group size (rows through tmp)
   // adjoint extensions (zero in the forward stages):
   int out_conj;            // 1: outputs transformed with the + sign
   int nout_a;              // > 0: outputs [nout_a, nout) go to out2 instead
@@ -1054,7 +1053,7 @@ struct ColFftArgs {
   const cplx* in;          // [js][out_w][n]
   cplx* out;               // [js][box h][box w]
   Box box;                 // output box (modes)
-  int n, log2n;            // compact grid along y
+  int n;                   // compact grid along y
   int nsrc;                // spectra per job
   int jobs_per_unit;
   const unsigned char* mask;   // [unit][h][w] or null

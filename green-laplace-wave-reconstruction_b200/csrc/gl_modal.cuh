@@ -58,9 +58,9 @@ struct SFft {
   const int* live;       // non-null: columns *live and up hold zeros, and are left alone
   double scale;          // applied to the outputs
   int tw_log2p;          // > 0: output k times w^(k grp), w = e^{SIGN 2 pi i / 2^tw_log2p}
-  int fields;            // arrays transformed alike (grid z), fstride elements apart
+  int fields;            // arrays transformed alike (grid y), fstride elements apart
   long long fstride;
-  int nbanks;            // > 0: field z is read from bank z
+  int nbanks;            // > 0: field k is read from bank k
   ModalBank bank[MODAL_BANKS];
   ModalGeo geo;
   int row_step;          // bank: element i of group grp is row i * row_step + grp
