@@ -147,7 +147,7 @@ __global__ void geo_kernel(double* geo, Box box, int nx, int ny, double lx, doub
 }
 
 // Factor planes of a box behind its geometry planes (Fac, the first `nfac`),
-// column-major [x][y]: the products in apply_mult's order of operations.
+// column-major [x][y]: the products in the reference's order of operations.
 __global__ void factor_kernel(double* geo, Box box, int nfac) {
   const int plane = box.w * box.h;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < plane; j += gridDim.x * blockDim.x) {

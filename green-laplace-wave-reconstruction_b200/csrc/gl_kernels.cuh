@@ -88,7 +88,9 @@ struct GeoRef {
 
 // value = multiplier(bin) * s, in the evaluation order of the reference's
 // NumPy expressions (_order3.py:151-193, spatial.py:196-203); only the
-// geometry planes a multiplier needs are read.
+// geometry planes a multiplier needs are read.  For the adjoint's combining
+// columns (orders 1 to 3) and the general final columns; the inverse columns
+// read factor planes (Fac) or call mult_direct.
 GL_D cplx apply_mult(int m, const GeoRef& g, cplx s) {
   switch (m) {
     case M_ONE: return s;
@@ -115,31 +117,12 @@ GL_D cplx apply_mult(int m, const GeoRef& g, cplx s) {
     case M_QX_DIVNU: { const cplx t = cscale(g.qx(), s); const double sn = safe_nu(g.nu()); return cmk(t.x / sn, t.y / sn); }
     case M_QY_DIVNU: { const cplx t = cscale(g.qy(), s); const double sn = safe_nu(g.nu()); return cmk(t.x / sn, t.y / sn); }
     case M_Q2_DIVNU: { const double q = g.q(); const cplx t = cscale(q * q, s); const double sn = safe_nu(g.nu()); return cmk(t.x / sn, t.y / sn); }
-    case M_MI_NU2QX: { const double nu = g.nu(); return cmulmi(cscale(nu * nu * g.qx(), s)); }
-    case M_MI_NU2QY: { const double nu = g.nu(); return cmulmi(cscale(nu * nu * g.qy(), s)); }
-    case M_MINUS_Q2A: { const double q = g.q(); return cscale(-(q * q * g.a()), s); }
-    case M_I_ANU: return cmuli(cscale(g.a() * g.nu(), s));
-    case M_PHI_IQXQ2: case M_PHI_IQYQ2: case M_PHI_Q4: {
-      // phi = (-i s)/nu where nu > 0, then the vertical-derivative multiplier
-      const double nu = g.nu();
-      if (!(nu > 0.0)) return czero();
-      const cplx phi = cmk(s.y / nu, -s.x / nu);
-      const double q = g.q();
-      if (m == M_PHI_Q4) return cscale(q * q * q * q, phi);
-      return cmuli(cscale((m == M_PHI_IQXQ2 ? g.qx() : g.qy()) * q * q, phi));
-    }
-    case M_NU4: { const double nu = g.nu(); return cscale(nu * nu * nu * nu, s); }
-    case M_Q2NU: { const double q = g.q(); return cscale(q * q * g.nu(), s); }
-    case M_NU2QX: { const double nu = g.nu(); return cscale(nu * nu * g.qx(), s); }
-    case M_NU2QY: { const double nu = g.nu(); return cscale(nu * nu * g.qy(), s); }
-    case M_IQXA: return cmuli(cscale(g.qx() * g.a(), s));
-    case M_IQYA: return cmuli(cscale(g.qy() * g.a(), s));
-    case M_Q2A: { const double q = g.q(); return cscale(q * q * g.a(), s); }
   }
   return czero();
 }
 
-// The multipliers that divide, as apply_mult forms them.
+// The multipliers that divide: those of orders 1 to 3 as apply_mult forms them,
+// and order 4's vertical derivatives of phi.
 GL_D cplx mult_direct(int m, const GeoRef& g, cplx s) {
   const double nu = g.nu();
   if (m == M_QX_DIVNU || m == M_QY_DIVNU || m == M_Q2_DIVNU) {
@@ -293,12 +276,12 @@ GL_D cplx col_base(const ColArgs& a, int job, int i, double nu) {
 // f a real factor of the bin and rot a multiple of 90 degrees, read their
 // factor from a table behind the geometry planes (column-major, so that a
 // transform group's lanes read it contiguously).  The rest (divisions after
-// or before the product) are formed by apply_mult.
+// or before the product) are formed by mult_direct.
 enum Fac : int {
   F_A = 0, F_Q2, F_QX, F_QY, F_QXA, F_QYA, F_Q2A, F_NU, F_NU2, F_NU3, F_QX_SNU, F_QY_SNU, F_Q2_SNU, F_NUQX,
   F_NUQY, F_Q2NU, F_NU4, F_NU2QX, F_NU2QY, F_ANU, N_FAC,
   F_ONE = -1,      // no factor
-  F_DIRECT = -2,   // apply_mult
+  F_DIRECT = -2,   // mult_direct
 };
 constexpr int GEO_PLANES = 6;
 constexpr int ROT_SWAP = 1, ROT_NEG_RE = 2, ROT_NEG_IM = 4;
