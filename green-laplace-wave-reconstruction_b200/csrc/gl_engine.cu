@@ -879,8 +879,10 @@ static size_t stage_scratch(gl_plan* p, int g, size_t base) {
       widths += p->comp_ids[k] <= GL_COMP_PSI11 ? p->b1.w : (p->comp_ids[k] <= GL_COMP_PSI22 ? p->b2.w : p->b3.w);
     main = std::max(main, align_up((size_t)g * widths * p->d.ny * c));
   }
-  // Branches pay while the stages' launches leave SMs idle, i.e. while their
-  // buffers are a fraction of L2.
+  // Side by side the stages need regions of their own: the bound is one on memory.
+  // They gain on both sides of it (us a call in turn -> side by side; below:
+  // 128^2 x4 order 3 249 -> 219, 512^2 x1 312 -> 248; above: 256^2 x4 314 -> 245, 1024^2 x1
+  // 433 -> 357, x8 1768 -> 1704; order 2, 512^2 x8 420 -> 365).
   const int chains = (p->want_eta22 ? 1 : 0) + (p->want_psi22 ? 1 : 0) + (p->want_o3 ? 2 : 0);
   p->branches = chains >= 2 && eta + psi + first <= BRANCH_BYTES;
   if (!p->branches) {
@@ -1352,7 +1354,9 @@ struct FinalComp {
 
 // Final transforms of `n` components to the reference grid.  The components
 // share launches (a 128^2 call with six: 8 launches of 8 to 22 us became 2) as
-// long as their intermediate columns stay well inside L2.
+// long as their intermediate columns stay well inside L2: a bound of 12 MB
+// instead of 48 measured 0 to 4 % slower a call from 256^2 x8 on, none at all
+// within 1.5 % either way (1024^2 x8 1777 -> 1754 us, x1 437 both).
 static gl_status final_outputs(gl_plan* p, int gu, const FinalComp* f, int n, void* outputs, void* scratch,
                                cudaStream_t st, UnitScalars* us) {
   const double scale = 1.0 / ((double)p->d.nx * (double)p->d.ny);
@@ -3949,7 +3953,7 @@ extern "C" gl_status gl_fft2(int batch, int nx, int ny, const void* d_in, void* 
 // `fields` arrays of one shape, `stride` elements apart, transformed by the same
 // launch: a record's banks are small (a 1024 x 256 array fills a third of the
 // GPU) and many, and one launch per bank and axis left most of it idle (122
-// launches of 20 us, 2.5 ms, for a 1024-sample record; now 22 launches, 1.4 ms).
+// launches of 20 us, 2.5 ms, for a 1024-sample record; now 26 launches, 0.55 ms).
 struct Fields {
   cplx* data;
   int count;
@@ -4679,7 +4683,7 @@ extern "C" gl_status gl_wit_sector_range(int sector, int n_modes, const int* d_m
   const Wit44Path path = wit44_path(sector, n_modes, count);
   if (path.pairs) {
     // Real arithmetic over tabulated pair and triple states; 100 modes (4.4 M
-    // quartets): 13.4 ms by the general kernel below, 0.37 so.
+    // quartets): 13.4 ms by the general kernel below, 0.34 so.
     Wit44Tables t;
     t.n_modes = n_modes;
     t.n_pairs = wit_pairs(n_modes);

@@ -72,7 +72,7 @@ struct SFft {
 // Staged element by element through shared memory, with divisions by the
 // column count, the 22 launches of a 1024-sample record took 1408 us (and the
 // multiplier banks 164 in kernels of their own); these and the
-// line transforms, banks included, take 622.
+// line transforms, banks included, take 550.
 template <int N>
 struct StridedLen {
   static constexpr int T = FftLen<N>::T;

@@ -512,10 +512,13 @@ __global__ void __launch_bounds__(128) wit44_kernel(WitArgs a) {
 // share a potential block collapse into one elevation factor per order
 // (unordered partitions; the block orders cancel the factorials).
 //
-// What bounds it: FP64 issue (about 250 operations a quartet) and the loads
-// of four triple and six pair states, which the lanes of a warp read
-// contiguously because consecutive candidates differ in their lowest mode,
-// and four FP64 atomics per quartet.
+// What bounds it: instruction issue and the FP64 chain's latency -- 1300
+// instructions a quartet, 420 of them FP64 (600 operations), at 10.5 warps per SM
+// (164 registers): 53 % of issue slots, the FP64 pipe 38 %, fixed-latency
+// waits the first stall.  The four triple and six pair states are read
+// contiguously by the lanes of a warp, because consecutive candidates differ in
+// their lowest mode (71 % of the sectors from L1); the four FP64 atomics per
+// quartet keep the L2 units 15 % busy, the busiest 64 %.
 // 100 modes (4.4 M quartets): 0.31 ms and 0.03 ms for the tables, against
 // 13.4 ms for the general kernel; 382 modes (901 M): 0.06 s against 3.2 s.
 
